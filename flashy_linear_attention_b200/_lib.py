@@ -193,5 +193,19 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host side of a call on torch tensors (csrc/fla_host.cpp), loaded once."""
+    global _host
+    if _host is None:
+        load()
+        from . import _hostcalls
+
+        _host = _hostcalls
+    return _host
+
+
 def strerror(code: int) -> str:
     return load().fla_sm100_strerror(code).decode()

@@ -1,0 +1,240 @@
+// Host side of one forward / backward call on torch tensors: checks, output and scratch tensors,
+// argument block and the C-ABI call, in one native function each. Python's part of a call is then a
+// few attribute reads; doing the same through torch's Python API and ctypes (about 45 stride reads,
+// 40 structure fields and four device guards) took longer than the kernels of a small layer.
+//
+// Both functions return None for calls they do not cover (wrong types, shapes that do not match,
+// head dims above 384, running states with head dims above 128): the caller then takes the general path in
+// ops.py, which reports the errors and handles the rest.
+#include <torch/extension.h>
+
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <algorithm>
+#include <optional>
+#include <string>
+
+#include "../../include/flashlinear_sm100.h"
+
+namespace {
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+constexpr int64_t kKernelHeadDim = 128;  // widest head dim of the running-state kernels
+constexpr int64_t kWideHeadDim = 384;    // widest head dim one library call covers
+
+// What a TMA tensor map needs: unit innermost stride, 16-byte aligned base and outer strides.
+bool addressable(const Tensor& t) {
+  if (t.stride(3) != 1 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0 || t.stride(2) < t.size(3))
+    return false;
+  for (int d = 0; d < 3; ++d)
+    if (t.size(d) > 1 && t.stride(d) % 8 != 0) return false;
+  return true;
+}
+
+bool usable(const Tensor& t, const Tensor& ref) {
+  return t.layout() == at::kStrided && t.dim() == 4 && t.is_cuda() && t.device() == ref.device() &&
+         t.scalar_type() == ref.scalar_type() && !t.is_neg();
+}
+
+bool same_rows(const Tensor& a, const Tensor& b) {  // batch, heads, tokens
+  return a.size(0) == b.size(0) && a.size(1) == b.size(1) && a.size(2) == b.size(2);
+}
+
+bool is_state(const OptTensor& s, const Tensor& ref, int64_t bh, int64_t dk, int64_t dv) {
+  return !s.has_value() || (s->is_cuda() && s->device() == ref.device() && s->scalar_type() == at::kFloat &&
+                            s->is_contiguous() && s->dim() == 3 && s->size(0) == bh && s->size(1) == dk &&
+                            s->size(2) == dv);
+}
+
+FlaTensor desc(const Tensor& t) {
+  FlaTensor d;
+  d.ptr = t.data_ptr();
+  d.stride_b = t.stride(0);
+  d.stride_h = t.stride(1);
+  d.stride_n = t.stride(2);
+  return d;
+}
+
+// View [..., :d] of a fresh tensor whose rows are padded to a multiple of 8 elements.
+Tensor padded_empty(const Tensor& like) {
+  const int64_t d = like.size(3);
+  return at::empty({like.size(0), like.size(1), like.size(2), (d + 7) / 8 * 8}, like.options()).narrow(3, 0, d);
+}
+
+void check(int rc, const char* name) {
+  if (rc != FLA_OK)
+    throw std::runtime_error(std::string("flashlinear: ") + name + " returned " + std::to_string(rc) + ": " +
+                             fla_sm100_strerror(rc));
+}
+
+// The library's pad / unpad kernels work on contiguous tensors of any row length.
+bool contiguous_rows(const Tensor& t) {
+  return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 4 == 0;
+}
+
+// `t`, or a copy with padded rows when the kernels cannot address it in place.
+Tensor kernel_view(const Tensor& t, void* stream) {
+  if (addressable(t)) return t;
+  Tensor v = padded_empty(t);
+  if (contiguous_rows(t))
+    check(fla_sm100_pad_rows(t.data_ptr(), v.data_ptr(), t.numel() / t.size(3), static_cast<int>(t.size(3)),
+                             static_cast<int>(v.stride(2)), stream),
+          "fla_sm100_pad_rows");
+  else
+    v.copy_(t);
+  return v;
+}
+
+// An output with the layout of empty_like(t) and what the kernel writes to: the output itself, or a
+// row-padded scratch tensor that is copied back. keep_padded: the padded tensor IS the output.
+struct Output {
+  Tensor full, view;
+};
+Output output_like(const Tensor& t, bool keep_padded) {
+  Output o;
+  if (keep_padded && t.size(3) % 8 != 0) {
+    o.full = o.view = padded_empty(t);
+    return o;
+  }
+  o.full = at::empty_like(t);
+  o.view = addressable(o.full) ? o.full : padded_empty(o.full);
+  return o;
+}
+void copy_back(const Output& o, void* stream) {
+  if (o.view.is_same(o.full)) return;
+  if (contiguous_rows(o.full))
+    check(fla_sm100_unpad_rows(o.view.data_ptr(), o.full.data_ptr(), o.full.numel() / o.full.size(3),
+                               static_cast<int>(o.full.size(3)), static_cast<int>(o.view.stride(2)), stream),
+          "fla_sm100_unpad_rows");
+  else
+    o.full.copy_(o.view);
+}
+
+bool covered_dims(const Tensor& q, const Tensor& v) {
+  if (q.numel() == 0 || v.numel() == 0) return false;
+  if (q.size(0) > INT32_MAX || q.size(1) > INT32_MAX || q.size(2) > INT32_MAX) return false;
+  const int64_t m = std::max(q.size(3), v.size(3));
+  if (q.scalar_type() == at::kBFloat16) return m <= kWideHeadDim;
+  return q.scalar_type() == at::kHalf && m <= kKernelHeadDim;
+}
+
+void set_sizes(FlaArgs& a, const Tensor& q, const Tensor& v, unsigned debug_flags, uintptr_t status) {
+  a = FlaArgs{};
+  a.batch = static_cast<int32_t>(q.size(0));
+  a.heads = static_cast<int32_t>(q.size(1));
+  a.seqlen = static_cast<int32_t>(q.size(2));
+  a.dk = static_cast<int32_t>(q.size(3));
+  a.dv = static_cast<int32_t>(v.size(3));
+  a.dtype = q.scalar_type() == at::kHalf ? FLA_DTYPE_F16 : FLA_DTYPE_BF16;
+  a.debug_flags = debug_flags;
+  a.status = reinterpret_cast<int32_t*>(status);
+}
+
+Tensor scratch(FlaArgs& a, int pass, const Tensor& ref) {
+  const size_t need = fla_sm100_workspace_bytes(&a, pass);
+  if (need == 0) return Tensor();
+  Tensor ws = at::empty({static_cast<int64_t>(need)}, ref.options().dtype(at::kByte));
+  a.workspace = ws.data_ptr();
+  a.workspace_bytes = need;
+  return ws;
+}
+
+// state: 0 none; 1 always return the final state, [B, H, dk, dv]; 2 return what the backward of
+// these shapes uses (final state and boundary states, each a tensor or None).
+py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init, int state,
+                   unsigned debug_flags, uintptr_t status) {
+  if (!usable(q, q) || !usable(k, q) || !usable(v, q) || !covered_dims(q, v) || !same_rows(q, k) ||
+      !same_rows(q, v) || q.size(3) != k.size(3))
+    return py::none();
+  const int64_t bh = q.size(0) * q.size(1), dk = q.size(3), dv = v.size(3);
+  const bool wide = dk > kKernelHeadDim || dv > kKernelHeadDim;
+  if (wide && (s_init.has_value() || state == 1)) return py::none();
+  if (!is_state(s_init, q, bh, dk, dv)) return py::none();
+  const c10::cuda::CUDAGuard guard(q.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  Output out = output_like(v, false);
+  const Tensor qv = kernel_view(q, stream), kv = kernel_view(k, stream), vv = kernel_view(v, stream);
+  FlaArgs a;
+  set_sizes(a, q, v, debug_flags, status);
+  a.stream = stream;
+  OptTensor s_final, seg_states;
+  if (!wide && (state == 1 || (state == 2 && fla_sm100_bwd_uses_final_state(&a) != 0))) {
+    s_final = state == 1 ? at::empty({q.size(0), q.size(1), dk, dv}, q.options().dtype(at::kFloat))
+                         : at::empty({bh, dk, dv}, q.options().dtype(at::kFloat));
+    if (state == 2) {
+      const size_t need = fla_sm100_seg_states_bytes(&a);
+      if (need > 0) {
+        seg_states = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
+        a.seg_states = seg_states->data_ptr();
+        a.seg_states_bytes = need;
+      }
+    }
+  }
+  a.q = desc(qv);
+  a.k = desc(kv);
+  a.v = desc(vv);
+  a.o = desc(out.view);
+  if (s_init.has_value()) a.s_init = s_init->data_ptr<float>();
+  if (s_final.has_value()) a.s_final = s_final->data_ptr<float>();
+  const Tensor ws = scratch(a, 0, q);
+  check(fla_sm100_fwd(&a), "libflashlinear_sm100");
+  copy_back(out, stream);
+  return py::make_tuple(out.full, s_final, seg_states);
+}
+
+py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init,
+                    const OptTensor& r_init, bool want_r_final, const OptTensor& s_last,
+                    const OptTensor& seg_states, bool keep_padded, unsigned debug_flags, uintptr_t status) {
+  if (!usable(q, q) || !usable(k, q) || !usable(v, q) || !usable(g, q) || !covered_dims(q, v) ||
+      !same_rows(q, k) || !same_rows(q, v) || !same_rows(q, g) || q.size(3) != k.size(3) ||
+      g.size(3) != v.size(3))
+    return py::none();
+  const int64_t bh = q.size(0) * q.size(1), dk = q.size(3), dv = v.size(3);
+  if ((dk > kKernelHeadDim || dv > kKernelHeadDim) &&
+      (s_init.has_value() || r_init.has_value() || want_r_final || s_last.has_value()))
+    return py::none();
+  if (!is_state(s_init, q, bh, dk, dv) || !is_state(r_init, q, bh, dk, dv) || !is_state(s_last, q, bh, dk, dv))
+    return py::none();
+  const c10::cuda::CUDAGuard guard(q.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  Output dq = output_like(q, keep_padded), dkk = output_like(k, keep_padded), dvv = output_like(v, keep_padded);
+  const Tensor gv = kernel_view(g, stream), qv = kernel_view(q, stream), kv = kernel_view(k, stream),
+               vv = kernel_view(v, stream);
+  FlaArgs a;
+  set_sizes(a, q, v, debug_flags, status);
+  a.stream = stream;
+  a.q = desc(qv);
+  a.k = desc(kv);
+  a.v = desc(vv);
+  a.d_o = desc(gv);
+  a.d_q = desc(dq.view);
+  a.d_k = desc(dkk.view);
+  a.d_v = desc(dvv.view);
+  OptTensor r_final;
+  if (want_r_final) r_final = at::empty({bh, dk, dv}, q.options().dtype(at::kFloat));
+  if (s_init.has_value()) a.s_init = s_init->data_ptr<float>();
+  if (r_init.has_value()) a.r_init = r_init->data_ptr<float>();
+  if (r_final.has_value()) a.r_final = r_final->data_ptr<float>();
+  if (s_last.has_value()) a.s_last = s_last->data_ptr<float>();
+  if (seg_states.has_value()) {
+    a.seg_states = seg_states->data_ptr();
+    a.seg_states_bytes = static_cast<size_t>(seg_states->numel() * seg_states->element_size());
+  }
+  const Tensor ws = scratch(a, 1, q);
+  check(fla_sm100_bwd(&a), "libflashlinear_sm100");
+  copy_back(dq, stream);
+  copy_back(dkk, stream);
+  copy_back(dvv, stream);
+  return py::make_tuple(dq.full, dkk.full, dvv.full, r_final);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_hostcalls, m) {
+  m.def("forward", &forward);
+  m.def("backward", &backward);
+}

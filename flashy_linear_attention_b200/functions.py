@@ -8,94 +8,86 @@ the reference's ``custom_fwd(cast_inputs=torch.bfloat16)`` does.
 """
 from __future__ import annotations
 
+import functools
 from typing import Any, Tuple
 
 import torch
 from torch.autograd import Function
 
 from . import ops
-from .ops import (
-    linear_flash_wrapper_bwd,
-    linear_flash_wrapper_bwd_smallv_hd,
-    linear_flash_wrapper_fwd,
-    linear_flash_wrapper_fwd_smallv_hd,
-)
+
+
+def _autocast_to_bf16(forward):
+    """``custom_fwd(cast_inputs=torch.bfloat16)``, entered only where autocast is on. The backward
+    needs no counterpart: nothing it calls depends on the autocast state."""
+    cast = torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)(forward)
+
+    @functools.wraps(forward)
+    def wrapper(ctx: Any, *args):
+        return cast(ctx, *args) if torch.is_autocast_enabled("cuda") else forward(ctx, *args)
+
+    return wrapper
 
 
 def _forward_with_state(ctx: Any, q, k, v, smallv: bool):
     """Forward through the reference-named wrapper's checks; when a backward will follow and can
     use it, also keeps the final state S = sum k^T v (fp32, batch*heads x dk x dv), which lets the
-    backward read q, k, v, dO from HBM once instead of twice."""
-    want_state = any(ctx.needs_input_grad[:3]) and q.is_cuda and ops.backward_uses_final_state(q, v)
+    backward read q, k, v, dO from HBM once instead of twice, and with few heads per GPU the states
+    at the boundaries of the forward's segments."""
+    ops.check_forward_preconditions(q, v, smallv)
+    need_grad = any(ctx.needs_input_grad[:3])
     ctx.keep_padded = False
-    if smallv and q.is_cuda and q.shape[-1] % 8 != 0 and any(ctx.needs_input_grad[:3]):
+    if smallv and need_grad and q.is_cuda and q.shape[-1] % 8 != 0:
         # Head dims such as 273 have rows the kernels cannot address in place. Repack q and k once,
         # keep the repacked views for the backward, and let the backward return dQ and dK as views
         # of row-padded tensors (same values and shape as the reference's gradients, which are
         # contiguous, linear_attn_kernels_smallv_hd.py:384-386; one copy pass per tensor less).
-        ops.check_forward_preconditions(q, v, smallv)
         q, k = ops.kernel_view(q), ops.kernel_view(k)
         ctx.keep_padded = True
-    if not want_state:
-        out = linear_flash_wrapper_fwd_smallv_hd(q, k, v) if smallv else linear_flash_wrapper_fwd(q, k, v)
+    res = ops.host_forward(q, k, v, None, 2 if need_grad else 0)
+    if res is None:
+        res = (ops.causal_dot_product_fwd(q, k, v), None, None)
+    out, s_final, seg_states = res
+    if s_final is None:
         ctx.save_for_backward(q, k, v)
-        ctx.has_state = False
-        return out
-    ops.check_forward_preconditions(q, v, smallv)
-    B, H, _, dk = q.shape
-    s_final = torch.empty(B * H, dk, v.shape[-1], dtype=torch.float32, device=q.device)
-    # few heads per GPU: the forward is split into segments and also hands the state at the segment
-    # boundaries to the backward
-    seg_states = ops.segment_states_buffer(q, v)
-    out = ops.causal_dot_product_fwd(q, k, v, s_final=s_final, seg_states=seg_states)
-    if seg_states is None:
+    elif seg_states is None:
         ctx.save_for_backward(q, k, v, s_final)
     else:
         ctx.save_for_backward(q, k, v, s_final, seg_states)
-    ctx.has_state = True
     return out
 
 
-def _backward_with_state(ctx: Any, grad_output, smallv: bool):
-    if not ctx.has_state:
-        query, key, value = ctx.saved_tensors
-        if ctx.keep_padded:
-            return ops.causal_dot_product_bwd(grad_output, query, key, value, keep_padded=True)
-        fn = linear_flash_wrapper_bwd_smallv_hd if smallv else linear_flash_wrapper_bwd
-        return fn(grad_output, query, key, value)
-    query, key, value, s_final = ctx.saved_tensors[:4]
-    seg_states = ctx.saved_tensors[4] if len(ctx.saved_tensors) > 4 else None
-    return ops.causal_dot_product_bwd(grad_output, query, key, value, s_last=s_final, seg_states=seg_states)
+def _backward_with_state(ctx: Any, grad_output):
+    saved = ctx.saved_tensors
+    return ops.causal_dot_product_bwd(
+        grad_output, saved[0], saved[1], saved[2], s_last=saved[3] if len(saved) > 3 else None,
+        seg_states=saved[4] if len(saved) > 4 else None, keep_padded=ctx.keep_padded)
 
 
 class LinearAttention(Function):
     """Causal linear attention with dk == dv."""
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    @_autocast_to_bf16
     def forward(ctx: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
         return _forward_with_state(ctx, q, k, v, smallv=False)
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx: Any, grad_output: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-        gradq, gradk, gradv = _backward_with_state(ctx, grad_output, smallv=False)
-        return gradq, gradk, gradv
+        return _backward_with_state(ctx, grad_output)
 
 
 class LinearAttentionSmallVHD(Function):
     """Causal linear attention where q/k have head dim hd_qk and v has a smaller hd_v."""
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    @_autocast_to_bf16
     def forward(ctx: Any, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
         return _forward_with_state(ctx, q, k, v, smallv=True)
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx: Any, grad_output: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-        gradq, gradk, gradv = _backward_with_state(ctx, grad_output, smallv=True)
-        return gradq, gradk, gradv
+        return _backward_with_state(ctx, grad_output)
 
 
 class LinearAttentionResumable(Function):
@@ -116,7 +108,7 @@ class LinearAttentionResumable(Function):
     """
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    @_autocast_to_bf16
     def forward(ctx: Any, q, k, v, s_init=None):
         assert q.shape[-1] <= ops.KERNEL_HEAD_DIM and v.shape[-1] <= ops.KERNEL_HEAD_DIM, \
             f"Only head_dims <= {ops.KERNEL_HEAD_DIM} are supported."
@@ -127,15 +119,17 @@ class LinearAttentionResumable(Function):
             s_init = s_init.to(torch.float32).contiguous()
             if tuple(s_init.shape) != (B, H, dk, dv):
                 raise ValueError(f"s_init must have shape {(B, H, dk, dv)}")
-        s_final = torch.empty(B, H, dk, dv, dtype=torch.float32, device=q.device)
-        out = ops.causal_dot_product_fwd(
-            q, k, v, s_init=None if s_init is None else s_init.view(B * H, dk, dv),
-            s_final=s_final.view(B * H, dk, dv))
+        flat_init = None if s_init is None else s_init.view(B * H, dk, dv)
+        res = ops.host_forward(q, k, v, flat_init, 1)
+        if res is not None:
+            out, s_final, _ = res
+        else:
+            s_final = torch.empty(B, H, dk, dv, dtype=torch.float32, device=q.device)
+            out = ops.causal_dot_product_fwd(q, k, v, s_init=flat_init, s_final=s_final.view(B * H, dk, dv))
         ctx.save_for_backward(q, k, v, s_init, s_final)
         return out, s_final
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx: Any, grad_output, grad_s_final):
         q, k, v, s_init, s_final = ctx.saved_tensors
         B, H, _, dk = q.shape
@@ -163,7 +157,7 @@ class LinearAttentionNormalized(Function):
     """
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    @_autocast_to_bf16
     def forward(ctx: Any, q, k, v, eps: float = 1e-5):
         ops.check_forward_preconditions(q, v, smallv=q.shape[-1] != v.shape[-1])
         if v.shape[-1] % 8 != 0:
@@ -186,7 +180,6 @@ class LinearAttentionNormalized(Function):
         return out
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx: Any, grad_output):
         q, k, v, out, den = ctx.saved_tensors[:5]
         s_final = ctx.saved_tensors[5] if ctx.has_state else None
@@ -209,7 +202,7 @@ class TaylorLinearAttention(Function):
     """
 
     @staticmethod
-    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    @_autocast_to_bf16
     def forward(ctx: Any, xq, xk, v):
         pq, pk = ops.taylor_features(xq), ops.taylor_features(xk)
         ops.check_forward_preconditions(pq, v, smallv=True)
@@ -218,7 +211,6 @@ class TaylorLinearAttention(Function):
         return out
 
     @staticmethod
-    @torch.amp.custom_bwd(device_type="cuda")
     def backward(ctx: Any, grad_output):
         xq, xk, v, pq, pk = ctx.saved_tensors
         dpq, dpk, dv = ops.causal_dot_product_bwd(grad_output, pq, pk, v, keep_padded=True)

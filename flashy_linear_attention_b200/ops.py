@@ -262,6 +262,42 @@ def _call(pass_id: int, args: FlaArgs, device: torch.device, which: int = 0,
     return ws
 
 
+_status_ptrs: dict = {}  # device index -> address of its status word
+
+
+def _status_ptr(t: torch.Tensor) -> int:
+    ptr = _status_ptrs.get(t.get_device())
+    if ptr is None:
+        ptr = _status_word(t.device).data_ptr()
+        _status_ptrs[t.get_device()] = ptr
+    return ptr
+
+
+def host_forward(q, k, v, s_init: Optional[torch.Tensor] = None, state: int = 0):
+    """One forward call through the native host path: (out, s_final, seg_states), or None for calls
+    it does not cover (they take the general path below). `state`: 0 no state is returned, 1 the
+    final state [B, H, dk, dv], 2 whatever the backward of these shapes makes use of."""
+    if not q.is_cuda:
+        return None
+    res = _lib.host().forward(q, k, v, s_init, state, _debug_flags, _status_ptr(q))
+    if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
+        check_status(q.device)
+    return res
+
+
+def host_backward(grad_output, q, k, v, s_init=None, r_init=None, want_r_final: bool = False, s_last=None,
+                  seg_states=None, keep_padded: bool = False):
+    """One backward call through the native host path: (dQ, dK, dV, r_final), or None (see
+    host_forward)."""
+    if not q.is_cuda:
+        return None
+    res = _lib.host().backward(grad_output, q, k, v, s_init, r_init, want_r_final, s_last, seg_states,
+                               keep_padded, _debug_flags, _status_ptr(q))
+    if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
+        check_status(q.device)
+    return res
+
+
 def _product_call(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, out: torch.Tensor, anticausal: bool) -> None:
     """out = causal (or anti-causal) product of kernel-addressable views, head dims <= 128."""
     B, H, N, da = a.shape
@@ -330,6 +366,10 @@ def causal_dot_product_fwd(
     segment boundaries there, and causal_dot_product_bwd(..., s_last=..., seg_states=...) then runs
     the backward as one launch split at those boundaries (few heads per GPU).
     """
+    if s_init is None and s_final is None and segments == 0 and segment_workspace is None and seg_states is None:
+        res = host_forward(q, k, v)
+        if res is not None:
+            return res[0]
     _check_inputs(q, k, v, allow_half=True)
     B, H, N, dk = q.shape
     dv = v.shape[-1]
@@ -376,6 +416,10 @@ def causal_dot_product_bwd(
     `s_final`; with it the backward reads q, k, v, dO from HBM only once.
     keep_padded=True: gradients whose head dim is not a multiple of 8 are returned as views of the
     row-padded tensors the kernels wrote, instead of being copied to the contiguous layout."""
+    if s_init is None and r_init is None and r_final is None and segments == 0:
+        res = host_backward(grad_output, q, k, v, s_last=s_last, seg_states=seg_states, keep_padded=keep_padded)
+        if res is not None:
+            return res[:3]
     _check_inputs(grad_output, q, k, v, allow_half=True)
     B, H, N, dk = q.shape
     dv = v.shape[-1]
