@@ -21,7 +21,7 @@ HOST_PATH = os.path.join(HERE, "_hostcalls.so")
 
 SOURCES = ["fla_api.cu"]
 HOST_SOURCES = ["fla_host.cpp", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
-HEADERS = ["fla_kernel.cuh", "fla_wide_kernel.cuh", "fla_normalize.cuh", "fla_taylor.cuh", "ptx.cuh", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
+HEADERS = ["fla_kernel.cuh", "fla_wide_kernel.cuh", "fla_normalize.cuh", "fla_taylor.cuh", "fla_decode.cuh", "ptx.cuh", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
