@@ -100,6 +100,8 @@ EXPORTED_SYMBOLS = (
     "fla_sm100_taylor_features_bwd",
     "fla_sm100_pad_rows",
     "fla_sm100_unpad_rows",
+    "fla_sm100_pad_rows_batch",
+    "fla_sm100_unpad_rows_batch",
     "fla_sm100_exchange_bytes",
     "fla_sm100_exchange_workspace_bytes",
     "fla_sm100_state_exchange",
@@ -153,6 +155,11 @@ def load() -> ctypes.CDLL:
         fn.restype = ctypes.c_int
         fn.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_int,
                        ctypes.c_void_p]
+    for name in ("fla_sm100_pad_rows_batch", "fla_sm100_unpad_rows_batch"):
+        fn = getattr(lib, name)
+        fn.restype = ctypes.c_int
+        fn.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p), ctypes.c_int,
+                       ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_void_p]
     lib.fla_sm100_normalize_workspace_bytes.restype = ctypes.c_size_t
     lib.fla_sm100_normalize_workspace_bytes.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_normalize_fwd.restype = ctypes.c_int

@@ -76,17 +76,37 @@ bool contiguous_rows(const Tensor& t) {
   return t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 4 == 0;
 }
 
-// `t`, or a copy with padded rows when the kernels cannot address it in place.
-Tensor kernel_view(const Tensor& t, void* stream) {
-  if (addressable(t)) return t;
-  Tensor v = padded_empty(t);
-  if (contiguous_rows(t))
-    check(fla_sm100_pad_rows(t.data_ptr(), v.data_ptr(), t.numel() / t.size(3), static_cast<int>(t.size(3)),
-                             static_cast<int>(v.stride(2)), stream),
-          "fla_sm100_pad_rows");
-  else
-    v.copy_(t);
-  return v;
+// Replaces every tensor the kernels cannot address in place by a copy with padded rows. Contiguous
+// tensors of one row length share a launch of the pad kernel.
+void kernel_views(Tensor* t, int n, void* stream) {
+  constexpr int kMax = 4;
+  const void* src[kMax];
+  void* dst[kMax];
+  Tensor copies[kMax];
+  bool done[kMax] = {};
+  for (int i = 0; i < n; ++i) {
+    if (addressable(t[i])) done[i] = true;
+    else copies[i] = padded_empty(t[i]);
+    if (!done[i] && !contiguous_rows(t[i])) {
+      copies[i].copy_(t[i]);
+      done[i] = true;
+    }
+  }
+  for (int i = 0; i < n; ++i) {
+    if (done[i]) continue;
+    int count = 0;
+    for (int j = i; j < n; ++j) {
+      if (done[j] || t[j].size(3) != t[i].size(3)) continue;
+      src[count] = t[j].data_ptr();
+      dst[count++] = copies[j].data_ptr();
+      done[j] = true;
+    }
+    check(fla_sm100_pad_rows_batch(src, dst, count, t[i].numel() / t[i].size(3), static_cast<int>(t[i].size(3)),
+                                   static_cast<int>(copies[i].stride(2)), stream),
+          "fla_sm100_pad_rows_batch");
+  }
+  for (int i = 0; i < n; ++i)
+    if (copies[i].defined()) t[i] = copies[i];
 }
 
 // An output with the layout of empty_like(t) and what the kernel writes to: the output itself, or a
@@ -104,14 +124,33 @@ Output output_like(const Tensor& t, bool keep_padded) {
   o.view = addressable(o.full) ? o.full : padded_empty(o.full);
   return o;
 }
-void copy_back(const Output& o, void* stream) {
-  if (o.view.is_same(o.full)) return;
-  if (contiguous_rows(o.full))
-    check(fla_sm100_unpad_rows(o.view.data_ptr(), o.full.data_ptr(), o.full.numel() / o.full.size(3),
-                               static_cast<int>(o.full.size(3)), static_cast<int>(o.view.stride(2)), stream),
-          "fla_sm100_unpad_rows");
-  else
-    o.full.copy_(o.view);
+// Results from the padded scratch rows into the caller-layout outputs, grouped like kernel_views().
+void copy_back(const Output* o, int n, void* stream) {
+  constexpr int kMax = 4;
+  const void* src[kMax];
+  void* dst[kMax];
+  bool done[kMax] = {};
+  for (int i = 0; i < n; ++i) {
+    done[i] = o[i].view.is_same(o[i].full);
+    if (!done[i] && !contiguous_rows(o[i].full)) {
+      o[i].full.copy_(o[i].view);
+      done[i] = true;
+    }
+  }
+  for (int i = 0; i < n; ++i) {
+    if (done[i]) continue;
+    int count = 0;
+    const int64_t d = o[i].full.size(3);
+    for (int j = i; j < n; ++j) {
+      if (done[j] || o[j].full.size(3) != d) continue;
+      src[count] = o[j].view.data_ptr();
+      dst[count++] = o[j].full.data_ptr();
+      done[j] = true;
+    }
+    check(fla_sm100_unpad_rows_batch(src, dst, count, o[i].full.numel() / d, static_cast<int>(d),
+                                     static_cast<int>(o[i].view.stride(2)), stream),
+          "fla_sm100_unpad_rows_batch");
+  }
 }
 
 bool covered_dims(const Tensor& q, const Tensor& v) {
@@ -157,7 +196,8 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
   Output out = output_like(v, false);
-  const Tensor qv = kernel_view(q, stream), kv = kernel_view(k, stream), vv = kernel_view(v, stream);
+  Tensor in[3] = {q, k, v};
+  kernel_views(in, 3, stream);
   FlaArgs a;
   set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
@@ -174,15 +214,15 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
       }
     }
   }
-  a.q = desc(qv);
-  a.k = desc(kv);
-  a.v = desc(vv);
+  a.q = desc(in[0]);
+  a.k = desc(in[1]);
+  a.v = desc(in[2]);
   a.o = desc(out.view);
   if (s_init.has_value()) a.s_init = s_init->data_ptr<float>();
   if (s_final.has_value()) a.s_final = s_final->data_ptr<float>();
   const Tensor ws = scratch(a, 0, q);
   check(fla_sm100_fwd(&a), "libflashlinear_sm100");
-  copy_back(out, stream);
+  copy_back(&out, 1, stream);
   return py::make_tuple(out.full, s_final, seg_states);
 }
 
@@ -201,19 +241,19 @@ py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Ten
     return py::none();
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  Output dq = output_like(q, keep_padded), dkk = output_like(k, keep_padded), dvv = output_like(v, keep_padded);
-  const Tensor gv = kernel_view(g, stream), qv = kernel_view(q, stream), kv = kernel_view(k, stream),
-               vv = kernel_view(v, stream);
+  const Output out[3] = {output_like(q, keep_padded), output_like(k, keep_padded), output_like(v, keep_padded)};
+  Tensor in[4] = {q, k, v, g};
+  kernel_views(in, 4, stream);
   FlaArgs a;
   set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
-  a.q = desc(qv);
-  a.k = desc(kv);
-  a.v = desc(vv);
-  a.d_o = desc(gv);
-  a.d_q = desc(dq.view);
-  a.d_k = desc(dkk.view);
-  a.d_v = desc(dvv.view);
+  a.q = desc(in[0]);
+  a.k = desc(in[1]);
+  a.v = desc(in[2]);
+  a.d_o = desc(in[3]);
+  a.d_q = desc(out[0].view);
+  a.d_k = desc(out[1].view);
+  a.d_v = desc(out[2].view);
   OptTensor r_final;
   if (want_r_final) r_final = at::empty({bh, dk, dv}, q.options().dtype(at::kFloat));
   if (s_init.has_value()) a.s_init = s_init->data_ptr<float>();
@@ -226,10 +266,8 @@ py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Ten
   }
   const Tensor ws = scratch(a, 1, q);
   check(fla_sm100_bwd(&a), "libflashlinear_sm100");
-  copy_back(dq, stream);
-  copy_back(dkk, stream);
-  copy_back(dvv, stream);
-  return py::make_tuple(dq.full, dkk.full, dvv.full, r_final);
+  copy_back(out, 3, stream);
+  return py::make_tuple(out[0].full, out[1].full, out[2].full, r_final);
 }
 
 }  // namespace

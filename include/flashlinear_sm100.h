@@ -269,6 +269,11 @@ int fla_sm100_pad_rows(const void* src, void* dst, long long rows, int d, int dp
 /* dst[r][0..d) = src[r][0..d) for src rows of dpad elements: the inverse copy, for gradients that
  * must come back in the contiguous layout of torch.empty_like (linear_attn_kernels_smallv_hd.py:384). */
 int fla_sm100_unpad_rows(const void* src, void* dst, long long rows, int d, int dpad, void* stream);
+/* The same for `count` (at most 4) tensors of one shape in one launch. */
+int fla_sm100_pad_rows_batch(const void* const* src, void* const* dst, int count, long long rows, int d, int dpad,
+                             void* stream);
+int fla_sm100_unpad_rows_batch(const void* const* src, void* const* dst, int count, long long rows, int d, int dpad,
+                               void* stream);
 
 /* ---- normalised attention: the denominator of README.md:27-30 as kernels ----
  * The reference returns the unnormalised product and leaves

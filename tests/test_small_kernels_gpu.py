@@ -1,0 +1,75 @@
+"""GPU tests of the small kernels beside the attention kernels: the recurrent kernel that takes
+forward calls of a few tokens, and the row pad / unpad kernels."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# tokens: one, an odd few, the longest call of the recurrent kernel (16) and the shortest beyond it;
+# head dims: a whole tile, columns that are no multiple of 4 or of a block's 32, one block, dk != dv
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens", [1, 5, 16, 17])
+@pytest.mark.parametrize("dk,dv", [(128, 128), (83, 83), (64, 40), (8, 128), (128, 8)])
+def test_few_tokens_from_a_state(tokens, dk, dv, dtype):
+    from flashy_linear_attention_b200 import LinearAttentionResumable
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens * 1000 + dk + dv)
+    B, H = 2, 3
+    q, k = (torch.randn(B, tokens, H, dk, device="cuda", generator=gen).to(dtype).transpose(1, 2) / dk**0.5
+            for _ in range(2))
+    v = torch.randn(B, H, tokens, dv, device="cuda", generator=gen).to(dtype)
+    s0 = torch.randn(B, H, dk, dv, device="cuda", generator=gen)
+    for state in (s0, None):
+        out, s1 = LinearAttentionResumable.apply(q, k, v, state)
+        qd, kd, vd = q.double(), k.double(), v.double()
+        start = torch.zeros_like(s0).double() if state is None else s0.double()
+        want = qd @ start + torch.tril(qd @ kd.transpose(-1, -2)) @ vd
+        want_s = start + kd.transpose(-1, -2) @ vd
+        # fp32 sums of at most tokens + 1 terms of size <= max|s|
+        assert (s1.double() - want_s).abs().max() <= 2e-6 * (tokens + 1) * want_s.abs().max()
+        # one rounding of the result (half an ulp: 2^-9 / 2^-12 relative); from 17 tokens on the state
+        # and the scores are rounded to 16 bits as well, three roundings that add up in norm
+        ulp = 2.0**-9 if dtype == torch.bfloat16 else 2.0**-12
+        rounds = 1 if tokens <= 16 else 3
+        rel = (out.double() - want).norm() / want.norm()
+        assert rel <= rounds * ulp, (rel.item(), rounds * ulp)
+
+
+def test_few_tokens_state_in_place():
+    from flashy_linear_attention_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(1, 4, 3, 128, device="cuda", generator=gen).bfloat16() for _ in range(3))
+    state = torch.randn(4, 128, 128, device="cuda", generator=gen)
+    other = torch.empty_like(state)
+    out = ops.causal_dot_product_fwd(q, k, v, s_init=state, s_final=other)
+    out2 = ops.causal_dot_product_fwd(q, k, v, s_init=state, s_final=state)
+    assert torch.equal(out, out2) and torch.equal(state, other)
+
+
+# rows of one element, pieces that cross one row end, several, none; a last block with few rows;
+# destinations that are 16-byte aligned and only 4-byte aligned
+@pytest.mark.parametrize("rows", [1, 31, 33, 1000])
+@pytest.mark.parametrize("d", [1, 3, 7, 9, 16, 83, 273])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_pad_and_unpad_rows_batch(rows, d, offset):
+    from flashy_linear_attention_b200 import _lib
+
+    lib = _lib.load()
+    dpad = (d + 7) // 8 * 8
+    n = 3
+    src = [torch.randn(rows * d + 8, device="cuda").bfloat16()[offset:offset + rows * d] for _ in range(n)]
+    mid = [torch.full((rows, dpad), 7.0, device="cuda").bfloat16() for _ in range(n)]
+    buf = [torch.full((rows * d + 64,), 5.0, device="cuda").bfloat16() for _ in range(n)]
+    dst = [b[8 + offset:8 + offset + rows * d] for b in buf]
+    stream = torch.cuda.current_stream().cuda_stream
+    arr = lambda ts: (ctypes.c_void_p * n)(*[t.data_ptr() for t in ts])  # noqa: E731
+    assert lib.fla_sm100_pad_rows_batch(arr(src), arr(mid), n, rows, d, dpad, stream) == 0
+    assert lib.fla_sm100_unpad_rows_batch(arr(mid), arr(dst), n, rows, d, dpad, stream) == 0
+    for s, m, t, b in zip(src, mid, dst, buf):
+        assert torch.equal(m[:, :d], s.view(rows, d)) and not m[:, d:].any()
+        assert torch.equal(t, s)
+        assert (b[:8 + offset] == 5).all() and (b[8 + offset + rows * d:] == 5).all()  # nothing beyond
