@@ -566,7 +566,31 @@ int current_sm_count_early() {
   return sm;
 }
 
-int auto_segments(int nprob, int bh, int nchunks, int sm_count) {
+// Splitting a sequence pays when the chunks it saves every CTA from walking cost more than the two
+// barriers, the scan and the state loads of a segmented launch. Both times are close to linear in the
+// number of chunks n; fitted to 1 - 96 heads, 4 - 64 chunks, bf16 (microseconds, s segments that fill
+// the SMs once):
+//                          unsegmented     segmented
+//   128-wide, forward      9 + 1.85 n      22 + (0.35 + 3.0 / s) n
+//   128-wide, backward     9 + 1.8 n       22 + 2.9 n / s             (one fused launch)
+//    64-wide, forward      7 + 1.14 n      15 + 1.8 n / s
+//    64-wide, backward     6 + 1.17 n      15.6 + 1.6 n / s
+// so two segments of a 128-wide forward never pay (64 heads, 8 chunks: 23 us whole, 38 us split; 72
+// heads, 16 chunks: 42 and 54) and three pay from about 27 chunks on. Sequences of at most 2048
+// tokens run a split backward as three launches, which cost 6 to 9 us more.
+bool split_pays(int nprob, int nseg, int nchunks, int width) {
+  const double n = nchunks, per_seg = n / nseg;
+  const bool three_launches = nprob > 1 && nchunks < kSingleSweepMinChunks;
+  if (width > 64) {
+    if (nprob == 1) return 1.5 * n - 3.0 * per_seg > 13.0;
+    return 1.8 * n - 2.9 * per_seg > (three_launches ? 22.0 : 13.0);
+  }
+  if (nprob == 1) return 1.14 * n - 1.8 * per_seg > 8.0;
+  return 1.17 * n - 1.6 * per_seg > (three_launches ? 13.0 : 9.6);
+}
+
+// `width`: the wider of the two head dims (it selects the kernel's tile).
+int auto_segments(int nprob, int bh, int nchunks, int sm_count, int width) {
   const long ctas = static_cast<long>(nprob) * bh;
   if (ctas * 4 >= static_cast<long>(sm_count) * 3) return 1;  // already >= 75 % of the SMs
   // One wave: as many segments as fit the SMs once (every CTA pays a fixed start-up cost, and the
@@ -576,6 +600,7 @@ int auto_segments(int nprob, int bh, int nchunks, int sm_count) {
   if (max_seg < 1) max_seg = 1;
   if (want > max_seg) want = max_seg;
   if (want < 1) want = 1;
+  if (want > 1 && !split_pays(nprob, want, nchunks, width)) return 1;
   // make segments equal: seg_chunks = ceil(nchunks / want), then recompute the count
   const int seg_chunks = (nchunks + want - 1) / want;
   return (nchunks + seg_chunks - 1) / seg_chunks;
@@ -610,7 +635,7 @@ SegPlan make_plan(int want, int nchunks) {
 // Segments of a forward call (one product per head).
 SegPlan forward_plan(const FlaArgs* a, int sm_count) {
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  const int want = a->segments > 0 ? a->segments : auto_segments(1, a->batch * a->heads, nchunks, sm_count);
+  const int want = a->segments > 0 ? a->segments : auto_segments(1, a->batch * a->heads, nchunks, sm_count, std::max(a->dk, a->dv));
   SegPlan p = make_plan(want, nchunks);
   if (a->segments <= 0 && p.nseg > 1 && nchunks % p.seg_chunks != 0) {
     // An automatic split prefers equal segments (up to a quarter longer than the even share): the
@@ -633,7 +658,7 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   const int bh = a->batch * a->heads;
   const SegPlan none = {1, nchunks};
-  const SegPlan base = make_plan(auto_segments(3, bh, nchunks, sm_count), nchunks);
+  const SegPlan base = make_plan(auto_segments(3, bh, nchunks, sm_count, std::max(a->dk, a->dv)), nchunks);
   if (base.nseg <= 1 || f.nseg <= 1 || nchunks % f.seg_chunks != 0) return none;
   SegPlan b;
   b.seg_chunks = (base.seg_chunks + f.seg_chunks - 1) / f.seg_chunks * f.seg_chunks;
@@ -731,7 +756,7 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
   const int bh = B * H;
   const int nchunks = (N + fla::kChunk - 1) / fla::kChunk;
   int nseg = segments;
-  if (nseg <= 0) nseg = auto_segments(nprob, bh, nchunks, dev.sm_count);
+  if (nseg <= 0) nseg = auto_segments(nprob, bh, nchunks, dev.sm_count, std::max(da, dc));
   if (nseg > nchunks) nseg = nchunks;
   const int seg_chunks = seg_chunks_in > 0 ? seg_chunks_in : (nchunks + nseg - 1) / nseg;
   nseg = (nchunks + seg_chunks - 1) / seg_chunks;
@@ -903,7 +928,7 @@ int run_state(const Operand& bop, const Operand& cop, int B, int H, int N, int d
   const int bh = B * H;
   const int nchunks = (N + fla::kChunk - 1) / fla::kChunk;
   int nseg = segments;
-  if (nseg <= 0) nseg = auto_segments(1, bh, nchunks, dev.sm_count);
+  if (nseg <= 0) nseg = auto_segments(1, bh, nchunks, dev.sm_count, std::max(da, dc));
   if (nseg > nchunks) nseg = nchunks;
   const int seg_chunks = (nchunks + nseg - 1) / nseg;
   nseg = (nchunks + seg_chunks - 1) / seg_chunks;
@@ -1163,7 +1188,7 @@ int fla_sm100_auto_segments(const FlaArgs* a, int pass) {
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  return auto_segments(pass == 1 ? 3 : 1, a->batch * a->heads, nchunks, sm);
+  return auto_segments(pass == 1 ? 3 : 1, a->batch * a->heads, nchunks, sm, std::max(a->dk, a->dv));
 }
 
 size_t fla_sm100_workspace_bytes(const FlaArgs* a, int pass) {
@@ -1196,7 +1221,7 @@ int fla_sm100_bwd_uses_final_state(const FlaArgs* a) {
   if (!(nchunks >= kSingleSweepMinChunks || (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP))) return 0;
   if (fla_sm100_seg_states_bytes(a) > 0) return 1;
   int nseg = a->segments > 0 ? a->segments
-                             : auto_segments(3, a->batch * a->heads, nchunks, current_sm_count_early());
+                             : auto_segments(3, a->batch * a->heads, nchunks, current_sm_count_early(), std::max(a->dk, a->dv));
   return nseg <= 1 ? 1 : 0;
 }
 
@@ -1311,7 +1336,7 @@ int fla_sm100_bwd(const FlaArgs* a) {
     }
   }
   int nseg = a->segments > 0 ? a->segments
-                             : auto_segments(3, a->batch * a->heads, nchunks, dev->sm_count);
+                             : auto_segments(3, a->batch * a->heads, nchunks, dev->sm_count, std::max(a->dk, a->dv));
   if (nseg > nchunks) nseg = nchunks;
   if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks)) {
     // The forward state after this call's tokens is known: dQ can walk the sequence in the same
@@ -1377,7 +1402,7 @@ int fla_sm100_fwd_static_scratch(const FlaArgs* a) {
   // How much scratch this shape needs with the segment count the call will use.
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   int nseg = a->segments > 0 ? a->segments
-                             : auto_segments(1, a->batch * a->heads, nchunks, dev->sm_count);
+                             : auto_segments(1, a->batch * a->heads, nchunks, dev->sm_count, std::max(a->dk, a->dv));
   if (nseg > nchunks) nseg = nchunks;
   if (nseg > 1) {
     const int seg_chunks = (nchunks + nseg - 1) / nseg;
@@ -1727,7 +1752,7 @@ namespace {
 // Segment count and scratch size of the exchange path (scratch is needed even for one segment).
 int exchange_segments(const FlaArgs* a, int sm_count) {
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  int nseg = a->segments > 0 ? a->segments : auto_segments(1, a->batch * a->heads, nchunks, sm_count);
+  int nseg = a->segments > 0 ? a->segments : auto_segments(1, a->batch * a->heads, nchunks, sm_count, std::max(a->dk, a->dv));
   if (nseg > nchunks) nseg = nchunks;
   if (nseg < 1) nseg = 1;
   const int seg_chunks = (nchunks + nseg - 1) / nseg;
