@@ -531,6 +531,13 @@ int device_info(DeviceInfo** out) {
       ok &= cudaFuncSetAttribute(fla::fla_wide_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  fla::WideCfg<3>::SMEM_BYTES) == cudaSuccess;
       constexpr int kMaxSmem = 232448;
+      auto norm_smem = [&](const void* fn, int bytes) {
+        ok &= cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+      };
+      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<64, 64, false, 1>), fla::Cfg<64, 64>::NORM_SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<64, 64, false, 2>), fla::Cfg<64, 64>::NORM_SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<128, 128, false, 1>), fla::Cfg<128, 128>::NORM_SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<128, 128, false, 2>), fla::Cfg<128, 128>::NORM_SMEM_BYTES);
       auto big_smem = [&](const void* fn) {
         ok &= cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess;
       };
@@ -683,11 +690,15 @@ size_t seg_states_bytes(const FlaArgs* a, int sm_count, SegPlan* fwd_out, SegPla
 }
 
 template <int D>
-int launch_kernel(const KernelParams& kp_in, dim3 grid, cudaStream_t stream) {
+int launch_kernel(const KernelParams& kp_in, dim3 grid, cudaStream_t stream, int norm) {
   KernelParams kp = kp_in;
   kp.wait_limit_us = g_wait_limit_us;
   kp.debug_withhold = g_debug_withhold;
-  if (g_half)
+  if (norm == 1)
+    fla::fla_chunk_kernel<D, D, false, 1><<<grid, fla::kThreads, fla::Cfg<D, D>::NORM_SMEM_BYTES, stream>>>(kp);
+  else if (norm == 2)
+    fla::fla_chunk_kernel<D, D, false, 2><<<grid, fla::kThreads, fla::Cfg<D, D>::NORM_SMEM_BYTES, stream>>>(kp);
+  else if (g_half)
     fla::fla_chunk_kernel<D, D, true><<<grid, fla::kThreads, fla::Cfg<D, D>::SMEM_BYTES, stream>>>(kp);
   else
     fla::fla_chunk_kernel<D, D><<<grid, fla::kThreads, fla::Cfg<D, D>::SMEM_BYTES, stream>>>(kp);
@@ -699,9 +710,10 @@ int launch_kernel(const KernelParams& kp_in, dim3 grid, cudaStream_t stream) {
   return e == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
 }
 
-int launch_template(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t stream) {
-  if (tmpl == 64) return launch_kernel<64>(kp, grid, stream);
-  if (tmpl == 128) return launch_kernel<128>(kp, grid, stream);
+// norm: the kernel's NORM variant, 0 for attention without its denominator
+int launch_template(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t stream, int norm = 0) {
+  if (tmpl == 64) return launch_kernel<64>(kp, grid, stream, norm);
+  if (tmpl == 128) return launch_kernel<128>(kp, grid, stream, norm);
   return FLA_ERR_UNSUPPORTED;
 }
 
@@ -744,13 +756,23 @@ int launch_fused(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t strea
   return FLA_ERR_UNSUPPORTED;
 }
 
+// What the NORM variants of the kernel take beside the products, see KernelParams.
+struct NormLaunch {
+  int variant;  // 1 forward, 2 backward
+  float eps;
+  float* den;
+  float* k_sums;
+  const float* bias;
+  const float* w_sums;
+};
+
 // Runs `nprob` products that share shapes (da, dc) in one grid (plus, with segments, a state pass
 // and a scan before it).
 // `seg_chunks_in` > 0 fixes the segment length (in chunks) instead of deriving it from `segments`.
 int run_products(const Product* prods, int nprob, int B, int H, int N, int da, int dc,
                  int segments, void* workspace, size_t workspace_bytes, int32_t* status,
                  cudaStream_t stream, const DeviceInfo& dev, bool states_ready = false,
-                 int seg_chunks_in = 0) {
+                 int seg_chunks_in = 0, const NormLaunch* norm = nullptr) {
   const int tmpl = pick_template(da, dc);
   if (tmpl == 0) return FLA_ERR_UNSUPPORTED;
   const int bh = B * H;
@@ -814,8 +836,16 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
       kp.prob[i].st_trans = prods[i].ext_trans;
     }
     kp.mode = 0;
-    return launch_template(tmpl, kp, dim3(nprob, 1, bh), stream);
+    if (norm != nullptr) {
+      kp.eps = norm->eps;
+      kp.den = norm->den;
+      kp.k_sums = norm->k_sums;
+      kp.bias = norm->bias;
+      kp.w_sums = norm->w_sums;
+    }
+    return launch_template(tmpl, kp, dim3(nprob, 1, bh), stream, norm != nullptr ? norm->variant : 0);
   }
+  if (norm != nullptr) return FLA_ERR_UNSUPPORTED;
 
   float* ws = static_cast<float*>(workspace);
   // The fused form sums ONE state per (head, segment). Products that start from the partial sums
@@ -1045,9 +1075,12 @@ int run_wide_any(const Product& pd, int B, int H, int N, int da, int dc, int32_t
 
 // Forward calls of a few tokens go to the recurrent kernel. 256 heads of 128 x 128, one token: 8.4 us
 // against 36 us for the chunk kernel, which moves the state through tensor memory and works on a
-// whole 128-token tile whatever the call holds. DECODE_LINE
+// whole 128-token tile whatever the call holds. It takes 0.5 us a token (a dependent chain) once few
+// blocks share an SM: at 128 columns 16 tokens still win on 16 heads (11.4 against 15.1 us) and on 1024
+// (82 against 112), at 64 columns only 8 do (16 heads: 6.8 against 8.5 us, 11.1 against 8.4 with 16).
 bool use_decode(const FlaArgs* a) {
-  return a->seqlen <= fla::kDecodeMaxTokens && a->dk <= fla::kDecodeRows && a->dv <= 128 &&
+  const int most = std::max(a->dk, a->dv) > 64 ? fla::kDecodeMaxTokens : fla::kDecodeMaxTokens / 2;
+  return a->seqlen <= most && a->dk <= fla::kDecodeRows && a->dv <= 128 &&
          a->segment_states_ready == 0 && a->segments <= 1 && g_debug_withhold == 0 &&
          reinterpret_cast<uintptr_t>(a->s_init) % 16 == 0 && reinterpret_cast<uintptr_t>(a->s_final) % 16 == 0;
 }
@@ -1138,6 +1171,37 @@ int static_scratch_address(void** out) {
   }
   *out = addr[dev];
   return FLA_OK;
+}
+
+// The three gradients as products, see the top of this file.
+void backward_products(const FlaArgs* a, Product* pq, Product* pv, Product* pk) {
+  // dQ: causal, state sum v^T k = S^T (dv x dk)
+  pq->a = operand(a->d_o, a->dv);
+  pq->b = operand(a->v, a->dv);
+  pq->c = operand(a->k, a->dk);
+  pq->out = operand(a->d_q, a->dk);
+  pq->flags = 0;
+  pq->ext_init = a->s_init;
+  pq->ext_final = nullptr;
+  pq->ext_trans = 1;
+  // dV: anti-causal, state sum q^T dO = R (dk x dv)
+  pv->a = operand(a->k, a->dk);
+  pv->b = operand(a->q, a->dk);
+  pv->c = operand(a->d_o, a->dv);
+  pv->out = operand(a->d_v, a->dv);
+  pv->flags = fla::kFlagDescending | fla::kFlagUpperMask;
+  pv->ext_init = a->r_init;
+  pv->ext_final = a->r_final;
+  pv->ext_trans = 0;
+  // dK: anti-causal, state sum dO^T q = R^T (dv x dk)
+  pk->a = operand(a->v, a->dv);
+  pk->b = operand(a->d_o, a->dv);
+  pk->c = operand(a->q, a->dk);
+  pk->out = operand(a->d_k, a->dk);
+  pk->flags = fla::kFlagDescending | fla::kFlagUpperMask;
+  pk->ext_init = a->r_init;
+  pk->ext_final = nullptr;
+  pk->ext_trans = 1;
 }
 
 }  // namespace
@@ -1266,36 +1330,8 @@ int fla_sm100_bwd(const FlaArgs* a) {
   int rc = check_common(a, &dev);
   if (rc) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
-  // dQ: causal, state sum v^T k = S^T (dv x dk)
-  Product pq;
-  pq.a = operand(a->d_o, a->dv);
-  pq.b = operand(a->v, a->dv);
-  pq.c = operand(a->k, a->dk);
-  pq.out = operand(a->d_q, a->dk);
-  pq.flags = 0;
-  pq.ext_init = a->s_init;
-  pq.ext_final = nullptr;
-  pq.ext_trans = 1;
-  // dV: anti-causal, state sum q^T dO = R (dk x dv)
-  Product pv;
-  pv.a = operand(a->k, a->dk);
-  pv.b = operand(a->q, a->dk);
-  pv.c = operand(a->d_o, a->dv);
-  pv.out = operand(a->d_v, a->dv);
-  pv.flags = fla::kFlagDescending | fla::kFlagUpperMask;
-  pv.ext_init = a->r_init;
-  pv.ext_final = a->r_final;
-  pv.ext_trans = 0;
-  // dK: anti-causal, state sum dO^T q = R^T (dv x dk)
-  Product pk;
-  pk.a = operand(a->v, a->dv);
-  pk.b = operand(a->d_o, a->dv);
-  pk.c = operand(a->q, a->dk);
-  pk.out = operand(a->d_k, a->dk);
-  pk.flags = fla::kFlagDescending | fla::kFlagUpperMask;
-  pk.ext_init = a->r_init;
-  pk.ext_final = nullptr;
-  pk.ext_trans = 1;
+  Product pq, pv, pk;
+  backward_products(a, &pq, &pv, &pk);
 
   if (a->dk > 128 || a->dv > 128) {
     // Head dims above the 128-wide tiles (SmallVHD shapes: dQ and dK have the wide head dim on the
@@ -1724,6 +1760,103 @@ int fla_sm100_normalize_bwd_sweep(const FlaArgs* a, const float* dden) {
     fla::fla_normalize_bwd_sweep_kernel<16, 0><<<grid, fla::kNormThreads, smem, stream>>>(p);
   ++g_last_launches;
   return cudaGetLastError() == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
+}
+
+// ---- attention with its denominator, fused into the chunk kernel
+int fla_sm100_normalized_fused(const FlaArgs* a) {
+  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0) return 0;
+  if (a->dk != a->dv || a->dk > 128 || a->dk % 8 != 0 || a->dtype != FLA_DTYPE_BF16) return 0;
+  if (a->segments > 1) return 0;
+  const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
+  const int bh = a->batch * a->heads, sm = current_sm_count_early();
+  return a->segments == 1 || (auto_segments(1, bh, nchunks, sm, a->dk) == 1 && auto_segments(3, bh, nchunks, sm, a->dk) == 1);
+}
+
+size_t fla_sm100_normalized_sums_bytes(const FlaArgs* a) {
+  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0) return 0;
+  const int tmpl = pick_template(a->dk, a->dv);
+  const size_t nchunks = (static_cast<size_t>(a->seqlen) + fla::kChunk - 1) / fla::kChunk;
+  return static_cast<size_t>(a->batch) * a->heads * nchunks * tmpl * sizeof(float);
+}
+
+int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den, float* k_sums) {
+  DeviceInfo* dev = nullptr;
+  g_last_launches = 0;
+  int rc = check_common(a, &dev);
+  if (rc) return rc;
+  if (den == nullptr) return FLA_ERR_INVALID;
+  if (reinterpret_cast<uintptr_t>(k_sums) % 16 != 0) return FLA_ERR_ALIGNMENT;
+  if (a->s_init != nullptr || !fla_sm100_normalized_fused(a)) return FLA_ERR_UNSUPPORTED;
+  Product p;
+  p.a = operand(a->q, a->dk);
+  p.b = operand(a->k, a->dk);
+  p.c = operand(a->v, a->dv);
+  p.out = operand(a->o, a->dv);
+  p.flags = 0;
+  p.ext_init = nullptr;
+  p.ext_final = a->s_final;
+  p.ext_trans = 0;
+  const NormLaunch norm = {1, eps, den, k_sums, nullptr, nullptr};
+  return run_products(&p, 1, a->batch, a->heads, a->seqlen, a->dk, a->dv, 1, nullptr, 0, a->status,
+                      static_cast<cudaStream_t>(a->stream), *dev, false, 0, &norm);
+}
+
+int fla_sm100_normalized_bwd_prepare(const FlaArgs* a, const float* den, float* dden, float* w_sums) {
+  DeviceInfo* dev = nullptr;
+  g_last_launches = 0;
+  int rc = check_common(a, &dev);
+  if (rc) return rc;
+  if (den == nullptr || dden == nullptr || w_sums == nullptr) return FLA_ERR_INVALID;
+  if (!fla_sm100_normalized_fused(a)) return FLA_ERR_UNSUPPORTED;
+  if ((rc = check_operand(operand(a->d_o, a->dv), a->batch, a->heads)) ||
+      (rc = check_operand(operand(a->o, a->dv), a->batch, a->heads)) ||
+      (rc = check_operand(operand(a->q, a->dk), a->batch, a->heads)) ||
+      (rc = check_operand(operand(a->d_v, a->dv), a->batch, a->heads)))
+    return rc;
+  fla::NormParams p;
+  memset(&p, 0, sizeof(p));
+  p.x = norm_tensor(a->d_o);
+  p.y = norm_tensor(a->o);
+  p.z = norm_tensor(a->d_v);
+  p.q = norm_tensor(a->q);
+  p.den = const_cast<float*>(den);
+  p.dden = dden;
+  p.sums_out = w_sums;
+  p.heads = a->heads;
+  p.n = a->seqlen;
+  p.dk = a->dk;
+  p.dv = a->dv;
+  cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  const dim3 grid((a->seqlen + fla::kNormChunk - 1) / fla::kNormChunk, a->batch * a->heads, 1);
+  const int cols = pick_template(a->dk, a->dv);
+  if (a->dk == 128)
+    fla::fla_normalize_bwd_prepare_sums_kernel<128><<<grid, fla::kNormThreads, 0, stream>>>(p, cols);
+  else if (a->dk == 64)
+    fla::fla_normalize_bwd_prepare_sums_kernel<64><<<grid, fla::kNormThreads, 0, stream>>>(p, cols);
+  else
+    fla::fla_normalize_bwd_prepare_sums_kernel<0><<<grid, fla::kNormThreads, 0, stream>>>(p, cols);
+  ++g_last_launches;
+  return cudaGetLastError() == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
+}
+
+int fla_sm100_normalized_bwd(const FlaArgs* a, const float* dden, const float* k_sums, const float* w_sums) {
+  DeviceInfo* dev = nullptr;
+  g_last_launches = 0;
+  int rc = check_common(a, &dev);
+  if (rc) return rc;
+  if (dden == nullptr || k_sums == nullptr || w_sums == nullptr) return FLA_ERR_INVALID;
+  if (a->s_init || a->r_init || a->r_final || !fla_sm100_normalized_fused(a)) return FLA_ERR_UNSUPPORTED;
+  Product all[3];  // dQ, dV, dK
+  backward_products(a, &all[0], &all[1], &all[2]);
+  all[0].flags |= fla::kFlagRowBias;
+  all[2].flags |= fla::kFlagColBias;
+  if (a->s_last != nullptr && single_sweep_allowed((a->seqlen + fla::kChunk - 1) / fla::kChunk)) {
+    all[0].flags |= fla::kFlagDescending | fla::kFlagTotalMinusSuffix | fla::kFlagFirstChunkExact;
+    all[0].ext_init = a->s_last;
+  }
+  const NormLaunch norm = {2, 0.f, nullptr, const_cast<float*>(k_sums), dden, w_sums};
+  return run_products(all, 3, a->batch, a->heads, a->seqlen, a->dk, a->dv, 1, nullptr, 0, a->status,
+                      static_cast<cudaStream_t>(a->stream), *dev, false, 0, &norm);
 }
 
 int fla_sm100_product(const FlaArgs* a, int anticausal) {

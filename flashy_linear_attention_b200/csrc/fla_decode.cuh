@@ -33,7 +33,7 @@ struct DecodeParams {
 constexpr int kDecodeThreads = 128;
 constexpr int kDecodeCols = 32;       // columns of the state per block
 constexpr int kDecodeRows = 128;      // rows a block covers: 16 groups of 8
-constexpr int kDecodeMaxTokens = 16;  // longest call that takes this kernel, see use_decode()
+constexpr int kDecodeMaxTokens = 16;  // longest call the kernel has room for, see use_decode()
 
 template <bool HALF>
 __device__ __forceinline__ float decode_load(const void* base, long long idx) {

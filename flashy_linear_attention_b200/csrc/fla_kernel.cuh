@@ -71,6 +71,11 @@ constexpr int kFlagTotalMinusSuffix = 4;
 // score tile alone (ordinary lower mask, no state term); otherwise its first rows would be the
 // small difference of two 128-term sums and lose accuracy.
 constexpr int kFlagFirstChunkExact = 8;
+// Gradients of attention WITH its denominator (NORM == 2 below): the score (a_i . b_j) is taken plus
+// bias_i (row) or plus bias_j (column), and what that adds to the state term comes from column sums
+// of c that other kernels formed per chunk.
+constexpr int kFlagRowBias = 16;
+constexpr int kFlagColBias = 32;
 
 struct KernelParams {
   Problem prob[3];
@@ -98,6 +103,13 @@ struct KernelParams {
   int pre_prob;
   float* part_out;
   unsigned bar_slot;   // which pair of g_grid_barriers this launch uses
+  // ---- attention with its denominator (NORM != 0, unsegmented launches only)
+  float eps;           // NORM 1: den_i = q_i . (sum of k_j, j <= i) + eps, and o_i is divided by it
+  float* den;          // NORM 1: [bh][tokens], out
+  float* k_sums;       // [bh][chunk][DK]: sum of k over all tokens up to the end of the chunk (NORM 1:
+                       // out; NORM 2: in, for the problem with kFlagRowBias)
+  const float* bias;   // NORM 2: [bh][tokens], d(loss)/d(den)
+  const float* w_sums; // NORM 2: [bh][chunk][DK]: sum of bias_i q_i over the chunk's own tokens
 };
 
 // Barrier words of the fused form. Only the CTAs of one head exchange data, so every head has its
@@ -138,6 +150,16 @@ struct Cfg {
   static constexpr int S_COL = 256 + O_BUFS * DV;  // S fp32: DV columns, lane = dk index
   static constexpr int TMEM_COLS = 512;
   static_assert(S_COL + DV <= TMEM_COLS, "TMEM budget");
+  // Attention with its denominator: two vectors of DK floats, then 128 floats (NORM 1: row sums of
+  // the score tile's lower column half, NORM 2: the chunk's bias), then NORM 1's row sums of the
+  // upper column half for rows 64 .. 127 (the causal mask leaves none elsewhere), which at DK = 128
+  // sit in the unused end of the barrier area: shared memory is full to the byte.
+  static constexpr int NORM_VEC_BYTES = 2 * DK * 4;
+  static constexpr int NORM_BYTES = NORM_VEC_BYTES + 512 + (DK == 128 ? 0 : 256);
+  static constexpr int NORM_HI_OFF = DK == 128 ? -256 : NORM_VEC_BYTES + 512;  // from the end of the barriers
+  static constexpr int NORM_SMEM_BYTES = SMEM_BYTES + NORM_BYTES;
+  static_assert(NORM_SMEM_BYTES <= SMEM_LIMIT, "shared memory budget");
+  static_assert(DK != 128 || (2 * NSLOT + 15) * 8 + 16 <= BAR_BYTES - 256, "barrier area");
 };
 
 // Arguments of converter_prologue(): where the CTA is and where its buffers and barriers are.
@@ -523,7 +545,18 @@ __device__ __noinline__ bool converter_prologue(const KernelParams& p, const Pro
 
 // HALF: operands and outputs are fp16 instead of bf16 (same tiles, same pipeline; only the MMA
 // operand format and the fp32 -> 16-bit roundings differ).
-template <int DK, int DV, bool HALF = false>
+//
+// NORM: attention with its denominator, den_i = q_i . z_i + eps with z_i = sum_{j<=i} k_j, in the
+// same pass (see fla_normalize.cuh for the formulas as separate kernels). The score tile already
+// holds the part of den_i that comes from the chunk itself, as its row sums in fp32, and a bias on
+// the scores is the whole of what den's gradient adds to dQ and dK inside a chunk; what is left is
+// one vector of DK floats per chunk (a running column sum) and a rank-1 term in the epilogue.
+//   1  forward: the epilogue warps form q_i . z and the column sums of the k tile from the tiles in
+//      the ring before they wait for the accumulator, and divide while they round.
+//   2  backward: bias_i = d(loss)/d(den_i) goes onto the scores of dQ (rows) and dK (columns); the
+//      epilogue adds bias_i z (dQ) or the suffix sum of bias_i q_i (dK).
+// NORM_TIMES
+template <int DK, int DV, bool HALF = false, int NORM = 0>
 __global__ void __launch_bounds__(kThreads, 1)
 fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   using cfg = Cfg<DK, DV>;
@@ -563,8 +596,14 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   const uint32_t s_full = bar_base + 8u * (2 * NSLOT + 4);
   const uint32_t part_done = bar_base + 8u * (2 * NSLOT + 10);  // fused: partial sum stored (256 arrivals)
   const uint32_t grid_done = bar_base + 8u * (2 * NSLOT + 11);  // fused: the grid barrier was passed
-  const uint32_t holder_off =
-      NSLOT * cfg::TILE_BYTES + cfg::SB_BYTES + cfg::OST_BYTES + 8u * (2 * NSLOT + 12);
+  const uint32_t rs_full = bar_base + 8u * (2 * NSLOT + 12);  // NORM 1: row sums written (256 arrivals)
+  const uint32_t rs_free = bar_base + 8u * (2 * NSLOT + 13);  // NORM 1: and read (128)
+  const uint32_t vec_ready = bar_base + 8u * (2 * NSLOT + 14);  // NORM: the epilogue's vector written (128)
+  const uint32_t norm_base = bar_base + cfg::BAR_BYTES;
+  const uint32_t norm_lo = norm_base + cfg::NORM_VEC_BYTES;
+  const uint32_t norm_hi = norm_base + cfg::NORM_HI_OFF;
+  const uint32_t holder_off = NSLOT * cfg::TILE_BYTES + cfg::SB_BYTES + cfg::OST_BYTES +
+                              8u * (2 * NSLOT + (NORM != 0 ? 15 : 12));
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem_gen + holder_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + holder_off + 4);
 
@@ -622,7 +661,8 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     for (int s = 0; s < NSLOT; ++s) {
       ptx::mbar_init(full_bar(s), 1);
       // mode 0: every tile is read by two MMA groups, each followed by a tcgen05.commit arrival
-      ptx::mbar_init(empty_bar(s), mode == 0 ? 2 : 1);
+      // (NORM 1: and by the four epilogue warps)
+      ptx::mbar_init(empty_bar(s), mode == 0 ? (NORM == 1 ? 6 : 2) : 1);
     }
     ptx::mbar_init(p_full, 1);
     ptx::mbar_init(pb_ready, 256);
@@ -636,6 +676,11 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     ptx::mbar_init(s_full, 1);
     ptx::mbar_init(part_done, 256);
     ptx::mbar_init(grid_done, 1);
+    if (NORM != 0) {
+      ptx::mbar_init(rs_full, 256);
+      ptx::mbar_init(rs_free, 128);
+      ptx::mbar_init(vec_ready, 128);
+    }
     ptx::fence_barrier_init();
     ptx::fence_proxy_async_smem();
   }
@@ -978,12 +1023,30 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     // phase A, if it ran, used the first phase of s_full
     const uint32_t s_off = a_iter > 0 ? 1u : 0u;
     if (mode == 0) {
+      const bool row_bias = NORM == 2 && (pr.flags & kFlagRowBias) != 0;
+      const bool col_bias = NORM == 2 && (pr.flags & kFlagColBias) != 0;
+      float row_sum = 0.f;
       for (int i = 0; conv_ok && i < n_iter; ++i) {
+        float bias0 = 0.f, bias1 = 0.f;  // this row's, or those of two columns of this warp's half
+        if (NORM == 2 && (row_bias || col_bias)) {
+          const float* src = p.bias + static_cast<size_t>(bh) * pr.n_tokens;
+          const int tok0 = mem_chunk(i) * kChunk + (row_bias ? row : half * 64 + lane);
+          if (tok0 < pr.n_tokens) bias0 = __ldg(src + tok0);
+          if (col_bias && tok0 + 32 < pr.n_tokens) bias1 = __ldg(src + tok0 + 32);
+        }
         // ---------------- P: fp32 -> causal mask -> bf16 A operand (this group's 64 columns)
         int ok = ptx::mbar_wait(p_full, i & 1, abort_flag) ? 1 : 0;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         ptx::tc_fence_after();
+        if (NORM == 2 && col_bias) {
+          // The four warps of a half write the same values. The buffer is free: every converter
+          // thread arrived on p_read after it had used the last chunk's, and p_full came after that.
+          ptx::st_shared_b32(norm_lo + (half * 64 + lane) * 4, __float_as_uint(bias0));
+          ptx::st_shared_b32(norm_lo + (half * 64 + 32 + lane) * 4, __float_as_uint(bias1));
+          __syncwarp();
+        }
+        row_sum = 0.f;
         // Column blocks of 32: relative to this warp's 32 rows a block is entirely kept, entirely
         // masked, or (block index == quadrant) the diagonal block that needs per-element tests.
         // The three mask modes are compiled separately (MODE 0: keep col <= row; 1: keep
@@ -1004,7 +1067,31 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           } else if (!masked1) {
             ptx::tmem_ld32(lane_base + cfg::P_COL + cb1 * 32, rb);
           }
-          auto convert_block = [&](int cb, bool masked, const uint32_t (&r)[32]) {
+          auto convert_block = [&](int cb, bool masked, uint32_t (&r)[32]) {
+            if (NORM == 2 && !masked) {
+              if (row_bias) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + bias0);
+              } else if (col_bias) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                  const float4 x = ptx::ld_shared_f4(norm_lo + (cb * 32 + j) * 4);
+                  r[j] = __float_as_uint(__uint_as_float(r[j]) + x.x);
+                  r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + x.y);
+                  r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + x.z);
+                  r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + x.w);
+                }
+              }
+            }
+            if (NORM == 1 && !masked) {
+              float even = 0.f, odd = 0.f;
+#pragma unroll
+              for (int j = 0; j < 32; j += 2) {
+                even += (cb != quad || j <= lane) ? __uint_as_float(r[j]) : 0.f;
+                odd += (cb != quad || j + 1 <= lane) ? __uint_as_float(r[j + 1]) : 0.f;
+              }
+              row_sum += even + odd;
+            }
             if (masked) {
 #pragma unroll
               for (int j = 0; j < 16; ++j) pk[j] = 0u;
@@ -1071,6 +1158,15 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
             ptx::mbar_arrive(sb_ready);
           }
         }
+        if (NORM == 1) {
+          // One buffer: chunk i - 1's sums have been read (its epilogue needs nothing more from here).
+          ok = i == 0 || ptx::mbar_wait(rs_free, (i - 1) & 1, abort_flag) ? 1 : 0;
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          if (half == 0) ptx::st_shared_b32(norm_lo + row * 4, __float_as_uint(row_sum));
+          else if (row >= 64) ptx::st_shared_b32(norm_hi + (row - 64) * 4, __float_as_uint(row_sum));
+          ptx::mbar_arrive(rs_full);
+        }
       }
     } else {
       // state only: one read-out after the last chunk
@@ -1089,7 +1185,105 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
       const uint32_t swz = static_cast<uint32_t>(row & 7);
       uint32_t ra[32], rb[32];
+      // NORM 1: running column sums of k, 8 columns in each of the first kPieces lanes of a warp.
+      // NORM 2: column `tid` of the vector that the state term takes (dK: a running suffix sum).
+      constexpr int kPieces = DK / 32;  // 16-byte pieces of a k row that one warp sums
+      float z_run[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      float q_dot = 0.f, w_run = 0.f;
+      const bool row_bias = NORM == 2 && (pr.flags & kFlagRowBias) != 0;
+      const bool col_bias = NORM == 2 && (pr.flags & kFlagColBias) != 0;
       for (int i = 0; i < n_iter; ++i) {
+        const uint32_t vec = norm_base + (i & 1) * (DK * 4);  // this chunk's vector
+        if (NORM == 1) {
+          const int tq = 3 * i;
+          bool up = wait_uniform(full_bar(tq % NSLOT), (tq / NSLOT) & 1);  // q and k tiles
+          // the vector of chunk i was written by all warps during chunk i - 1
+          if (up && i > 0) up = wait_uniform(vec_ready, (i - 1) & 1);
+          if (!up) break;
+          q_dot = 0.f;
+          if (i > 0) {
+            float d0 = 0.f, d1 = 0.f;
+            const uint32_t q_row = slot_addr(tq) + row * 128;
+#pragma unroll
+            for (int pc = 0; pc < DK / 8; ++pc) {
+              const uint4 x = ptx::ld_shared_u4(q_row + (pc >> 3) * kGroupBytes + (((pc & 7) ^ swz) << 4));
+              const float4 z0 = ptx::ld_shared_f4(vec + pc * 32), z1 = ptx::ld_shared_f4(vec + pc * 32 + 16);
+              d0 += ptx::bf16_lo(x.x) * z0.x + ptx::bf16_lo(x.y) * z0.z;
+              d1 += ptx::bf16_hi(x.x) * z0.y + ptx::bf16_hi(x.y) * z0.w;
+              d0 += ptx::bf16_lo(x.z) * z1.x + ptx::bf16_lo(x.w) * z1.z;
+              d1 += ptx::bf16_hi(x.z) * z1.y + ptx::bf16_hi(x.w) * z1.w;
+            }
+            q_dot = d0 + d1;
+          }
+          // Column sums of the k tile: a warp takes kPieces 16-byte pieces of every row, 32 / kPieces
+          // rows at a time, chosen so that each quarter of the warp reads eight different 16-byte
+          // columns of the swizzled tile.
+          {
+            const int piece = quad * kPieces + lane % kPieces;
+            const int sub = lane / kPieces;
+            const int r0 = (sub % (8 / kPieces)) * kPieces + (sub / (8 / kPieces)) % kPieces +
+                           8 * ((sub / (8 / kPieces)) / kPieces);
+            const uint32_t k_col = slot_addr(tq + 1) + (piece >> 3) * kGroupBytes;
+            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+            for (int it = 0; it < 4 * kPieces; ++it) {
+              const int r = r0 + it * (32 / kPieces);
+              const uint4 x = ptx::ld_shared_u4(k_col + r * 128 + (((piece & 7) ^ (r & 7)) << 4));
+              acc[0] += ptx::bf16_lo(x.x); acc[1] += ptx::bf16_hi(x.x);
+              acc[2] += ptx::bf16_lo(x.y); acc[3] += ptx::bf16_hi(x.y);
+              acc[4] += ptx::bf16_lo(x.z); acc[5] += ptx::bf16_hi(x.z);
+              acc[6] += ptx::bf16_lo(x.w); acc[7] += ptx::bf16_hi(x.w);
+            }
+#pragma unroll
+            for (int o = kPieces; o < 32; o <<= 1)
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) z_run[j] += acc[j];
+            if (lane < kPieces) {
+              const uint32_t next = norm_base + ((i + 1) & 1) * (DK * 4) + piece * 32;
+              ptx::st_shared_v4(next, __float_as_uint(z_run[0]), __float_as_uint(z_run[1]),
+                                __float_as_uint(z_run[2]), __float_as_uint(z_run[3]));
+              ptx::st_shared_v4(next + 16, __float_as_uint(z_run[4]), __float_as_uint(z_run[5]),
+                                __float_as_uint(z_run[6]), __float_as_uint(z_run[7]));
+              if (p.k_sums != nullptr) {
+                float4* dst = reinterpret_cast<float4*>(
+                    p.k_sums + (static_cast<size_t>(bh) * p.nchunks + i) * DK + piece * 8);
+                dst[0] = make_float4(z_run[0], z_run[1], z_run[2], z_run[3]);
+                dst[1] = make_float4(z_run[4], z_run[5], z_run[6], z_run[7]);
+              }
+            }
+          }
+          // Every thread has read this chunk's vector and written its part of the next.
+          ptx::mbar_arrive(vec_ready);
+          __syncwarp();
+          if (lane == 0) {
+            ptx::mbar_arrive(empty_bar(tq % NSLOT));
+            ptx::mbar_arrive(empty_bar((tq + 1) % NSLOT));
+          }
+        }
+        float bias_row = 1.f;
+        if (NORM == 2 && (row_bias || col_bias)) {
+          const int c = mem_chunk(i);
+          const int tid = static_cast<int>(threadIdx.x) - 320;  // 0 .. 127, a column here
+          float x = 0.f;
+          if (row_bias) {
+            // ascending: the sum before this chunk; descending: its own tokens included, as in the
+            // state; the chunk computed without the state: none
+            const int upto = tms ? c : c - 1;
+            if (tid < DK && upto >= 0 && !plain_chunk(i))
+              x = __ldg(p.k_sums + (static_cast<size_t>(bh) * p.nchunks + upto) * DK + tid);
+            const int tok = c * kChunk + row;
+            bias_row = tok < pr.n_tokens ? __ldg(p.bias + static_cast<size_t>(bh) * pr.n_tokens + tok) : 0.f;
+          } else {
+            x = w_run;
+            if (tid < DK) w_run += __ldg(p.w_sums + (static_cast<size_t>(bh) * p.nchunks + c) * DK + tid);
+          }
+          // two buffers: chunk i - 2's vector has been read by every thread that arrived for i - 1
+          if (tid < DK) ptx::st_shared_b32(vec + tid * 4, __float_as_uint(x));
+          ptx::mbar_arrive(vec_ready);
+          if (!wait_uniform(vec_ready, i & 1)) break;
+        }
         int ok = ptx::mbar_wait((i & 1) ? o_full1 : o_full0, (i >> 1) & 1, abort_flag) ? 1 : 0;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -1099,6 +1293,17 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         // before overwriting its rows, lane 0 checks that the previous store has read them.
         if (lane == 0) ptx::bulk_wait_group_read0();
         __syncwarp();
+        float inv = 1.f;
+        if (NORM == 1) {
+          if (lane == 0) ptx::mbar_arrive(empty_bar((3 * i + 2) % NSLOT));  // v: not read here, see empty_bar
+          if (!wait_uniform(rs_full, i & 1)) break;
+          float den = q_dot + p.eps + __uint_as_float(ptx::ld_shared_b32(norm_lo + row * 4));
+          if (row >= 64) den += __uint_as_float(ptx::ld_shared_b32(norm_hi + (row - 64) * 4));
+          const int tok = mem_chunk(i) * kChunk + row;
+          if (tok < pr.n_tokens) p.den[static_cast<size_t>(bh) * pr.n_tokens + tok] = den;
+          inv = 1.f / den;
+          ptx::mbar_arrive(rs_free);
+        }
         const uint32_t obuf = ost_addr + row * 128;
         // One 64-column group at a time: two TMEM loads in flight, rounded and written to the
         // staging rows straight away (16-byte pieces XOR-swizzled by row % 8), so that only 64
@@ -1107,6 +1312,27 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         for (int gg = 0; gg < cfg::GV; ++gg) {
           const uint32_t o_col = cfg::O_COL + (cfg::O_BUFS == 2 ? (i & 1) * DV : 0) + gg * 64;
           ptx::tmem_ld32x2(lane_base + o_col, ra, lane_base + o_col + 32, rb);
+          if (NORM == 1) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              ra[j] = __float_as_uint(__uint_as_float(ra[j]) * inv);
+              rb[j] = __float_as_uint(__uint_as_float(rb[j]) * inv);
+            }
+          }
+          if (NORM == 2 && (row_bias || col_bias)) {
+            auto add_vec = [&](uint32_t at, uint32_t (&r)[32]) {
+#pragma unroll
+              for (int j = 0; j < 32; j += 4) {
+                const float4 x = ptx::ld_shared_f4(at + j * 4);
+                r[j] = __float_as_uint(__uint_as_float(r[j]) + bias_row * x.x);
+                r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + bias_row * x.y);
+                r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + bias_row * x.z);
+                r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + bias_row * x.w);
+              }
+            };
+            add_vec(vec + gg * 256, ra);
+            add_vec(vec + gg * 256 + 128, rb);
+          }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             ptx::st_shared_v4(

@@ -165,6 +165,12 @@ class LinearAttentionNormalized(Function):
         q, k = ops.kernel_view(q), ops.kernel_view(k)  # repacked once if the rows are not 16-byte multiples
         B, H, _, dk = q.shape
         need_grad = any(ctx.needs_input_grad[:3])
+        ctx.fused = ops.normalized_fused(q, k, v)
+        if ctx.fused:
+            out, den, k_sums, s_final = ops.normalized_fwd(q, k, v, eps, need_grad)
+            ctx.has_state = s_final is not None
+            ctx.save_for_backward(q, k, v, out, den, k_sums, *((s_final,) if ctx.has_state else ()))
+            return out
         s_final = None
         if need_grad and ops.backward_uses_final_state(q, v):
             s_final = torch.empty(B * H, dk, v.shape[-1], dtype=torch.float32, device=q.device)
@@ -181,8 +187,12 @@ class LinearAttentionNormalized(Function):
 
     @staticmethod
     def backward(ctx: Any, grad_output):
-        q, k, v, out, den = ctx.saved_tensors[:5]
-        s_final = ctx.saved_tensors[5] if ctx.has_state else None
+        saved = ctx.saved_tensors
+        q, k, v, out, den = saved[:5]
+        if ctx.fused:
+            return ops.normalized_bwd(grad_output, q, k, v, out, den, saved[5],
+                                      saved[6] if ctx.has_state else None) + (None,)
+        s_final = saved[5] if ctx.has_state else None
         dnum, dden = ops.normalize_bwd_prepare(grad_output, out, den)
         dq, dk, dv = ops.causal_dot_product_bwd(dnum, q, k, v, s_last=s_final, keep_padded=True)
         ops.normalize_bwd_sweep(q, k, dq, dk, dden)
