@@ -96,10 +96,7 @@ EXPORTED_SYMBOLS = (
     "fla_sm100_normalize_bwd_prepare",
     "fla_sm100_normalize_bwd_sweep",
     "fla_sm100_normalized_fused",
-    "fla_sm100_normalized_sums_bytes",
     "fla_sm100_normalized_fwd",
-    "fla_sm100_normalized_bwd_prepare",
-    "fla_sm100_normalized_bwd",
     "fla_sm100_taylor_dims",
     "fla_sm100_taylor_features",
     "fla_sm100_taylor_features_bwd",
@@ -175,14 +172,8 @@ def load() -> ctypes.CDLL:
     lib.fla_sm100_normalize_bwd_sweep.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_void_p]
     lib.fla_sm100_normalized_fused.restype = ctypes.c_int
     lib.fla_sm100_normalized_fused.argtypes = [ctypes.POINTER(FlaArgs)]
-    lib.fla_sm100_normalized_sums_bytes.restype = ctypes.c_size_t
-    lib.fla_sm100_normalized_sums_bytes.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_normalized_fwd.restype = ctypes.c_int
-    lib.fla_sm100_normalized_fwd.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_float, ctypes.c_void_p, ctypes.c_void_p]
-    for name in ("fla_sm100_normalized_bwd_prepare", "fla_sm100_normalized_bwd"):
-        fn = getattr(lib, name)
-        fn.restype = ctypes.c_int
-        fn.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.fla_sm100_normalized_fwd.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_float, ctypes.c_void_p]
     lib.fla_sm100_taylor_dims.restype = ctypes.c_int
     lib.fla_sm100_taylor_dims.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
     lib.fla_sm100_taylor_features.restype = ctypes.c_int

@@ -534,10 +534,8 @@ int device_info(DeviceInfo** out) {
       auto norm_smem = [&](const void* fn, int bytes) {
         ok &= cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
       };
-      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<64, 64, false, 1>), fla::Cfg<64, 64>::NORM_SMEM_BYTES);
-      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<64, 64, false, 2>), fla::Cfg<64, 64>::NORM_SMEM_BYTES);
-      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<128, 128, false, 1>), fla::Cfg<128, 128>::NORM_SMEM_BYTES);
-      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<128, 128, false, 2>), fla::Cfg<128, 128>::NORM_SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<64, 64, false, true>), fla::Cfg<64, 64>::NORM_SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<128, 128, false, true>), fla::Cfg<128, 128>::NORM_SMEM_BYTES);
       auto big_smem = [&](const void* fn) {
         ok &= cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess;
       };
@@ -566,6 +564,9 @@ int pick_template(int da, int dc) {
   if (m <= 128) return 128;
   return 0;
 }
+
+// Token rows of the boxes that fla_chunk_kernel<tmpl, tmpl> loads.
+int load_rows(int tmpl) { return tmpl == 64 ? fla::Cfg<64, 64>::LOAD_ROWS : fla::Cfg<128, 128>::LOAD_ROWS; }
 
 int current_sm_count_early() {
   int sm = 148, dev = 0;
@@ -690,14 +691,12 @@ size_t seg_states_bytes(const FlaArgs* a, int sm_count, SegPlan* fwd_out, SegPla
 }
 
 template <int D>
-int launch_kernel(const KernelParams& kp_in, dim3 grid, cudaStream_t stream, int norm) {
+int launch_kernel(const KernelParams& kp_in, dim3 grid, cudaStream_t stream, bool norm) {
   KernelParams kp = kp_in;
   kp.wait_limit_us = g_wait_limit_us;
   kp.debug_withhold = g_debug_withhold;
-  if (norm == 1)
-    fla::fla_chunk_kernel<D, D, false, 1><<<grid, fla::kThreads, fla::Cfg<D, D>::NORM_SMEM_BYTES, stream>>>(kp);
-  else if (norm == 2)
-    fla::fla_chunk_kernel<D, D, false, 2><<<grid, fla::kThreads, fla::Cfg<D, D>::NORM_SMEM_BYTES, stream>>>(kp);
+  if (norm)
+    fla::fla_chunk_kernel<D, D, false, true><<<grid, fla::kThreads, fla::Cfg<D, D>::NORM_SMEM_BYTES, stream>>>(kp);
   else if (g_half)
     fla::fla_chunk_kernel<D, D, true><<<grid, fla::kThreads, fla::Cfg<D, D>::SMEM_BYTES, stream>>>(kp);
   else
@@ -710,8 +709,8 @@ int launch_kernel(const KernelParams& kp_in, dim3 grid, cudaStream_t stream, int
   return e == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
 }
 
-// norm: the kernel's NORM variant, 0 for attention without its denominator
-int launch_template(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t stream, int norm = 0) {
+// norm: attention with its denominator (the kernel's NORM variant)
+int launch_template(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t stream, bool norm = false) {
   if (tmpl == 64) return launch_kernel<64>(kp, grid, stream, norm);
   if (tmpl == 128) return launch_kernel<128>(kp, grid, stream, norm);
   return FLA_ERR_UNSUPPORTED;
@@ -756,14 +755,10 @@ int launch_fused(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t strea
   return FLA_ERR_UNSUPPORTED;
 }
 
-// What the NORM variants of the kernel take beside the products, see KernelParams.
+// What the kernel's NORM variant takes beside the product, see KernelParams.
 struct NormLaunch {
-  int variant;  // 1 forward, 2 backward
   float eps;
   float* den;
-  float* k_sums;
-  const float* bias;
-  const float* w_sums;
 };
 
 // Runs `nprob` products that share shapes (da, dc) in one grid (plus, with segments, a state pass
@@ -804,8 +799,9 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
         (rc = check_operand(pd.c, B, H)) || (rc = check_operand(pd.out, B, H)))
       return rc;
     Problem& pr = kp.prob[i];
-    if ((rc = encode_map(&pr.q, pd.a, B, H, N)) || (rc = encode_map(&pr.k, pd.b, B, H, N)) ||
-        (rc = encode_map(&pr.v, pd.c, B, H, N)) || (rc = encode_map(&pr.o, pd.out, B, H, N, 32)))
+    const int rows = load_rows(tmpl);
+    if ((rc = encode_map(&pr.q, pd.a, B, H, N, rows)) || (rc = encode_map(&pr.k, pd.b, B, H, N, rows)) ||
+        (rc = encode_map(&pr.v, pd.c, B, H, N, rows)) || (rc = encode_map(&pr.o, pd.out, B, H, N, 32)))
       return rc;
     pr.flags = pd.flags;
     pr.n_tokens = N;
@@ -839,11 +835,8 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
     if (norm != nullptr) {
       kp.eps = norm->eps;
       kp.den = norm->den;
-      kp.k_sums = norm->k_sums;
-      kp.bias = norm->bias;
-      kp.w_sums = norm->w_sums;
     }
-    return launch_template(tmpl, kp, dim3(nprob, 1, bh), stream, norm != nullptr ? norm->variant : 0);
+    return launch_template(tmpl, kp, dim3(nprob, 1, bh), stream, norm != nullptr);
   }
   if (norm != nullptr) return FLA_ERR_UNSUPPORTED;
 
@@ -976,7 +969,8 @@ int run_state(const Operand& bop, const Operand& cop, int B, int H, int N, int d
   kp.st_cols = dc;
   kp.status = status;
   kp.mode = 1;
-  if ((rc = encode_map(&kp.prob[0].k, bop, B, H, N)) || (rc = encode_map(&kp.prob[0].v, cop, B, H, N)))
+  if ((rc = encode_map(&kp.prob[0].k, bop, B, H, N, load_rows(tmpl))) ||
+      (rc = encode_map(&kp.prob[0].v, cop, B, H, N, load_rows(tmpl))))
     return rc;
   kp.prob[0].s_final = (nseg == 1) ? final : static_cast<float*>(workspace);
   kp.prob[0].st_trans = (nseg == 1) ? 0 : 1;  // the scratch keeps states transposed
@@ -1769,23 +1763,15 @@ int fla_sm100_normalized_fused(const FlaArgs* a) {
   if (a->segments > 1) return 0;
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   const int bh = a->batch * a->heads, sm = current_sm_count_early();
-  return a->segments == 1 || (auto_segments(1, bh, nchunks, sm, a->dk) == 1 && auto_segments(3, bh, nchunks, sm, a->dk) == 1);
+  return a->segments == 1 || auto_segments(1, bh, nchunks, sm, a->dk) == 1;
 }
 
-size_t fla_sm100_normalized_sums_bytes(const FlaArgs* a) {
-  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0) return 0;
-  const int tmpl = pick_template(a->dk, a->dv);
-  const size_t nchunks = (static_cast<size_t>(a->seqlen) + fla::kChunk - 1) / fla::kChunk;
-  return static_cast<size_t>(a->batch) * a->heads * nchunks * tmpl * sizeof(float);
-}
-
-int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den, float* k_sums) {
+int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den) {
   DeviceInfo* dev = nullptr;
   g_last_launches = 0;
   int rc = check_common(a, &dev);
   if (rc) return rc;
   if (den == nullptr) return FLA_ERR_INVALID;
-  if (reinterpret_cast<uintptr_t>(k_sums) % 16 != 0) return FLA_ERR_ALIGNMENT;
   if (a->s_init != nullptr || !fla_sm100_normalized_fused(a)) return FLA_ERR_UNSUPPORTED;
   Product p;
   p.a = operand(a->q, a->dk);
@@ -1796,66 +1782,8 @@ int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den, float* k_s
   p.ext_init = nullptr;
   p.ext_final = a->s_final;
   p.ext_trans = 0;
-  const NormLaunch norm = {1, eps, den, k_sums, nullptr, nullptr};
+  const NormLaunch norm = {eps, den};
   return run_products(&p, 1, a->batch, a->heads, a->seqlen, a->dk, a->dv, 1, nullptr, 0, a->status,
-                      static_cast<cudaStream_t>(a->stream), *dev, false, 0, &norm);
-}
-
-int fla_sm100_normalized_bwd_prepare(const FlaArgs* a, const float* den, float* dden, float* w_sums) {
-  DeviceInfo* dev = nullptr;
-  g_last_launches = 0;
-  int rc = check_common(a, &dev);
-  if (rc) return rc;
-  if (den == nullptr || dden == nullptr || w_sums == nullptr) return FLA_ERR_INVALID;
-  if (!fla_sm100_normalized_fused(a)) return FLA_ERR_UNSUPPORTED;
-  if ((rc = check_operand(operand(a->d_o, a->dv), a->batch, a->heads)) ||
-      (rc = check_operand(operand(a->o, a->dv), a->batch, a->heads)) ||
-      (rc = check_operand(operand(a->q, a->dk), a->batch, a->heads)) ||
-      (rc = check_operand(operand(a->d_v, a->dv), a->batch, a->heads)))
-    return rc;
-  fla::NormParams p;
-  memset(&p, 0, sizeof(p));
-  p.x = norm_tensor(a->d_o);
-  p.y = norm_tensor(a->o);
-  p.z = norm_tensor(a->d_v);
-  p.q = norm_tensor(a->q);
-  p.den = const_cast<float*>(den);
-  p.dden = dden;
-  p.sums_out = w_sums;
-  p.heads = a->heads;
-  p.n = a->seqlen;
-  p.dk = a->dk;
-  p.dv = a->dv;
-  cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
-  const dim3 grid((a->seqlen + fla::kNormChunk - 1) / fla::kNormChunk, a->batch * a->heads, 1);
-  const int cols = pick_template(a->dk, a->dv);
-  if (a->dk == 128)
-    fla::fla_normalize_bwd_prepare_sums_kernel<128><<<grid, fla::kNormThreads, 0, stream>>>(p, cols);
-  else if (a->dk == 64)
-    fla::fla_normalize_bwd_prepare_sums_kernel<64><<<grid, fla::kNormThreads, 0, stream>>>(p, cols);
-  else
-    fla::fla_normalize_bwd_prepare_sums_kernel<0><<<grid, fla::kNormThreads, 0, stream>>>(p, cols);
-  ++g_last_launches;
-  return cudaGetLastError() == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
-}
-
-int fla_sm100_normalized_bwd(const FlaArgs* a, const float* dden, const float* k_sums, const float* w_sums) {
-  DeviceInfo* dev = nullptr;
-  g_last_launches = 0;
-  int rc = check_common(a, &dev);
-  if (rc) return rc;
-  if (dden == nullptr || k_sums == nullptr || w_sums == nullptr) return FLA_ERR_INVALID;
-  if (a->s_init || a->r_init || a->r_final || !fla_sm100_normalized_fused(a)) return FLA_ERR_UNSUPPORTED;
-  Product all[3];  // dQ, dV, dK
-  backward_products(a, &all[0], &all[1], &all[2]);
-  all[0].flags |= fla::kFlagRowBias;
-  all[2].flags |= fla::kFlagColBias;
-  if (a->s_last != nullptr && single_sweep_allowed((a->seqlen + fla::kChunk - 1) / fla::kChunk)) {
-    all[0].flags |= fla::kFlagDescending | fla::kFlagTotalMinusSuffix | fla::kFlagFirstChunkExact;
-    all[0].ext_init = a->s_last;
-  }
-  const NormLaunch norm = {2, 0.f, nullptr, const_cast<float*>(k_sums), dden, w_sums};
-  return run_products(all, 3, a->batch, a->heads, a->seqlen, a->dk, a->dv, 1, nullptr, 0, a->status,
                       static_cast<cudaStream_t>(a->stream), *dev, false, 0, &norm);
 }
 
@@ -2025,8 +1953,8 @@ int fla_sm100_state_exchange(const FlaArgs* a, int which, const FlaExchange* x) 
   kp.st_cols = dc;
   kp.status = a->status;
   kp.mode = 1;
-  if ((rc = encode_map(&kp.prob[0].k, bop, a->batch, a->heads, a->seqlen)) ||
-      (rc = encode_map(&kp.prob[0].v, cop, a->batch, a->heads, a->seqlen)))
+  if ((rc = encode_map(&kp.prob[0].k, bop, a->batch, a->heads, a->seqlen, load_rows(tmpl))) ||
+      (rc = encode_map(&kp.prob[0].v, cop, a->batch, a->heads, a->seqlen, load_rows(tmpl))))
     return rc;
   kp.prob[0].s_final = static_cast<float*>(a->workspace);
   kp.prob[0].st_trans = 1;

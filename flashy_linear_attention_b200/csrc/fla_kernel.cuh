@@ -8,8 +8,13 @@
 // product with the operands permuted (see fla_api.cu), which replaces the quadratic tile loops of
 // flashlinear/kernels/linear_attn_kernels.py:63-85 (fwd), :171-200 and :283-302 (bwd).
 //
-// CTA layout (480 threads, one CTA per SM):
-//   warp 0        TMA producer: Q, K, V chunk tiles -> a ring of shared-memory slots (128B swizzle)
+// CTA layout (512 threads, one CTA per SM):
+//   warps 0, 15   TMA producers: Q, K, V chunk tiles -> a ring of shared-memory slots (128B swizzle),
+//                 each warp one half of every tile. One warp issuing TMA loads gets 24 - 27 bytes a
+//                 cycle into an SM (640 cycles per 16 KB box, whatever the depth of the ring, also
+//                 with one CTA on the whole GPU), two get 38, more than two no more: with one
+//                 producer its 96 KB (D = 128) or 48 KB (D = 64) a chunk were the chunk period.
+//                 PRODUCER_TIMES
 //   warp 1        MMA issuer X (one elected lane) and TMEM owner: S += K^T V, P = Q K^T
 //   warp 14       MMA issuer Y (one elected lane): O = Q Sb, O += Pb V
 //   warps 2-5     converter group A  } P fp32 (TMEM) -> mask -> bf16 (TMEM, A operand of P V)
@@ -29,11 +34,11 @@
 namespace fla {
 
 constexpr int kChunk = 128;                // tokens per chunk (= MMA M)
-constexpr int kThreads = 480;              // 15 warps
+constexpr int kThreads = 512;              // 16 warps
 constexpr int kGroupBytes = kChunk * 128;  // one 64-column group of a chunk tile: 128 rows x 128 B
 
 struct Problem {
-  CUtensorMap q, k, v;     // 4-D maps (dim, token, head, batch), box 64 x 128 x 1 x 1, 128B swizzle
+  CUtensorMap q, k, v;     // 4-D maps (dim, token, head, batch), box 64 x Cfg::LOAD_ROWS x 1 x 1, 128B swizzle
   CUtensorMap o;           // output map with a 64 x 32 box: every epilogue warp stores its own rows
   const float* s_init;     // [bh * segments + g][st_rows][st_cols] fp32, or null
   float* s_final;          // same indexing, or null
@@ -71,11 +76,6 @@ constexpr int kFlagTotalMinusSuffix = 4;
 // score tile alone (ordinary lower mask, no state term); otherwise its first rows would be the
 // small difference of two 128-term sums and lose accuracy.
 constexpr int kFlagFirstChunkExact = 8;
-// Gradients of attention WITH its denominator (NORM == 2 below): the score (a_i . b_j) is taken plus
-// bias_i (row) or plus bias_j (column), and what that adds to the state term comes from column sums
-// of c that other kernels formed per chunk.
-constexpr int kFlagRowBias = 16;
-constexpr int kFlagColBias = 32;
 
 struct KernelParams {
   Problem prob[3];
@@ -103,13 +103,9 @@ struct KernelParams {
   int pre_prob;
   float* part_out;
   unsigned bar_slot;   // which pair of g_grid_barriers this launch uses
-  // ---- attention with its denominator (NORM != 0, unsegmented launches only)
-  float eps;           // NORM 1: den_i = q_i . (sum of k_j, j <= i) + eps, and o_i is divided by it
-  float* den;          // NORM 1: [bh][tokens], out
-  float* k_sums;       // [bh][chunk][DK]: sum of k over all tokens up to the end of the chunk (NORM 1:
-                       // out; NORM 2: in, for the problem with kFlagRowBias)
-  const float* bias;   // NORM 2: [bh][tokens], d(loss)/d(den)
-  const float* w_sums; // NORM 2: [bh][chunk][DK]: sum of bias_i q_i over the chunk's own tokens
+  // ---- attention with its denominator (NORM, unsegmented launches only)
+  float eps;           // den_i = q_i . (sum of k_j, j <= i) + eps, and o_i is divided by it
+  float* den;          // [bh][tokens], out
 };
 
 // Barrier words of the fused form. Only the CTAs of one head exchange data, so every head has its
@@ -128,6 +124,7 @@ struct Cfg {
   static constexpr int GK = DK / 64;
   static constexpr int GV = DV / 64;
   static constexpr int TILE_BYTES = GK * kGroupBytes;  // one chunk tile of q, k or v
+  static constexpr int LOAD_ROWS = GK == 2 ? kChunk : kChunk / 2;  // token rows of one load box
   static constexpr int SB_BYTES = GV * DK * 128;       // bf16 state as MMA B operand
   static constexpr int OST_BYTES = GV * kGroupBytes;   // output staging for the TMA store
   static constexpr int BAR_BYTES = 512;
@@ -150,10 +147,10 @@ struct Cfg {
   static constexpr int S_COL = 256 + O_BUFS * DV;  // S fp32: DV columns, lane = dk index
   static constexpr int TMEM_COLS = 512;
   static_assert(S_COL + DV <= TMEM_COLS, "TMEM budget");
-  // Attention with its denominator: two vectors of DK floats, then 128 floats (NORM 1: row sums of
-  // the score tile's lower column half, NORM 2: the chunk's bias), then NORM 1's row sums of the
-  // upper column half for rows 64 .. 127 (the causal mask leaves none elsewhere), which at DK = 128
-  // sit in the unused end of the barrier area: shared memory is full to the byte.
+  // Attention with its denominator: two vectors of DK floats, 128 row sums of the score tile's lower
+  // column half, then those of the upper column half for rows 64 .. 127 (the causal mask leaves none
+  // elsewhere), which at DK = 128 sit in the unused end of the barrier area: shared memory is full to
+  // the byte.
   static constexpr int NORM_VEC_BYTES = 2 * DK * 4;
   static constexpr int NORM_BYTES = NORM_VEC_BYTES + 512 + (DK == 128 ? 0 : 256);
   static constexpr int NORM_HI_OFF = DK == 128 ? -256 : NORM_VEC_BYTES + 512;  // from the end of the barriers
@@ -547,16 +544,11 @@ __device__ __noinline__ bool converter_prologue(const KernelParams& p, const Pro
 // operand format and the fp32 -> 16-bit roundings differ).
 //
 // NORM: attention with its denominator, den_i = q_i . z_i + eps with z_i = sum_{j<=i} k_j, in the
-// same pass (see fla_normalize.cuh for the formulas as separate kernels). The score tile already
-// holds the part of den_i that comes from the chunk itself, as its row sums in fp32, and a bias on
-// the scores is the whole of what den's gradient adds to dQ and dK inside a chunk; what is left is
-// one vector of DK floats per chunk (a running column sum) and a rank-1 term in the epilogue.
-//   1  forward: the epilogue warps form q_i . z and the column sums of the k tile from the tiles in
-//      the ring before they wait for the accumulator, and divide while they round.
-//   2  backward: bias_i = d(loss)/d(den_i) goes onto the scores of dQ (rows) and dK (columns); the
-//      epilogue adds bias_i z (dQ) or the suffix sum of bias_i q_i (dK).
-// NORM_TIMES
-template <int DK, int DV, bool HALF = false, int NORM = 0>
+// same pass (fla_normalize.cuh has it as separate kernels). The score tile already holds the part of
+// den_i that comes from the chunk itself, as its row sums in fp32; what is left is q_i . z with the
+// column sums z of the chunks before. The epilogue warps, idle in that time, form both from the q and
+// k tiles in the ring before they wait for the accumulator, and divide while they round. NORM_TIMES
+template <int DK, int DV, bool HALF = false, bool NORM = false>
 __global__ void __launch_bounds__(kThreads, 1)
 fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   using cfg = Cfg<DK, DV>;
@@ -596,14 +588,14 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   const uint32_t s_full = bar_base + 8u * (2 * NSLOT + 4);
   const uint32_t part_done = bar_base + 8u * (2 * NSLOT + 10);  // fused: partial sum stored (256 arrivals)
   const uint32_t grid_done = bar_base + 8u * (2 * NSLOT + 11);  // fused: the grid barrier was passed
-  const uint32_t rs_full = bar_base + 8u * (2 * NSLOT + 12);  // NORM 1: row sums written (256 arrivals)
-  const uint32_t rs_free = bar_base + 8u * (2 * NSLOT + 13);  // NORM 1: and read (128)
+  const uint32_t rs_full = bar_base + 8u * (2 * NSLOT + 12);  // NORM: row sums written (256 arrivals)
+  const uint32_t rs_free = bar_base + 8u * (2 * NSLOT + 13);  // NORM: and read (128)
   const uint32_t vec_ready = bar_base + 8u * (2 * NSLOT + 14);  // NORM: the epilogue's vector written (128)
   const uint32_t norm_base = bar_base + cfg::BAR_BYTES;
   const uint32_t norm_lo = norm_base + cfg::NORM_VEC_BYTES;
   const uint32_t norm_hi = norm_base + cfg::NORM_HI_OFF;
   const uint32_t holder_off = NSLOT * cfg::TILE_BYTES + cfg::SB_BYTES + cfg::OST_BYTES +
-                              8u * (2 * NSLOT + (NORM != 0 ? 15 : 12));
+                              8u * (2 * NSLOT + (NORM ? 15 : 12));
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem_gen + holder_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + holder_off + 4);
 
@@ -659,10 +651,10 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     abort_flag[0] = 0;
     abort_flag[1] = static_cast<int>(p.wait_limit_us);
     for (int s = 0; s < NSLOT; ++s) {
-      ptx::mbar_init(full_bar(s), 1);
+      ptx::mbar_init(full_bar(s), 2);  // both producers
       // mode 0: every tile is read by two MMA groups, each followed by a tcgen05.commit arrival
-      // (NORM 1: and by the four epilogue warps)
-      ptx::mbar_init(empty_bar(s), mode == 0 ? (NORM == 1 ? 6 : 2) : 1);
+      // (NORM: and by the four epilogue warps)
+      ptx::mbar_init(empty_bar(s), mode == 0 ? (NORM ? 6 : 2) : 1);
     }
     ptx::mbar_init(p_full, 1);
     ptx::mbar_init(pb_ready, 256);
@@ -676,7 +668,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     ptx::mbar_init(s_full, 1);
     ptx::mbar_init(part_done, 256);
     ptx::mbar_init(grid_done, 1);
-    if (NORM != 0) {
+    if (NORM) {
       ptx::mbar_init(rs_full, 256);
       ptx::mbar_init(rs_free, 128);
       ptx::mbar_init(vec_ready, 128);
@@ -720,11 +712,18 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     return smem_base + static_cast<uint32_t>(t % NSLOT) * cfg::TILE_BYTES;
   };
 
-  if (warp == 0) {
-    // ================================================================ TMA producer
+  if (warp == 0 || warp == 15) {
+    // ================================================================ TMA producers
     // The whole warp runs the loop (so that addresses and coordinates stay warp-uniform); one
     // elected lane issues. In mode 0 the q and k tiles of a chunk complete on the q tile's barrier.
+    // Each producer loads its half of every tile: one 64-column group, or 64 of the 128 rows where
+    // a tile is one group wide.
     const bool leader = ptx::elect_one();
+    const int part = warp == 0 ? 0 : 1;
+    constexpr int kPartBytes = cfg::TILE_BYTES / 2;
+    constexpr int kPartRows = cfg::LOAD_ROWS;
+    const int part_col = cfg::GK == 2 ? part * 64 : 0;
+    const int part_row = cfg::GK == 2 ? 0 : part * kPartRows;
     const int n_tiles = t0 + n_iter * tpc;
     for (int t = 0; t < n_tiles; ++t) {
       const int s = t % NSLOT;
@@ -742,16 +741,13 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       // barrier that the tile's bytes complete on, and the bytes armed on it at this point
       const uint32_t bar = (paired && which == 1) ? full_bar((t - 1) % NSLOT) : full_bar(s);
       if (leader) {
-        if (paired && which == 0) ptx::mbar_expect_tx(bar, 2 * cfg::TILE_BYTES);
-        if (!paired || which == 2) ptx::mbar_expect_tx(bar, cfg::TILE_BYTES);
+        if (paired && which == 0) ptx::mbar_expect_tx(bar, 2 * kPartBytes);
+        if (!paired || which == 2) ptx::mbar_expect_tx(bar, kPartBytes);
         // The k slot's own barrier is not waited on; complete its phase so that the parity of
         // later ring passes stays in step.
         if (paired && which == 1) ptx::mbar_arrive(full_bar(s));
-        if (!(p.debug_withhold && t == 0)) {
-#pragma unroll
-          for (int gg = 0; gg < cfg::GK; ++gg)
-            ptx::tma_load_4d(dst + gg * kGroupBytes, map, bar, gg * 64, tok, h, b);
-        }
+        if (!(p.debug_withhold && t == 0))
+          ptx::tma_load_4d(dst + part * kPartBytes, map, bar, part_col, tok + part_row, h, b);
       }
       __syncwarp();
     }
@@ -1023,29 +1019,13 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     // phase A, if it ran, used the first phase of s_full
     const uint32_t s_off = a_iter > 0 ? 1u : 0u;
     if (mode == 0) {
-      const bool row_bias = NORM == 2 && (pr.flags & kFlagRowBias) != 0;
-      const bool col_bias = NORM == 2 && (pr.flags & kFlagColBias) != 0;
       float row_sum = 0.f;
       for (int i = 0; conv_ok && i < n_iter; ++i) {
-        float bias0 = 0.f, bias1 = 0.f;  // this row's, or those of two columns of this warp's half
-        if (NORM == 2 && (row_bias || col_bias)) {
-          const float* src = p.bias + static_cast<size_t>(bh) * pr.n_tokens;
-          const int tok0 = mem_chunk(i) * kChunk + (row_bias ? row : half * 64 + lane);
-          if (tok0 < pr.n_tokens) bias0 = __ldg(src + tok0);
-          if (col_bias && tok0 + 32 < pr.n_tokens) bias1 = __ldg(src + tok0 + 32);
-        }
         // ---------------- P: fp32 -> causal mask -> bf16 A operand (this group's 64 columns)
         int ok = ptx::mbar_wait(p_full, i & 1, abort_flag) ? 1 : 0;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         ptx::tc_fence_after();
-        if (NORM == 2 && col_bias) {
-          // The four warps of a half write the same values. The buffer is free: every converter
-          // thread arrived on p_read after it had used the last chunk's, and p_full came after that.
-          ptx::st_shared_b32(norm_lo + (half * 64 + lane) * 4, __float_as_uint(bias0));
-          ptx::st_shared_b32(norm_lo + (half * 64 + 32 + lane) * 4, __float_as_uint(bias1));
-          __syncwarp();
-        }
         row_sum = 0.f;
         // Column blocks of 32: relative to this warp's 32 rows a block is entirely kept, entirely
         // masked, or (block index == quadrant) the diagonal block that needs per-element tests.
@@ -1067,23 +1047,8 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           } else if (!masked1) {
             ptx::tmem_ld32(lane_base + cfg::P_COL + cb1 * 32, rb);
           }
-          auto convert_block = [&](int cb, bool masked, uint32_t (&r)[32]) {
-            if (NORM == 2 && !masked) {
-              if (row_bias) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + bias0);
-              } else if (col_bias) {
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) {
-                  const float4 x = ptx::ld_shared_f4(norm_lo + (cb * 32 + j) * 4);
-                  r[j] = __float_as_uint(__uint_as_float(r[j]) + x.x);
-                  r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + x.y);
-                  r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + x.z);
-                  r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + x.w);
-                }
-              }
-            }
-            if (NORM == 1 && !masked) {
+          auto convert_block = [&](int cb, bool masked, const uint32_t (&r)[32]) {
+            if (NORM && !masked) {
               float even = 0.f, odd = 0.f;
 #pragma unroll
               for (int j = 0; j < 32; j += 2) {
@@ -1158,7 +1123,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
             ptx::mbar_arrive(sb_ready);
           }
         }
-        if (NORM == 1) {
+        if (NORM) {
           // One buffer: chunk i - 1's sums have been read (its epilogue needs nothing more from here).
           ok = i == 0 || ptx::mbar_wait(rs_free, (i - 1) & 1, abort_flag) ? 1 : 0;
           ok = __all_sync(0xffffffffu, ok);
@@ -1185,16 +1150,13 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
       const uint32_t swz = static_cast<uint32_t>(row & 7);
       uint32_t ra[32], rb[32];
-      // NORM 1: running column sums of k, 8 columns in each of the first kPieces lanes of a warp.
-      // NORM 2: column `tid` of the vector that the state term takes (dK: a running suffix sum).
+      // running column sums of k, 8 columns in each of the first kPieces lanes of a warp
       constexpr int kPieces = DK / 32;  // 16-byte pieces of a k row that one warp sums
       float z_run[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      float q_dot = 0.f, w_run = 0.f;
-      const bool row_bias = NORM == 2 && (pr.flags & kFlagRowBias) != 0;
-      const bool col_bias = NORM == 2 && (pr.flags & kFlagColBias) != 0;
+      float q_dot = 0.f;
       for (int i = 0; i < n_iter; ++i) {
         const uint32_t vec = norm_base + (i & 1) * (DK * 4);  // this chunk's vector
-        if (NORM == 1) {
+        if (NORM) {
           const int tq = 3 * i;
           bool up = wait_uniform(full_bar(tq % NSLOT), (tq / NSLOT) & 1);  // q and k tiles
           // the vector of chunk i was written by all warps during chunk i - 1
@@ -1246,12 +1208,6 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
                                 __float_as_uint(z_run[2]), __float_as_uint(z_run[3]));
               ptx::st_shared_v4(next + 16, __float_as_uint(z_run[4]), __float_as_uint(z_run[5]),
                                 __float_as_uint(z_run[6]), __float_as_uint(z_run[7]));
-              if (p.k_sums != nullptr) {
-                float4* dst = reinterpret_cast<float4*>(
-                    p.k_sums + (static_cast<size_t>(bh) * p.nchunks + i) * DK + piece * 8);
-                dst[0] = make_float4(z_run[0], z_run[1], z_run[2], z_run[3]);
-                dst[1] = make_float4(z_run[4], z_run[5], z_run[6], z_run[7]);
-              }
             }
           }
           // Every thread has read this chunk's vector and written its part of the next.
@@ -1261,28 +1217,6 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
             ptx::mbar_arrive(empty_bar(tq % NSLOT));
             ptx::mbar_arrive(empty_bar((tq + 1) % NSLOT));
           }
-        }
-        float bias_row = 1.f;
-        if (NORM == 2 && (row_bias || col_bias)) {
-          const int c = mem_chunk(i);
-          const int tid = static_cast<int>(threadIdx.x) - 320;  // 0 .. 127, a column here
-          float x = 0.f;
-          if (row_bias) {
-            // ascending: the sum before this chunk; descending: its own tokens included, as in the
-            // state; the chunk computed without the state: none
-            const int upto = tms ? c : c - 1;
-            if (tid < DK && upto >= 0 && !plain_chunk(i))
-              x = __ldg(p.k_sums + (static_cast<size_t>(bh) * p.nchunks + upto) * DK + tid);
-            const int tok = c * kChunk + row;
-            bias_row = tok < pr.n_tokens ? __ldg(p.bias + static_cast<size_t>(bh) * pr.n_tokens + tok) : 0.f;
-          } else {
-            x = w_run;
-            if (tid < DK) w_run += __ldg(p.w_sums + (static_cast<size_t>(bh) * p.nchunks + c) * DK + tid);
-          }
-          // two buffers: chunk i - 2's vector has been read by every thread that arrived for i - 1
-          if (tid < DK) ptx::st_shared_b32(vec + tid * 4, __float_as_uint(x));
-          ptx::mbar_arrive(vec_ready);
-          if (!wait_uniform(vec_ready, i & 1)) break;
         }
         int ok = ptx::mbar_wait((i & 1) ? o_full1 : o_full0, (i >> 1) & 1, abort_flag) ? 1 : 0;
         ok = __all_sync(0xffffffffu, ok);
@@ -1294,7 +1228,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         if (lane == 0) ptx::bulk_wait_group_read0();
         __syncwarp();
         float inv = 1.f;
-        if (NORM == 1) {
+        if (NORM) {
           if (lane == 0) ptx::mbar_arrive(empty_bar((3 * i + 2) % NSLOT));  // v: not read here, see empty_bar
           if (!wait_uniform(rs_full, i & 1)) break;
           float den = q_dot + p.eps + __uint_as_float(ptx::ld_shared_b32(norm_lo + row * 4));
@@ -1312,26 +1246,18 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         for (int gg = 0; gg < cfg::GV; ++gg) {
           const uint32_t o_col = cfg::O_COL + (cfg::O_BUFS == 2 ? (i & 1) * DV : 0) + gg * 64;
           ptx::tmem_ld32x2(lane_base + o_col, ra, lane_base + o_col + 32, rb);
-          if (NORM == 1) {
+          if (NORM) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              ra[j] = __float_as_uint(__uint_as_float(ra[j]) * inv);
-              rb[j] = __float_as_uint(__uint_as_float(rb[j]) * inv);
+            for (int j = 0; j < 32; j += 2) {
+              // rounded to 16 bits before the division, as the separate kernels do: the gradients,
+              // sums of two cancelling parts that both depend on this value, then stay what they are
+              const uint32_t a = ptx::pack_bf16x2(__uint_as_float(ra[j]), __uint_as_float(ra[j + 1]));
+              const uint32_t c = ptx::pack_bf16x2(__uint_as_float(rb[j]), __uint_as_float(rb[j + 1]));
+              ra[j] = __float_as_uint(ptx::bf16_lo(a) * inv);
+              ra[j + 1] = __float_as_uint(ptx::bf16_hi(a) * inv);
+              rb[j] = __float_as_uint(ptx::bf16_lo(c) * inv);
+              rb[j + 1] = __float_as_uint(ptx::bf16_hi(c) * inv);
             }
-          }
-          if (NORM == 2 && (row_bias || col_bias)) {
-            auto add_vec = [&](uint32_t at, uint32_t (&r)[32]) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 4) {
-                const float4 x = ptx::ld_shared_f4(at + j * 4);
-                r[j] = __float_as_uint(__uint_as_float(r[j]) + bias_row * x.x);
-                r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + bias_row * x.y);
-                r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + bias_row * x.z);
-                r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + bias_row * x.w);
-              }
-            };
-            add_vec(vec + gg * 256, ra);
-            add_vec(vec + gg * 256 + 128, rb);
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {

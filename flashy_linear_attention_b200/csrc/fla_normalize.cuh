@@ -359,92 +359,6 @@ fla_normalize_bwd_prepare_kernel(const NormParams p_in) {
   }
 }
 
-// The same for the fused form (NORM in fla_kernel.cuh), one block per 128-token chunk, which also
-// leaves the chunk's column sums of dden_i q_i in sums_out[bh][chunk][sum_cols] (zero beyond dk): the
-// chunk's dden are in shared memory at that point. dk == dv <= 128. Bound by HBM: g, out, q in, dnum out. PREPARE_TIME
-constexpr int kNormChunk = 128;
-template <int D>
-__global__ void __launch_bounds__(kNormThreads)
-fla_normalize_bwd_prepare_sums_kernel(const NormParams p_in, int sum_cols) {
-  NormParams p = p_in;
-  if (D != 0) p.dk = p.dv = D;
-  __shared__ float weight[kNormChunk];
-  __shared__ float part[kNormThreads * 8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int bh = blockIdx.y;
-  const int b = bh / p.heads, h = bh % p.heads;
-  const int tok0 = blockIdx.x * kNormChunk;
-  const int rows = min(kNormChunk, p.n - tok0);
-  const int dvp = (p.dv + 7) / 8 * 8;
-  const int lpr = lanes_per_row(dvp);
-  const int rpw = 32 / lpr;
-  const int sub = lane % lpr, rsel = lane / lpr;
-  const int c = sub * 8;  // at most 16 pieces a row: one step
-  const bool valid = c < dvp;
-  const float* den = p.den + static_cast<size_t>(bh) * p.n;
-  float* dden = p.dden + static_cast<size_t>(bh) * p.n;
-#pragma unroll 4
-  for (int r0 = warp * rpw; r0 < kNormChunk; r0 += (kNormThreads / 32) * rpw) {
-    const int r = r0 + rsel;
-    const bool live = r < rows;
-    const int tok = tok0 + (live ? r : rows - 1);  // keep the whole warp in the shuffles
-    uint4 gv = make_uint4(0u, 0u, 0u, 0u), ov = gv;
-    if (valid) {
-      gv = *reinterpret_cast<const uint4*>(norm_row(p.x, b, h, tok) + c);
-      ov = *reinterpret_cast<const uint4*>(norm_row(p.y, b, h, tok) + c);
-    }
-    const float inv = 1.f / den[tok];
-    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
-    const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w};
-    uint32_t res[4];
-    float acc = 0.f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {  // dv is a multiple of 8: no ragged piece
-      const float2 gg = bf2_to_f2(gw[j]), oo = bf2_to_f2(ow[j]);
-      acc += gg.x * oo.x + gg.y * oo.y;
-      res[j] = f2_to_bf2(gg.x * inv, gg.y * inv);
-    }
-    if (live && valid)
-      *reinterpret_cast<uint4*>(const_cast<__nv_bfloat16*>(norm_row(p.z, b, h, tok)) + c) =
-          make_uint4(res[0], res[1], res[2], res[3]);
-    for (int o2 = lpr >> 1; o2 > 0; o2 >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o2);
-    if (sub == 0) {
-      weight[r] = live ? -acc * inv : 0.f;
-      if (live) dden[tok] = -acc * inv;
-    }
-  }
-  __syncthreads();
-  const int pieces = dvp >> 3;
-  const int rows_per_pass = kNormThreads / pieces;
-  const int piece = threadIdx.x % pieces, rgrp = threadIdx.x / pieces;
-  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (rgrp < rows_per_pass) {
-#pragma unroll 4
-    for (int r = rgrp; r < rows; r += rows_per_pass) {
-      const uint4 v = *reinterpret_cast<const uint4*>(norm_row(p.q, b, h, tok0 + r) + piece * 8);
-      const float w = weight[r];
-      const uint32_t words[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = bf2_to_f2(words[j]);
-        sum[2 * j] += w * f.x;
-        sum[2 * j + 1] += w * f.y;
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) part[threadIdx.x * 8 + j] = sum[j];
-  __syncthreads();
-  for (int col = threadIdx.x; col < sum_cols; col += kNormThreads) {
-    float tot = 0.f;
-    if (col < p.dk) {
-      const int pc = col >> 3, j = col & 7;
-      for (int g = 0; g < rows_per_pass; ++g) tot += part[(g * pieces + pc) * 8 + j];
-    }
-    p.sums_out[(static_cast<size_t>(bh) * gridDim.x + blockIdx.x) * sum_cols + col] = tot;
-  }
-}
-
 // Shared memory: kNormStages x ((src tile, dst tile) bf16 + T floats of dden)
 __host__ __device__ inline size_t norm_sweep_smem_bytes(int dk, int tile) {
   const size_t dkp = (dk + 7) / 8 * 8;

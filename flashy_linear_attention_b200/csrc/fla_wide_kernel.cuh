@@ -12,10 +12,12 @@
 //     S_t += B_t^T C            (state rows of pair t, fp32 in tensor memory)
 // and the chunk ends with O += mask(P) C. The state S (128*NT x 64 fp32) never leaves tensor memory.
 //
-// CTA layout (448 threads, one CTA per (batch, head)):
-//   warp 0       TMA producer: c tile of the chunk (own double buffer), then the a/b tile pairs
+// CTA layout (480 threads, one CTA per (batch, head)):
+//   warps 0, 14  TMA producers: c tile of the chunk (own double buffer), then the a/b tile pairs
 //                into a ring of eight 16 KB slots (one 64-column group each; a tile takes the one
-//                or two groups that hold valid columns, so padding costs no ring space)
+//                or two groups that hold valid columns, so padding costs no ring space). They take
+//                turns, group by group: one warp alone issues at most 27 bytes a cycle (see
+//                fla_kernel.cuh), two get 38. PRODUCER_TIMES
 //   warp 1       MMA issuer (one elected lane) and TMEM owner
 //   warps 2-9    converters: P fp32 -> mask -> bf16 (TMEM), S fp32 -> bf16 (shared memory)
 //   warps 10-13  epilogue: O fp32 -> bf16 -> staging -> TMA store (each warp its own 32 rows)
@@ -42,7 +44,7 @@ struct WideParams {
   int debug_withhold;  // test hook: the first c tile is never loaded, so the waits on it run out
 };
 
-constexpr int kWideThreads = 448;
+constexpr int kWideThreads = 480;
 constexpr int kWideChunk = 128;
 constexpr int kWideGroupBytes = kWideChunk * 128;   // 64 columns x 128 rows
 constexpr int kWideSlots = 8;  // ring slots of one 64-column group (16 KB) each
@@ -168,24 +170,29 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
     return smem_base + static_cast<uint32_t>(g % kWideSlots) * kWideGroupBytes;
   };
 
-  if (warp == 0) {
-    // ================================================================ TMA producer
+  if (warp == 0 || warp == 14) {
+    // ================================================================ TMA producers
+    // Producer `part` loads the groups of its parity and every second c tile.
     const bool leader = ptx::elect_one();
+    const int part = warp == 0 ? 0 : 1;
     bool ok = true;
     for (int i = 0; ok && i < n_iter; ++i) {
       const int tok = mem_chunk(i) * kWideChunk;
       const int cs = i & 1;
-      if (!wait_uniform(cempty_bar(cs), ((i >> 1) & 1) ^ 1u)) break;
-      if (leader) {
-        ptx::mbar_expect_tx(cfull_bar(cs), kWideGroupBytes);
-        if (!(p.debug_withhold && i == 0))
-          ptx::tma_load_4d(c_addr + cs * kWideGroupBytes, &p.c, cfull_bar(cs), c_col0, tok, h, b);
+      if (cs == part) {
+        if (!wait_uniform(cempty_bar(cs), ((i >> 1) & 1) ^ 1u)) break;
+        if (leader) {
+          ptx::mbar_expect_tx(cfull_bar(cs), kWideGroupBytes);
+          if (!(p.debug_withhold && i == 0))
+            ptx::tma_load_4d(c_addr + cs * kWideGroupBytes, &p.c, cfull_bar(cs), c_col0, tok, h, b);
+        }
       }
       for (int t = 0; t < NT; ++t) {
         const int groups = pair_groups(t);  // a group that is all padding is not loaded
         for (int w = 0; w < 2; ++w) {
           for (int gg = 0; gg < groups; ++gg) {
             const int g = tile_group(i, t, w) + gg;
+            if ((g & 1) != part) continue;
             const int s = g % kWideSlots;
             if (!wait_uniform(empty_bar(s), ((g / kWideSlots) & 1) ^ 1u)) { ok = false; break; }
             if (leader) {
@@ -368,7 +375,7 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
         ptx::mbar_arrive(sb_ready);
       }
     }
-  } else {
+  } else if (warp < 14) {
     // ================================================================ epilogue
     const int quad = warp & 3;
     const int row = quad * 32 + lane;

@@ -165,11 +165,10 @@ class LinearAttentionNormalized(Function):
         q, k = ops.kernel_view(q), ops.kernel_view(k)  # repacked once if the rows are not 16-byte multiples
         B, H, _, dk = q.shape
         need_grad = any(ctx.needs_input_grad[:3])
-        ctx.fused = ops.normalized_fused(q, k, v)
-        if ctx.fused:
-            out, den, k_sums, s_final = ops.normalized_fwd(q, k, v, eps, need_grad)
+        if ops.normalized_fused(q, k, v):
+            out, den, s_final = ops.normalized_fwd(q, k, v, eps, need_grad)
             ctx.has_state = s_final is not None
-            ctx.save_for_backward(q, k, v, out, den, k_sums, *((s_final,) if ctx.has_state else ()))
+            ctx.save_for_backward(q, k, v, out, den, *((s_final,) if ctx.has_state else ()))
             return out
         s_final = None
         if need_grad and ops.backward_uses_final_state(q, v):
@@ -189,9 +188,6 @@ class LinearAttentionNormalized(Function):
     def backward(ctx: Any, grad_output):
         saved = ctx.saved_tensors
         q, k, v, out, den = saved[:5]
-        if ctx.fused:
-            return ops.normalized_bwd(grad_output, q, k, v, out, den, saved[5],
-                                      saved[6] if ctx.has_state else None) + (None,)
         s_final = saved[5] if ctx.has_state else None
         dnum, dden = ops.normalize_bwd_prepare(grad_output, out, den)
         dq, dk, dv = ops.causal_dot_product_bwd(dnum, q, k, v, s_last=s_final, keep_padded=True)

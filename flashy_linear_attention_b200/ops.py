@@ -530,7 +530,7 @@ def normalize_bwd_sweep(q: torch.Tensor, k: torch.Tensor, dq: torch.Tensor, dk: 
 
 def normalized_fused(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
     """True when attention with its denominator runs inside the product kernels for these tensors
-    (normalized_fwd / normalized_bwd); otherwise it is product + normalize_fwd and so on."""
+    (normalized_fwd); otherwise the forward is product + normalize_fwd."""
     if not all(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 4 and _addressable(t) for t in (q, k, v)):
         return False
     if q.shape != k.shape or q.shape != v.shape or q.device != k.device or q.device != v.device:
@@ -541,14 +541,9 @@ def normalized_fused(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> bool:
         return _lib.load().fla_sm100_normalized_fused(ctypes.byref(a)) != 0
 
 
-def _norm_sums(a: FlaArgs, device: torch.device) -> torch.Tensor:
-    need = _lib.load().fla_sm100_normalized_sums_bytes(ctypes.byref(a))
-    return torch.empty(need // 4, dtype=torch.float32, device=device)
-
-
 def normalized_fwd(q, k, v, eps: float, need_grad: bool):
-    """(out, den, k_sums, s_final): the normalised output, its denominator (fp32 [B*H, N]) and, for a
-    backward, the column sums of k per chunk and the final state (None where it has no use for one)."""
+    """(out, den, s_final): the normalised output, its denominator (fp32 [B*H, N]) and, for a backward
+    that has a use for it, the final state (else None)."""
     B, H, N, d = q.shape
     out = torch.empty(v.shape, dtype=v.dtype, device=v.device)
     den = torch.empty(B * H, N, dtype=torch.float32, device=q.device)
@@ -556,49 +551,15 @@ def normalized_fwd(q, k, v, eps: float, need_grad: bool):
         a = _norm_args(q, d, d)
         a.debug_flags = _debug_flags
         a.q, a.k, a.v, a.o = _desc(q), _desc(k), _desc(v), _desc(out)
-        k_sums = s_final = None
-        if need_grad:
-            k_sums = _norm_sums(a, q.device)
-            if backward_uses_final_state(q, v):
-                s_final = torch.empty(B * H, d, d, dtype=torch.float32, device=q.device)
-                a.s_final = s_final.data_ptr()
-        _norm_check(_lib.load().fla_sm100_normalized_fwd(ctypes.byref(a), float(eps), den.data_ptr(),
-                                                         None if k_sums is None else k_sums.data_ptr()),
+        s_final = None
+        if need_grad and backward_uses_final_state(q, v):
+            s_final = torch.empty(B * H, d, d, dtype=torch.float32, device=q.device)
+            a.s_final = s_final.data_ptr()
+        _norm_check(_lib.load().fla_sm100_normalized_fwd(ctypes.byref(a), float(eps), den.data_ptr()),
                     "fla_sm100_normalized_fwd")
     if os.environ.get("FLA_DEBUG", "0") == "1":
         check_status(q.device)
-    return out, den, k_sums, s_final
-
-
-def normalized_bwd(grad_output, q, k, v, out, den, k_sums, s_final):
-    """Gradients (dQ, dK, dV) of normalized_fwd's output."""
-    _check_inputs(grad_output, q, k, v)
-    B, H, N, d = q.shape
-    g = _kernel_view(grad_output)
-    dnum = torch.empty(out.shape, dtype=out.dtype, device=out.device)
-    dden = torch.empty(B * H, N, dtype=torch.float32, device=out.device)
-    dq, dk, dv = (torch.empty_like(t) for t in (q, k, v))
-    dqv, dkv, dvv = (_kernel_view_for_output(t) for t in (dq, dk, dv))
-    lib = _lib.load()
-    with torch.cuda.device(out.device):
-        a = _norm_args(q, d, d)
-        a.debug_flags = _debug_flags
-        w_sums = _norm_sums(a, q.device)
-        a.d_o, a.o, a.q, a.d_v = _desc(g), _desc(out), _desc(q), _desc(dnum)
-        _norm_check(lib.fla_sm100_normalized_bwd_prepare(ctypes.byref(a), den.data_ptr(), dden.data_ptr(),
-                                                         w_sums.data_ptr()),
-                    "fla_sm100_normalized_bwd_prepare")
-        a.k, a.v, a.d_o = _desc(k), _desc(v), _desc(dnum)
-        a.d_q, a.d_k, a.d_v = _desc(dqv), _desc(dkv), _desc(dvv)
-        a.s_last = None if s_final is None else s_final.data_ptr()
-        _norm_check(lib.fla_sm100_normalized_bwd(ctypes.byref(a), dden.data_ptr(), k_sums.data_ptr(),
-                                                 w_sums.data_ptr()),
-                    "fla_sm100_normalized_bwd")
-    if os.environ.get("FLA_DEBUG", "0") == "1":
-        check_status(q.device)
-    for full, view in ((dq, dqv), (dk, dkv), (dv, dvv)):
-        _copy_back(full, view)
-    return dq, dk, dv
+    return out, den, s_final
 
 
 def taylor_features(x: torch.Tensor) -> torch.Tensor:

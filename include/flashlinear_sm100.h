@@ -298,20 +298,13 @@ int fla_sm100_normalize_fwd(const FlaArgs* args, float eps, float* den);
 int fla_sm100_normalize_bwd_prepare(const FlaArgs* args, const float* den, float* dden);
 int fla_sm100_normalize_bwd_sweep(const FlaArgs* args, const float* dden);
 
-/* The same operation with the denominator inside the product kernels: two passes over q, k, v less
- * than product + normalize. fla_sm100_normalized_fused() says whether a shape runs that way (1) or
- * through the separate calls above (0): bf16, dk == dv <= 128 and a multiple of 8, neither pass split
- * into segments. sums: fla_sm100_normalized_sums_bytes() bytes each, private to the library.
- *   fwd          q, k, v -> o (normalised), den [batch*heads, seqlen], k_sums (NULL without a
- *                backward), s_final optional
- *   bwd_prepare  d_o, o, q, den -> d_v := d_o / den, dden [batch*heads, seqlen], w_sums
- *   bwd          d_o := what bwd_prepare left in d_v, q, k, v, dden, k_sums, w_sums, s_last optional
- *                -> d_q, d_k, d_v */
+/* The forward of the same operation with the denominator inside the product kernel: q, k, v -> o
+ * (normalised), den [batch*heads, seqlen] fp32, s_final optional; 512 bytes a token-head less at head
+ * dim 128 than product + normalize_fwd read and write. fla_sm100_normalized_fused() says whether a
+ * shape runs that way (1) or through the separate calls above (0): bf16, dk == dv <= 128 and a
+ * multiple of 8, the forward not split into segments. */
 int fla_sm100_normalized_fused(const FlaArgs* args);
-size_t fla_sm100_normalized_sums_bytes(const FlaArgs* args);
-int fla_sm100_normalized_fwd(const FlaArgs* args, float eps, float* den, float* k_sums);
-int fla_sm100_normalized_bwd_prepare(const FlaArgs* args, const float* den, float* dden, float* w_sums);
-int fla_sm100_normalized_bwd(const FlaArgs* args, const float* dden, const float* k_sums, const float* w_sums);
+int fla_sm100_normalized_fwd(const FlaArgs* args, float eps, float* den);
 
 /* ---- second-order Taylor feature map (benchmark configuration 4) ----
  * phi(x) = [1, x / d^(1/4), vec(x x^T) / (sqrt(2) sqrt(d))]: 1 + d + d^2 features, so that

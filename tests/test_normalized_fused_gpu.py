@@ -1,4 +1,4 @@
-"""GPU tests of attention with its denominator inside the product kernels (the NORM variants of the
+"""GPU tests of attention with its denominator inside the product kernel (the NORM variant of the
 chunk kernel) against the closed form in fp64."""
 import pytest
 import torch
@@ -42,7 +42,7 @@ def test_fused_denominator_against_closed_form(shape, layout, single_sweep):
     try:
         out = LinearAttentionNormalized.apply(q, k, v, 1e-5)
         grads = torch.autograd.grad(out, (q, k, v), g)
-        _, den, _, _ = ops.normalized_fwd(q.detach(), k.detach(), v.detach(), 1e-5, False)
+        _, den, _ = ops.normalized_fwd(q.detach(), k.detach(), v.detach(), 1e-5, False)
     finally:
         ops.set_debug_flags(old)
     ops.check_status()
