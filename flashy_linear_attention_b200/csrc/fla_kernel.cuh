@@ -14,7 +14,7 @@
 //                 cycle into an SM (640 cycles per 16 KB box, whatever the depth of the ring, also
 //                 with one CTA on the whole GPU), two get 38, more than two no more: with one
 //                 producer its 96 KB (D = 128) or 48 KB (D = 64) a chunk were the chunk period.
-//                 PRODUCER_TIMES
+//                 128 heads, backward: 8192 x 128 428 -> 423 us, 4096 x 64 134 -> 128 us.
 //   warp 1        MMA issuer X (one elected lane) and TMEM owner: S += K^T V, P = Q K^T
 //   warp 14       MMA issuer Y (one elected lane): O = Q Sb, O += Pb V
 //   warps 2-5     converter group A  } P fp32 (TMEM) -> mask -> bf16 (TMEM, A operand of P V)
@@ -77,8 +77,10 @@ constexpr int kFlagTotalMinusSuffix = 4;
 // small difference of two 128-term sums and lose accuracy.
 constexpr int kFlagFirstChunkExact = 8;
 
+// Problems of one launch (block x): three gradients, or up to three column slices each of two.
+constexpr int kMaxProblems = 6;
 struct KernelParams {
-  Problem prob[3];
+  Problem prob[kMaxProblems];
   int heads;       // heads per batch entry (block z = b * heads + h; block x = problem)
   int nchunks;     // ceil(seqlen / 128)
   int seg_chunks;  // chunks per segment (block y = segment index in scan order)
@@ -547,7 +549,10 @@ __device__ __noinline__ bool converter_prologue(const KernelParams& p, const Pro
 // same pass (fla_normalize.cuh has it as separate kernels). The score tile already holds the part of
 // den_i that comes from the chunk itself, as its row sums in fp32; what is left is q_i . z with the
 // column sums z of the chunks before. The epilogue warps, idle in that time, form both from the q and
-// k tiles in the ring before they wait for the accumulator, and divide while they round. NORM_TIMES
+// k tiles in the ring before they wait for the accumulator, and divide while they round.
+// What it costs is shared-memory bandwidth next to the MMA operands (80 KB a chunk at DK = 128). 128
+// heads x 4096 x 128: 166 us against 91 + 31 + 129 for product, column sums and division; forming the
+// vector one chunk ahead of the accumulator made no difference (169).
 template <int DK, int DV, bool HALF = false, bool NORM = false>
 __global__ void __launch_bounds__(kThreads, 1)
 fla_chunk_kernel(const __grid_constant__ KernelParams p) {

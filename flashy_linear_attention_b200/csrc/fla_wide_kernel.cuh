@@ -17,7 +17,8 @@
 //                into a ring of eight 16 KB slots (one 64-column group each; a tile takes the one
 //                or two groups that hold valid columns, so padding costs no ring space). They take
 //                turns, group by group: one warp alone issues at most 27 bytes a cycle (see
-//                fla_kernel.cuh), two get 38. PRODUCER_TIMES
+//                fla_kernel.cuh), two get 38. (This kernel's
+//                times did not move, 91.5 us at 32 heads x 4096 x 256: shared memory bounds it.)
 //   warp 1       MMA issuer (one elected lane) and TMEM owner
 //   warps 2-9    converters: P fp32 -> mask -> bf16 (TMEM), S fp32 -> bf16 (shared memory)
 //   warps 10-13  epilogue: O fp32 -> bf16 -> staging -> TMA store (each warp its own 32 rows)
