@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <optional>
 #include <string>
+#include <vector>
 
 #include "../../include/flashlinear_sm100.h"
 
@@ -111,17 +112,20 @@ void kernel_views(Tensor* t, int n, void* stream) {
 
 // An output with the layout of empty_like(t) and what the kernel writes to: the output itself, or a
 // row-padded scratch tensor that is copied back. keep_padded: the padded tensor IS the output.
+// can_pack: the kernels of this call write a contiguous output of any head dim (packed_outputs).
 struct Output {
   Tensor full, view;
 };
-Output output_like(const Tensor& t, bool keep_padded) {
+Output output_like(const Tensor& t, bool keep_padded, bool can_pack) {
   Output o;
   if (keep_padded && t.size(3) % 8 != 0) {
     o.full = o.view = padded_empty(t);
     return o;
   }
   o.full = at::empty_like(t);
-  o.view = addressable(o.full) ? o.full : padded_empty(o.full);
+  const bool packs = can_pack && o.full.size(3) % 8 != 0 && o.full.is_contiguous() &&
+                     reinterpret_cast<uintptr_t>(o.full.data_ptr()) % 16 == 0;
+  o.view = packs || addressable(o.full) ? o.full : padded_empty(o.full);
   return o;
 }
 // Results from the padded scratch rows into the caller-layout outputs, grouped like kernel_views().
@@ -182,6 +186,8 @@ Tensor scratch(FlaArgs& a, int pass, const Tensor& ref) {
   return ws;
 }
 
+// Returns (out, s_final, seg_states, views); views: with state 2, the q, k, v the kernels read where
+// one of them had to be repacked, for the backward of the same call.
 // state: 0 none; 1 always return the final state, [B, H, dk, dv]; 2 return what the backward of
 // these shapes uses (final state and boundary states, each a tensor or None).
 py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init, int state,
@@ -195,12 +201,14 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
   if (!is_state(s_init, q, bh, dk, dv)) return py::none();
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  Output out = output_like(v, false);
+  const bool can_pack = !wide && q.size(2) % 32 == 0;
+  const Output out = output_like(v, false, can_pack);
   Tensor in[3] = {q, k, v};
   kernel_views(in, 3, stream);
   FlaArgs a;
   set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
+  a.packed_outputs = can_pack ? 1 : 0;
   OptTensor s_final, seg_states;
   if (!wide && (state == 1 || (state == 2 && fla_sm100_bwd_uses_final_state(&a) != 0))) {
     s_final = state == 1 ? at::empty({q.size(0), q.size(1), dk, dv}, q.options().dtype(at::kFloat))
@@ -223,12 +231,22 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
   const Tensor ws = scratch(a, 0, q);
   check(fla_sm100_fwd(&a), "libflashlinear_sm100");
   copy_back(&out, 1, stream);
-  return py::make_tuple(out.full, s_final, seg_states);
+  py::object views = py::none();
+  if (state == 2 && !(in[0].is_same(q) && in[1].is_same(k) && in[2].is_same(v)))
+    views = py::make_tuple(in[0], in[1], in[2]);
+  return py::make_tuple(out.full, s_final, seg_states, views);
 }
 
 py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init,
                     const OptTensor& r_init, bool want_r_final, const OptTensor& s_last,
-                    const OptTensor& seg_states, bool keep_padded, unsigned debug_flags, uintptr_t status) {
+                    const OptTensor& seg_states, bool keep_padded,
+                    const std::optional<std::vector<Tensor>>& views, unsigned debug_flags, uintptr_t status) {
+  if (views.has_value()) {
+    if (views->size() != 3) return py::none();
+    const Tensor* full[3] = {&q, &k, &v};
+    for (int i = 0; i < 3; ++i)
+      if (!usable((*views)[i], q) || (*views)[i].sizes() != full[i]->sizes()) return py::none();
+  }
   if (!usable(q, q) || !usable(k, q) || !usable(v, q) || !usable(g, q) || !covered_dims(q, v) ||
       !same_rows(q, k) || !same_rows(q, v) || !same_rows(q, g) || q.size(3) != k.size(3) ||
       g.size(3) != v.size(3))
@@ -241,12 +259,16 @@ py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Ten
     return py::none();
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  const Output out[3] = {output_like(q, keep_padded), output_like(k, keep_padded), output_like(v, keep_padded)};
+  const bool can_pack = dk <= kKernelHeadDim && dv <= kKernelHeadDim && q.size(2) % 32 == 0;
+  const Output out[3] = {output_like(q, keep_padded, can_pack), output_like(k, keep_padded, can_pack),
+                         output_like(v, keep_padded, can_pack)};
   Tensor in[4] = {q, k, v, g};
+  if (views.has_value()) std::copy(views->begin(), views->end(), in);
   kernel_views(in, 4, stream);
   FlaArgs a;
   set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
+  a.packed_outputs = can_pack ? 1 : 0;
   a.q = desc(in[0]);
   a.k = desc(in[1]);
   a.v = desc(in[2]);

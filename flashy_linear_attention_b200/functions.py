@@ -46,22 +46,26 @@ def _forward_with_state(ctx: Any, q, k, v, smallv: bool):
         ctx.keep_padded = True
     res = ops.host_forward(q, k, v, None, 2 if need_grad else 0)
     if res is None:
-        res = (ops.causal_dot_product_fwd(q, k, v), None, None)
-    out, s_final, seg_states = res
-    if s_final is None:
-        ctx.save_for_backward(q, k, v)
-    elif seg_states is None:
-        ctx.save_for_backward(q, k, v, s_final)
-    else:
-        ctx.save_for_backward(q, k, v, s_final, seg_states)
+        res = (ops.causal_dot_product_fwd(q, k, v), None, None, None)
+    out, s_final, seg_states, views = res
+    # Head dims whose rows had to be repacked: the backward reads the repacked copies again (a pad
+    # pass over three tensors less); q, k, v themselves are saved too, for their version checks and
+    # because the gradients take their layout.
+    ctx.has_views = views is not None
+    ctx.save_for_backward(q, k, v, s_final, seg_states, *(views or ()))
     return out
 
 
 def _backward_with_state(ctx: Any, grad_output):
     saved = ctx.saved_tensors
-    return ops.causal_dot_product_bwd(
-        grad_output, saved[0], saved[1], saved[2], s_last=saved[3] if len(saved) > 3 else None,
-        seg_states=saved[4] if len(saved) > 4 else None, keep_padded=ctx.keep_padded)
+    q, k, v, s_final, seg_states = saved[:5]
+    if ctx.has_views:
+        res = ops.host_backward(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,
+                                keep_padded=ctx.keep_padded, views=saved[5:8])
+        if res is not None:
+            return res[:3]
+    return ops.causal_dot_product_bwd(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,
+                                      keep_padded=ctx.keep_padded)
 
 
 class LinearAttention(Function):
@@ -99,8 +103,8 @@ class LinearAttentionResumable(Function):
     as ``s_init`` of the next gives what one call over the concatenated tokens gives: chunked
     prefill, decoding a few tokens at a time, or training on a long sequence piece by piece. Any
     number of tokens per call is accepted (the reference's multiple-of-64 rule,
-    linear_attn_kernels.py:323-325, is a property of its tiling; a call of one token still costs a
-    whole 128-token tile here, so decode in blocks where possible). The state is
+    linear_attn_kernels.py:323-325, is a property of its tiling; calls of up to 16 tokens run the
+    recurrence itself in fp32 instead of a 128-token tile). The state is
     differentiable: the backward returns the gradient of ``s_init`` and accepts one for ``s_final``.
 
     Not part of the reference, whose Functions (flashlinear/linear_attn.py:11-31) always start from
@@ -122,7 +126,7 @@ class LinearAttentionResumable(Function):
         flat_init = None if s_init is None else s_init.view(B * H, dk, dv)
         res = ops.host_forward(q, k, v, flat_init, 1)
         if res is not None:
-            out, s_final, _ = res
+            out, s_final = res[:2]
         else:
             s_final = torch.empty(B, H, dk, dv, dtype=torch.float32, device=q.device)
             out = ops.causal_dot_product_fwd(q, k, v, s_init=flat_init, s_final=s_final.view(B * H, dk, dv))

@@ -274,9 +274,10 @@ def _status_ptr(t: torch.Tensor) -> int:
 
 
 def host_forward(q, k, v, s_init: Optional[torch.Tensor] = None, state: int = 0):
-    """One forward call through the native host path: (out, s_final, seg_states), or None for calls
-    it does not cover (they take the general path below). `state`: 0 no state is returned, 1 the
-    final state [B, H, dk, dv], 2 whatever the backward of these shapes makes use of."""
+    """One forward call through the native host path: (out, s_final, seg_states, views), or None for
+    calls it does not cover (they take the general path below). `state`: 0 no state is returned, 1 the
+    final state [B, H, dk, dv], 2 whatever the backward of these shapes makes use of: states and, where
+    q, k or v had to be repacked, `views`, the three tensors as the kernels read them."""
     if not q.is_cuda:
         return None
     res = _lib.host().forward(q, k, v, s_init, state, _debug_flags, _status_ptr(q))
@@ -286,13 +287,13 @@ def host_forward(q, k, v, s_init: Optional[torch.Tensor] = None, state: int = 0)
 
 
 def host_backward(grad_output, q, k, v, s_init=None, r_init=None, want_r_final: bool = False, s_last=None,
-                  seg_states=None, keep_padded: bool = False):
+                  seg_states=None, keep_padded: bool = False, views=None):
     """One backward call through the native host path: (dQ, dK, dV, r_final), or None (see
-    host_forward)."""
+    host_forward). `views`: what host_forward returned for the same q, k, v."""
     if not q.is_cuda:
         return None
     res = _lib.host().backward(grad_output, q, k, v, s_init, r_init, want_r_final, s_last, seg_states,
-                               keep_padded, _debug_flags, _status_ptr(q))
+                               keep_padded, views, _debug_flags, _status_ptr(q))
     if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
         check_status(q.device)
     return res

@@ -74,3 +74,40 @@ def test_pad_and_unpad_rows_batch(rows, d, offset):
         assert torch.equal(m[:, :d], s.view(rows, d)) and not m[:, d:].any()
         assert torch.equal(t, s)
         assert (b[:8 + offset] == 5).all() and (b[8 + offset + rows * d:] == 5).all()  # nothing beyond
+
+
+# head dims that are no multiple of 8: odd and even ones, one column, one column into the second
+# 64-column group, one short of a tile; lengths with whole and partly used chunks, and one that is no
+# multiple of 32 (row-padded outputs and a copy)
+@pytest.mark.parametrize("layout", ["bhnd", "bnhd"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N,dk,dv", [(64, 83, 83), (320, 63, 63), (192, 1, 1), (256, 65, 65), (352, 127, 127),
+                                     (2240, 90, 90), (192, 20, 64), (160, 64, 20), (200, 83, 83)])
+def test_head_dims_that_are_no_multiple_of_8(N, dk, dv, dtype, layout):
+    from flashy_linear_attention_b200 import LinearAttentionResumable, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(N + dk)
+    B, H = 2, 3
+
+    def draw(d, scale=1.0):
+        x = (torch.randn(B, N, H, d, device="cuda", generator=gen) * scale).to(dtype).transpose(1, 2)
+        return x if layout == "bnhd" else x.contiguous()
+
+    q, k, v, g = draw(dk, dk**-0.5), draw(dk), draw(dv), draw(dv)
+    out, s_final, seg_states, views = ops.host_forward(q, k, v, None, 2)
+    grads = ops.host_backward(g, q, k, v, s_last=s_final, seg_states=seg_states, views=views)[:3]
+    plain = ops.host_backward(g, q, k, v, s_last=s_final, seg_states=seg_states)[:3]
+    for a, b, t in zip(grads, plain, (q, k, v)):
+        assert torch.equal(a, b) and a.stride() == torch.empty_like(t).stride()
+    assert out.stride() == torch.empty_like(v).stride()
+    qd, kd, vd, gd = (t.double() for t in (q, k, v, g))
+    P, dP = torch.tril(qd @ kd.transpose(-1, -2)), torch.tril(gd @ vd.transpose(-1, -2))
+    want = (P @ vd, dP @ kd, dP.transpose(-1, -2) @ qd, P.transpose(-1, -2) @ gd)
+    # scores, state and result rounded to 16 bits: three roundings of half an ulp, and room for the
+    # cancellation of the total-minus-suffix form at 2240 tokens
+    bound = 1e-2 if dtype == torch.bfloat16 else 2e-3
+    for got, ref in zip((out,) + tuple(grads), want):
+        assert (got.double() - ref).norm() / ref.norm() < bound
+    if N % 32 == 0:
+        o2, s2 = LinearAttentionResumable.apply(q, k, v)
+        assert torch.equal(o2, ops.causal_dot_product_fwd(q, k, v)) and s2.shape == (B, H, dk, dv)
