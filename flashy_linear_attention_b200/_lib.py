@@ -11,7 +11,7 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libflashlinear_sm100.so")
 
-FLA_ABI_VERSION = 10
+FLA_ABI_VERSION = 9
 FLA_DEBUG_WITHHOLD_FIRST_TILE = 1
 FLA_DEBUG_NO_FUSED_SEGMENTS = 2
 FLA_DEBUG_FORCE_SINGLE_SWEEP = 4
@@ -60,7 +60,6 @@ class FlaArgs(ctypes.Structure):
         ("dtype", ctypes.c_int32),
         ("wait_limit_us", ctypes.c_uint32),
         ("debug_flags", ctypes.c_uint32),
-        ("packed_outputs", ctypes.c_int32),
     ]
 
 

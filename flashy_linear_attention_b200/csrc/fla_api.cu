@@ -63,7 +63,6 @@ thread_local int g_debug_withhold = 0;
 thread_local int g_no_fused = 0;  // FLA_DEBUG_NO_FUSED_SEGMENTS: keep the three-launch segmented path
 thread_local int g_force_single_sweep = 0;  // FLA_DEBUG_FORCE_SINGLE_SWEEP
 thread_local int g_half = 0;  // FlaArgs::dtype == FLA_DTYPE_F16
-thread_local int g_packed = 0;  // FlaArgs::packed_outputs
 
 // The single-sweep backward computes dQ as "total minus suffix": every chunk's own share comes out
 // as the difference of two sums over the whole chunk, which costs the early rows of a chunk a few
@@ -114,13 +113,6 @@ int check_operand(const Operand& o, int B, int H) {
   if (H > 1 && (o.sh * 2) % 16 != 0) return FLA_ERR_ALIGNMENT;
   if (B > 1 && (o.sb * 2) % 16 != 0) return FLA_ERR_ALIGNMENT;
   return FLA_OK;
-}
-
-// An output that the kernels write with its rows packed (FlaArgs::packed_outputs): contiguous, and
-// its head dim not a multiple of 8, so that a row-padded tensor is never meant.
-bool is_packed(const Operand& o, int B, int H, int N) {
-  return g_packed && o.dim % 8 != 0 && o.sn == o.dim && (H == 1 || o.sh == static_cast<int64_t>(N) * o.dim) &&
-         (B == 1 || o.sb == static_cast<int64_t>(H) * N * o.dim);
 }
 
 // 4-D tensor map (dim, token, head, batch); box = 64 columns x box_rows tokens, 128-byte swizzle.
@@ -803,21 +795,14 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
   for (int i = 0; i < nprob; ++i) {
     const Product& pd = prods[i];
     int rc;
-    const bool packed = is_packed(pd.out, B, H, N);
     if ((rc = check_operand(pd.a, B, H)) || (rc = check_operand(pd.b, B, H)) ||
-        (rc = check_operand(pd.c, B, H)) || (!packed && (rc = check_operand(pd.out, B, H))))
+        (rc = check_operand(pd.c, B, H)) || (rc = check_operand(pd.out, B, H)))
       return rc;
-    if (packed) {
-      if (pd.out.ptr == nullptr) return FLA_ERR_INVALID;
-      if (N % 32 != 0 || reinterpret_cast<uintptr_t>(pd.out.ptr) % 16 != 0) return FLA_ERR_ALIGNMENT;
-    }
     Problem& pr = kp.prob[i];
     const int rows = load_rows(tmpl);
     if ((rc = encode_map(&pr.q, pd.a, B, H, N, rows)) || (rc = encode_map(&pr.k, pd.b, B, H, N, rows)) ||
-        (rc = encode_map(&pr.v, pd.c, B, H, N, rows)) || (!packed && (rc = encode_map(&pr.o, pd.out, B, H, N, 32))))
+        (rc = encode_map(&pr.v, pd.c, B, H, N, rows)) || (rc = encode_map(&pr.o, pd.out, B, H, N, 32)))
       return rc;
-    pr.o_packed = packed ? static_cast<uint16_t*>(const_cast<void*>(pd.out.ptr)) : nullptr;
-    pr.o_dim = pd.out.dim;
     pr.flags = pd.flags;
     pr.n_tokens = N;
     want_final |= (pd.ext_final != nullptr);
@@ -1149,7 +1134,6 @@ int check_common(const FlaArgs* a, DeviceInfo** dev) {
   g_force_single_sweep = (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP) ? 1 : 0;
   if (a->dtype != FLA_DTYPE_BF16 && a->dtype != FLA_DTYPE_F16) return FLA_ERR_INVALID;
   g_half = a->dtype == FLA_DTYPE_F16 ? 1 : 0;
-  g_packed = a->packed_outputs != 0 ? 1 : 0;
   return FLA_OK;
 }
 

@@ -112,20 +112,17 @@ void kernel_views(Tensor* t, int n, void* stream) {
 
 // An output with the layout of empty_like(t) and what the kernel writes to: the output itself, or a
 // row-padded scratch tensor that is copied back. keep_padded: the padded tensor IS the output.
-// can_pack: the kernels of this call write a contiguous output of any head dim (packed_outputs).
 struct Output {
   Tensor full, view;
 };
-Output output_like(const Tensor& t, bool keep_padded, bool can_pack) {
+Output output_like(const Tensor& t, bool keep_padded) {
   Output o;
   if (keep_padded && t.size(3) % 8 != 0) {
     o.full = o.view = padded_empty(t);
     return o;
   }
   o.full = at::empty_like(t);
-  const bool packs = can_pack && o.full.size(3) % 8 != 0 && o.full.is_contiguous() &&
-                     reinterpret_cast<uintptr_t>(o.full.data_ptr()) % 16 == 0;
-  o.view = packs || addressable(o.full) ? o.full : padded_empty(o.full);
+  o.view = addressable(o.full) ? o.full : padded_empty(o.full);
   return o;
 }
 // Results from the padded scratch rows into the caller-layout outputs, grouped like kernel_views().
@@ -201,14 +198,12 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
   if (!is_state(s_init, q, bh, dk, dv)) return py::none();
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  const bool can_pack = !wide && q.size(2) % 32 == 0;
-  const Output out = output_like(v, false, can_pack);
+  const Output out = output_like(v, false);
   Tensor in[3] = {q, k, v};
   kernel_views(in, 3, stream);
   FlaArgs a;
   set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
-  a.packed_outputs = can_pack ? 1 : 0;
   OptTensor s_final, seg_states;
   if (!wide && (state == 1 || (state == 2 && fla_sm100_bwd_uses_final_state(&a) != 0))) {
     s_final = state == 1 ? at::empty({q.size(0), q.size(1), dk, dv}, q.options().dtype(at::kFloat))
@@ -259,16 +254,13 @@ py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Ten
     return py::none();
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  const bool can_pack = dk <= kKernelHeadDim && dv <= kKernelHeadDim && q.size(2) % 32 == 0;
-  const Output out[3] = {output_like(q, keep_padded, can_pack), output_like(k, keep_padded, can_pack),
-                         output_like(v, keep_padded, can_pack)};
+  const Output out[3] = {output_like(q, keep_padded), output_like(k, keep_padded), output_like(v, keep_padded)};
   Tensor in[4] = {q, k, v, g};
   if (views.has_value()) std::copy(views->begin(), views->end(), in);
   kernel_views(in, 4, stream);
   FlaArgs a;
   set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
-  a.packed_outputs = can_pack ? 1 : 0;
   a.q = desc(in[0]);
   a.k = desc(in[1]);
   a.v = desc(in[2]);

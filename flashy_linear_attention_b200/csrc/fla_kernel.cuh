@@ -40,8 +40,6 @@ constexpr int kGroupBytes = kChunk * 128;  // one 64-column group of a chunk til
 struct Problem {
   CUtensorMap q, k, v;     // 4-D maps (dim, token, head, batch), box 64 x Cfg::LOAD_ROWS x 1 x 1, 128B swizzle
   CUtensorMap o;           // output map with a 64 x 32 box: every epilogue warp stores its own rows
-  uint16_t* o_packed;      // or the output itself, contiguous with rows of o_dim elements (no map then)
-  int o_dim;
   const float* s_init;     // [bh * segments + g][st_rows][st_cols] fp32, or null
   float* s_final;          // same indexing, or null
   int flags;               // kFlag* bits below
@@ -690,7 +688,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   if (warp == 0 && lane == 0) {
     if (mode == 0) {
       ptx::prefetch_tensormap(&pr.q);
-      if (pr.o_packed == nullptr) ptx::prefetch_tensormap(&pr.o);
+      ptx::prefetch_tensormap(&pr.o);
     }
     ptx::prefetch_tensormap(&pr.k);
     ptx::prefetch_tensormap(&pr.v);
@@ -1244,52 +1242,6 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           if (tok < pr.n_tokens) p.den[static_cast<size_t>(bh) * pr.n_tokens + tok] = den;
           inv = 1.f / den;
           ptx::mbar_arrive(rs_free);
-        }
-        // An output whose rows are no multiple of 16 bytes cannot be written through a tensor map. If it
-        // is contiguous, a warp's 32 rows are one run of 64 o_dim bytes: they are packed in the staging
-        // buffer and stored with one bulk copy. (Row-padded scratch plus a copy kernel: 12 to 15 us per
-        // 24 MB output.) Odd rows of an odd o_dim start in the middle of a word; their words pair
-        // the upper half of one accumulator pair with the lower half of the next.
-        if (pr.o_packed != nullptr) {
-          const uint32_t stage = ost_addr + quad * (cfg::OST_BYTES / 4);
-          const uint32_t rowb = stage + static_cast<uint32_t>(lane * pr.o_dim) * 2;
-          const bool odd = ((lane * pr.o_dim) & 1) != 0;
-          const int d = pr.o_dim;
-          uint32_t prev = 0;
-#pragma unroll
-          for (int gg = 0; gg < cfg::GV; ++gg) {
-            if (gg * 64 >= d) break;
-            const uint32_t o_col = cfg::O_COL + (cfg::O_BUFS == 2 ? (i & 1) * DV : 0) + gg * 64;
-            ptx::tmem_ld32x2(lane_base + o_col, ra, lane_base + o_col + 32, rb);
-            auto put = [&](int e, uint32_t w) {  // columns e, e + 1 (compile-time e)
-              if (!odd) {
-                if (e + 1 < d) ptx::st_shared_b32(rowb + e * 2, w);
-                else if (e < d) ptx::st_shared_b16(rowb + e * 2, w);
-              } else {
-                if (e == 0) ptx::st_shared_b16(rowb, w);
-                else if (e < d) ptx::st_shared_b32(rowb + e * 2 - 2, __funnelshift_r(prev, w, 16));
-                prev = w;
-              }
-            };
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              put(gg * 64 + 2 * j, ptx::pack16x2<HALF>(__uint_as_float(ra[2 * j]), __uint_as_float(ra[2 * j + 1])));
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              put(gg * 64 + 32 + 2 * j,
-                  ptx::pack16x2<HALF>(__uint_as_float(rb[2 * j]), __uint_as_float(rb[2 * j + 1])));
-          }
-          ptx::tc_fence_before();
-          ptx::mbar_arrive((cfg::O_BUFS == 2 && (i & 1)) ? o_free1 : o_free0);
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
-          const int tok = mem_chunk(i) * kChunk + quad * 32;
-          if (lane == 0 && tok < pr.n_tokens) {  // n_tokens is a multiple of 32: all rows or none
-            ptx::bulk_store(pr.o_packed + (static_cast<size_t>(bh) * pr.n_tokens + tok) * d, stage,
-                            static_cast<uint32_t>(64 * d));
-            ptx::bulk_commit_group();
-          }
-          continue;
         }
         const uint32_t obuf = ost_addr + row * 128;
         // One 64-column group at a time: two TMEM loads in flight, rounded and written to the

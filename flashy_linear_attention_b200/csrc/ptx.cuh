@@ -178,11 +178,6 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, uint32_t src,
       "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-// Untiled copy to global memory: both addresses and the size are multiples of 16 bytes.
-__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void bulk_commit_group() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -388,9 +383,6 @@ __device__ __forceinline__ void keep_together(uint32_t (&r)[32]) {
 }
 __device__ __forceinline__ void st_shared_b32(uint32_t addr, uint32_t v) {
   asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_shared_b16(uint32_t addr, uint32_t v) {  // the low half of v
-  asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(static_cast<uint16_t>(v)) : "memory");
 }
 __device__ __forceinline__ uint32_t ld_shared_b32(uint32_t addr) {
   uint32_t v;

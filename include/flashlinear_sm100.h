@@ -33,7 +33,7 @@
 extern "C" {
 #endif
 
-#define FLA_ABI_VERSION 10
+#define FLA_ABI_VERSION 9
 #define FLA_DTYPE_BF16 0
 #define FLA_DTYPE_F16 1
 
@@ -126,11 +126,6 @@ typedef struct FlaArgs {
   uint32_t wait_limit_us;
   /* FLA_DEBUG_* bits, 0 in production. */
   uint32_t debug_flags;
-  /* Non-zero: an output (o, d_q, d_k, d_v) whose head dim is not a multiple of 8 may be a contiguous
-   * [batch, heads, seqlen, dim] tensor; it is written as it is, without padded rows and a copy. Such a
-   * tensor starts on a 16-byte boundary and seqlen is a multiple of 32 (else FLA_ERR_ALIGNMENT); head
-   * dims up to 128. */
-  int32_t packed_outputs;
 } FlaArgs;
 
 /* Test hook for the status path: the kernel never loads its first tile, so the waits that depend

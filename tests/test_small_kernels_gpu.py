@@ -77,8 +77,7 @@ def test_pad_and_unpad_rows_batch(rows, d, offset):
 
 
 # head dims that are no multiple of 8: odd and even ones, one column, one column into the second
-# 64-column group, one short of a tile; lengths with whole and partly used chunks, and one that is no
-# multiple of 32 (row-padded outputs and a copy)
+# 64-column group, one short of a tile; lengths with whole and partly used chunks
 @pytest.mark.parametrize("layout", ["bhnd", "bnhd"])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("N,dk,dv", [(64, 83, 83), (320, 63, 63), (192, 1, 1), (256, 65, 65), (352, 127, 127),
