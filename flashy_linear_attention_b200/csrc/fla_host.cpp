@@ -1,7 +1,8 @@
 // Host side of one forward / backward call on torch tensors: checks, output and scratch tensors,
 // argument block and the C-ABI call, in one native function each. Python's part of a call is then a
 // few attribute reads; doing the same through torch's Python API and ctypes (about 45 stride reads,
-// 40 structure fields and four device guards) took longer than the kernels of a small layer.
+// 40 structure fields and four device guards) took longer than the kernels of a small layer: a
+// training step of 8 heads x 256 x 64 took 195 us that way, 95 us this way (18 us of kernels).
 //
 // Both functions return None for calls they do not cover (wrong types, shapes that do not match,
 // head dims above 384, running states with head dims above 128): the caller then takes the general path in
