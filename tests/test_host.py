@@ -201,3 +201,30 @@ def test_segment_planning_queries_without_a_gpu():
     assert query(1, 16, 8192, 256, 64)["states"] == 0
     # an explicit segment count is honoured
     assert query(1, 4, 8192, 128, 128, segments=4)["seg_fwd"] == 4
+
+
+@pytest.mark.parametrize("heads,seqlen,dim,fwd,bwd", [
+    (64, 1024, 128, 1, 1),     # two segments of a 128-wide forward never pay
+    (72, 8192, 128, 1, 1),
+    (48, 3072, 128, 1, 1),     # three pay from 27 chunks on
+    (48, 4096, 128, 3, 1),
+    (16, 1024, 128, 1, 1),     # 8 chunks: too short for any split
+    (16, 2048, 128, 8, 1),     # up to 2048 tokens a split backward takes three launches
+    (16, 3072, 128, 8, 3),
+    (1, 2048, 128, 8, 8),
+    (72, 3072, 64, 1, 1),
+    (72, 8192, 64, 2, 1),
+    (8, 1024, 64, 1, 1),
+    (8, 2048, 64, 8, 6),
+])
+def test_sequences_are_split_only_where_it_pays(heads, seqlen, dim, fwd, bwd):
+    from flashy_linear_attention_b200 import _lib
+    from flashy_linear_attention_b200._lib import FlaArgs
+
+    lib = _lib.load()
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, seqlen, dim, dim
+    got = [lib.fla_sm100_auto_segments(ctypes.byref(a), p) for p in (0, 1)]
+    assert got == [fwd, bwd]
+    for p, nseg in enumerate(got):  # scratch is asked for exactly where the call is split
+        assert (lib.fla_sm100_workspace_bytes(ctypes.byref(a), p) > 0) == (nseg > 1)
