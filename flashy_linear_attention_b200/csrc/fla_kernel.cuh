@@ -137,7 +137,7 @@ struct Cfg {
   static_assert(NSLOT >= 5, "need at least five tile slots");
   static constexpr int SMEM_BYTES = 1024 + NSLOT * TILE_BYTES + SB_BYTES + OST_BYTES + BAR_BYTES;
   static_assert(SMEM_BYTES <= SMEM_LIMIT, "shared memory budget");
-  static_assert((2 * NSLOT + 12) * 8 + 16 <= BAR_BYTES, "barrier area");
+  static_assert((2 * NSLOT + 15) * 8 + 16 <= BAR_BYTES, "barrier area");
   // TMEM columns (32-bit each, 128 lanes)
   static constexpr int P_COL = 0;         // P fp32: 128 columns
   static constexpr int PB_COL = 128;      // P bf16 (two per column): two buffers of 64 columns
@@ -158,7 +158,7 @@ struct Cfg {
   static constexpr int NORM_HI_OFF = DK == 128 ? -256 : NORM_VEC_BYTES + 512;  // from the end of the barriers
   static constexpr int NORM_SMEM_BYTES = SMEM_BYTES + NORM_BYTES;
   static_assert(NORM_SMEM_BYTES <= SMEM_LIMIT, "shared memory budget");
-  static_assert(DK != 128 || (2 * NSLOT + 15) * 8 + 16 <= BAR_BYTES - 256, "barrier area");
+  static_assert(DK != 128 || (2 * NSLOT + 18) * 8 + 16 <= BAR_BYTES - 256, "barrier area");
 };
 
 // Arguments of converter_prologue(): where the CTA is and where its buffers and barriers are.
@@ -579,9 +579,16 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (NSLOT + s); };
   const uint32_t p_full = bar_base + 8u * (2 * NSLOT + 0);
-  const uint32_t pb_ready = bar_base + 8u * (2 * NSLOT + 1);
-  // One o_full barrier per bf16-P buffer (chunk parity): a waiter that needs "chunk i-1 is done"
-  // must not be overtaken by the completion for chunk i, which a shared barrier would allow.
+  // A wait for phase n of a barrier must not be overtaken by the completion of phase n + 1: the wait
+  // tests a parity only and would then block for good. Where nothing in the protocol keeps the next
+  // completion behind the waiter, the phases alternate between two barriers (chunk parity):
+  //   o_full   issuer X waits for chunk i-1 while chunk i may complete
+  //   pb_ready issuer Y, late by a microsecond between its Q Sb of chunk i and this wait, could find the
+  //            converters done with chunk i+1, which they may start as soon as Q Sb is done (with
+  //            one barrier this was seen as a wait that ran out, 64-wide, about once in 30,000
+  //            launches). The phase after next needs Y's own P V of chunk i.
+  const uint32_t pb_ready0 = bar_base + 8u * (2 * NSLOT + 1);
+  const uint32_t pb_ready1 = bar_base + 8u * (2 * NSLOT + 12);
   const uint32_t o_full0 = bar_base + 8u * (2 * NSLOT + 2);
   const uint32_t o_full1 = bar_base + 8u * (2 * NSLOT + 7);
   const uint32_t qs_done = bar_base + 8u * (2 * NSLOT + 6);
@@ -593,14 +600,16 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   const uint32_t s_full = bar_base + 8u * (2 * NSLOT + 4);
   const uint32_t part_done = bar_base + 8u * (2 * NSLOT + 10);  // fused: partial sum stored (256 arrivals)
   const uint32_t grid_done = bar_base + 8u * (2 * NSLOT + 11);  // fused: the grid barrier was passed
-  const uint32_t rs_full = bar_base + 8u * (2 * NSLOT + 12);  // NORM: row sums written (256 arrivals)
-  const uint32_t rs_free = bar_base + 8u * (2 * NSLOT + 13);  // NORM: and read (128)
-  const uint32_t vec_ready = bar_base + 8u * (2 * NSLOT + 14);  // NORM: the epilogue's vector written (128)
+  const uint32_t drained_x = bar_base + 8u * (2 * NSLOT + 13);  // everything issuer X resp. Y issued has
+  const uint32_t drained_y = bar_base + 8u * (2 * NSLOT + 14);  // completed, its commits included
+  const uint32_t rs_full = bar_base + 8u * (2 * NSLOT + 15);  // NORM: row sums written (256 arrivals)
+  const uint32_t rs_free = bar_base + 8u * (2 * NSLOT + 16);  // NORM: and read (128)
+  const uint32_t vec_ready = bar_base + 8u * (2 * NSLOT + 17);  // NORM: the epilogue's vector written (128)
   const uint32_t norm_base = bar_base + cfg::BAR_BYTES;
   const uint32_t norm_lo = norm_base + cfg::NORM_VEC_BYTES;
   const uint32_t norm_hi = norm_base + cfg::NORM_HI_OFF;
   const uint32_t holder_off = NSLOT * cfg::TILE_BYTES + cfg::SB_BYTES + cfg::OST_BYTES +
-                              8u * (2 * NSLOT + (NORM ? 15 : 12));
+                              8u * (2 * NSLOT + (NORM ? 18 : 15));
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem_gen + holder_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + holder_off + 4);
 
@@ -662,7 +671,10 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       ptx::mbar_init(empty_bar(s), mode == 0 ? (NORM ? 6 : 2) : 1);
     }
     ptx::mbar_init(p_full, 1);
-    ptx::mbar_init(pb_ready, 256);
+    ptx::mbar_init(pb_ready0, 256);
+    ptx::mbar_init(pb_ready1, 256);
+    ptx::mbar_init(drained_x, 1);
+    ptx::mbar_init(drained_y, 1);
     ptx::mbar_init(o_full0, 1);
     ptx::mbar_init(o_full1, 1);
     ptx::mbar_init(qs_done, 1);
@@ -716,6 +728,8 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   auto slot_addr = [&](int t) {
     return smem_base + static_cast<uint32_t>(t % NSLOT) * cfg::TILE_BYTES;
   };
+
+  bool issuer = false;  // the one lane of an issuer warp that executes tcgen05.mma / tcgen05.commit
 
   if (warp == 0 || warp == 15) {
     // ================================================================ TMA producers
@@ -772,6 +786,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     const uint32_t tP = tmem_base + cfg::P_COL;
     const uint32_t tS = tmem_base + cfg::S_COL;
     const bool leader = ptx::elect_one();
+    issuer = leader;
     auto wait_tile = [&](int t) { return wait_uniform(full_bar(t % NSLOT), (t / NSLOT) & 1); };
     auto release_tile = [&](int t) {
       if (leader) ptx::tc_commit(empty_bar(t % NSLOT));
@@ -884,6 +899,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       const uint32_t tO0 = tmem_base + cfg::O_COL;
       const uint32_t sb_lo = ptx::desc_lo(sb_addr, DK * 128);  // MN-major, groups DK*128 B apart
       const bool leader = ptx::elect_one();
+      issuer = leader;
       auto wait_tile = [&](int t) { return wait_uniform(full_bar(t % NSLOT), (t / NSLOT) & 1); };
       uint32_t sb_waits = 0;
       for (int i = 0; i < n_iter; ++i) {
@@ -916,7 +932,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           ptx::tc_commit(qs_done);
           ptx::tc_commit(empty_bar((t0 + 3 * i) % NSLOT));  // second arrival on q
         }
-        if (!wait_uniform(pb_ready, i & 1)) break;
+        if (!wait_uniform((i & 1) ? pb_ready1 : pb_ready0, (i >> 1) & 1)) break;
         if (!wait_tile(t0 + 3 * i + 2)) break;
         ptx::tc_fence_after();
         if (leader) {
@@ -1108,7 +1124,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         }
         ptx::tc_wait_st();
         ptx::tc_fence_before();
-        ptx::mbar_arrive(pb_ready);
+        ptx::mbar_arrive((i & 1) ? pb_ready1 : pb_ready0);
 
         // ---------------- S: fp32 -> bf16 B operand for the next chunk (or -> s_final)
         const bool last = (i == n_iter - 1);
@@ -1304,6 +1320,14 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
 
   // ------------------------------------------------------------------ teardown
   __syncwarp();
+  // The issuers' last instructions (S += K^T V of the last chunk, the releases of its tiles) have no
+  // reader that waits for them; tensor memory and the barriers have to outlive them all the same.
+  if (warp == 1 || (warp == 14 && mode == 0)) {
+    const uint32_t drained = warp == 1 ? drained_x : drained_y;
+    if (issuer) ptx::tc_commit(drained);
+    __syncwarp();
+    wait_uniform(drained, 0);
+  }
   if (*abort_flag) {
     // A wait gave up: let copies in flight land before the shared memory is released.
     __nanosleep(100000);

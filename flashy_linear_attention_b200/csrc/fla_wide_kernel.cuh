@@ -103,8 +103,9 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
   const uint32_t sb_ready = bar_base + 8u * (2 * kWideSlots + 7);
   const uint32_t o_full = bar_base + 8u * (2 * kWideSlots + 8);
   const uint32_t o_free = bar_base + 8u * (2 * kWideSlots + 9);
+  const uint32_t drained = bar_base + 8u * (2 * kWideSlots + 10);  // all the issuer issued has completed
   const uint32_t holder_off = cfg::RING_BYTES + cfg::C_BYTES + cfg::SB_BYTES + cfg::OST_BYTES +
-                              8u * (2 * kWideSlots + 10);
+                              8u * (2 * kWideSlots + 11);
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem_gen + holder_off);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + holder_off + 4);
 
@@ -131,6 +132,7 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
     ptx::mbar_init(sb_ready, 256);
     ptx::mbar_init(o_full, 1);
     ptx::mbar_init(o_free, 128);
+    ptx::mbar_init(drained, 1);
     ptx::fence_barrier_init();
     ptx::fence_proxy_async_smem();
   }
@@ -289,6 +291,10 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
       }
       __syncwarp();
     }
+    // Nobody waits for the last chunk's releases; the barriers have to outlive them all the same.
+    if (leader) ptx::tc_commit(drained);
+    __syncwarp();
+    wait_uniform(drained, 0);
   } else if (warp < 10) {
     // ================================================================ converters
     const int half = (warp - 2) >> 2;  // column half this group owns

@@ -60,9 +60,7 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // Default limit of one wait: 2 s of the GPU's global timer, far above any legitimate wait of these
 // kernels, which are microseconds. Waits are timed with %globaltimer, not clock64(): a CTA that is
 // preempted (another context's time slice on a shared GPU) may resume on another SM, whose cycle
-// counter has nothing to do with the one read before, and the time it spent switched out must not
-// count against a 0.4 s limit either (a wait of a process's first launch, taken while the previous
-// process's context was still being torn down, did run out that way).
+// counter has nothing to do with the one read before.
 constexpr unsigned long long kWaitLimitNs = 2000ull * 1000ull * 1000ull;
 __device__ __forceinline__ unsigned long long global_timer_ns() {
   unsigned long long t;

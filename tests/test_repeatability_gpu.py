@@ -65,6 +65,16 @@ def test_forward_and_single_sweep_backward_repeat_bit_for_bit(shape, repeats):
     assert _repeat(step, repeats, batch=16) == {}
 
 
+def test_product_of_more_heads_than_sms_never_waits_in_vain():
+    """The 64-wide product of 160 heads x 2048 tokens: with one barrier for the bf16 score tiles of all
+    chunks, issuer Y was now and then (about once in 30,000 launches) overtaken by two of them and
+    waited until its limit."""
+    from flashy_linear_attention_b200 import ops
+
+    q, k, v, _ = _inputs(1, 160, 2048, 64, seed=6)
+    assert _repeat(lambda: (ops.causal_dot_product_fwd(q, k, v),), 30000, batch=32) == {}
+
+
 def test_sequence_shard_with_states_from_both_sides_repeats_bit_for_bit():
     """What one of eight GPUs computes for the sequence-sharded 65536-token job: state pass, forward
     from the scratch prefixes plus the state of the tokens before, backward with that state, the
