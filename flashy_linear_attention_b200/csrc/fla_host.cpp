@@ -28,11 +28,13 @@ using OptTensor = std::optional<Tensor>;
 constexpr int64_t kKernelHeadDim = 128;  // widest head dim of the running-state kernels
 constexpr int64_t kWideHeadDim = 384;    // widest head dim one library call covers
 
-// What a TMA tensor map needs: unit innermost stride, 16-byte aligned base and outer strides.
+// What a TMA tensor map needs: unit innermost stride, 16-byte aligned base and outer strides. The row
+// stride counts even where there is one row: the library checks it without looking at the length.
 bool addressable(const Tensor& t) {
-  if (t.stride(3) != 1 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0 || t.stride(2) < t.size(3))
+  if (t.stride(3) != 1 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0 ||
+      t.stride(2) < (t.size(3) + 7) / 8 * 8 || t.stride(2) % 8 != 0)
     return false;
-  for (int d = 0; d < 3; ++d)
+  for (int d = 0; d < 2; ++d)
     if (t.size(d) > 1 && t.stride(d) % 8 != 0) return false;
   return true;
 }

@@ -130,10 +130,11 @@ def _check_inputs(*tensors: torch.Tensor, allow_half: bool = False) -> None:
 
 def _addressable(t: torch.Tensor) -> bool:
     """True if the kernels can read or write `t` in place: unit innermost stride, 16-byte aligned
-    base and row/head/batch strides (what a TMA tensor map needs)."""
+    base and row/head/batch strides (what a TMA tensor map needs). The row stride counts even where
+    there is one row: the library checks it without looking at the length."""
     d = t.shape[-1]
-    ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and t.stride(2) >= d
-    for dim in (0, 1, 2):
+    ok = t.stride(3) == 1 and t.data_ptr() % 16 == 0 and t.stride(2) >= (d + 7) // 8 * 8 and t.stride(2) % 8 == 0
+    for dim in (0, 1):
         if t.shape[dim] > 1 and t.stride(dim) % 8 != 0:
             ok = False
     return ok

@@ -228,3 +228,18 @@ def test_sequences_are_split_only_where_it_pays(heads, seqlen, dim, fwd, bwd):
     assert got == [fwd, bwd]
     for p, nseg in enumerate(got):  # scratch is asked for exactly where the call is split
         assert (lib.fla_sm100_workspace_bytes(ctypes.byref(a), p) > 0) == (nseg > 1)
+
+
+@pytest.mark.parametrize("size,strides", [((1, 1, 1, 83), (83, 83, 83, 1)), ((1, 1, 1, 64), (64, 64, 64, 1)),
+                                          ((1, 3, 1, 83), (64 * 83 * 3, 64 * 83, 83, 1)), ((2, 3, 1, 20), (1920, 640, 20, 1)),
+                                          ((1, 1, 1, 83), (88, 88, 88, 1)), ((1, 1, 1, 83), (84, 84, 84, 1)),
+                                          ((1, 2, 64, 128), (0, 0, 128, 1)), ((1, 1, 5, 64), (8, 8, 0, 1))])
+def test_addressable_is_what_the_library_accepts(size, strides):
+    """A tensor that is read in place must pass the library's operand check (row stride a multiple of 8
+    elements that holds the padded row, whatever the length; head and batch strides where they count)."""
+    from flashy_linear_attention_b200 import ops
+
+    t = torch.empty(64 * 83 * 3 + 512, dtype=torch.bfloat16).as_strided(size, strides)
+    sb, sh, sn = strides[:3]
+    accepted = sn % 8 == 0 and sn >= (size[3] + 7) // 8 * 8 and (size[1] == 1 or sh % 8 == 0) and (size[0] == 1 or sb % 8 == 0)
+    assert ops._addressable(t) == accepted

@@ -39,6 +39,36 @@ def test_few_tokens_from_a_state(tokens, dk, dv, dtype):
         assert rel <= rounds * ulp, (rel.item(), rounds * ulp)
 
 
+# one token whose row is no multiple of 16 bytes although its head and batch strides are or do not
+# count: a tensor of its own, one step of a longer contiguous one (at a 16-byte boundary and not)
+@pytest.mark.parametrize("d", [83, 20])
+@pytest.mark.parametrize("step", [None, 0, 8, 3])
+def test_one_token_with_an_odd_row(d, step):
+    from flashy_linear_attention_b200 import LinearAttentionResumable, ops
+
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    H = 1 if step is None else 3
+
+    def draw():
+        n = 1 if step is None else 64
+        t = torch.randn(1, H, n, d, device="cuda", generator=gen).bfloat16()
+        return t if step is None else t[:, :, step:step + 1]
+
+    q, k, v, g = (draw() for _ in range(4))
+    s0 = torch.randn(1, H, d, d, device="cuda", generator=gen)
+    out, s1 = LinearAttentionResumable.apply(q, k, v, s0)
+    want_s = s0.double() + k.double().transpose(-1, -2) @ v.double()
+    want = q.double() @ want_s
+    assert (s1.double() - want_s).abs().max() <= 4e-6 * want_s.abs().max()
+    assert (out.double() - want).norm() <= 2.0**-9 * want.norm()  # one rounding of the result
+    general = ops.causal_dot_product_fwd(q, k, v, s_init=s0.view(H, d, d), s_final=torch.empty(H, d, d, device="cuda"))
+    assert torch.equal(out, general)  # the Python path judges the strides like the native one
+    dq, dk, dv = ops.causal_dot_product_bwd(g, q, k, v)
+    p, dp = (q.double() * k.double()).sum(-1, keepdim=True), (g.double() * v.double()).sum(-1, keepdim=True)
+    for got, ref in ((dq, dp * k.double()), (dk, dp * q.double()), (dv, p * g.double())):
+        assert (got.double() - ref).norm() <= 1e-2 * ref.norm()
+
+
 def test_few_tokens_state_in_place():
     from flashy_linear_attention_b200 import ops
 
