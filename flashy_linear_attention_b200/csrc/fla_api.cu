@@ -1075,9 +1075,9 @@ int run_wide_any(const Product& pd, int B, int H, int N, int da, int dc, int32_t
 
 // Forward calls of a few tokens go to the recurrent kernel. 256 heads of 128 x 128, one token: 8.4 us
 // against 36 us for the chunk kernel, which moves the state through tensor memory and works on a
-// whole 128-token tile whatever the call holds. It takes 0.5 us a token (a dependent chain) once few
-// blocks share an SM: at 128 columns 16 tokens still win on 16 heads (11.4 against 15.1 us) and on 1024
-// (82 against 112), at 64 columns only 8 do (16 heads: 6.8 against 8.5 us, 11.1 against 8.4 with 16).
+// whole 128-token tile whatever the call holds. It takes about 0.5 us a token on top where
+// few blocks share an SM: at 128 columns 16 tokens still win on 16 heads (10.8 against 15.1 us) and on 1024
+// (86 against 112), at 64 columns only 8 do (16 heads: 6.9 against 8.5 us; 16 tokens took 11.1 against 8.4).
 bool use_decode(const FlaArgs* a) {
   const int most = std::max(a->dk, a->dv) > 64 ? fla::kDecodeMaxTokens : fla::kDecodeMaxTokens / 2;
   return a->seqlen <= most && a->dk <= fla::kDecodeRows && a->dv <= 128 &&
@@ -1106,10 +1106,15 @@ int run_decode(const FlaArgs* a) {
   p.dv = a->dv;
   const dim3 grid((a->dv + fla::kDecodeCols - 1) / fla::kDecodeCols, a->batch * a->heads, 1);
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
-  if (g_half)
-    fla::fla_decode_kernel<true><<<grid, fla::kDecodeThreads, 0, stream>>>(p);
+  const bool multi = a->seqlen > 1;
+  if (g_half && multi)
+    fla::fla_decode_kernel<true, true><<<grid, fla::kDecodeThreads, 0, stream>>>(p);
+  else if (g_half)
+    fla::fla_decode_kernel<true, false><<<grid, fla::kDecodeThreads, 0, stream>>>(p);
+  else if (multi)
+    fla::fla_decode_kernel<false, true><<<grid, fla::kDecodeThreads, 0, stream>>>(p);
   else
-    fla::fla_decode_kernel<false><<<grid, fla::kDecodeThreads, 0, stream>>>(p);
+    fla::fla_decode_kernel<false, false><<<grid, fla::kDecodeThreads, 0, stream>>>(p);
   ++g_last_launches;
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) FLA_LOG_FAILURE("launch of fla_decode_kernel failed: %s", cudaGetErrorString(e));

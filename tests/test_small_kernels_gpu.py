@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 # and the shortest beyond them;
 # head dims: a whole tile, columns that are no multiple of 4 or of a block's 32, one block, dk != dv
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("tokens", [1, 5, 8, 9, 16, 17])
+@pytest.mark.parametrize("tokens", [1, 3, 4, 5, 8, 9, 16, 17])
 @pytest.mark.parametrize("dk,dv", [(128, 128), (83, 83), (64, 40), (8, 128), (128, 8)])
 def test_few_tokens_from_a_state(tokens, dk, dv, dtype):
     from flashy_linear_attention_b200 import LinearAttentionResumable
@@ -37,6 +37,24 @@ def test_few_tokens_from_a_state(tokens, dk, dv, dtype):
         rounds = 1 if tokens <= (16 if max(dk, dv) > 64 else 8) else 3
         rel = (out.double() - want).norm() / want.norm()
         assert rel <= rounds * ulp, (rel.item(), rounds * ulp)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens", [1, 2, 5, 8, 16])
+def test_few_tokens_round_the_state_once(tokens, dtype):
+    """A running state much larger than what a call adds to it, as after a few hundred tokens: the new one
+    is the exact sum rounded to fp32 once. The sum of the call's own tokens, itself in fp32, is off by at most
+    tokens x 2^-24 of its size, which is 1 / 16 or less of the state's here: a tenth of the rounding in norm."""
+    from flashy_linear_attention_b200 import LinearAttentionResumable
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    B, H, d = 2, 8, 128
+    q, k, v = (torch.randn(B, H, tokens, d, device="cuda", generator=gen).to(dtype) for _ in range(3))
+    s0 = torch.randn(B, H, d, d, device="cuda", generator=gen) * 64
+    _, s1 = LinearAttentionResumable.apply(q, k, v, s0)
+    want = s0.double() + k.double().transpose(-1, -2) @ v.double()
+    once = (want.float().double() - want).norm()
+    assert (s1.double() - want).norm() <= 1.1 * once
 
 
 # one token whose row is no multiple of 16 bytes although its head and batch strides are or do not
