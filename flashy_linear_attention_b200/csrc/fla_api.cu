@@ -574,32 +574,59 @@ int current_sm_count_early() {
   return sm;
 }
 
-// Splitting a sequence pays when the chunks it saves every CTA from walking cost more than the two
-// barriers, the scan and the state loads of a segmented launch. Both times are close to linear in the
-// number of chunks n; fitted to 1 - 96 heads, 4 - 64 chunks, bf16 (microseconds, s segments that fill
-// the SMs once):
-//                          unsegmented     segmented
-//   128-wide, forward      9 + 1.85 n      22 + (0.35 + 3.0 / s) n
-//   128-wide, backward     9 + 1.8 n       22 + 2.9 n / s             (one fused launch)
-//    64-wide, forward      7 + 1.14 n      15 + 1.8 n / s
-//    64-wide, backward     6 + 1.17 n      15.6 + 1.6 n / s
-// so two segments of a 128-wide forward never pay (64 heads, 8 chunks: 23 us whole, 38 us split; 72
-// heads, 16 chunks: 42 and 54) and three pay from about 27 chunks on. Sequences of at most 2048
-// tokens run a split backward as three launches, which cost 6 to 9 us more.
-bool split_pays(int nprob, int nseg, int nchunks, int width) {
-  const double n = nchunks, per_seg = n / nseg;
-  const bool three_launches = nprob > 1 && nchunks < kSingleSweepMinChunks;
-  if (width > 64) {
-    if (nprob == 1) return 1.5 * n - 3.0 * per_seg > 13.0;
-    return 1.8 * n - 2.9 * per_seg > (three_launches ? 22.0 : 13.0);
+// What a call does with a split sequence, which decides when splitting pays.
+enum class SplitForm {
+  kForward,         // one product, its states summed in the same call
+  kBackwardStates,  // three gradients in one launch that starts from the forward's boundary states
+  kBackward,        // three gradients without those: state pass, scan, products (dk != dv: twice)
+  kState,           // state pass whose segment prefixes a forward reads (segment_states_ready)
+  kStateOnly,       // state pass of which only the total is wanted
+};
+
+// Splitting a sequence pays when the chunks it saves every CTA from walking cost more than what a
+// segmented call does on top: launches or barriers, the scan, and state traffic that grows with the
+// heads. Fitted to 1 - 96 heads, 4 - 64 chunks, bf16, in microseconds: n chunks, s segments that fill the
+// SMs once, c = ceil(n / s), h heads.
+//                                 unsegmented            segmented
+//   128-wide, kForward            9 + 1.85 n             22 + (0.35 + 3.0 / s) n
+//   128-wide, kBackwardStates     9 + 1.8 n              22 + 2.9 n / s
+//   128-wide, kBackward           4.5 + 1.68 n           17 + h + 3.4 c
+//     (dk != dv)                  9 + 3.2 n              39 + 0.25 h + 5.1 c
+//   128-wide, kState + forward    10.5 + (2.2 + h/110) n 15 + 0.35 h + 4.2 c
+//   128-wide, kStateOnly          8 + (0.65 + h/370) n   9 + 0.31 h + 1.7 c
+//    64-wide, kForward            7 + 1.14 n             15 + 1.8 n / s
+//    64-wide, kBackwardStates     6 + 1.17 n             15.6 + 1.6 n / s
+//    64-wide, kBackward           4.3 + 1.15 n           12.5 + 0.25 h + 1.85 c
+//     (dk != dv)                  8 + 2.3 n              28 + 0.08 h + 3.3 c
+//    64-wide, kState + forward    10 + 1.8 n             13 + 0.07 h + 2.2 c
+//    64-wide, kStateOnly          6 + 0.65 n             8.5 + 0.06 h + 0.75 c
+// So two segments of a 128-wide forward never pay (64 heads, 8 chunks: 23 us whole, 38 us split; 72
+// heads, 16 chunks: 42 and 54) and three pay from about 27 chunks on, but a state pass and the forward
+// that reads its prefixes do split 64 heads x 64 chunks (187 and 168 us; 64-wide: 128 and 84).
+// Without boundary states 24 heads x 64 chunks run the backward whole (117 us, split 147; 64-wide: 81
+// and 78), and 16 heads x 32 chunks (62 and 69).
+bool split_pays(SplitForm form, int heads, int nseg, int nchunks, int width, bool square) {
+  const double n = nchunks, per_seg = n / nseg, c = (nchunks + nseg - 1) / nseg, h = heads;
+  const bool wide = width > 64;
+  switch (form) {
+    case SplitForm::kForward:
+      return wide ? 1.5 * n - 3.0 * per_seg > 13.0 : 1.14 * n - 1.8 * per_seg > 8.0;
+    case SplitForm::kBackwardStates:
+      return wide ? 1.8 * n - 2.9 * per_seg > 13.0 : 1.17 * n - 1.6 * per_seg > 9.6;
+    case SplitForm::kBackward:
+      if (square) return wide ? 1.68 * n - 3.4 * c > 12.5 + h : 1.15 * n - 1.85 * c > 8.2 + 0.25 * h;
+      return wide ? 3.2 * n - 5.1 * c > 30.0 + 0.25 * h : 2.3 * n - 3.3 * c > 20.0 + 0.08 * h;
+    case SplitForm::kState:
+      return wide ? (2.2 + h / 110.0) * n - 4.2 * c > 4.5 + 0.35 * h : 1.8 * n - 2.2 * c > 3.0 + 0.07 * h;
+    case SplitForm::kStateOnly:
+      return wide ? (0.65 + h / 370.0) * n - 1.7 * c > 1.0 + 0.31 * h : 0.65 * n - 0.75 * c > 2.5 + 0.06 * h;
   }
-  if (nprob == 1) return 1.14 * n - 1.8 * per_seg > 8.0;
-  return 1.17 * n - 1.6 * per_seg > (three_launches ? 13.0 : 9.6);
+  return false;
 }
 
-// `width`: the wider of the two head dims (it selects the kernel's tile).
-int auto_segments(int nprob, int bh, int nchunks, int sm_count, int width) {
-  const long ctas = static_cast<long>(nprob) * bh;
+int auto_segments(SplitForm form, int bh, int nchunks, int sm_count, int dk, int dv) {
+  const bool backward = form == SplitForm::kBackwardStates || form == SplitForm::kBackward;
+  const long ctas = (backward ? 3l : 1l) * bh;
   if (ctas * 4 >= static_cast<long>(sm_count) * 3) return 1;  // already >= 75 % of the SMs
   // One wave: as many segments as fit the SMs once (every CTA pays a fixed start-up cost, and the
   // state pass re-reads b and c, so more, shorter segments do not pay).
@@ -608,7 +635,7 @@ int auto_segments(int nprob, int bh, int nchunks, int sm_count, int width) {
   if (max_seg < 1) max_seg = 1;
   if (want > max_seg) want = max_seg;
   if (want < 1) want = 1;
-  if (want > 1 && !split_pays(nprob, want, nchunks, width)) return 1;
+  if (want > 1 && !split_pays(form, bh, want, nchunks, std::max(dk, dv), dk == dv)) return 1;
   // make segments equal: seg_chunks = ceil(nchunks / want), then recompute the count
   const int seg_chunks = (nchunks + want - 1) / want;
   return (nchunks + seg_chunks - 1) / seg_chunks;
@@ -643,7 +670,8 @@ SegPlan make_plan(int want, int nchunks) {
 // Segments of a forward call (one product per head).
 SegPlan forward_plan(const FlaArgs* a, int sm_count) {
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  const int want = a->segments > 0 ? a->segments : auto_segments(1, a->batch * a->heads, nchunks, sm_count, std::max(a->dk, a->dv));
+  const int want = a->segments > 0 ? a->segments
+                                   : auto_segments(SplitForm::kForward, a->batch * a->heads, nchunks, sm_count, a->dk, a->dv);
   SegPlan p = make_plan(want, nchunks);
   if (a->segments <= 0 && p.nseg > 1 && nchunks % p.seg_chunks != 0) {
     // An automatic split prefers equal segments (up to a quarter longer than the even share): the
@@ -666,7 +694,7 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   const int bh = a->batch * a->heads;
   const SegPlan none = {1, nchunks};
-  const SegPlan base = make_plan(auto_segments(3, bh, nchunks, sm_count, std::max(a->dk, a->dv)), nchunks);
+  const SegPlan base = make_plan(auto_segments(SplitForm::kBackwardStates, bh, nchunks, sm_count, a->dk, a->dv), nchunks);
   if (base.nseg <= 1 || f.nseg <= 1 || nchunks % f.seg_chunks != 0) return none;
   SegPlan b;
   b.seg_chunks = (base.seg_chunks + f.seg_chunks - 1) / f.seg_chunks * f.seg_chunks;
@@ -773,7 +801,9 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
   const int bh = B * H;
   const int nchunks = (N + fla::kChunk - 1) / fla::kChunk;
   int nseg = segments;
-  if (nseg <= 0) nseg = auto_segments(nprob, bh, nchunks, dev.sm_count, std::max(da, dc));
+  // (the backward passes its segment count in)
+  if (nseg <= 0)
+    nseg = auto_segments(states_ready ? SplitForm::kState : SplitForm::kForward, bh, nchunks, dev.sm_count, da, dc);
   if (nseg > nchunks) nseg = nchunks;
   const int seg_chunks = seg_chunks_in > 0 ? seg_chunks_in : (nchunks + nseg - 1) / nseg;
   nseg = (nchunks + seg_chunks - 1) / seg_chunks;
@@ -943,7 +973,7 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
 // Sum over all tokens of b^T c (fp32, [bh][da][dc]) into `final`: the per-shard state that
 // sequence-sharded callers exchange between GPUs. Uses segments to fill the GPU when bh is small.
 int run_state(const Operand& bop, const Operand& cop, int B, int H, int N, int da, int dc,
-              int segments, float* final, void* workspace, size_t workspace_bytes,
+              int segments, SplitForm form, float* final, void* workspace, size_t workspace_bytes,
               int32_t* status, cudaStream_t stream, const DeviceInfo& dev) {
   const int tmpl = pick_template(da, dc);
   if (tmpl == 0) return FLA_ERR_UNSUPPORTED;
@@ -951,7 +981,7 @@ int run_state(const Operand& bop, const Operand& cop, int B, int H, int N, int d
   const int bh = B * H;
   const int nchunks = (N + fla::kChunk - 1) / fla::kChunk;
   int nseg = segments;
-  if (nseg <= 0) nseg = auto_segments(1, bh, nchunks, dev.sm_count, std::max(da, dc));
+  if (nseg <= 0) nseg = auto_segments(form, bh, nchunks, dev.sm_count, da, dc);
   if (nseg > nchunks) nseg = nchunks;
   const int seg_chunks = (nchunks + nseg - 1) / nseg;
   nseg = (nchunks + seg_chunks - 1) / seg_chunks;
@@ -1257,7 +1287,14 @@ int fla_sm100_auto_segments(const FlaArgs* a, int pass) {
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  return auto_segments(pass == 1 ? 3 : 1, a->batch * a->heads, nchunks, sm, std::max(a->dk, a->dv));
+  const int bh = a->batch * a->heads;
+  auto count = [&](SplitForm form) { return auto_segments(form, bh, nchunks, sm, a->dk, a->dv); };
+  if (pass == 0) return count(a->segment_states_ready ? SplitForm::kState : SplitForm::kForward);
+  if (pass == 1) {
+    const int n = count(SplitForm::kBackward);
+    return fla_sm100_seg_states_bytes(a) > 0 ? std::max(n, count(SplitForm::kBackwardStates)) : n;
+  }
+  return std::max(count(SplitForm::kState), count(SplitForm::kStateOnly));
 }
 
 size_t fla_sm100_workspace_bytes(const FlaArgs* a, int pass) {
@@ -1290,7 +1327,8 @@ int fla_sm100_bwd_uses_final_state(const FlaArgs* a) {
   if (!(nchunks >= kSingleSweepMinChunks || (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP))) return 0;
   if (fla_sm100_seg_states_bytes(a) > 0) return 1;
   int nseg = a->segments > 0 ? a->segments
-                             : auto_segments(3, a->batch * a->heads, nchunks, current_sm_count_early(), std::max(a->dk, a->dv));
+                             : auto_segments(SplitForm::kBackward, a->batch * a->heads, nchunks,
+                                             current_sm_count_early(), a->dk, a->dv);
   return nseg <= 1 ? 1 : 0;
 }
 
@@ -1382,7 +1420,7 @@ int fla_sm100_bwd(const FlaArgs* a) {
     }
   }
   int nseg = a->segments > 0 ? a->segments
-                             : auto_segments(3, a->batch * a->heads, nchunks, dev->sm_count, std::max(a->dk, a->dv));
+                             : auto_segments(SplitForm::kBackward, a->batch * a->heads, nchunks, dev->sm_count, a->dk, a->dv);
   if (nseg > nchunks) nseg = nchunks;
   if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks)) {
     // The forward state after this call's tokens is known: dQ can walk the sequence in the same
@@ -1418,11 +1456,11 @@ int fla_sm100_state(const FlaArgs* a, int which) {
   cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
   if (which == 0)
     return run_state(operand(a->k, a->dk), operand(a->v, a->dv), a->batch, a->heads, a->seqlen,
-                     a->dk, a->dv, a->segments, a->s_final, a->workspace, a->workspace_bytes,
+                     a->dk, a->dv, a->segments, SplitForm::kState, a->s_final, a->workspace, a->workspace_bytes,
                      a->status, stream, *dev);
   if (which == 1)
     return run_state(operand(a->q, a->dk), operand(a->d_o, a->dv), a->batch, a->heads, a->seqlen,
-                     a->dk, a->dv, a->segments, a->r_final, a->workspace, a->workspace_bytes,
+                     a->dk, a->dv, a->segments, SplitForm::kStateOnly, a->r_final, a->workspace, a->workspace_bytes,
                      a->status, stream, *dev);
   return FLA_ERR_INVALID;
 }
@@ -1448,7 +1486,7 @@ int fla_sm100_fwd_static_scratch(const FlaArgs* a) {
   // How much scratch this shape needs with the segment count the call will use.
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   int nseg = a->segments > 0 ? a->segments
-                             : auto_segments(1, a->batch * a->heads, nchunks, dev->sm_count, std::max(a->dk, a->dv));
+                             : auto_segments(SplitForm::kForward, a->batch * a->heads, nchunks, dev->sm_count, a->dk, a->dv);
   if (nseg > nchunks) nseg = nchunks;
   if (nseg > 1) {
     const int seg_chunks = (nchunks + nseg - 1) / nseg;
@@ -1781,7 +1819,7 @@ int fla_sm100_normalized_fused(const FlaArgs* a) {
   if (a->segments > 1) return 0;
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   const int bh = a->batch * a->heads, sm = current_sm_count_early();
-  return a->segments == 1 || auto_segments(1, bh, nchunks, sm, a->dk) == 1;
+  return a->segments == 1 || auto_segments(SplitForm::kForward, bh, nchunks, sm, a->dk, a->dv) == 1;
 }
 
 int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den) {
@@ -1831,7 +1869,8 @@ namespace {
 // Segment count and scratch size of the exchange path (scratch is needed even for one segment).
 int exchange_segments(const FlaArgs* a, int sm_count) {
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  int nseg = a->segments > 0 ? a->segments : auto_segments(1, a->batch * a->heads, nchunks, sm_count, std::max(a->dk, a->dv));
+  int nseg = a->segments > 0 ? a->segments
+                             : auto_segments(SplitForm::kState, a->batch * a->heads, nchunks, sm_count, a->dk, a->dv);
   if (nseg > nchunks) nseg = nchunks;
   if (nseg < 1) nseg = 1;
   const int seg_chunks = (nchunks + nseg - 1) / nseg;

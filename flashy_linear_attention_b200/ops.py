@@ -652,10 +652,13 @@ def chunk_state(b: torch.Tensor, c: torch.Tensor, segments: int = 0, keep_worksp
     a = FlaArgs()
     a.batch, a.heads, a.seqlen, a.dk, a.dv = B, H, N, db, dc
     a.dtype = _dtype_code(b)
-    a.k, a.v = _desc(bv), _desc(cv)
-    a.s_final = out.data_ptr()
+    # both sum b^T c; a state whose segment prefixes nobody reads (which = 1) is split less readily
+    if keep_workspace:
+        a.k, a.v, a.s_final = _desc(bv), _desc(cv), out.data_ptr()
+    else:
+        a.q, a.d_o, a.r_final = _desc(bv), _desc(cv), out.data_ptr()
     a.segments = segments
-    ws = _call(2, a, b.device, which=0)
+    ws = _call(2, a, b.device, which=0 if keep_workspace else 1)
     if keep_workspace:
         if ws is None:  # unsegmented call: nothing to reuse, but keep the calling convention
             ws = torch.empty(0, dtype=torch.uint8, device=b.device)

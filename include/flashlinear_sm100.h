@@ -158,7 +158,9 @@ int fla_sm100_timeout_records(unsigned* out, int max_records);
 int fla_sm100_abi_version(void);
 const char* fla_sm100_strerror(int code);
 size_t fla_sm100_workspace_bytes(const FlaArgs* args, int pass);
-/* Number of segments the call will use for args->segments == 0. */
+/* Number of segments the call will use for args->segments == 0 (pass 0 looks at segment_states_ready). A
+ * backward without the seg_states that its shapes could use, and a state pass with which = 1, whose
+ * prefixes nobody reads, may use fewer; scratch of fla_sm100_workspace_bytes() covers both. */
 int fla_sm100_auto_segments(const FlaArgs* args, int pass);
 /* Bytes for FlaArgs::seg_states, or 0 when forward + backward of these shapes do not use them (many
  * heads: nothing is segmented; dk != dv; head dims above 128). The reference has no counterpart: its

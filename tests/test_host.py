@@ -230,6 +230,40 @@ def test_sequences_are_split_only_where_it_pays(heads, seqlen, dim, fwd, bwd):
         assert (lib.fla_sm100_workspace_bytes(ctypes.byref(a), p) > 0) == (nseg > 1)
 
 
+@pytest.mark.parametrize("heads,seqlen,dk,dv,state,bwd", [
+    (64, 8192, 128, 128, 2, 1),  # a state pass and the forward that reads its prefixes: 187 us whole, 168 split
+    (64, 4096, 128, 128, 1, 1),  # (104 and 108)
+    (56, 8192, 128, 128, 2, 1),
+    (64, 1024, 64, 64, 1, 1),    # (25.0 and 25.3)
+    (64, 2048, 64, 64, 2, 1),    # (40 and 33)
+    (4, 1024, 128, 128, 4, 1),   # (29 and 24)
+    (24, 8192, 128, 128, 6, 1),  # backward without boundary states: 117 us whole, 147 split
+    (16, 4096, 128, 128, 8, 1),  # (62 and 69)
+    (16, 8192, 128, 128, 8, 3),  # (114 and 109)
+    (8, 3072, 128, 128, 12, 6),  # (46 and 38)
+    (24, 4096, 64, 64, 6, 1),    # (43 and 48)
+    (8, 2048, 128, 64, 8, 6),    # dk != dv, two calls: (57 and 54)
+    (12, 2048, 128, 64, 8, 1),   # (58 and 63)
+    (16, 3072, 64, 32, 8, 3),    # (65 and 55)
+])
+def test_split_rule_follows_what_the_call_does(heads, seqlen, dk, dv, state, bwd):
+    from flashy_linear_attention_b200 import _lib
+    from flashy_linear_attention_b200._lib import FLA_DEBUG_NO_FUSED_SEGMENTS, FlaArgs
+
+    lib = _lib.load()
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, seqlen, dk, dv
+    assert lib.fla_sm100_auto_segments(ctypes.byref(a), 2) == state
+    a.segment_states_ready = 1  # the forward that reads the prefixes must count the same segments
+    assert lib.fla_sm100_auto_segments(ctypes.byref(a), 0) == state
+    a.segment_states_ready = 0
+    with_states = lib.fla_sm100_workspace_bytes(ctypes.byref(a), 1)
+    a.debug_flags = FLA_DEBUG_NO_FUSED_SEGMENTS  # no boundary states
+    assert lib.fla_sm100_auto_segments(ctypes.byref(a), 1) == bwd
+    # scratch asked for with boundary states in mind covers the call that comes without
+    assert with_states >= lib.fla_sm100_workspace_bytes(ctypes.byref(a), 1)
+
+
 @pytest.mark.parametrize("size,strides", [((1, 1, 1, 83), (83, 83, 83, 1)), ((1, 1, 1, 64), (64, 64, 64, 1)),
                                           ((1, 3, 1, 83), (64 * 83 * 3, 64 * 83, 83, 1)), ((2, 3, 1, 20), (1920, 640, 20, 1)),
                                           ((1, 1, 1, 83), (88, 88, 88, 1)), ((1, 1, 1, 83), (84, 84, 84, 1)),
