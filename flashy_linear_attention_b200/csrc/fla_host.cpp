@@ -6,13 +6,16 @@
 //
 // Both functions return None for calls they do not cover (wrong types, shapes that do not match,
 // head dims above 384, running states with head dims above 128): the caller then takes the general path in
-// ops.py, which reports the errors and handles the rest.
+// ops.py, which reports the errors and handles the rest. The interpreter lock is given up while they
+// work, as ctypes does: an allocation or a full launch queue can block, and other Python threads, that
+// drive other streams or GPUs, have to go on meanwhile.
 #include <torch/extension.h>
 
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <algorithm>
+#include <array>
 #include <optional>
 #include <string>
 #include <vector>
@@ -186,19 +189,24 @@ Tensor scratch(FlaArgs& a, int pass, const Tensor& ref) {
   return ws;
 }
 
-// Returns (out, s_final, seg_states, views); views: with state 2, the q, k, v the kernels read where
+// views: with state 2, the q, k, v the kernels read where
 // one of them had to be repacked, for the backward of the same call.
 // state: 0 none; 1 always return the final state, [B, H, dk, dv]; 2 return what the backward of
 // these shapes uses (final state and boundary states, each a tensor or None).
-py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init, int state,
-                   unsigned debug_flags, uintptr_t status) {
+struct Forward {
+  Tensor out;
+  OptTensor s_final, seg_states;
+  std::optional<std::array<Tensor, 3>> views;
+};
+std::optional<Forward> forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init, int state,
+                               unsigned debug_flags, uintptr_t status) {
   if (!usable(q, q) || !usable(k, q) || !usable(v, q) || !covered_dims(q, v) || !same_rows(q, k) ||
       !same_rows(q, v) || q.size(3) != k.size(3))
-    return py::none();
+    return std::nullopt;
   const int64_t bh = q.size(0) * q.size(1), dk = q.size(3), dv = v.size(3);
   const bool wide = dk > kKernelHeadDim || dv > kKernelHeadDim;
-  if (wide && (s_init.has_value() || state == 1)) return py::none();
-  if (!is_state(s_init, q, bh, dk, dv)) return py::none();
+  if (wide && (s_init.has_value() || state == 1)) return std::nullopt;
+  if (!is_state(s_init, q, bh, dk, dv)) return std::nullopt;
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
   const Output out = output_like(v, false);
@@ -229,32 +237,29 @@ py::object forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptT
   const Tensor ws = scratch(a, 0, q);
   check(fla_sm100_fwd(&a), "libflashlinear_sm100");
   copy_back(&out, 1, stream);
-  py::object views = py::none();
+  Forward res{out.full, s_final, seg_states, std::nullopt};
   if (state == 2 && !(in[0].is_same(q) && in[1].is_same(k) && in[2].is_same(v)))
-    views = py::make_tuple(in[0], in[1], in[2]);
-  return py::make_tuple(out.full, s_final, seg_states, views);
+    res.views = std::array<Tensor, 3>{in[0], in[1], in[2]};
+  return res;
 }
 
-py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init,
-                    const OptTensor& r_init, bool want_r_final, const OptTensor& s_last,
-                    const OptTensor& seg_states, bool keep_padded,
-                    const std::optional<std::vector<Tensor>>& views, unsigned debug_flags, uintptr_t status) {
+std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v,
+                                              const OptTensor& s_last, const OptTensor& seg_states, bool keep_padded,
+                                              const std::optional<std::vector<Tensor>>& views, unsigned debug_flags,
+                                              uintptr_t status) {
   if (views.has_value()) {
-    if (views->size() != 3) return py::none();
+    if (views->size() != 3) return std::nullopt;
     const Tensor* full[3] = {&q, &k, &v};
     for (int i = 0; i < 3; ++i)
-      if (!usable((*views)[i], q) || (*views)[i].sizes() != full[i]->sizes()) return py::none();
+      if (!usable((*views)[i], q) || (*views)[i].sizes() != full[i]->sizes()) return std::nullopt;
   }
   if (!usable(q, q) || !usable(k, q) || !usable(v, q) || !usable(g, q) || !covered_dims(q, v) ||
       !same_rows(q, k) || !same_rows(q, v) || !same_rows(q, g) || q.size(3) != k.size(3) ||
       g.size(3) != v.size(3))
-    return py::none();
+    return std::nullopt;
   const int64_t bh = q.size(0) * q.size(1), dk = q.size(3), dv = v.size(3);
-  if ((dk > kKernelHeadDim || dv > kKernelHeadDim) &&
-      (s_init.has_value() || r_init.has_value() || want_r_final || s_last.has_value()))
-    return py::none();
-  if (!is_state(s_init, q, bh, dk, dv) || !is_state(r_init, q, bh, dk, dv) || !is_state(s_last, q, bh, dk, dv))
-    return py::none();
+  if ((dk > kKernelHeadDim || dv > kKernelHeadDim) && s_last.has_value()) return std::nullopt;
+  if (!is_state(s_last, q, bh, dk, dv)) return std::nullopt;
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
   const Output out[3] = {output_like(q, keep_padded), output_like(k, keep_padded), output_like(v, keep_padded)};
@@ -271,11 +276,6 @@ py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Ten
   a.d_q = desc(out[0].view);
   a.d_k = desc(out[1].view);
   a.d_v = desc(out[2].view);
-  OptTensor r_final;
-  if (want_r_final) r_final = at::empty({bh, dk, dv}, q.options().dtype(at::kFloat));
-  if (s_init.has_value()) a.s_init = s_init->data_ptr<float>();
-  if (r_init.has_value()) a.r_init = r_init->data_ptr<float>();
-  if (r_final.has_value()) a.r_final = r_final->data_ptr<float>();
   if (s_last.has_value()) a.s_last = s_last->data_ptr<float>();
   if (seg_states.has_value()) {
     a.seg_states = seg_states->data_ptr();
@@ -284,12 +284,33 @@ py::object backward(const Tensor& g, const Tensor& q, const Tensor& k, const Ten
   const Tensor ws = scratch(a, 1, q);
   check(fla_sm100_bwd(&a), "libflashlinear_sm100");
   copy_back(out, 3, stream);
-  return py::make_tuple(out[0].full, out[1].full, out[2].full, r_final);
+  return std::array<Tensor, 3>{out[0].full, out[1].full, out[2].full};
 }
 
 }  // namespace
 
 PYBIND11_MODULE(_hostcalls, m) {
-  m.def("forward", &forward);
-  m.def("backward", &backward);
+  m.def("forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init, int state,
+                      unsigned debug_flags, uintptr_t status) -> py::object {
+    std::optional<Forward> r;
+    {
+      const py::gil_scoped_release unlocked;
+      r = forward(q, k, v, s_init, state, debug_flags, status);
+    }
+    if (!r.has_value()) return py::none();
+    py::object views = py::none();
+    if (r->views.has_value()) views = py::make_tuple((*r->views)[0], (*r->views)[1], (*r->views)[2]);
+    return py::make_tuple(r->out, r->s_final, r->seg_states, views);
+  });
+  m.def("backward", [](const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_last,
+                       const OptTensor& seg_states, bool keep_padded, const std::optional<std::vector<Tensor>>& views,
+                       unsigned debug_flags, uintptr_t status) -> py::object {
+    std::optional<std::array<Tensor, 3>> r;
+    {
+      const py::gil_scoped_release unlocked;
+      r = backward(g, q, k, v, s_last, seg_states, keep_padded, views, debug_flags, status);
+    }
+    if (!r.has_value()) return py::none();
+    return py::make_tuple((*r)[0], (*r)[1], (*r)[2]);
+  });
 }

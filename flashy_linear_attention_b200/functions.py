@@ -63,7 +63,7 @@ def _backward_with_state(ctx: Any, grad_output):
         res = ops.host_backward(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,
                                 keep_padded=ctx.keep_padded, views=saved[5:8])
         if res is not None:
-            return res[:3]
+            return res
     return ops.causal_dot_product_bwd(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,
                                       keep_padded=ctx.keep_padded)
 

@@ -283,14 +283,12 @@ def host_forward(q, k, v, s_init: Optional[torch.Tensor] = None, state: int = 0)
     return res
 
 
-def host_backward(grad_output, q, k, v, s_init=None, r_init=None, want_r_final: bool = False, s_last=None,
-                  seg_states=None, keep_padded: bool = False, views=None):
-    """One backward call through the native host path: (dQ, dK, dV, r_final), or None (see
-    host_forward). `views`: what host_forward returned for the same q, k, v."""
+def host_backward(grad_output, q, k, v, s_last=None, seg_states=None, keep_padded: bool = False, views=None):
+    """One backward call through the native host path: (dQ, dK, dV), or None (see host_forward). `views`: what host_forward returned for the same q, k, v."""
     if not q.is_cuda:
         return None
-    res = _lib.host().backward(grad_output, q, k, v, s_init, r_init, want_r_final, s_last, seg_states,
-                               keep_padded, views, _debug_flags, _status_ptr(q))
+    res = _lib.host().backward(grad_output, q, k, v, s_last, seg_states, keep_padded, views,
+                               _debug_flags, _status_ptr(q))
     if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
         check_status(q.device)
     return res
@@ -417,7 +415,7 @@ def causal_dot_product_bwd(
     if s_init is None and r_init is None and r_final is None and segments == 0:
         res = host_backward(grad_output, q, k, v, s_last=s_last, seg_states=seg_states, keep_padded=keep_padded)
         if res is not None:
-            return res[:3]
+            return res
     _check_inputs(grad_output, q, k, v, allow_half=True)
     B, H, N, dk = q.shape
     dv = v.shape[-1]
