@@ -6,7 +6,9 @@ build it, and every call fails loudly when the current device is not an sm_100 G
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import warnings
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libflashlinear_sm100.so")
@@ -206,18 +208,37 @@ def load() -> ctypes.CDLL:
     return lib
 
 
-_host = None
+_host = None  # the extension, or False where there is none for this Python and torch
 
 
 def host():
-    """The native host side of a call on torch tensors (csrc/fla_host.cpp), loaded once."""
+    """The native host side of a call on torch tensors (csrc/fla_host.cpp), loaded once. None, with one
+    warning, where it has not been built for the running Python, the installed torch and this version of the
+    library: the caller then prepares the call in Python and reaches the same kernels through ctypes."""
     global _host
     if _host is None:
         load()
-        from . import _hostcalls
+        _host = _load_host()
+    return _host or None
 
-        _host = _hostcalls
-    return _host
+
+def _load_host():
+    from . import build
+
+    path = build.host_path()
+    try:
+        spec = importlib.util.spec_from_file_location(__package__ + "._hostcalls", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        if module.abi_version != FLA_ABI_VERSION:
+            raise ImportError(f"built for version {module.abi_version} of the C interface, not {FLA_ABI_VERSION}")
+    except (ImportError, OSError) as exc:
+        warnings.warn(
+            f"flashlinear: no native host path ({exc}); calls take more host time. Build it with "
+            "`python -m flashy_linear_attention_b200.build` (needs g++ and the installed torch's headers).",
+            RuntimeWarning, stacklevel=2)
+        return False
+    return module
 
 
 def strerror(code: int) -> str:

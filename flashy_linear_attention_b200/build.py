@@ -1,8 +1,11 @@
-"""Builds libflashlinear_sm100.so in-tree with nvcc for sm_100a, and _hostcalls.so beside it.
+"""Builds libflashlinear_sm100.so in-tree with nvcc for sm_100a, and _hostcalls.*.so beside it.
 
 Usage: python -m flashy_linear_attention_b200.build [--force]
-The library has no Python or torch dependency; it links the static CUDA runtime only. _hostcalls.so
-is the host side of a call on torch tensors (csrc/fla_host.cpp), a Python extension on top of it.
+The library has no Python or torch dependency; it links the static CUDA runtime only. _hostcalls.*.so
+is the host side of a call on torch tensors (csrc/fla_host.cpp), a Python extension on top of it that
+needs g++. It is bound to one torch and one Python, so its name carries both versions: after an
+upgrade it counts as missing, calls go through ctypes (same kernels, more host time) and say so once,
+until this module has run again.
 """
 from __future__ import annotations
 
@@ -16,8 +19,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_NAME = "libflashlinear_sm100.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
-
-HOST_PATH = os.path.join(HERE, "_hostcalls.so")
 
 SOURCES = ["fla_api.cu"]
 HOST_SOURCES = ["fla_host.cpp", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
@@ -38,6 +39,13 @@ def find_nvcc() -> str:
     return nvcc
 
 
+def host_path() -> str:
+    """Where the extension for the running Python and the installed torch is built."""
+    import torch
+
+    return os.path.join(HERE, f"_hostcalls.torch-{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
 def _stale(built_path: str, sources) -> bool:
     if not os.path.exists(built_path):
         return True
@@ -46,7 +54,7 @@ def _stale(built_path: str, sources) -> bool:
 
 
 def is_stale() -> bool:
-    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(HOST_PATH, HOST_SOURCES)
+    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(host_path(), HOST_SOURCES)
 
 
 def _run(cmd, what: str) -> str:
@@ -58,8 +66,9 @@ def _run(cmd, what: str) -> str:
 
 def build_host(force: bool = False) -> str:
     """Compiles the Python extension (host code only; links the library, found beside it)."""
-    if not force and not _stale(HOST_PATH, HOST_SOURCES):
-        return HOST_PATH
+    path = host_path()
+    if not force and not _stale(path, HOST_SOURCES):
+        return path
     import torch
     from torch.utils.cpp_extension import include_paths, library_paths
 
@@ -68,12 +77,12 @@ def build_host(force: bool = False) -> str:
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"]
     cmd += [f"-I{p}" for p in includes]
-    cmd += [os.path.join(CSRC, HOST_SOURCES[0]), "-o", HOST_PATH]
+    cmd += [os.path.join(CSRC, HOST_SOURCES[0]), "-o", path]
     cmd += [f"-L{p}" for p in library_paths()]
     cmd += [f"-L{HERE}", "-l:" + LIB_NAME, "-Wl,-rpath,$ORIGIN"]
     cmd += ["-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu", "-ltorch_python"]
     _run(cmd, "g++")
-    return HOST_PATH
+    return path
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -290,6 +290,7 @@ std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, 
 }  // namespace
 
 PYBIND11_MODULE(_hostcalls, m) {
+  m.attr("abi_version") = FLA_ABI_VERSION;
   m.def("forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_init, int state,
                       unsigned debug_flags, uintptr_t status) -> py::object {
     std::optional<Forward> r;

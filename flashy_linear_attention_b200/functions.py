@@ -46,7 +46,7 @@ def _forward_with_state(ctx: Any, q, k, v, smallv: bool):
         ctx.keep_padded = True
     res = ops.host_forward(q, k, v, None, 2 if need_grad else 0)
     if res is None:
-        res = (ops.causal_dot_product_fwd(q, k, v), None, None, None)
+        res = ops.general_forward(q, k, v) if need_grad else (ops.causal_dot_product_fwd(q, k, v), None, None, None)
     out, s_final, seg_states, views = res
     # Head dims whose rows had to be repacked: the backward reads the repacked copies again (a pad
     # pass over three tensors less); q, k, v themselves are saved too, for their version checks and

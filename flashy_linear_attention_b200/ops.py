@@ -275,19 +275,31 @@ def host_forward(q, k, v, s_init: Optional[torch.Tensor] = None, state: int = 0)
     calls it does not cover (they take the general path below). `state`: 0 no state is returned, 1 the
     final state [B, H, dk, dv], 2 whatever the backward of these shapes makes use of: states and, where
     q, k or v had to be repacked, `views`, the three tensors as the kernels read them."""
-    if not q.is_cuda:
+    native = _lib.host() if q.is_cuda else None
+    if native is None:
         return None
-    res = _lib.host().forward(q, k, v, s_init, state, _debug_flags, _status_ptr(q))
+    res = native.forward(q, k, v, s_init, state, _debug_flags, _status_ptr(q))
     if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
         check_status(q.device)
     return res
 
 
+def general_forward(q, k, v):
+    """What host_forward(q, k, v, state=2) returns, prepared in Python, for calls that it leaves to others."""
+    _check_inputs(q, k, v, allow_half=True)
+    s_final = seg_states = None
+    if backward_uses_final_state(q, v):
+        s_final = torch.empty(q.shape[0] * q.shape[1], q.shape[3], v.shape[3], dtype=torch.float32, device=q.device)
+        seg_states = segment_states_buffer(q, v)
+    return causal_dot_product_fwd(q, k, v, s_final=s_final, seg_states=seg_states), s_final, seg_states, None
+
+
 def host_backward(grad_output, q, k, v, s_last=None, seg_states=None, keep_padded: bool = False, views=None):
     """One backward call through the native host path: (dQ, dK, dV), or None (see host_forward). `views`: what host_forward returned for the same q, k, v."""
-    if not q.is_cuda:
+    native = _lib.host() if q.is_cuda else None
+    if native is None:
         return None
-    res = _lib.host().backward(grad_output, q, k, v, s_last, seg_states, keep_padded, views,
+    res = native.backward(grad_output, q, k, v, s_last, seg_states, keep_padded, views,
                                _debug_flags, _status_ptr(q))
     if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
         check_status(q.device)

@@ -277,3 +277,31 @@ def test_addressable_is_what_the_library_accepts(size, strides):
     sb, sh, sn = strides[:3]
     accepted = sn % 8 == 0 and sn >= (size[3] + 7) // 8 * 8 and (size[1] == 1 or sh % 8 == 0) and (size[0] == 1 or sb % 8 == 0)
     assert ops._addressable(t) == accepted
+
+
+def test_native_host_path_belongs_to_one_torch_and_python(monkeypatch, tmp_path):
+    """The extension's file name carries both versions: after an upgrade it counts as not built (so build()
+    makes it anew), and calls fall back to the ctypes path with one warning instead of an ImportError."""
+    import sysconfig
+    import warnings
+
+    from flashy_linear_attention_b200 import _lib, build
+
+    path = build.host_path()
+    assert torch.__version__ in path and path.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert _lib.host() is not None
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    assert build.host_path() != path and build.is_stale()
+    monkeypatch.setattr(_lib, "_host", None)
+    with pytest.warns(RuntimeWarning, match="flashy_linear_attention_b200.build"):
+        assert _lib.host() is None
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert _lib.host() is None  # said once
+    # a file that cannot be loaded (another ABI, for one) counts the same
+    bad = tmp_path / "_hostcalls.so"
+    bad.write_bytes(b"not an extension")
+    monkeypatch.setattr(build, "host_path", lambda: str(bad))
+    monkeypatch.setattr(_lib, "_host", None)
+    with pytest.warns(RuntimeWarning):
+        assert _lib.host() is None

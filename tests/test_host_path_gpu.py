@@ -45,3 +45,22 @@ def test_other_threads_run_while_a_call_blocks():
     gaps = [b - a for a, b in zip(ticks, ticks[1:])]
     assert blocked > 0.3, "the launch queue never filled: the test shows nothing"
     assert max(gaps) < 0.2, max(gaps)
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 192, 83), (1, 2, 2240, 64), (1, 4, 4096, 128), (1, 2, 128, 192)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_calls_without_the_native_host_path_give_the_same(shape, monkeypatch):
+    """Same kernels, same plan (final state and boundary states included), other host code."""
+    from flashy_linear_attention_b200 import LinearAttention, _lib
+
+    q, k, v, g = (_draw(*shape, seed=i) for i in range(4))
+
+    def step():
+        x = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        out = LinearAttention.apply(*x)
+        return (out,) + torch.autograd.grad(out, x, g)
+
+    want = step()
+    monkeypatch.setattr(_lib, "_host", False)
+    for a, b in zip(step(), want):
+        assert torch.equal(a, b) and a.stride() == b.stride()
