@@ -67,9 +67,9 @@ FlaTensor desc(const Tensor& t) {
 }
 
 // View [..., :d] of a fresh tensor whose rows are padded to a multiple of 8 elements.
-Tensor padded_empty(const Tensor& like) {
+Tensor padded_empty(const Tensor& like, const at::TensorOptions& options) {
   const int64_t d = like.size(3);
-  return at::empty({like.size(0), like.size(1), like.size(2), (d + 7) / 8 * 8}, like.options()).narrow(3, 0, d);
+  return at::empty({like.size(0), like.size(1), like.size(2), (d + 7) / 8 * 8}, options).narrow(3, 0, d);
 }
 
 void check(int rc, const char* name) {
@@ -93,7 +93,7 @@ void kernel_views(Tensor* t, int n, void* stream) {
   bool done[kMax] = {};
   for (int i = 0; i < n; ++i) {
     if (addressable(t[i])) done[i] = true;
-    else copies[i] = padded_empty(t[i]);
+    else copies[i] = padded_empty(t[i], t[i].options());
     if (!done[i] && !contiguous_rows(t[i])) {
       copies[i].copy_(t[i]);
       done[i] = true;
@@ -121,14 +121,14 @@ void kernel_views(Tensor* t, int n, void* stream) {
 struct Output {
   Tensor full, view;
 };
-Output output_like(const Tensor& t, bool keep_padded) {
+Output output_like(const Tensor& t, bool keep_padded, const at::TensorOptions& options) {
   Output o;
   if (keep_padded && t.size(3) % 8 != 0) {
-    o.full = o.view = padded_empty(t);
+    o.full = o.view = padded_empty(t, options);
     return o;
   }
-  o.full = at::empty_like(t);
-  o.view = addressable(o.full) ? o.full : padded_empty(o.full);
+  o.full = at::empty_like(t, options);
+  o.view = addressable(o.full) ? o.full : padded_empty(o.full, options);
   return o;
 }
 // Results from the padded scratch rows into the caller-layout outputs, grouped like kernel_views().
@@ -209,7 +209,7 @@ std::optional<Forward> forward(const Tensor& q, const Tensor& k, const Tensor& v
   if (!is_state(s_init, q, bh, dk, dv)) return std::nullopt;
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  const Output out = output_like(v, false);
+  const Output out = output_like(v, false, v.options());
   Tensor in[3] = {q, k, v};
   kernel_views(in, 3, stream);
   FlaArgs a;
@@ -247,27 +247,30 @@ std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, 
                                               const OptTensor& s_last, const OptTensor& seg_states, bool keep_padded,
                                               const std::optional<std::vector<Tensor>>& views, unsigned debug_flags,
                                               uintptr_t status) {
+  // With views, q, k and v only say what layout the gradients have (stand_ins()).
+  const Tensor like[3] = {q, k, v};
+  Tensor in[4] = {q, k, v, g};
   if (views.has_value()) {
     if (views->size() != 3) return std::nullopt;
-    const Tensor* full[3] = {&q, &k, &v};
-    for (int i = 0; i < 3; ++i)
-      if (!usable((*views)[i], q) || (*views)[i].sizes() != full[i]->sizes()) return std::nullopt;
+    for (int i = 0; i < 3; ++i) {
+      if ((*views)[i].sizes() != like[i].sizes()) return std::nullopt;
+      in[i] = (*views)[i];
+    }
   }
-  if (!usable(q, q) || !usable(k, q) || !usable(v, q) || !usable(g, q) || !covered_dims(q, v) ||
-      !same_rows(q, k) || !same_rows(q, v) || !same_rows(q, g) || q.size(3) != k.size(3) ||
-      g.size(3) != v.size(3))
-    return std::nullopt;
+  for (const Tensor& t : in)
+    if (!usable(t, in[0]) || !same_rows(t, in[0])) return std::nullopt;
+  if (!covered_dims(in[0], in[2]) || q.size(3) != k.size(3) || g.size(3) != v.size(3)) return std::nullopt;
   const int64_t bh = q.size(0) * q.size(1), dk = q.size(3), dv = v.size(3);
   if ((dk > kKernelHeadDim || dv > kKernelHeadDim) && s_last.has_value()) return std::nullopt;
-  if (!is_state(s_last, q, bh, dk, dv)) return std::nullopt;
-  const c10::cuda::CUDAGuard guard(q.device());
-  void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  const Output out[3] = {output_like(q, keep_padded), output_like(k, keep_padded), output_like(v, keep_padded)};
-  Tensor in[4] = {q, k, v, g};
-  if (views.has_value()) std::copy(views->begin(), views->end(), in);
+  if (!is_state(s_last, g, bh, dk, dv)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(g.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(g.device().index()).stream();
+  const at::TensorOptions options = g.options();
+  const Output out[3] = {output_like(q, keep_padded, options), output_like(k, keep_padded, options),
+                         output_like(v, keep_padded, options)};
   kernel_views(in, 4, stream);
   FlaArgs a;
-  set_sizes(a, q, v, debug_flags, status);
+  set_sizes(a, in[0], in[2], debug_flags, status);
   a.stream = stream;
   a.q = desc(in[0]);
   a.k = desc(in[1]);
@@ -281,10 +284,22 @@ std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, 
     a.seg_states = seg_states->data_ptr();
     a.seg_states_bytes = static_cast<size_t>(seg_states->numel() * seg_states->element_size());
   }
-  const Tensor ws = scratch(a, 1, q);
+  const Tensor ws = scratch(a, 1, g);
   check(fla_sm100_bwd(&a), "libflashlinear_sm100");
   copy_back(out, 3, stream);
   return std::array<Tensor, 3>{out[0].full, out[1].full, out[2].full};
+}
+
+// What stands in for an input whose repacked copy is kept for the backward instead of itself, so that
+// the layer holds it once: its layout (a tensor without storage), for the gradient, and an empty
+// tensor that shares its version count, for autograd to see that it was changed in place. (An inference
+// tensor has none; it is returned itself, and autograd refuses it as it always does.)
+std::pair<Tensor, Tensor> stand_ins(const Tensor& t) {
+  const Tensor layout = at::empty_strided(t.sizes(), t.strides(), t.options().device(at::kMeta));
+  if (t.is_inference()) return {layout, t};
+  const Tensor version = at::empty({0}, t.options());
+  torch::autograd::impl::set_version_counter(version, torch::autograd::impl::version_counter(t));
+  return {layout, version};
 }
 
 }  // namespace
@@ -303,6 +318,7 @@ PYBIND11_MODULE(_hostcalls, m) {
     if (r->views.has_value()) views = py::make_tuple((*r->views)[0], (*r->views)[1], (*r->views)[2]);
     return py::make_tuple(r->out, r->s_final, r->seg_states, views);
   });
+  m.def("stand_ins", &stand_ins);
   m.def("backward", [](const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_last,
                        const OptTensor& seg_states, bool keep_padded, const std::optional<std::vector<Tensor>>& views,
                        unsigned debug_flags, uintptr_t status) -> py::object {

@@ -49,19 +49,20 @@ def _forward_with_state(ctx: Any, q, k, v, smallv: bool):
         res = ops.general_forward(q, k, v) if need_grad else (ops.causal_dot_product_fwd(q, k, v), None, None, None)
     out, s_final, seg_states, views = res
     # Head dims whose rows had to be repacked: the backward reads the repacked copies again (a pad
-    # pass over three tensors less); q, k, v themselves are saved too, for their version checks and
-    # because the gradients take their layout.
-    ctx.has_views = views is not None
-    ctx.save_for_backward(q, k, v, s_final, seg_states, *(views or ()))
+    # pass over three tensors less). They are kept in place of q, k, v, not beside them; what is left of
+    # those is their layout, which the gradients take, and their version counts.
+    ctx.layouts, versions = (None, ()) if views is None else ops.stand_ins(q, k, v)
+    if views is not None:
+        q, k, v = views
+    ctx.save_for_backward(q, k, v, s_final, seg_states, *versions)
     return out
 
 
 def _backward_with_state(ctx: Any, grad_output):
-    saved = ctx.saved_tensors
-    q, k, v, s_final, seg_states = saved[:5]
-    if ctx.has_views:
-        res = ops.host_backward(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,
-                                keep_padded=ctx.keep_padded, views=saved[5:8])
+    q, k, v, s_final, seg_states = ctx.saved_tensors[:5]
+    if ctx.layouts is not None:
+        res = ops.host_backward(grad_output, *ctx.layouts, s_last=s_final, seg_states=seg_states,
+                                keep_padded=ctx.keep_padded, views=(q, k, v))
         if res is not None:
             return res
     return ops.causal_dot_product_bwd(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,

@@ -295,15 +295,23 @@ def general_forward(q, k, v):
 
 
 def host_backward(grad_output, q, k, v, s_last=None, seg_states=None, keep_padded: bool = False, views=None):
-    """One backward call through the native host path: (dQ, dK, dV), or None (see host_forward). `views`: what host_forward returned for the same q, k, v."""
-    native = _lib.host() if q.is_cuda else None
+    """One backward call through the native host path: (dQ, dK, dV), or None (see host_forward). `views`: what
+    host_forward returned for the same q, k, v, of which only the layout then counts (stand_ins())."""
+    native = _lib.host() if grad_output.is_cuda else None
     if native is None:
         return None
     res = native.backward(grad_output, q, k, v, s_last, seg_states, keep_padded, views,
-                               _debug_flags, _status_ptr(q))
+                               _debug_flags, _status_ptr(grad_output))
     if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
-        check_status(q.device)
+        check_status(grad_output.device)
     return res
+
+
+def stand_ins(*tensors: torch.Tensor):
+    """(layouts, versions) of inputs that are not kept for the backward because their repacked copies are:
+    tensors without storage that have their sizes and strides, and empty ones that share their version
+    counts."""
+    return tuple(zip(*(_lib.host().stand_ins(t) for t in tensors)))
 
 
 def _product_call(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, out: torch.Tensor, anticausal: bool) -> None:

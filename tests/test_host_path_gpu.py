@@ -64,3 +64,97 @@ def test_calls_without_the_native_host_path_give_the_same(shape, monkeypatch):
     monkeypatch.setattr(_lib, "_host", False)
     for a, b in zip(step(), want):
         assert torch.equal(a, b) and a.stride() == b.stride()
+
+
+def _odd(layout, B=2, H=3, N=192, d=83, seed=0):
+    x = _draw(B, N, H, d, seed=seed).transpose(1, 2)
+    return x if layout == "bnhd" else x.contiguous()
+
+
+def _step(x, g):
+    from flashy_linear_attention_b200 import LinearAttention
+
+    out = LinearAttention.apply(*x)
+    return (out,) + torch.autograd.grad(out, x, g)
+
+
+@pytest.mark.parametrize("layout", ["bhnd", "bnhd"])
+def test_a_layer_holds_one_copy_of_an_odd_head_dim(layout):
+    """Between forward and backward an odd head dim costs what its repacked rows take (88 columns for 83), not
+    that and q, k, v as well, and the gradients have the layout of q, k, v."""
+    from flashy_linear_attention_b200 import LinearAttention
+
+    leaf = [_odd(layout, N=2048, seed=i).requires_grad_(True) for i in range(3)]
+    g = _odd(layout, N=2048, seed=3)
+    _step(leaf, g)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    out = LinearAttention.apply(*(t * 1 for t in leaf))  # nobody else keeps the three products
+    torch.cuda.synchronize()
+    rows = leaf[0].numel() // 83
+    held = torch.cuda.memory_allocated() - before - rows * 83 * 2  # without the output
+    assert held < 1.1 * 3 * rows * 88 * 2, held / (3 * rows * 88 * 2)
+    x = [t.detach().requires_grad_(True) for t in leaf]
+    for got, want, t in zip(torch.autograd.grad(out, leaf, g), _step(x, g)[1:], leaf):
+        assert torch.equal(got, want) and want.stride() == torch.empty_like(t).stride()
+
+
+@pytest.mark.parametrize("which", [0, 1, 2])
+@pytest.mark.parametrize("d", [83, 64])
+def test_an_input_changed_in_place_before_the_backward_is_refused(which, d):
+    from flashy_linear_attention_b200 import LinearAttention
+
+    leaf = [_odd("bhnd", d=d, seed=i).requires_grad_(True) for i in range(3)]
+    x = [t * 1 for t in leaf]
+    out = LinearAttention.apply(*x)
+    with torch.no_grad():
+        x[which].add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(out.sum(), leaf)
+
+
+@pytest.mark.parametrize("layout", ["bhnd", "bnhd"])
+@pytest.mark.parametrize("d", [83, 64])
+def test_saved_tensors_may_come_back_elsewhere_and_contiguous(layout, d):
+    """saved_tensors_hooks that move what is saved to the host and bring back plain contiguous tensors."""
+    x = [_odd(layout, N=2240, d=d, seed=i).requires_grad_(True) for i in range(3)]
+    g = _odd(layout, N=2240, d=d, seed=3)
+    want = _step(x, g)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu().contiguous(), lambda t: t.to(DEV)):
+        got = _step(x, g)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    with torch.autograd.graph.save_on_cpu():
+        got = _step(x, g)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b) and a.stride() == b.stride()
+
+
+@pytest.mark.parametrize("d", [83, 64])
+def test_two_threads_on_streams_of_their_own(d):
+    """Each thread's forward and backward on its own stream, inputs made there; many at once."""
+    results, errors = {}, []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for rep in range(20):
+                    x = [_odd("bhnd", N=512, d=d, seed=10 * i + j).requires_grad_(True) for j in range(3)]
+                    got = [t.clone() for t in _step(x, _odd("bhnd", N=512, d=d, seed=10 * i + 9))]
+                    first = results.setdefault(i, got)
+                    torch.cuda.current_stream().synchronize()
+                    assert all(torch.equal(a, b) for a, b in zip(first, got)), (i, rep)
+        except Exception as exc:  # reported by the main thread
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    torch.cuda.synchronize()
+    for i, got in results.items():
+        x = [_odd("bhnd", N=512, d=d, seed=10 * i + j).requires_grad_(True) for j in range(3)]
+        for a, b in zip(got, _step(x, _odd("bhnd", N=512, d=d, seed=10 * i + 9))):
+            assert torch.equal(a, b)
