@@ -7,6 +7,7 @@ Tolerances (bf16 in / bf16 out, fp32 accumulation):
     max relative error  max|a-b| / max|b|  <= 2e-2     (north-star bound for bf16)
     Frobenius relative error               <  1e-2     (the reference tests' bound, test_attn.py:17)
 """
+import ctypes
 import glob
 import os
 
@@ -637,14 +638,21 @@ def test_taylor_attention_function_against_oracle(shape):
     _check("dxk", _np(gk), orc.taylor_feature_map_grad(k64, dpk))
 
 
-@pytest.mark.parametrize("shape", [(1, 4, 1024, 128, 128), (2, 16, 512, 64, 64)], ids=["segmented", "one-wave"])
+@pytest.mark.parametrize("shape", [(1, 4, 4096, 128, 128), (1, 4, 1024, 128, 128), (2, 16, 512, 64, 64)],
+                         ids=["segmented", "few-heads", "one-wave"])
 def test_cuda_graph_capture_replays_the_same_results(shape):
     """The entry points only enqueue work, so a forward + backward over fixed buffers can be captured
     in a CUDA graph; a replay after the inputs changed in place gives what an eager call gives."""
+    from flashy_linear_attention_b200 import _lib
+    from flashy_linear_attention_b200._lib import FlaArgs
     from flashy_linear_attention_b200.graphs import capture_step
 
     ops = _ops()
     B, H, N, dk, dv = shape
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = shape
+    for p in (0, 1):  # the first shape is split, and uses scratch, in both passes
+        assert (_lib.load().fla_sm100_workspace_bytes(ctypes.byref(a), p) > 0) == (N == 4096)
     torch.manual_seed(5)
     q = (torch.nn.functional.elu(torch.randn(B, H, N, dk, device=DEV)) + 1).to(torch.bfloat16)
     k = (torch.nn.functional.elu(torch.randn(B, H, N, dk, device=DEV)) + 1).to(torch.bfloat16)

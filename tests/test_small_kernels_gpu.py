@@ -57,6 +57,28 @@ def test_few_tokens_round_the_state_once(tokens, dtype):
     assert (s1.double() - want).norm() <= 1.1 * once
 
 
+@pytest.mark.parametrize("tokens", [4, 7, 16])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_few_tokens_keep_what_comes_before_a_bad_one(tokens, value):
+    from flashy_linear_attention_b200 import LinearAttentionResumable
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    q, k, v = (torch.randn(1, 3, tokens, 128, device="cuda", generator=gen).bfloat16() for _ in range(3))
+    s0 = torch.randn(1, 3, 128, 128, device="cuda", generator=gen)
+    clean, state = LinearAttentionResumable.apply(q, k, v, s0)
+    at = tokens - 2
+    for which in range(3):
+        x = [q.clone(), k.clone(), v.clone()]
+        x[which][0, 1, at, 5] = value
+        out, s1 = LinearAttentionResumable.apply(*x, s0)
+        assert torch.equal(out[0, ::2], clean[0, ::2]) and torch.equal(s1[0, ::2], state[0, ::2])
+        assert torch.equal(out[0, 1, :at], clean[0, 1, :at]) and not out[0, 1, at].isfinite().all()
+        if which == 0:  # a query leaves no trace
+            assert torch.equal(out[0, 1, at + 1:], clean[0, 1, at + 1:]) and torch.equal(s1, state)
+        else:
+            assert not out[0, 1, at + 1].isfinite().all() and not s1[0, 1].isfinite().all()
+
+
 # one token whose row is no multiple of 16 bytes although its head and batch strides are or do not
 # count: a tensor of its own, one step of a longer contiguous one (at a 16-byte boundary and not)
 @pytest.mark.parametrize("d", [83, 20])
