@@ -67,9 +67,26 @@ FlaTensor desc(const Tensor& t) {
 }
 
 // View [..., :d] of a fresh tensor whose rows are padded to a multiple of 8 elements.
-Tensor padded_empty(const Tensor& like, const at::TensorOptions& options) {
+Tensor padded_empty(const Tensor& like) {
   const int64_t d = like.size(3);
-  return at::empty({like.size(0), like.size(1), like.size(2), (d + 7) / 8 * 8}, options).narrow(3, 0, d);
+  return at::empty({like.size(0), like.size(1), like.size(2), (d + 7) / 8 * 8}, like.options()).narrow(3, 0, d);
+}
+
+// empty_like() of a tensor of these sizes and strides that is not at hand any more.
+Tensor empty_like_of(const Tensor& sizes_of, at::IntArrayRef strides) {
+  const at::IntArrayRef sizes = sizes_of.sizes();
+  // strides without gaps or overlaps are kept as they are: walk the dimensions from the inside out
+  int order[4] = {3, 2, 1, 0};
+  std::stable_sort(order, order + 4, [&](int a, int b) { return strides[a] < strides[b]; });
+  int64_t next = 1;
+  bool dense = true;
+  for (int d : order) {
+    if (sizes[d] == 1) continue;
+    dense = dense && strides[d] == next;
+    next *= sizes[d];
+  }
+  if (dense) return at::empty_strided(sizes, strides, sizes_of.options());
+  return at::empty_like(at::empty_strided(sizes, strides, sizes_of.options().device(at::kMeta)), sizes_of.options());
 }
 
 void check(int rc, const char* name) {
@@ -93,7 +110,7 @@ void kernel_views(Tensor* t, int n, void* stream) {
   bool done[kMax] = {};
   for (int i = 0; i < n; ++i) {
     if (addressable(t[i])) done[i] = true;
-    else copies[i] = padded_empty(t[i], t[i].options());
+    else copies[i] = padded_empty(t[i]);
     if (!done[i] && !contiguous_rows(t[i])) {
       copies[i].copy_(t[i]);
       done[i] = true;
@@ -121,14 +138,14 @@ void kernel_views(Tensor* t, int n, void* stream) {
 struct Output {
   Tensor full, view;
 };
-Output output_like(const Tensor& t, bool keep_padded, const at::TensorOptions& options) {
+Output output_like(const Tensor& t, bool keep_padded, const std::vector<int64_t>* strides) {
   Output o;
   if (keep_padded && t.size(3) % 8 != 0) {
-    o.full = o.view = padded_empty(t, options);
+    o.full = o.view = padded_empty(t);
     return o;
   }
-  o.full = at::empty_like(t, options);
-  o.view = addressable(o.full) ? o.full : padded_empty(o.full, options);
+  o.full = strides != nullptr ? empty_like_of(t, *strides) : at::empty_like(t);
+  o.view = addressable(o.full) ? o.full : padded_empty(o.full);
   return o;
 }
 // Results from the padded scratch rows into the caller-layout outputs, grouped like kernel_views().
@@ -209,7 +226,7 @@ std::optional<Forward> forward(const Tensor& q, const Tensor& k, const Tensor& v
   if (!is_state(s_init, q, bh, dk, dv)) return std::nullopt;
   const c10::cuda::CUDAGuard guard(q.device());
   void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
-  const Output out = output_like(v, false, v.options());
+  const Output out = output_like(v, false, nullptr);
   Tensor in[3] = {q, k, v};
   kernel_views(in, 3, stream);
   FlaArgs a;
@@ -243,34 +260,28 @@ std::optional<Forward> forward(const Tensor& q, const Tensor& k, const Tensor& v
   return res;
 }
 
+// strides: those of the three tensors that q, k, v are repacked copies of; the gradients take their layout.
+using Strides = std::optional<std::array<std::vector<int64_t>, 3>>;
 std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v,
                                               const OptTensor& s_last, const OptTensor& seg_states, bool keep_padded,
-                                              const std::optional<std::vector<Tensor>>& views, unsigned debug_flags,
-                                              uintptr_t status) {
-  // With views, q, k and v only say what layout the gradients have (stand_ins()).
-  const Tensor like[3] = {q, k, v};
+                                              const Strides& strides, unsigned debug_flags, uintptr_t status) {
   Tensor in[4] = {q, k, v, g};
-  if (views.has_value()) {
-    if (views->size() != 3) return std::nullopt;
-    for (int i = 0; i < 3; ++i) {
-      if ((*views)[i].sizes() != like[i].sizes()) return std::nullopt;
-      in[i] = (*views)[i];
-    }
-  }
   for (const Tensor& t : in)
-    if (!usable(t, in[0]) || !same_rows(t, in[0])) return std::nullopt;
-  if (!covered_dims(in[0], in[2]) || q.size(3) != k.size(3) || g.size(3) != v.size(3)) return std::nullopt;
+    if (!usable(t, q) || !same_rows(t, q)) return std::nullopt;
+  if (!covered_dims(q, v) || q.size(3) != k.size(3) || g.size(3) != v.size(3)) return std::nullopt;
+  if (strides.has_value())
+    for (const auto& s : *strides)
+      if (s.size() != 4) return std::nullopt;
   const int64_t bh = q.size(0) * q.size(1), dk = q.size(3), dv = v.size(3);
   if ((dk > kKernelHeadDim || dv > kKernelHeadDim) && s_last.has_value()) return std::nullopt;
   if (!is_state(s_last, g, bh, dk, dv)) return std::nullopt;
   const c10::cuda::CUDAGuard guard(g.device());
   void* stream = c10::cuda::getCurrentCUDAStream(g.device().index()).stream();
-  const at::TensorOptions options = g.options();
-  const Output out[3] = {output_like(q, keep_padded, options), output_like(k, keep_padded, options),
-                         output_like(v, keep_padded, options)};
+  Output out[3];
+  for (int i = 0; i < 3; ++i) out[i] = output_like(in[i], keep_padded, strides.has_value() ? &(*strides)[i] : nullptr);
   kernel_views(in, 4, stream);
   FlaArgs a;
-  set_sizes(a, in[0], in[2], debug_flags, status);
+  set_sizes(a, q, v, debug_flags, status);
   a.stream = stream;
   a.q = desc(in[0]);
   a.k = desc(in[1]);
@@ -290,16 +301,14 @@ std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, 
   return std::array<Tensor, 3>{out[0].full, out[1].full, out[2].full};
 }
 
-// What stands in for an input whose repacked copy is kept for the backward instead of itself, so that
-// the layer holds it once: its layout (a tensor without storage), for the gradient, and an empty
-// tensor that shares its version count, for autograd to see that it was changed in place. (An inference
-// tensor has none; it is returned itself, and autograd refuses it as it always does.)
-std::pair<Tensor, Tensor> stand_ins(const Tensor& t) {
-  const Tensor layout = at::empty_strided(t.sizes(), t.strides(), t.options().device(at::kMeta));
-  if (t.is_inference()) return {layout, t};
+// What is saved beside the repacked copy of an input that is not kept itself: an empty tensor that shares
+// its version count, for autograd to see that it was changed in place. (An inference tensor has none;
+// it is returned itself, and autograd refuses it as it always does.)
+Tensor version_of(const Tensor& t) {
+  if (t.is_inference()) return t;
   const Tensor version = at::empty({0}, t.options());
   torch::autograd::impl::set_version_counter(version, torch::autograd::impl::version_counter(t));
-  return {layout, version};
+  return version;
 }
 
 }  // namespace
@@ -318,14 +327,14 @@ PYBIND11_MODULE(_hostcalls, m) {
     if (r->views.has_value()) views = py::make_tuple((*r->views)[0], (*r->views)[1], (*r->views)[2]);
     return py::make_tuple(r->out, r->s_final, r->seg_states, views);
   });
-  m.def("stand_ins", &stand_ins);
+  m.def("version_of", &version_of);
   m.def("backward", [](const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_last,
-                       const OptTensor& seg_states, bool keep_padded, const std::optional<std::vector<Tensor>>& views,
-                       unsigned debug_flags, uintptr_t status) -> py::object {
+                       const OptTensor& seg_states, bool keep_padded, const Strides& strides, unsigned debug_flags,
+                       uintptr_t status) -> py::object {
     std::optional<std::array<Tensor, 3>> r;
     {
       const py::gil_scoped_release unlocked;
-      r = backward(g, q, k, v, s_last, seg_states, keep_padded, views, debug_flags, status);
+      r = backward(g, q, k, v, s_last, seg_states, keep_padded, strides, debug_flags, status);
     }
     if (!r.has_value()) return py::none();
     return py::make_tuple((*r)[0], (*r)[1], (*r)[2]);

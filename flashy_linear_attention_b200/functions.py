@@ -51,8 +51,9 @@ def _forward_with_state(ctx: Any, q, k, v, smallv: bool):
     # Head dims whose rows had to be repacked: the backward reads the repacked copies again (a pad
     # pass over three tensors less). They are kept in place of q, k, v, not beside them; what is left of
     # those is their layout, which the gradients take, and their version counts.
-    ctx.layouts, versions = (None, ()) if views is None else ops.stand_ins(q, k, v)
+    ctx.strides, versions = None, ()
     if views is not None:
+        ctx.strides, versions = [t.stride() for t in (q, k, v)], ops.versions_of(q, k, v)
         q, k, v = views
     ctx.save_for_backward(q, k, v, s_final, seg_states, *versions)
     return out
@@ -60,9 +61,9 @@ def _forward_with_state(ctx: Any, q, k, v, smallv: bool):
 
 def _backward_with_state(ctx: Any, grad_output):
     q, k, v, s_final, seg_states = ctx.saved_tensors[:5]
-    if ctx.layouts is not None:
-        res = ops.host_backward(grad_output, *ctx.layouts, s_last=s_final, seg_states=seg_states,
-                                keep_padded=ctx.keep_padded, views=(q, k, v))
+    if ctx.strides is not None:
+        res = ops.host_backward(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,
+                                keep_padded=ctx.keep_padded, strides=ctx.strides)
         if res is not None:
             return res
     return ops.causal_dot_product_bwd(grad_output, q, k, v, s_last=s_final, seg_states=seg_states,

@@ -294,24 +294,28 @@ def general_forward(q, k, v):
     return causal_dot_product_fwd(q, k, v, s_final=s_final, seg_states=seg_states), s_final, seg_states, None
 
 
-def host_backward(grad_output, q, k, v, s_last=None, seg_states=None, keep_padded: bool = False, views=None):
+def host_backward(grad_output, q, k, v, s_last=None, seg_states=None, keep_padded: bool = False, views=None,
+                  strides=None):
     """One backward call through the native host path: (dQ, dK, dV), or None (see host_forward). `views`: what
-    host_forward returned for the same q, k, v, of which only the layout then counts (stand_ins())."""
+    host_forward returned for the same q, k, v, of which only the layout then counts; a caller that has kept
+    nothing else of them passes the views as q, k, v and the `strides` of the three tensors."""
+    if views is not None:
+        strides = [t.stride() for t in (q, k, v)]
+        q, k, v = views
     native = _lib.host() if grad_output.is_cuda else None
     if native is None:
         return None
-    res = native.backward(grad_output, q, k, v, s_last, seg_states, keep_padded, views,
+    res = native.backward(grad_output, q, k, v, s_last, seg_states, keep_padded, strides,
                                _debug_flags, _status_ptr(grad_output))
     if res is not None and os.environ.get("FLA_DEBUG", "0") == "1":
         check_status(grad_output.device)
     return res
 
 
-def stand_ins(*tensors: torch.Tensor):
-    """(layouts, versions) of inputs that are not kept for the backward because their repacked copies are:
-    tensors without storage that have their sizes and strides, and empty ones that share their version
-    counts."""
-    return tuple(zip(*(_lib.host().stand_ins(t) for t in tensors)))
+def versions_of(*tensors: torch.Tensor):
+    """Empty tensors that share the version counts of `tensors`, whose repacked copies are kept for the backward
+    instead of themselves: saved with those, they let autograd see an input that was changed in place."""
+    return tuple(_lib.host().version_of(t) for t in tensors)
 
 
 def _product_call(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, out: torch.Tensor, anticausal: bool) -> None:

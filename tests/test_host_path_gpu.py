@@ -158,3 +158,21 @@ def test_two_threads_on_streams_of_their_own(d):
         x = [_odd("bhnd", N=512, d=d, seed=10 * i + j).requires_grad_(True) for j in range(3)]
         for a, b in zip(got, _step(x, _odd("bhnd", N=512, d=d, seed=10 * i + 9))):
             assert torch.equal(a, b)
+
+
+def test_gradients_of_repacked_inputs_take_the_layout_of_empty_like():
+    """Permuted, expanded and sliced inputs whose rows have to be repacked."""
+    from flashy_linear_attention_b200 import LinearAttention
+
+    base = _draw(2, 3, 128, 90, seed=1)
+    forms = [base[..., :83].contiguous(), base[..., :83], base[..., 1:84], base[:, :, :, :83].transpose(1, 2).contiguous().transpose(1, 2),
+             base[..., :83].transpose(0, 1).contiguous().transpose(0, 1), base[:, :1, :, :83].expand(2, 3, 128, 83),
+             base[..., :83].transpose(2, 3).contiguous().transpose(2, 3), base[:1, ..., :83].contiguous().expand(2, 3, 128, 83)]
+    g = _draw(2, 3, 128, 83, seed=2)
+    for i, x in enumerate(forms):
+        leaf = [x.detach().requires_grad_(True)] + [forms[0].detach().clone().requires_grad_(True) for _ in range(2)]
+        got = torch.autograd.grad(LinearAttention.apply(*leaf), leaf, g)
+        plain = [t.detach().contiguous().requires_grad_(True) for t in leaf]
+        want = torch.autograd.grad(LinearAttention.apply(*plain), plain, g)
+        for a, b, t in zip(got, want, leaf):
+            assert torch.equal(a, b) and a.stride() == torch.empty_like(t).stride(), (i, a.stride(), t.stride())
