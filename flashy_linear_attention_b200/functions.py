@@ -105,8 +105,8 @@ class LinearAttentionResumable(Function):
     as ``s_init`` of the next gives what one call over the concatenated tokens gives: chunked
     prefill, decoding a few tokens at a time, or training on a long sequence piece by piece. Any
     number of tokens per call is accepted (the reference's multiple-of-64 rule,
-    linear_attn_kernels.py:323-325, is a property of its tiling; calls of up to 16 tokens run the
-    recurrence itself in fp32 instead of a 128-token tile). The state is
+    linear_attn_kernels.py:323-325, is a property of its tiling; calls of up to 16 tokens, 8
+    where both head dims are at most 64, run the recurrence itself in fp32 instead of a 128-token tile). The state is
     differentiable: the backward returns the gradient of ``s_init`` and accepts one for ``s_final``.
 
     Not part of the reference, whose Functions (flashlinear/linear_attn.py:11-31) always start from
@@ -157,9 +157,10 @@ class LinearAttentionNormalized(Function):
     """Causal linear attention WITH its denominator:
     ``out_i = sum_{j<=i} (q_i . k_j) v_j / (q_i . sum_{j<=i} k_j + eps)``, i.e. the whole recipe of
     the reference's README (README.md:27-30) in one Function. The product runs in the same kernels
-    as LinearAttention / LinearAttentionSmallVHD; the denominator, the division and their
-    gradients run in three streaming kernels with an fp32 running sum instead of PyTorch's
-    cumsum / multiply / sum / divide passes. ``apply(q, k, v, eps=1e-5)``; dv a multiple of 8.
+    as LinearAttention / LinearAttentionSmallVHD. The denominator and the division run inside the
+    forward product where ``ops.normalized_fused`` says so (bf16, dk == dv <= 128, enough heads),
+    otherwise, like their gradients, in streaming kernels with an fp32 running sum instead of
+    PyTorch's cumsum / multiply / sum / divide passes. ``apply(q, k, v, eps=1e-5)``; dv a multiple of 8.
     """
 
     @staticmethod

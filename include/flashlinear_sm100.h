@@ -301,8 +301,9 @@ int fla_sm100_normalize_bwd_prepare(const FlaArgs* args, const float* den, float
 int fla_sm100_normalize_bwd_sweep(const FlaArgs* args, const float* dden);
 
 /* The forward of the same operation with the denominator inside the product kernel: q, k, v -> o
- * (normalised), den [batch*heads, seqlen] fp32, s_final optional; 512 bytes a token-head less at head
- * dim 128 than product + normalize_fwd read and write. fla_sm100_normalized_fused() says whether a
+ * (normalised), den [batch*heads, seqlen] fp32, s_final optional. At head dim 128 product +
+ * normalize_fwd move 1024 bytes a token-head more (the product is written and read again, q and k are
+ * read again), 1280 where normalize_fwd takes column sums of k first. fla_sm100_normalized_fused() says whether a
  * shape runs that way (1) or through the separate calls above (0): bf16, dk == dv <= 128 and a
  * multiple of 8, the forward not split into segments. */
 int fla_sm100_normalized_fused(const FlaArgs* args);
