@@ -303,9 +303,10 @@ int fla_sm100_normalize_bwd_sweep(const FlaArgs* args, const float* dden);
 /* The forward of the same operation with the denominator inside the product kernel: q, k, v -> o
  * (normalised), den [batch*heads, seqlen] fp32, s_final optional. At head dim 128 product +
  * normalize_fwd move 1024 bytes a token-head more (the product is written and read again, q and k are
- * read again), 1280 where normalize_fwd takes column sums of k first. fla_sm100_normalized_fused() says whether a
- * shape runs that way (1) or through the separate calls above (0): bf16, dk == dv <= 128 and a
- * multiple of 8, the forward not split into segments. */
+ * read again), 1280 where normalize_fwd takes column sums of k first. normalized_fwd
+ * takes bf16, dk == dv <= 128 and a multiple of 8, where the forward is not split into segments;
+ * fla_sm100_normalized_fused() says whether it takes a shape and is the faster way for it (1), or the
+ * separate calls above are to be used (0). With args->segments == 1 only the former counts. */
 int fla_sm100_normalized_fused(const FlaArgs* args);
 int fla_sm100_normalized_fwd(const FlaArgs* args, float eps, float* den);
 

@@ -305,3 +305,18 @@ def test_native_host_path_belongs_to_one_torch_and_python(monkeypatch, tmp_path)
     monkeypatch.setattr(_lib, "_host", None)
     with pytest.warns(RuntimeWarning):
         assert _lib.host() is None
+
+
+@pytest.mark.parametrize("heads, tokens, fused", [(1, 128, 1), (2, 1024, 1), (60, 1024, 1), (60, 1025, 0), (75, 4096, 0),
+                                                  (76, 4096, 1), (128, 4096, 1), (2, 4096, 0)])
+@pytest.mark.parametrize("width", [64, 128])
+def test_rule_of_the_fused_denominator(heads, tokens, fused, width):
+    """Short calls and many heads take the fused forward; a caller that asks for one segment gets it."""
+    from flashy_linear_attention_b200 import _lib
+    from flashy_linear_attention_b200._lib import FlaArgs
+
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, tokens, width, width
+    assert _lib.load().fla_sm100_normalized_fused(ctypes.byref(a)) == fused
+    a.segments = 1
+    assert _lib.load().fla_sm100_normalized_fused(ctypes.byref(a)) == 1
