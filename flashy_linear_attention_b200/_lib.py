@@ -100,6 +100,8 @@ EXPORTED_SYMBOLS = (
     "fla_sm100_normalized_fused",
     "fla_sm100_normalized_fwd",
     "fla_sm100_taylor_dims",
+    "fla_sm100_taylor_fwd",
+    "fla_sm100_taylor_bwd",
     "fla_sm100_taylor_features",
     "fla_sm100_taylor_features_bwd",
     "fla_sm100_pad_rows",
@@ -176,6 +178,10 @@ def load() -> ctypes.CDLL:
     lib.fla_sm100_normalized_fused.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_normalized_fwd.restype = ctypes.c_int
     lib.fla_sm100_normalized_fwd.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_float, ctypes.c_void_p]
+    for name in ("fla_sm100_taylor_fwd", "fla_sm100_taylor_bwd"):
+        fn = getattr(lib, name)
+        fn.restype = ctypes.c_int
+        fn.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_taylor_dims.restype = ctypes.c_int
     lib.fla_sm100_taylor_dims.argtypes = [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
     lib.fla_sm100_taylor_features.restype = ctypes.c_int

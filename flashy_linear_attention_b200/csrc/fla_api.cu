@@ -15,6 +15,7 @@
 #include "fla_wide_kernel.cuh"
 #include "fla_normalize.cuh"
 #include "fla_taylor.cuh"
+#include "fla_taylor_attention.cuh"
 #include "fla_decode.cuh"
 
 #include <cuda_runtime.h>
@@ -536,6 +537,8 @@ int device_info(DeviceInfo** out) {
       };
       norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<64, 64, false, true>), fla::Cfg<64, 64>::NORM_SMEM_BYTES);
       norm_smem(reinterpret_cast<const void*>(fla::fla_chunk_kernel<128, 128, false, true>), fla::Cfg<128, 128>::NORM_SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_taylor_attention_kernel<8>), fla::TaylorCfg<8>::SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_taylor_attention_kernel<16>), fla::TaylorCfg<16>::SMEM_BYTES);
       auto big_smem = [&](const void* fn) {
         ok &= cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) == cudaSuccess;
       };
@@ -1504,6 +1507,69 @@ int fla_sm100_fwd_static_scratch(const FlaArgs* a) {
                       nseg > 1 ? FLA_STATIC_SCRATCH_BYTES : 0, a->status,
                       static_cast<cudaStream_t>(a->stream), *dev);
 }
+
+namespace {
+// What the kernel on raw rows takes: bf16, d = 8 or 16, values of up to 64 columns.
+int taylor_call(const FlaArgs* a, bool backward) {
+  DeviceInfo* dev = nullptr;
+  g_last_launches = 0;
+  int rc = check_common(a, &dev);
+  if (rc) return rc;
+  if ((a->dk != 8 && a->dk != 16) || a->dv > 64 || g_half) return FLA_ERR_UNSUPPORTED;
+  if (a->s_init || a->s_final || a->r_init || a->r_final) return FLA_ERR_UNSUPPORTED;
+  const int B = a->batch, H = a->heads, N = a->seqlen;
+  fla::TaylorParams p;
+  memset(&p, 0, sizeof(p));
+  auto map = [&](CUtensorMap* m, const FlaTensor& t, int rows) {
+    const Operand o = operand(t, a->dv);
+    const int r = check_operand(o, B, H);
+    return r ? r : encode_map(m, o, B, H, N, rows);
+  };
+  auto raw = [&](fla::RawRows* r, const FlaTensor& t) {
+    *r = {static_cast<const __nv_bfloat16*>(t.ptr), t.stride_b, t.stride_h, t.stride_n};
+    return check_operand(operand(t, a->dk), B, H);
+  };
+  if (!backward) {
+    fla::TaylorProblem& f = p.prob[0];
+    f.want_o = 1;
+    if ((rc = raw(&f.x, a->q)) || (rc = raw(&f.y, a->k)) || (rc = map(&f.b, a->v, fla::kChunk)) || (rc = map(&f.o, a->o, 32)))
+      return rc;
+  } else {
+    // dK and dV first: their CTAs take longer, and the grid has more CTAs than SMs for many heads
+    fla::TaylorProblem &kv = p.prob[0], &q = p.prob[1];
+    q.want_dx = 1;
+    if ((rc = raw(&q.x, a->q)) || (rc = raw(&q.y, a->k)) || (rc = raw(&q.dx, a->d_q)) ||
+        (rc = map(&q.a, a->d_o, fla::kChunk)) || (rc = map(&q.b, a->v, fla::kChunk)))
+      return rc;
+    kv.want_o = kv.want_dx = 1;
+    kv.flags = fla::kFlagDescending | fla::kFlagUpperMask;
+    kv.x = q.y;
+    kv.y = q.x;
+    kv.a = q.b;
+    kv.b = q.a;
+    if ((rc = raw(&kv.dx, a->d_k)) || (rc = map(&kv.o, a->d_v, 32))) return rc;
+  }
+  p.heads = H;
+  p.nchunks = (N + fla::kChunk - 1) / fla::kChunk;
+  p.n_tokens = N;
+  p.status = a->status;
+  p.wait_limit_us = g_wait_limit_us;
+  p.debug_withhold = g_debug_withhold;
+  const dim3 grid(backward ? 2 : 1, 1, B * H);
+  cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  if (a->dk == 16)
+    fla::fla_taylor_attention_kernel<16><<<grid, fla::kTaylorThreads, fla::TaylorCfg<16>::SMEM_BYTES, stream>>>(p);
+  else
+    fla::fla_taylor_attention_kernel<8><<<grid, fla::kTaylorThreads, fla::TaylorCfg<8>::SMEM_BYTES, stream>>>(p);
+  ++g_last_launches;
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) FLA_LOG_FAILURE("launch of fla_taylor_attention_kernel<%d> failed: %s", a->dk, cudaGetErrorString(e));
+  return e == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
+}
+}  // namespace
+
+int fla_sm100_taylor_fwd(const FlaArgs* a) { return taylor_call(a, false); }
+int fla_sm100_taylor_bwd(const FlaArgs* a) { return taylor_call(a, true); }
 
 int fla_sm100_taylor_dims(int d, int* features, int* padded) {
   if (d != 8 && d != 16) return FLA_ERR_UNSUPPORTED;

@@ -301,6 +301,54 @@ std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, 
   return std::array<Tensor, 3>{out[0].full, out[1].full, out[2].full};
 }
 
+// Attention on the Taylor features of raw q, k.
+bool taylor_covered(const Tensor& q, const Tensor& k, const Tensor& v) {
+  const int64_t d = q.dim() == 4 ? q.size(3) : 0, dv = v.dim() == 4 ? v.size(3) : 0;
+  return usable(q, q) && usable(k, q) && usable(v, q) && same_rows(q, k) && same_rows(q, v) && k.size(3) == d &&
+         (d == 8 || d == 16) && dv % 8 == 0 && dv <= 64 && q.scalar_type() == at::kBFloat16 && covered_dims(q, v);
+}
+std::optional<Tensor> taylor_forward(const Tensor& q, const Tensor& k, const Tensor& v, unsigned debug_flags, uintptr_t status) {
+  if (!taylor_covered(q, k, v)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(q.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  const Output out = output_like(v, false, nullptr);
+  Tensor in[3] = {q, k, v};
+  kernel_views(in, 3, stream);
+  FlaArgs a;
+  set_sizes(a, q, v, debug_flags, status);
+  a.stream = stream;
+  a.q = desc(in[0]);
+  a.k = desc(in[1]);
+  a.v = desc(in[2]);
+  a.o = desc(out.view);
+  check(fla_sm100_taylor_fwd(&a), "fla_sm100_taylor_fwd");
+  copy_back(&out, 1, stream);
+  return out.full;
+}
+std::optional<std::array<Tensor, 3>> taylor_backward(const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v,
+                                                     unsigned debug_flags, uintptr_t status) {
+  if (!taylor_covered(q, k, v) || !usable(g, q) || !same_rows(g, q) || g.size(3) != v.size(3)) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(g.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(g.device().index()).stream();
+  const Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options());
+  const Output dv = output_like(v, false, nullptr);
+  Tensor in[4] = {q, k, v, g};
+  kernel_views(in, 4, stream);
+  FlaArgs a;
+  set_sizes(a, q, v, debug_flags, status);
+  a.stream = stream;
+  a.q = desc(in[0]);
+  a.k = desc(in[1]);
+  a.v = desc(in[2]);
+  a.d_o = desc(in[3]);
+  a.d_q = desc(dq);
+  a.d_k = desc(dk);
+  a.d_v = desc(dv.view);
+  check(fla_sm100_taylor_bwd(&a), "fla_sm100_taylor_bwd");
+  copy_back(&dv, 1, stream);
+  return std::array<Tensor, 3>{dq, dk, dv.full};
+}
+
 // What is saved beside the repacked copy of an input that is not kept itself: an empty tensor that shares
 // its version count, for autograd to see that it was changed in place. (An inference tensor has none;
 // it is returned itself, and autograd refuses it as it always does.)
@@ -328,6 +376,8 @@ PYBIND11_MODULE(_hostcalls, m) {
     return py::make_tuple(r->out, r->s_final, r->seg_states, views);
   });
   m.def("version_of", &version_of);
+  m.def("taylor_forward", &taylor_forward, py::call_guard<py::gil_scoped_release>());
+  m.def("taylor_backward", &taylor_backward, py::call_guard<py::gil_scoped_release>());
   m.def("backward", [](const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_last,
                        const OptTensor& seg_states, bool keep_padded, const Strides& strides, unsigned debug_flags,
                        uintptr_t status) -> py::object {

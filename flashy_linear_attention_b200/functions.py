@@ -209,22 +209,28 @@ class TaylorLinearAttention(Function):
     vec(x x^T) / (sqrt(2) sqrt(d))]`` (benchmark configuration 4: d = 16 -> 273 features), and its
     backward returns gradients with respect to the raw xq, xk and v.
 
-    The feature map runs in its own kernels and writes rows the attention kernels read in place,
-    so the pad passes of ``LinearAttentionSmallVHD`` on contiguous 273-wide tensors disappear and the
-    273-wide tensors never have to exist on the caller's side. The reference has no counterpart.
+    The features are formed on chip and never exist in memory, in neither pass, and nothing but xq, xk and v
+    is kept for the backward (values wider than 64 columns, or of a width that is no multiple of 8, go through feature tensors in memory, in
+    both passes). The reference has no counterpart.
     """
 
     @staticmethod
     @_autocast_to_bf16
     def forward(ctx: Any, xq, xk, v):
-        pq, pk = ops.taylor_features(xq), ops.taylor_features(xk)
-        ops.check_forward_preconditions(pq, v, smallv=True)
-        out = ops.causal_dot_product_fwd(pq, pk, v)
-        ctx.save_for_backward(xq, xk, v, pq, pk)
+        out = ops.taylor_forward(xq, xk, v)
+        if out is None:  # errors, and values wider than 64 columns
+            pq, pk = ops.taylor_features(xq), ops.taylor_features(xk)
+            ops.check_forward_preconditions(pq, v, smallv=True)
+            out = ops.causal_dot_product_fwd(pq, pk, v)
+        ctx.save_for_backward(xq, xk, v)
         return out
 
     @staticmethod
     def backward(ctx: Any, grad_output):
-        xq, xk, v, pq, pk = ctx.saved_tensors
+        xq, xk, v = ctx.saved_tensors
+        grads = ops.taylor_backward(grad_output, xq, xk, v)
+        if grads is not None:
+            return tuple(grads)
+        pq, pk = ops.taylor_features(xq), ops.taylor_features(xk)
         dpq, dpk, dv = ops.causal_dot_product_bwd(grad_output, pq, pk, v, keep_padded=True)
         return ops.taylor_features_bwd(dpq, xq), ops.taylor_features_bwd(dpk, xk), dv

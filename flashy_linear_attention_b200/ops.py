@@ -582,6 +582,66 @@ def normalized_fwd(q, k, v, eps: float, need_grad: bool):
     return out, den, s_final
 
 
+def _taylor_on_chip(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> bool:
+    """True for calls that the kernel on raw rows takes: those that pass the checks of the feature map and of
+    the SmallVHD shapes, with values of 8 to 64 columns. What it does not take goes through the features in
+    memory, which report the errors."""
+    if not all(t.is_cuda and t.device == xq.device and t.dtype == torch.bfloat16 and t.dim() == 4 for t in (xq, xk, v)):
+        return False
+    d, dv = xq.shape[-1], v.shape[-1]
+    return (xq.shape == xk.shape and xq.shape[:3] == v.shape[:3] and xq.numel() > 0 and d in (8, 16)
+            and dv in (8, 16, 32, 64) and xq.shape[2] % (64 if d == 8 else 32) == 0)
+
+
+def _taylor_call(name: str, xq, xk, v, **tensors) -> None:
+    args = FlaArgs()
+    args.batch, args.heads, args.seqlen, args.dk, args.dv = *xq.shape, v.shape[-1]
+    for key, t in dict(tensors, q=_kernel_view(xq), k=_kernel_view(xk), v=_kernel_view(v)).items():
+        setattr(args, key, _desc(t))
+    with torch.cuda.device(xq.device):
+        args.stream = torch.cuda.current_stream(xq.device).cuda_stream
+        args.status = _status_word(xq.device).data_ptr()
+        args.debug_flags = _debug_flags
+        rc = getattr(_lib.load(), name)(ctypes.byref(args))
+    _norm_check(rc, name)
+
+
+def taylor_forward(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> Optional[torch.Tensor]:
+    """Causal linear attention on the Taylor features of raw q, k, formed on chip, or None for calls that
+    have to go through taylor_features()."""
+    if not _taylor_on_chip(xq, xk, v):
+        return None
+    native = _lib.host()
+    if native is not None:
+        out = native.taylor_forward(xq, xk, v, _debug_flags, _status_ptr(xq))
+    else:
+        out, view = _out_like(v)
+        _taylor_call("fla_sm100_taylor_fwd", xq, xk, v, o=view)
+        _copy_back(out, view)
+    if os.environ.get("FLA_DEBUG", "0") == "1":
+        check_status(xq.device)
+    return out
+
+
+def taylor_backward(grad_output: torch.Tensor, xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor):
+    """Gradients of taylor_forward() with respect to xq, xk and v, or None as there."""
+    g = grad_output
+    if not _taylor_on_chip(xq, xk, v) or g.shape != v.shape or g.dtype != v.dtype or g.device != v.device:
+        return None
+    native = _lib.host()
+    if native is not None:
+        grads = native.taylor_backward(g, xq, xk, v, _debug_flags, _status_ptr(xq))
+    else:
+        dq, dk = (torch.empty(x.shape, dtype=x.dtype, device=x.device) for x in (xq, xk))
+        dv, view = _out_like(v)
+        _taylor_call("fla_sm100_taylor_bwd", xq, xk, v, d_o=_kernel_view(g), d_q=dq, d_k=dk, d_v=view)
+        _copy_back(dv, view)
+        grads = dq, dk, dv
+    if os.environ.get("FLA_DEBUG", "0") == "1":
+        check_status(xq.device)
+    return grads
+
+
 def taylor_features(x: torch.Tensor) -> torch.Tensor:
     """Second-order Taylor features phi(x) = [1, x / d^(1/4), vec(x x^T) / (sqrt(2) sqrt(d))] of raw
     x [B, H, N, d] (bf16, d = 8 or 16): a [B, H, N, 1 + d + d^2] view of rows padded to a multiple

@@ -323,6 +323,12 @@ int fla_sm100_taylor_features(const void* x, void* phi, long long rows, int d, v
 int fla_sm100_taylor_features_bwd(const void* dphi, const void* x, void* dx, long long rows, int d,
                                   void* stream);
 
+/* Causal linear attention on those features from the RAW rows: q, k (and d_q, d_k) hold dk = d = 8 or 16
+ * columns, v, o, d_o, d_v up to 64, bf16; the features never leave the chip and the running state starts
+ * from zero. Other shapes: FLA_ERR_UNSUPPORTED. The backward needs q, k, v and d_o only. No scratch. */
+int fla_sm100_taylor_fwd(const FlaArgs* args);
+int fla_sm100_taylor_bwd(const FlaArgs* args);
+
 /* Forward pass for callers that cannot obtain device memory themselves.
  * It has no counterpart in the reference (whose wrappers allocate through torch).
  *
