@@ -241,6 +241,41 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_
       : "memory");
 }
 
+// D[tmem] (+)= A[smem desc] * B[smem desc], issued by the lane whose `on` is set. The predicate sits on the
+// instruction and not on a branch around it: in a warp that stays converged the compiler can keep
+// descriptors and addresses in uniform registers, where the instruction wants them.
+__device__ __forceinline__ void mma_ss_on(bool on, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
+                                          uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 da, {%1, %3};\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(on))
+      : "memory");
+}
+__device__ __forceinline__ void mma_ts_on(bool on, uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi,
+                                          uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(static_cast<uint32_t>(on))
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_on(bool on, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+      "r"(static_cast<uint32_t>(on))
+      : "memory");
+}
+
 // Instruction descriptor for kind::f16 with 16-bit operands (bf16, or fp16 when `half`) and an
 // fp32 accumulator.
 __host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool a_mn_major, bool b_mn_major,
