@@ -22,7 +22,7 @@ LIB_PATH = os.path.join(HERE, LIB_NAME)
 
 SOURCES = ["fla_api.cu"]
 HOST_SOURCES = ["fla_host.cpp", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
-HEADERS = ["fla_kernel.cuh", "fla_wide_kernel.cuh", "fla_normalize.cuh", "fla_taylor.cuh", "fla_taylor_attention.cuh", "fla_decode.cuh", "ptx.cuh", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
+HEADERS = ["fla_kernel.cuh", "fla_backward.cuh", "fla_wide_kernel.cuh", "fla_normalize.cuh", "fla_taylor.cuh", "fla_taylor_attention.cuh", "fla_decode.cuh", "ptx.cuh", os.path.join("..", "..", "include", "flashlinear_sm100.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
