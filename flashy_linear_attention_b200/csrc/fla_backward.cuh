@@ -54,7 +54,7 @@ struct BwdCfg {
   // next chunk's tiles in the order of their first use, v, g, k, q, so a tile has a third of a chunk's time
   // or more to arrive. (A fifth slot, with the outputs staged in the states' copies while those are dead,
   // was slower: the copy of S then waits for dK to leave it, 1000 cycles a chunk.)
-  static constexpr int NSLOT = D == 128 ? 4 : 10;
+  static constexpr int NSLOT = D == 128 ? 4 : 8;
   static constexpr int STAGE_BYTES = D == 128 ? TILE_BYTES : 3 * kGroupBytes;  // D = 64: one stage per gradient
   static constexpr int BAR_BYTES = 512;
   static constexpr int SB_OFF = NSLOT * TILE_BYTES;
@@ -242,6 +242,7 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
     // ================================================================ TMA producers
     if (ptx::elect_one()) {
       const int part = warp == 0 ? 0 : 1;
+      constexpr bool kPrefetch = D == 128;
       constexpr int kPartBytes = cfg::TILE_BYTES / 2;
       const int part_col = cfg::G == 2 ? part * 64 : 0;
       const int part_row = cfg::G == 2 ? 0 : part * cfg::LOAD_ROWS;
@@ -258,6 +259,7 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
         ptx::mbar_expect_tx(full_bar(s), kPartBytes);
         if (!(p.debug_withhold && t == 0))
           ptx::tma_load_4d(slot_addr(s) + part * kPartBytes, map, full_bar(s), part_col, chunk * kChunk + part_row, h, b);
+        if (kPrefetch && !phase_a && i + 1 < n_iter) ptx::tma_prefetch_4d(map, part_col, (chunk - 1) * kChunk + part_row, h, b);
       }
     }
   } else if (warp == 1) {

@@ -55,7 +55,7 @@ def backward_kernel(n_iter, double, has_r, a_iter, to_final, wait_dv=True):
     m = Buffers()
     conv, state, epi = ["convA", "convB"], ["stateA", "stateB"], ["epi0", "epi1"]  # two warps stand for each group
     roles = ["prod0", "prod1", "X"] + conv + state + epi
-    nslot = 10 if double else 4
+    nslot = 8 if double else 4
     t0 = 2 * a_iter
     V, G, K, Q = range(4)
 
