@@ -149,8 +149,13 @@ struct Product {
   const float* ext_init;  // caller's running state, or null
   float* ext_final;
   int ext_trans;  // the caller's state arrays hold the transpose of the product's [da][dc] state
-  // Fused segmented launch only: segments g >= 1 store the state they start from ([bh][segments - 1]
-  // [da*dc], scratch layout) for the backward.
+  // Fused segmented launch only. With bound_base set, segment 0 starts from ext_init and segment
+  // g >= 1 from the stored boundary state (bound_slot0 - g * bound_step) of bound_base
+  // ([bh][bound_stride][da*dc], layout flag bound_trans relative to this product's state) instead
+  // of from the partial sums of the launch. bound_out: segments g >= 1 store the state they start
+  // from ([bh][segments - 1][da*dc], scratch layout) for a later call to use as bound_base.
+  const float* bound_base = nullptr;
+  int bound_stride = 0, bound_slot0 = 0, bound_step = 0, bound_trans = 0;
   float* bound_out = nullptr;
 };
 
@@ -615,7 +620,7 @@ bool split_pays(SplitForm form, int heads, int nseg, int nchunks, int width, boo
     case SplitForm::kForward:
       return wide ? 1.5 * n - 3.0 * per_seg > 13.0 : 1.14 * n - 1.8 * per_seg > 8.0;
     case SplitForm::kBackwardStates:
-      return wide ? 1.8 * n - 5.2 * per_seg > 13.0 : 1.17 * n - 2.8 * per_seg > 9.6;
+      return wide ? 1.8 * n - 2.9 * per_seg > 13.0 : 1.17 * n - 1.6 * per_seg > 9.6;
     case SplitForm::kBackward:
       if (square) return wide ? 1.68 * n - 3.4 * c > 12.5 + h : 1.15 * n - 1.85 * c > 8.2 + 0.25 * h;
       return wide ? 3.2 * n - 5.1 * c > 30.0 + 0.25 * h : 2.3 * n - 3.3 * c > 20.0 + 0.08 * h;
@@ -628,7 +633,8 @@ bool split_pays(SplitForm form, int heads, int nseg, int nchunks, int width, boo
 }
 
 int auto_segments(SplitForm form, int bh, int nchunks, int sm_count, int dk, int dv) {
-  const long ctas = (form == SplitForm::kBackward ? 3l : 1l) * bh;
+  const bool backward = form == SplitForm::kBackwardStates || form == SplitForm::kBackward;
+  const long ctas = (backward ? 3l : 1l) * bh;
   if (ctas * 4 >= static_cast<long>(sm_count) * 3) return 1;  // already >= 75 % of the SMs
   // One wave: as many segments as fit the SMs once (every CTA pays a fixed start-up cost, and the
   // state pass re-reads b and c, so more, shorter segments do not pay).
@@ -689,38 +695,35 @@ SegPlan forward_plan(const FlaArgs* a, int sm_count) {
   return p;
 }
 
-// Whether the pair of calls runs its backward as one launch of fla_backward_kernel, split at the
-// boundaries of the forward's segments `f`, from the states that the forward stores there.
-bool backward_split(const FlaArgs* a, int sm_count, SegPlan* f) {
-  if (a->dk != a->dv || a->dk > 128 || g_no_fused) return false;
-  const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk, bh = a->batch * a->heads;
-  if (!single_sweep_allowed(nchunks) || bh * 4 > sm_count) return false;
-  *f = forward_plan(a, sm_count);
-  if (f->nseg <= 1 || !split_pays(SplitForm::kBackwardStates, bh, f->nseg, nchunks, a->dk, true)) return false;
-  // the two CTAs of a head cut in two share the sum over its last segment: not with one chunk in it
-  const int last = nchunks - (f->nseg - 1) * f->seg_chunks;
-  return !(f->nseg == 2 && last < 2) && static_cast<long>(f->nseg) * bh <= sm_count && bh <= fla::kBarHeads;
+// Segments of a backward call (three products per head) whose boundaries are boundaries of the
+// forward plan `f`, so that the states the forward stored at its boundaries can start dQ's
+// segments. nseg = 1 when no such plan exists or the backward would not be split anyway.
+SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) {
+  const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
+  const int bh = a->batch * a->heads;
+  const SegPlan none = {1, nchunks};
+  const SegPlan base = make_plan(auto_segments(SplitForm::kBackwardStates, bh, nchunks, sm_count, a->dk, a->dv), nchunks);
+  if (base.nseg <= 1 || f.nseg <= 1 || nchunks % f.seg_chunks != 0) return none;
+  SegPlan b;
+  b.seg_chunks = (base.seg_chunks + f.seg_chunks - 1) / f.seg_chunks * f.seg_chunks;
+  b.nseg = (nchunks + b.seg_chunks - 1) / b.seg_chunks;
+  if (b.nseg <= 1 || 3l * b.nseg * bh > sm_count) return none;
+  return b;
 }
 
-// backward_split() for the queries, which know the debug bits of the call from its arguments only.
-bool planned_backward_split(const FlaArgs* a, SegPlan* f) {
-  if (a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0 || a->segment_states_ready) return false;
-  const int saved = g_no_fused, saved_force = g_force_single_sweep;
-  g_no_fused = (a->debug_flags & FLA_DEBUG_NO_FUSED_SEGMENTS) ? 1 : 0;
-  g_force_single_sweep = (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP) ? 1 : 0;
-  const bool split = backward_split(a, current_sm_count_early(), f);
-  g_no_fused = saved;
-  g_force_single_sweep = saved_force;
-  return split;
-}
-
-// Bytes of the boundary states that the forward stores for it, and of its scratch: one partial sum of
-// q^T dO per CTA.
-size_t boundary_states_bytes(const FlaArgs* a, const SegPlan& f) {
-  return static_cast<size_t>(f.nseg - 1) * a->batch * a->heads * scratch_state_elems(a->dk, a->dv) * sizeof(float);
-}
-size_t split_backward_ws_bytes(const FlaArgs* a, const SegPlan& f) {
-  return static_cast<size_t>(f.nseg) * a->batch * a->heads * scratch_state_elems(a->dk, a->dv) * sizeof(float);
+// Bytes of the boundary states a fused forward stores for a fused backward, or 0 when the pair of
+// calls does not run that way for these shapes.
+size_t seg_states_bytes(const FlaArgs* a, int sm_count, SegPlan* fwd_out, SegPlan* bwd_out) {
+  if (a->dk != a->dv || a->dk > 128 || g_no_fused) return 0;
+  if (!single_sweep_allowed((a->seqlen + fla::kChunk - 1) / fla::kChunk)) return 0;
+  const int bh = a->batch * a->heads;
+  const SegPlan f = forward_plan(a, sm_count);
+  if (f.nseg <= 1 || static_cast<long>(f.nseg) * bh > sm_count || bh > fla::kBarHeads) return 0;
+  const SegPlan b = backward_aligned_plan(a, sm_count, f);
+  if (b.nseg <= 1) return 0;
+  if (fwd_out) *fwd_out = f;
+  if (bwd_out) *bwd_out = b;
+  return static_cast<size_t>(f.nseg - 1) * bh * scratch_state_elems(a->dk, a->dv) * sizeof(float);
 }
 
 template <int D>
@@ -786,29 +789,6 @@ int launch_fused(int tmpl, const KernelParams& kp, dim3 grid, cudaStream_t strea
   if (tmpl == 64) return launch_fused_kernel<64>(kp, grid, stream);
   if (tmpl == 128) return launch_fused_kernel<128>(kp, grid, stream);
   return FLA_ERR_UNSUPPORTED;
-}
-
-template <int D, bool HALF>
-int launch_backward(const fla::BackwardParams& p, int nseg, int bh, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(1, nseg, bh);
-  cfg.blockDim = dim3(fla::kBwdThreads, 1, 1);
-  cfg.dynamicSmemBytes = fla::BwdCfg<D>::SMEM_BYTES;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  memset(&attr, 0, sizeof(attr));
-  attr.id = cudaLaunchAttributeCooperative;
-  attr.val.cooperative = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = p.fused ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, fla::fla_backward_kernel<D, HALF>, p);
-  ++g_last_launches;
-  if (e != cudaSuccess) {
-    FLA_LOG_FAILURE("launch of fla_backward_kernel<%d> grid (1,%d,%d) failed: %s", D, nseg, bh, cudaGetErrorString(e));
-    (void)cudaGetLastError();
-  }
-  return e == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
 }
 
 // What the kernel's NORM variant takes beside the product, see KernelParams.
@@ -899,25 +879,67 @@ int run_products(const Product* prods, int nprob, int B, int H, int N, int da, i
   if (norm != nullptr) return FLA_ERR_UNSUPPORTED;
 
   float* ws = static_cast<float*>(workspace);
-  // Everything fits the GPU at once: ONE cooperative launch in which every CTA sums its share of
-  // its segment (phase A), the CTAs of a head meet at a barrier, and each then starts the attention
-  // loop from the sum of the partials of the earlier segments. The three-launch form below pays
-  // the pipeline fill and drain of a launch three times and reads b, c once more from HBM.
-  // (Gradients have states of their own: they are split by fla_backward_kernel, or in three launches.)
-  if (!g_no_fused && nprob == 1 && static_cast<long>(nseg) * bh <= dev.sm_count && bh <= fla::kBarHeads) {
-    Problem& pr = kp.prob[0];
-    const Product& pd = prods[0];
-    pr.s_add = pd.ext_init;
-    pr.add_trans = pd.ext_trans;
-    pr.s_final = pd.ext_final;   // written by the last segment's CTA
-    pr.st_trans = pd.ext_trans;
-    pr.init_kind = fla::kInitParts;
-    pr.init_base = ws;
-    pr.bound_out = pd.bound_out;
+  // The fused form sums ONE state per (head, segment). Products that start from the partial sums
+  // must therefore all carry that state or its transpose (dV and dK: q^T dO and dO^T q) and walk
+  // the sequence in the same direction; a product with another state (dQ: v^T k) can only ride
+  // along when its starting states come from stored boundary states.
+  bool fusable = !g_no_fused && static_cast<long>(nprob) * nseg * bh <= dev.sm_count && bh <= fla::kBarHeads;
+  {
+    const Product* first = nullptr;
+    for (int i = 0; i < nprob && fusable; ++i) {
+      const Product& pd = prods[i];
+      if (pd.bound_base != nullptr) continue;
+      if (first == nullptr) {
+        first = &pd;
+        continue;
+      }
+      const bool same = pd.b.ptr == first->b.ptr && pd.c.ptr == first->c.ptr && pd.ext_trans == first->ext_trans;
+      const bool swapped = pd.b.ptr == first->c.ptr && pd.c.ptr == first->b.ptr && pd.ext_trans != first->ext_trans;
+      const bool same_dir = ((pd.flags ^ first->flags) & fla::kFlagDescending) == 0;
+      if (!(same || swapped) || !same_dir || da != dc) fusable = false;
+    }
+    if (first == nullptr) fusable = false;
+  }
+  if (fusable) {
+    // Everything fits the GPU at once: ONE cooperative launch in which every CTA sums its share of
+    // its segment (phase A), all CTAs meet at a grid barrier, and each then starts the attention
+    // loop from the sum of the partials of the earlier segments. The three-launch form below pays
+    // the pipeline fill and drain of a launch three times and reads b, c once more from HBM.
+    int pre = 0;
+    for (int i = 0; i < nprob; ++i) {
+      Problem& pr = kp.prob[i];
+      const Product& pd = prods[i];
+      pr.s_init = nullptr;
+      pr.s_add = pd.ext_init;
+      pr.add_trans = pd.ext_trans;
+      pr.s_final = pd.ext_final;   // written by the last segment's CTA
+      pr.st_trans = pd.ext_trans;
+      if (pd.bound_base != nullptr) {
+        pr.init_kind = fla::kInitBound;
+        pr.init_base = pd.bound_base;
+        pr.init_trans = pd.bound_trans;
+        pr.init_stride = pd.bound_stride;
+        pr.bound_slot0 = pd.bound_slot0;
+        pr.bound_step = pd.bound_step;
+      } else {
+        pr.init_kind = fla::kInitParts;
+        pr.init_base = ws;
+        // The partials hold the state of problem `pre` in the scratch layout; a problem whose own
+        // state is the transpose of that one (dK beside dV) reads them the other way round.
+        pre = i;
+      }
+      pr.bound_out = pd.bound_out;
+    }
+    // `pre`: the (last) problem that starts from partial sums; its b, c operands and direction
+    // define phase A. Problems with the transposed state read the partials transposed.
+    for (int i = 0; i < nprob; ++i)
+      if (kp.prob[i].init_kind == fla::kInitParts)
+        kp.prob[i].init_trans = (prods[i].ext_trans == prods[pre].ext_trans) ? 1 : 0;
     kp.mode = 0;
     kp.fused = 1;
+    kp.pre_prob = pre;
     kp.part_out = ws;
-    return launch_fused(tmpl, kp, dim3(1, nseg, bh), stream);
+    return launch_fused(tmpl, kp, dim3(nprob, nseg, bh), stream);
   }
   // Pass A: per-segment sums of b^T c into the workspace (the last segment only when a final
   // state is wanted), exclusive scan over segments, then pass B with per-segment initial states.
@@ -1225,61 +1247,53 @@ void backward_products(const FlaArgs* a, Product* pq, Product* pv, Product* pk) 
   pk->ext_trans = 1;
 }
 
-// One CTA a head (nseg 1) or a head and segment: fla_backward_kernel. Needs s_last; with segments also
-// the forward's boundary states.
-int run_backward(const FlaArgs* a, const SegPlan& plan, cudaStream_t stream) {
-  const int B = a->batch, H = a->heads, N = a->seqlen, bh = B * H;
+// The three gradients of a head in one CTA: fla_backward_kernel. Needs s_last.
+int run_backward(const FlaArgs* a, cudaStream_t stream) {
+  const int B = a->batch, H = a->heads, N = a->seqlen;
   const int tmpl = pick_template(a->dk, a->dv);
   fla::BackwardParams p;
   memset(&p, 0, sizeof(p));
   struct Map {
     CUtensorMap* map;
     const FlaTensor& t;
-    int dim, rows;
+    int rows;
   };
   const int rows = load_rows(tmpl);
-  const Map maps[7] = {{&p.q, a->q, a->dk, rows},   {&p.k, a->k, a->dk, rows},   {&p.v, a->v, a->dv, rows}, {&p.g, a->d_o, a->dv, rows},
-                       {&p.dq, a->d_q, a->dk, 32}, {&p.dk, a->d_k, a->dk, 32}, {&p.dv, a->d_v, a->dv, 32}};
+  const Map maps[7] = {{&p.q, a->q, rows}, {&p.k, a->k, rows}, {&p.v, a->v, rows}, {&p.g, a->d_o, rows},
+                       {&p.dq, a->d_q, 32}, {&p.dk, a->d_k, 32}, {&p.dv, a->d_v, 32}};
   for (const Map& m : maps) {
-    const Operand o = operand(m.t, m.dim);
+    const Operand o = operand(m.t, a->dk);
     int rc;
     if ((rc = check_operand(o, B, H)) || (rc = encode_map(m.map, o, B, H, N, m.rows))) return rc;
   }
-  p.seg_chunks = plan.seg_chunks;
-  p.st_rows = a->dk;
-  p.st_cols = a->dv;
+  p.s_last = a->s_last;
+  p.r_init = a->r_init;
+  p.r_final = a->r_final;
+  p.dim = a->dk;
+  p.first_exact = a->s_init == nullptr ? 1 : 0;
   p.heads = H;
   p.nchunks = (N + fla::kChunk - 1) / fla::kChunk;
   p.n_tokens = N;
-  p.first_exact = a->s_init == nullptr ? 1 : 0;
-  p.r_final = a->r_final;
   p.status = a->status;
   p.wait_limit_us = g_wait_limit_us;
   p.debug_withhold = g_debug_withhold;
-  if (plan.nseg > 1) {
-    if (a->workspace == nullptr || a->workspace_bytes < split_backward_ws_bytes(a, plan)) return FLA_ERR_WORKSPACE;
-    p.fused = 1;
-    p.part_out = static_cast<float*>(a->workspace);
-    p.bar_slot = g_next_barrier_slot.fetch_add(1, std::memory_order_relaxed) % fla::kGridBarSlots;
-    p.r.init_kind = fla::kInitParts;
-    p.r.init_base = p.part_out;
-    p.r.s_add = a->r_init;
-    p.s.init_kind = fla::kInitBound;
-    p.s.init_base = static_cast<const float*>(a->seg_states);
-    p.s.init_stride = plan.nseg - 1;
-    p.s.bound_slot0 = plan.nseg - 1;  // the forward's segment nseg - g starts where segment g ends
-    p.s.s_add = a->s_last;
+  const dim3 grid(1, 1, B * H);
+  if (tmpl == 64) {
+    if (g_half) fla::fla_backward_kernel<64, true><<<grid, fla::kBwdThreads, fla::BwdCfg<64>::SMEM_BYTES, stream>>>(p);
+    else fla::fla_backward_kernel<64, false><<<grid, fla::kBwdThreads, fla::BwdCfg<64>::SMEM_BYTES, stream>>>(p);
   } else {
-    p.r.s_init = a->r_init;
-    p.s.s_init = a->s_last;
+    if (g_half) fla::fla_backward_kernel<128, true><<<grid, fla::kBwdThreads, fla::BwdCfg<128>::SMEM_BYTES, stream>>>(p);
+    else fla::fla_backward_kernel<128, false><<<grid, fla::kBwdThreads, fla::BwdCfg<128>::SMEM_BYTES, stream>>>(p);
   }
-  if (tmpl == 64)
-    return g_half ? launch_backward<64, true>(p, plan.nseg, bh, stream) : launch_backward<64, false>(p, plan.nseg, bh, stream);
-  return g_half ? launch_backward<128, true>(p, plan.nseg, bh, stream) : launch_backward<128, false>(p, plan.nseg, bh, stream);
+  ++g_last_launches;
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) FLA_LOG_FAILURE("launch of fla_backward_kernel<%d>, %d heads, failed: %s", tmpl, B * H, cudaGetErrorString(e));
+  return e == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
 }
 
-bool one_cta_backward_pays(int heads, int sm_count) {
+bool one_cta_backward_pays(int heads, int sm_count, int dim) {
   if (const char* e = getenv("FLA_ONE_CTA")) return atoi(e) != 0;
+  (void)dim;
   return heads > 2 * sm_count / 3;
 }
 
@@ -1336,9 +1350,7 @@ int fla_sm100_auto_segments(const FlaArgs* a, int pass) {
   if (pass == 0) return count(a->segment_states_ready ? SplitForm::kState : SplitForm::kForward);
   if (pass == 1) {
     const int n = count(SplitForm::kBackward);
-    SegPlan f;
-    // counted in threes of CTAs, as for the form that gives each gradient a CTA of its own
-    return planned_backward_split(a, &f) ? std::max(n, std::max(2, (f.nseg + 2) / 3)) : n;
+    return fla_sm100_seg_states_bytes(a) > 0 ? std::max(n, count(SplitForm::kBackwardStates)) : n;
   }
   return std::max(count(SplitForm::kState), count(SplitForm::kStateOnly));
 }
@@ -1348,19 +1360,22 @@ size_t fla_sm100_workspace_bytes(const FlaArgs* a, int pass) {
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   int nseg = fla_sm100_auto_segments(a, pass);
   if (nseg > nchunks) nseg = nchunks;
-  size_t split = 0;  // of a backward that starts from the forward's boundary states
-  SegPlan f;
-  if (pass == 1 && planned_backward_split(a, &f)) split = split_backward_ws_bytes(a, f);
-  if (nseg <= 1) return split > 0 ? split + 1024 : 0;
+  if (nseg <= 1) return 0;
   const int seg_chunks = (nchunks + nseg - 1) / nseg;
   nseg = (nchunks + seg_chunks - 1) / seg_chunks;
-  return std::max(split, segment_ws_bytes(pass == 1 ? 3 : 1, a->batch * a->heads, nseg, a->dk, a->dv)) + 1024;
+  return segment_ws_bytes(pass == 1 ? 3 : 1, a->batch * a->heads, nseg, a->dk, a->dv) + 1024;
 }
 
 size_t fla_sm100_seg_states_bytes(const FlaArgs* a) {
-  if (a == nullptr) return 0;
-  SegPlan f;
-  return planned_backward_split(a, &f) ? boundary_states_bytes(a, f) : 0;
+  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0) return 0;
+  if (a->segment_states_ready) return 0;
+  const int saved = g_no_fused, saved_force = g_force_single_sweep;
+  g_no_fused = (a->debug_flags & FLA_DEBUG_NO_FUSED_SEGMENTS) ? 1 : 0;
+  g_force_single_sweep = (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP) ? 1 : 0;
+  const size_t n = seg_states_bytes(a, current_sm_count_early(), nullptr, nullptr);
+  g_no_fused = saved;
+  g_force_single_sweep = saved_force;
+  return n;
 }
 
 int fla_sm100_bwd_uses_final_state(const FlaArgs* a) {
@@ -1394,11 +1409,12 @@ int fla_sm100_fwd(const FlaArgs* a) {
     return run_wide_any(p, a->batch, a->heads, a->seqlen, a->dk, a->dv, a->status,
                         static_cast<cudaStream_t>(a->stream), *dev);
   if (a->seg_states != nullptr && a->segment_states_ready == 0) {
-    SegPlan f;
-    if (backward_split(a, dev->sm_count, &f)) {
-      if (a->seg_states_bytes < boundary_states_bytes(a, f)) return FLA_ERR_WORKSPACE;
+    SegPlan f, b;
+    const size_t need = seg_states_bytes(a, dev->sm_count, &f, &b);
+    if (need > 0) {
+      if (a->seg_states_bytes < need) return FLA_ERR_WORKSPACE;
       p.bound_out = static_cast<float*>(a->seg_states);
-      // the segments the backward is split into
+      // the segments the backward's plan was made for
       return run_products(&p, 1, a->batch, a->heads, a->seqlen, a->dk, a->dv, f.nseg, a->workspace,
                           a->workspace_bytes, a->status, static_cast<cudaStream_t>(a->stream), *dev,
                           false, f.seg_chunks);
@@ -1440,20 +1456,33 @@ int fla_sm100_bwd(const FlaArgs* a) {
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   if (a->seg_states != nullptr && a->s_last != nullptr && single_sweep_allowed(nchunks)) {
     // Few heads: the forward ran as one fused segmented launch and stored the state at each of
-    // its segment boundaries. S of a segment starts from the state stored at its end, R from the partial
-    // sums of q^T dO that the same launch forms first.
-    SegPlan f;
-    if (backward_split(a, dev->sm_count, &f)) {
-      if (a->seg_states_bytes < boundary_states_bytes(a, f)) return FLA_ERR_WORKSPACE;
-      return run_backward(a, f, stream);
+    // its segment boundaries. The backward is split at a subset of those boundaries; dQ walks every
+    // segment end-to-start from the stored state at the segment's end (total minus suffix, as in
+    // the unsegmented case), dV and dK start from the partial sums of q^T dO that the same launch
+    // forms first. One launch, and the three products of a (head, segment) stream the same chunks.
+    SegPlan f, bp;
+    const size_t need = seg_states_bytes(a, dev->sm_count, &f, &bp);
+    if (need > 0) {
+      if (a->seg_states_bytes < need) return FLA_ERR_WORKSPACE;
+      pq.flags = fla::kFlagDescending | fla::kFlagTotalMinusSuffix;
+      if (a->s_init == nullptr) pq.flags |= fla::kFlagFirstChunkExact;
+      pq.ext_init = a->s_last;  // segment 0 of the descending walk: the end of the sequence
+      pq.bound_base = static_cast<const float*>(a->seg_states);
+      pq.bound_trans = 1;       // the forward stored S^T, which is this product's own state
+      pq.bound_stride = f.nseg - 1;
+      pq.bound_slot0 = nchunks / f.seg_chunks - 1;
+      pq.bound_step = bp.seg_chunks / f.seg_chunks;
+      Product all[3] = {pq, pv, pk};
+      return run_products(all, 3, a->batch, a->heads, a->seqlen, a->dk, a->dv, bp.nseg, a->workspace,
+                          a->workspace_bytes, a->status, stream, *dev, false, bp.seg_chunks);
     }
   }
   int nseg = a->segments > 0 ? a->segments
                              : auto_segments(SplitForm::kBackward, a->batch * a->heads, nchunks, dev->sm_count, a->dk, a->dv);
   if (nseg > nchunks) nseg = nchunks;
   if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks) && a->dk == a->dv &&
-      one_cta_backward_pays(a->batch * a->heads, dev->sm_count))
-    return run_backward(a, SegPlan{1, nchunks}, stream);
+      one_cta_backward_pays(a->batch * a->heads, dev->sm_count, a->dk))
+    return run_backward(a, stream);
   if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks)) {
     // The forward state after this call's tokens is known: dQ can walk the sequence in the same
     // descending order as dV and dK (state = total minus suffix), so the three products of a

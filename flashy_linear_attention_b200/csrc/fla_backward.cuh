@@ -1,5 +1,5 @@
-// All three gradients of causal linear attention (dk = dv <= 128) in one sweep of one CTA per head (or
-// per head and sequence segment), for sm_100a. Replaces flashlinear/kernels/linear_attn_kernels.py:103-307.
+// All three gradients of causal linear attention (dk = dv <= 128) in one sweep of one CTA per head, for
+// sm_100a. Replaces flashlinear/kernels/linear_attn_kernels.py:103-307 where there are heads enough.
 //
 // fla_kernel.cuh computes the gradients as three products, each in a CTA of its own: together they load
 // nine tiles a chunk, write three and run twelve MMA groups. Here one CTA walks the chunks from the last to the
@@ -20,7 +20,7 @@
 //   warps 0, 18   TMA producers, each half of every tile (see fla_kernel.cuh)
 //   warp 1        MMA issuer (one elected lane) and TMEM owner
 //   warps 2-9     converters of the scores: fp32 -> mask -> 16 bits, in place (TMEM); before the loop, the
-//                 states at the start (converter_prologue)
+//                 states at the start
 //   warps 10-13   epilogue: accumulator -> 16 bits -> staging -> TMA store
 //   warps 14-17   converters of the states: fp32 (TMEM) -> 16 bits (shared memory). With one group for scores
 //                 and states its five conversions a chunk, one behind the other, were the chunk period.
@@ -29,11 +29,14 @@
 
 namespace fla {
 
-struct BackwardParams : SegmentGeometry {
+struct BackwardParams {
   CUtensorMap q, k, v, g;     // 4-D maps, boxes as in Problem
   CUtensorMap dq, dk, dv;     // boxes of 64 columns x 32 rows
-  StateSource r, s;           // what R and S start from
-  float* r_final;             // [bh][st_rows][st_cols], optional: R including this call's tokens
+  // states, fp32 [bh][dk][dk]: S after this call's tokens; R before them (null: zero); R including them (or null)
+  const float* s_last;
+  const float* r_init;
+  float* r_final;
+  int dim;                    // dk
   int first_exact;            // nothing precedes token 0: the first chunk's S is zero, and is not used
   int heads, nchunks, n_tokens;
   int* status;                // see KernelParams
@@ -60,10 +63,13 @@ struct BwdCfg {
   static constexpr int SB_OFF = NSLOT * TILE_BYTES;
   static constexpr int RB_OFF = SB_OFF + STATE_BYTES;
   static constexpr int STAGE_OFF = RB_OFF + STATE_BYTES;
+  // 32 KB for the transposes of the states at the start (and, four warps, of R at the end): the stage
+  static constexpr int SCRATCH_OFF = STAGE_OFF;
+  static_assert(STAGE_BYTES >= 8 * 4096, "scratch of load_state()");
   static constexpr int BAR_OFF = STAGE_OFF + STAGE_BYTES;
   static constexpr int SMEM_BYTES = 1024 + BAR_OFF + BAR_BYTES;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-  static constexpr int NBARS = 2 * NSLOT + 17;
+  static constexpr int NBARS = 2 * NSLOT + 15;
   static_assert(NBARS * 8 + 16 <= BAR_BYTES, "barrier area");
   // tensor memory columns: fp32 scores, 128 each (their 16-bit form replaces each half in place), output
   // accumulators and states. D = 64 leaves room for two score tiles and two accumulators.
@@ -77,7 +83,7 @@ struct BwdCfg {
 // R -> the caller's array, a state-converter warp's 32 rows, at D = 128 through a 32 x 32 transpose in
 // `scratch` (4 KB a warp) so that global stores are whole 128-byte row segments. Out of line: once a CTA.
 template <int D>
-__device__ __noinline__ void write_final_rows(float* dst, int st_rows, int st_cols, uint32_t state, uint32_t scratch, int quad) {
+__device__ __noinline__ void write_final_rows(float* dst, int dim, uint32_t state, uint32_t scratch, int quad) {
   const int lane = static_cast<int>(threadIdx.x & 31), row = quad * 32 + lane;
   uint32_t r[32];
 #pragma unroll 1
@@ -92,13 +98,13 @@ __device__ __noinline__ void write_final_rows(float* dst, int st_rows, int st_co
       for (int rr = 0; rr < 32; ++rr) {
         const int grow = quad * 32 + rr;
         const uint32_t x = ptx::ld_shared_b32(scratch + (lane * 32 + (rr ^ lane)) * 4);
-        if (grow < st_rows && col < st_cols) dst[static_cast<size_t>(grow) * st_cols + col] = __uint_as_float(x);
+        if (grow < dim && col < dim) dst[static_cast<size_t>(grow) * dim + col] = __uint_as_float(x);
       }
       __syncwarp();
-    } else if (row < st_rows) {
+    } else if (row < dim) {
 #pragma unroll
       for (int j = 0; j < 32; ++j)
-        if (cb * 32 + j < st_cols) dst[static_cast<size_t>(row) * st_cols + cb * 32 + j] = __uint_as_float(r[j]);
+        if (cb * 32 + j < dim) dst[static_cast<size_t>(row) * dim + cb * 32 + j] = __uint_as_float(r[j]);
     }
   }
 }
@@ -122,6 +128,46 @@ __device__ __forceinline__ void issue_group(uint32_t d, Walk a, Walk b, uint32_t
   }
 }
 
+// A state at the start -> tensor memory (fp32, `state`: this warp's lane quadrant) and, with `copy`, the 16-bit
+// operand copy. A warp moves its 32 rows and half of the columns, in 32 x 32 blocks through `scratch` (4 KB a
+// warp), so that global loads are whole 128-byte row segments; what lies beyond dim x dim is zero. Out of
+// line: once or twice a CTA.
+template <int D, bool HALF>
+__device__ __noinline__ void load_state(const float* src, int dim, uint32_t state, uint32_t copy, uint32_t scratch, int quad, int half) {
+  const int lane = static_cast<int>(threadIdx.x & 31), row = quad * 32 + lane;
+  uint32_t r[32];
+#pragma unroll 1
+  for (int jb = 0; jb < D / 64; ++jb) {
+    const int cb = half * (D / 64) + jb, col = cb * 32 + lane;
+#pragma unroll
+    for (int rr = 0; rr < 32; ++rr) {
+      const int grow = quad * 32 + rr;
+      const bool valid = grow < dim && col < dim;
+      r[rr] = ptx::ld_global_cg_b32(src + (valid ? static_cast<size_t>(grow) * dim + col : 0));
+      r[rr] = valid ? r[rr] : 0u;
+    }
+#pragma unroll
+    for (int rr = 0; rr < 32; ++rr) ptx::st_shared_b32(scratch + (lane * 32 + (rr ^ lane)) * 4, r[rr]);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = ptx::ld_shared_b32(scratch + (j * 32 + (lane ^ j)) * 4);
+    __syncwarp();
+    ptx::tmem_st32(state + cb * 32, r);
+    if (copy != 0 && row < D) {
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj)
+        ptx::st_shared_v4(copy + (cb >> 1) * (D * 128) + row * 128 + ((((cb & 1) * 4 + jj) ^ (row & 7)) << 4),
+                          ptx::pack16x2<HALF>(__uint_as_float(r[jj * 8 + 0]), __uint_as_float(r[jj * 8 + 1])),
+                          ptx::pack16x2<HALF>(__uint_as_float(r[jj * 8 + 2]), __uint_as_float(r[jj * 8 + 3])),
+                          ptx::pack16x2<HALF>(__uint_as_float(r[jj * 8 + 4]), __uint_as_float(r[jj * 8 + 5])),
+                          ptx::pack16x2<HALF>(__uint_as_float(r[jj * 8 + 6]), __uint_as_float(r[jj * 8 + 7])));
+    }
+  }
+  ptx::tc_wait_st();
+  ptx::fence_proxy_async_smem();
+  ptx::tc_fence_before();
+}
+
 template <int D, bool HALF>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 fla_backward_kernel(const __grid_constant__ BackwardParams p) {
@@ -131,8 +177,6 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // provably warp-uniform
   const int lane = threadIdx.x & 31;
-  const int g = blockIdx.y;
-  const int nseg = gridDim.y;
   const int bh = blockIdx.z;
   const int h = bh % p.heads, b = bh / p.heads;
 
@@ -155,31 +199,13 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
   const uint32_t r_full = bar(10);    // R including this chunk is complete
   const uint32_t rb_ready = bar(11);  // and its 16-bit copy written (128)
   const uint32_t s_loaded = bar(12), r_loaded = bar(13);  // S, R at the start are in tensor memory (256)
-  const uint32_t part_done = bar(14), grid_done = bar(15);  // see converter_prologue()
-  const uint32_t drained = bar(16);   // everything the issuer issued has completed
+  const uint32_t drained = bar(14);   // everything the issuer issued has completed
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem_gen + cfg::BAR_OFF + cfg::NBARS * 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + cfg::BAR_OFF + cfg::NBARS * 8 + 4);
 
-  // Segments in scan order run from the end of the sequence; the one that is shorter than the others, if
-  // any, is the first of them, so that the boundaries are those of the forward, which counts from token 0.
-  const bool fused = p.fused != 0;
-  const int seg_lo = (nseg - 1 - g) * p.seg_chunks;  // first chunk in memory
-  const int n_iter = min(p.nchunks, seg_lo + p.seg_chunks) - seg_lo;
-  auto mem_chunk = [&](int i) { return seg_lo + n_iter - 1 - i; };
-  // Phase A of the fused form (see SegmentGeometry): chunks a_lo .. a_lo + a_iter - 1 of the sequence
-  int a_lo = 0, a_iter = 0;
-  if (fused && nseg > 1) {
-    const int shares = nseg / (nseg - 1);  // 2 for two segments, otherwise 1
-    if (g < shares * (nseg - 1)) {
-      const int sa = g / shares, xa = g - sa * shares;
-      const int lo = (nseg - 1 - sa) * p.seg_chunks;
-      const int len = min(p.nchunks, lo + p.seg_chunks) - lo;
-      a_lo = lo + len * xa / shares;
-      a_iter = lo + len * (xa + 1) / shares - a_lo;
-    }
-  }
-  const int t0 = 2 * a_iter;  // tiles of phase A (q, g) come first in the ring numbering
-  const bool has_r = fused || p.r.s_init != nullptr;  // R does not start from zero
+  const int n_iter = p.nchunks;
+  auto mem_chunk = [&](int i) { return n_iter - 1 - i; };
+  const bool has_r = p.r_init != nullptr;  // R does not start from zero
 
   // ------------------------------------------------------------------ setup
   if (threadIdx.x == 0) {
@@ -201,8 +227,6 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
     ptx::mbar_init(rb_ready, 128);
     ptx::mbar_init(s_loaded, 256);
     ptx::mbar_init(r_loaded, 256);
-    ptx::mbar_init(part_done, 256);
-    ptx::mbar_init(grid_done, 1);
     ptx::mbar_init(drained, 1);
     ptx::fence_barrier_init();
     ptx::fence_proxy_async_smem();
@@ -231,35 +255,32 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
     if (up) ptx::tc_fence_after();
     return up;
   };
-  // Tiles: phase A's are counted t = 0 .. t0 - 1 in ring order; chunk i then has v, g, k, q (w = 0 .. 3), at
-  // D = 64 further along the ring, at D = 128 in the slots in turn. use(): how often the slot was filled before.
+  // Chunk i has tiles v, g, k, q (w = 0 .. 3), in the order of their first use: at D = 64 along the ring, at
+  // D = 128 in the slots in turn. use(): how often the slot was filled before.
   constexpr int V = 0, G = 1, K = 2, Q = 3;
-  auto slot_of = [&](int i, int w) { return cfg::DOUBLE ? (t0 + 4 * i + w) % NSLOT : (w - i) & 3; };
-  auto use_of = [&](int i, int w) { return cfg::DOUBLE ? (t0 + 4 * i + w) / NSLOT : ((t0 + 3 - slot_of(i, w)) >> 2) + i; };
+  auto slot_of = [&](int i, int w) { return cfg::DOUBLE ? (4 * i + w) % NSLOT : (w - i) & 3; };
+  auto use_of = [&](int i, int w) { return cfg::DOUBLE ? (4 * i + w) / NSLOT : i; };
   auto slot_addr = [&](int s) { return smem_base + static_cast<uint32_t>(s) * cfg::TILE_BYTES; };
 
   if (warp == 0 || warp == 18) {
     // ================================================================ TMA producers
     if (ptx::elect_one()) {
       const int part = warp == 0 ? 0 : 1;
-      constexpr bool kPrefetch = D == 128;
       constexpr int kPartBytes = cfg::TILE_BYTES / 2;
       const int part_col = cfg::G == 2 ? part * 64 : 0;
       const int part_row = cfg::G == 2 ? 0 : part * cfg::LOAD_ROWS;
-      const int n_tiles = t0 + 4 * n_iter;
-      for (int t = 0; t < n_tiles; ++t) {
-        const bool phase_a = t < t0;
-        const int i = (t - t0) >> 2;
-        const int w = phase_a ? ((t & 1) ? G : Q) : ((t - t0) & 3);
-        const int s = phase_a ? t % NSLOT : slot_of(i, w);
-        const int use = phase_a ? t / NSLOT : use_of(i, w);
-        if (!ptx::mbar_wait(empty_bar(s), (use & 1) ^ 1u, abort_flag)) break;
-        const int chunk = phase_a ? a_lo + (t >> 1) : mem_chunk(i);
+      for (int t = 0; t < 4 * n_iter; ++t) {
+        const int i = t >> 2, w = t & 3;
+        const int s = slot_of(i, w);
+        if (!ptx::mbar_wait(empty_bar(s), (use_of(i, w) & 1) ^ 1u, abort_flag)) break;
+        const int tok = mem_chunk(i) * kChunk + part_row;
         const CUtensorMap* map = w == V ? &p.v : w == G ? &p.g : w == K ? &p.k : &p.q;
         ptx::mbar_expect_tx(full_bar(s), kPartBytes);
         if (!(p.debug_withhold && t == 0))
-          ptx::tma_load_4d(slot_addr(s) + part * kPartBytes, map, full_bar(s), part_col, chunk * kChunk + part_row, h, b);
-        if (kPrefetch && !phase_a && i + 1 < n_iter) ptx::tma_prefetch_4d(map, part_col, (chunk - 1) * kChunk + part_row, h, b);
+          ptx::tma_load_4d(slot_addr(s) + part * kPartBytes, map, full_bar(s), part_col, tok, h, b);
+        // At D = 128 a slot is free only shortly before its tile is wanted: the tile after that comes into L2
+        // now. (128 heads x 8192: 396 us without, 376 with; at D = 64, two chunks deep, no difference.)
+        if (D == 128 && i + 1 < n_iter) ptx::tma_prefetch_4d(map, part_col, tok - kChunk, h, b);
       }
     }
   } else if (warp == 1) {
@@ -298,18 +319,7 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       commit(o_full(n));
     };
 
-    bool ok = true;
-    for (int i = 0; ok && i < a_iter; ++i) {  // phase A: R of this CTA's share
-      const int sq = (2 * i) % NSLOT, sg = (2 * i + 1) % NSLOT;
-      ok = wait(full_bar(sq), (2 * i / NSLOT) & 1) && wait(full_bar(sg), ((2 * i + 1) / NSLOT) & 1);
-      if (!ok) break;
-      ptx::tc_fence_after();
-      state_add(tR, slot_addr(sq), slot_addr(sg), IDESC_ADD, i > 0);
-      commit(empty_bar(sq));
-      commit(empty_bar(sg));
-      if (i == a_iter - 1) commit(r_full);
-    }
-    ok = ok && wait(s_loaded, 0);
+    bool ok = wait(s_loaded, 0);
     auto tile = [&](int i, int w) { return slot_addr(slot_of(i, w)); };
     auto wait_tile = [&](int i, int w) { return wait(full_bar(slot_of(i, w)), use_of(i, w) & 1); };
     auto release = [&](int i, int w) { commit(empty_bar(slot_of(i, w))); };
@@ -347,7 +357,7 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       const int n = 3 * i;
       const bool have_r = i > 0 || has_r;
       const bool use_s = !(p.first_exact && mem_chunk(i) == 0);
-      const bool want_r = i + 1 < n_iter || (p.r_final != nullptr && g == nseg - 1);
+      const bool want_r = i + 1 < n_iter || p.r_final != nullptr;
       // ---- dK
       if (!(cfg::DOUBLE ? scores_v(i) : scores_k(i))) break;
       // S -= k^T v. The converters read the previous S before sb_ready, which was waited for.
@@ -394,29 +404,19 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
     const int half = (warp - 2) >> 2;  // column half this group owns
     const int quad = warp & 3;         // TMEM lane quadrant this warp may access
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    PrologueArgs pa;
-    pa.g = g;
-    pa.nseg = nseg;
-    pa.bh = bh;
-    pa.a_iter = a_iter;
-    pa.state = tmem_base + cfg::S_COL;
-    pa.sb_addr = 0;
-    pa.ost_addr = smem_base + cfg::STAGE_OFF;  // (D = 128) nothing is staged yet
-    pa.s_full = r_full;
-    pa.part_done = part_done;
-    pa.grid_done = grid_done;
-    pa.ready = s_loaded;
-    pa.meet = false;
-    pa.abort_flag = abort_flag;
-    bool ok = converter_prologue<D, D, HALF>(p, p.s, pa);
-    pa.state = tmem_base + cfg::R_COL;
-    pa.sb_addr = rb_addr;
-    pa.ready = r_loaded;
-    pa.meet = true;
-    if (has_r) ok = converter_prologue<D, D, HALF>(p, p.r, pa) && ok;
-
+    {
+      // (transposes go through the stage: nothing is staged before both states are in place)
+      const size_t offset = static_cast<size_t>(bh) * p.dim * p.dim;
+      const uint32_t scratch = smem_base + cfg::SCRATCH_OFF + static_cast<uint32_t>(warp - 2) * 4096u;
+      load_state<D, HALF>(p.s_last + offset, p.dim, lane_base + cfg::S_COL, 0u, scratch, quad, half);
+      ptx::mbar_arrive(s_loaded);
+      if (has_r) {
+        load_state<D, HALF>(p.r_init + offset, p.dim, lane_base + cfg::R_COL, rb_addr, scratch, quad, half);
+        ptx::mbar_arrive(r_loaded);
+      }
+    }
     uint32_t ra[32], rb[32];
-    for (int n = 0; ok && n < 3 * n_iter; ++n) {
+    for (int n = 0; n < 3 * n_iter; ++n) {
       // fp32 -> mask -> 16 bits, this group's 64 columns into the first half of their own place. Relative
       // to the warp's 32 rows a block of 32 columns is kept, masked, or (block index == quadrant) the
       // diagonal one. dK, dV: columns from the row on are kept (all but those up to the row before); dQ:
@@ -530,10 +530,9 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       ptx::fence_proxy_async_smem();
       ptx::tc_fence_before();
     };
-    const uint32_t r_off = a_iter > 0 ? 1u : 0u;  // phase A used the first phase of r_full
     for (int i = 0; i < n_iter; ++i) {
       const bool last = i + 1 == n_iter;
-      const bool to_final = last && p.r_final != nullptr && g == nseg - 1;
+      const bool to_final = last && p.r_final != nullptr;
       // S: its copy is free once dQ's first group of the last chunk is done, which this S being complete
       // implies (the groups were issued in that order)
       if (!wait_tmem(s_full, i & 1)) break;
@@ -543,13 +542,13 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       // below.)
       if (!last || to_final) {
         if (!wait_uniform(o_full(3 * i + 1), ((3 * i + 1) >> 1) & 1)) break;
-        if (!wait_tmem(r_full, (i + r_off) & 1)) break;
+        if (!wait_tmem(r_full, i & 1)) break;
         if (!last) {
           convert(lane_base + cfg::R_COL, rb_addr);
           ptx::mbar_arrive(rb_ready);
         } else {
-          write_final_rows<D>(p.r_final + static_cast<size_t>(bh) * p.st_rows * p.st_cols, p.st_rows, p.st_cols,
-                              lane_base + cfg::R_COL, rb_addr + static_cast<uint32_t>(warp - 14) * 4096u, quad);
+          write_final_rows<D>(p.r_final + static_cast<size_t>(bh) * p.dim * p.dim, p.dim, lane_base + cfg::R_COL,
+                              rb_addr + static_cast<uint32_t>(warp - 14) * 4096u, quad);
         }
       }
     }

@@ -37,31 +37,28 @@ constexpr int kChunk = 128;                // tokens per chunk (= MMA M)
 constexpr int kThreads = 512;              // 16 warps
 constexpr int kGroupBytes = kChunk * 128;  // one 64-column group of a chunk tile: 128 rows x 128 B
 
-// Where the running state that a CTA starts from comes from.
-struct StateSource {
+struct Problem {
+  CUtensorMap q, k, v;     // 4-D maps (dim, token, head, batch), box 64 x Cfg::LOAD_ROWS x 1 x 1, 128B swizzle
+  CUtensorMap o;           // output map with a 64 x 32 box: every epilogue warp stores its own rows
   const float* s_init;     // [bh * segments + g][st_rows][st_cols] fp32, or null
+  float* s_final;          // same indexing, or null
+  int flags;               // kFlag* bits below
   int st_trans;            // state arrays are stored transposed: element (row, col) at [col][row]
+  int n_tokens;            // sequence length
   int add_trans;           // layout of s_add: transposed like st_trans
   const float* s_add;      // optional [bh][st_rows][st_cols] fp32 added to s_init for every segment
-  // ---- fused segments only (SegmentGeometry::fused)
+  // ---- fused segments only (KernelParams::fused): where the state a segment starts from comes from
   int init_kind;           // kInitParts: s_add + the partial sums of all earlier segments;
                            // kInitBound: segment 0 starts from s_add, segment g >= 1 from ONE stored
-                           // boundary state, slot bound_slot0 - g of init_base
-  int bound_slot0;
-  const float* init_base;  // kInitParts: [bh][CTAs of a head][rows*cols] (SegmentGeometry::part_out);
+                           // boundary state, slot bound_slot0 - g * bound_step of init_base
+  int init_trans;          // layout of the init_base arrays relative to this product's state
+  const float* init_base;  // kInitParts: [bh][segments * splits][rows*cols] (KernelParams::part_out);
                            // kInitBound: [bh][init_stride][rows*cols]
   int init_stride;         // kInitBound: boundary states per head
+  int bound_slot0, bound_step;
   float* bound_out;        // optional: segment g >= 1 stores the state it starts from at slot g - 1 of
                            // [bh][segments - 1][rows*cols], scratch layout (a later pass reads it back
                            // through kInitBound)
-};
-
-struct Problem : StateSource {
-  CUtensorMap q, k, v;     // 4-D maps (dim, token, head, batch), box 64 x Cfg::LOAD_ROWS x 1 x 1, 128B swizzle
-  CUtensorMap o;           // output map with a 64 x 32 box: every epilogue warp stores its own rows
-  float* s_final;          // same indexing as s_init, or null
-  int flags;               // kFlag* bits below
-  int n_tokens;            // sequence length
 };
 constexpr int kInitParts = 0;
 constexpr int kInitBound = 1;
@@ -82,34 +79,32 @@ constexpr int kFlagFirstChunkExact = 8;
 
 // Problems of one launch (block x): three gradients, or up to three column slices each of two.
 constexpr int kMaxProblems = 6;
-// How a sequence is cut into segments, and the scratch of the fused form.
-struct SegmentGeometry {
-  int seg_chunks;  // chunks per segment (block y = segment index in scan order)
-  int st_rows;     // valid rows / cols of the state arrays in global memory
-  int st_cols;
-  // ---- fused segments: ONE launch does what mode 1 + the scan kernel + mode 0 do in three.
-  // Phase A: the sums of b^T c over segments 0 .. segments - 2 are needed; all gridDim.x * gridDim.y
-  // CTAs of a head share that work, CTA number c (= segment * gridDim.x + blockIdx.x) summing share
-  // c % shares of segment c / shares, and store their sums as slot c of the head in part_out. The CTAs
-  // of a head then meet at a barrier (the launch must be cooperative: every CTA resident), turn the
-  // partials into per-segment prefixes together (each CTA scans some of the state's elements over all
-  // slots, in place: the prefix of segment s lands in slot s * shares - 1), meet again, and each CTA
-  // takes the prefix of its segment as its starting state and runs the attention loop.
-  int fused;
-  unsigned bar_slot;   // which pair of g_grid_barriers this launch uses
-  float* part_out;
-};
-
-struct KernelParams : SegmentGeometry {
+struct KernelParams {
   Problem prob[kMaxProblems];
   int heads;       // heads per batch entry (block z = b * heads + h; block x = problem)
   int nchunks;     // ceil(seqlen / 128)
+  int seg_chunks;  // chunks per segment (block y = segment index in scan order)
   int mode;        // 0: attention, 1: state only (sum of K^T V over the segment -> s_final)
+  int st_rows;     // valid rows / cols of the state arrays in global memory
+  int st_cols;
   int skip_last_segment;  // mode 1: the last segment's sum is not needed
   int* status;     // device word, bit 0 set when a bounded wait ran out; may be null
   unsigned wait_limit_us;  // limit of one bounded wait in microseconds of the global timer; 0 = default
   int debug_withhold;  // test hook: the producer skips the load of its first tile, so that the
                        // consumers' bounded wait runs out and the status path is exercised
+  // ---- fused segments: ONE launch does what mode 1 + the scan kernel + mode 0 do in three.
+  // Phase A: the sums of b^T c over segments 0 .. segments - 2 are needed (operands and walking
+  // direction of problem `pre_prob`); all gridDim.x * gridDim.y CTAs of a head share that work,
+  // CTA number c (= segment * gridDim.x + blockIdx.x) summing share c % shares of segment
+  // c / shares, and store their sums as slot c of the head in part_out. The CTAs of a head then meet
+  // at a barrier (the launch must be cooperative: every CTA resident), turn the partials into
+  // per-segment prefixes together (each CTA scans some of the state's elements over all slots, in
+  // place: the prefix of segment s lands in slot s * shares - 1), meet again, and each CTA takes
+  // the prefix of its segment as its starting state and runs the attention loop.
+  int fused;
+  int pre_prob;
+  float* part_out;
+  unsigned bar_slot;   // which pair of g_grid_barriers this launch uses
   // ---- attention with its denominator (NORM, unsegmented launches only)
   float eps;           // den_i = q_i . (sum of k_j, j <= i) + eps, and o_i is divided by it
   float* den;          // [bh][tokens], out
@@ -168,11 +163,9 @@ struct Cfg {
 
 // Arguments of converter_prologue(): where the CTA is and where its buffers and barriers are.
 struct PrologueArgs {
-  int g, nseg, bh, a_iter;
-  uint32_t state;              // tensor-memory address of the fp32 state
-  uint32_t sb_addr, ost_addr;  // 16-bit operand buffer (0: none is wanted); scratch for transposes
-  uint32_t s_full, part_done, grid_done, ready;  // mbarrier addresses
-  bool meet;                   // fused form: this state is summed by the launch itself
+  int prob_idx, g, nseg, bh, a_iter;
+  uint32_t tmem_base, sb_addr, ost_addr;
+  uint32_t s_full, part_done, grid_done, sb_ready;  // mbarrier addresses
   volatile int* abort_flag;
 };
 
@@ -181,7 +174,7 @@ struct PrologueArgs {
 // state: fetch it, write it to TMEM (fp32) and to the operand buffer (16-bit) and release the MMA
 // issuers. Returns false when a bounded wait gave up.
 template <int DK, int DV, bool HALF>
-__device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const StateSource& pr, const PrologueArgs pa) {
+__device__ __noinline__ bool converter_prologue(const KernelParams& p, const PrologueArgs pa) {
   using cfg = Cfg<DK, DV>;
   const int warp = static_cast<int>(threadIdx.x >> 5);
   const int lane = static_cast<int>(threadIdx.x & 31);
@@ -189,6 +182,7 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
   // Copies of the parameters this function reads inside its loops: `p` is a generic reference here,
   // and the L2 loads below are volatile with memory clobbers, so a p.x in a loop would be fetched
   // again after every one of them.
+  const Problem& pr = p.prob[pa.prob_idx];
   const int st_rows = p.st_rows, st_cols = p.st_cols, seg_chunks = p.seg_chunks;
   float* const part_out = p.part_out;
   const unsigned bar_slot = p.bar_slot % kGridBarSlots;
@@ -196,7 +190,7 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
   const bool fused = p.fused != 0;
   const bool has_init = fused || pr.s_init != nullptr;
   const uint32_t sb_addr = pa.sb_addr, ost_addr = pa.ost_addr;
-  const uint32_t s_full = pa.s_full, part_done = pa.part_done, grid_done = pa.grid_done, ready = pa.ready;
+  const uint32_t s_full = pa.s_full, part_done = pa.part_done, grid_done = pa.grid_done, sb_ready = pa.sb_ready;
   volatile int* abort_flag = pa.abort_flag;
   const size_t st_elems = static_cast<size_t>(st_rows) * st_cols;
   const size_t st_index = (fused ? static_cast<size_t>(bh) : static_cast<size_t>(bh) * nseg + g) * st_elems;
@@ -204,7 +198,7 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
   const int half = (warp - 2) >> 2;
   const int quad = warp & 3;
   const int row = quad * 32 + lane;
-  const uint32_t state = pa.state + (static_cast<uint32_t>(quad * 32) << 16);
+  const uint32_t lane_base = pa.tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
   const uint32_t sb_row = sb_addr + row * 128;
   const uint32_t swz = static_cast<uint32_t>(row & 7);
   constexpr int SBLK = DV / 64;
@@ -256,14 +250,34 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
     });
     ptx::keep_together(r);
   };
+  // Stores the transpose: element (row, col) of the product goes to position (r = col, c = row).
+  // Stores are not waited for, so the 32 scalar instructions cost issue slots only; the reader
+  // (the dQ product of a later backward call, whose state is the transpose) then loads vectors.
+  auto store_frag_transposed = [&](float* state, int cb, const uint32_t (&r)[32]) {
+    float* ptr = state + (static_cast<size_t>(row >> 2) * DK + cb * 32) * 4 + (row & 3);
+    ptx::static_for<32>([&](auto j) {
+      constexpr int J = decltype(j)::value;
+      ptx::st_global_cg_b32_at<J * 16>(ptr, r[J]);
+    });
+  };
+  // The stored state is the transpose of this product's state: element (row, col) of the product
+  // is stored element (r = col, c = row).
+  auto load_frag_transposed = [&](const float* state, int cb, uint32_t (&r)[32]) {
+    const float* ptr = state + (static_cast<size_t>(row >> 2) * DK + cb * 32) * 4 + (row & 3);
+    ptx::static_for<32>([&](auto j) {
+      constexpr int J = decltype(j)::value;
+      r[J] = ptx::ld_global_cg_b32_at<J * 16>(ptr);
+    });
+    ptx::keep_together(r);
+  };
+
   bool conv_ok = true;
   unsigned gen0 = 0, gen1 = 0;  // barrier generations, fetched while phase A still runs
-  const bool meet = fused && pa.meet;
-  if (meet && warp == 2 && lane == 0) {
+  if (fused && warp == 2 && lane == 0) {
     gen0 = ptx::barrier_generation(&g_grid_barriers[((bar_slot * kBarHeads + bh) * 2 + 0) * 2]);
     gen1 = ptx::barrier_generation(&g_grid_barriers[((bar_slot * kBarHeads + bh) * 2 + 1) * 2]);
   }
-  if (meet) {
+  if (fused) {
     // ---------------- phase A read-out: this CTA's partial sum -> part_out (scratch layout,
     // one thread per state row), then the barrier of the head's CTAs. Every CTA takes part in
     // the barriers, whether it had chunks to sum or not.
@@ -278,7 +292,7 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
 #pragma unroll 1
         for (int jb = 0; jb < SBLK; ++jb) {
           const int cb = half * SBLK + jb;
-          ptx::tmem_ld32(state + cb * 32, ra);
+          ptx::tmem_ld32(lane_base + cfg::S_COL + cb * 32, ra);
           if (row < DK) store_frag(dst, cb, ra);
         }
         ptx::tc_fence_before();
@@ -474,21 +488,23 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
           for (int c = 0; c < 32; ++c)
             ra[c] = __float_as_uint(__uint_as_float(ra[c]) + __uint_as_float(rb[c]));
         }
-        ptx::tmem_st32(state + cb * 32, ra);
-        if (row < DK && sb_addr != 0) store_sb(cb, ra);
+        ptx::tmem_st32(lane_base + cfg::S_COL + cb * 32, ra);
+        if (row < DK) store_sb(cb, ra);
       }
     } else {
+      static_assert(DK == DV, "the transposed read of a stored state assumes square scratch states");
       // Fused form. Segment g >= 1 starts from ONE scratch state: the scanned prefix of its
       // segment (slot g * nsplit of the head) or a boundary state an earlier call stored; the
       // caller's state is added for every segment (partial sums) or is all segment 0 has (boundary
-      // states).
+      // states). `own`: the scratch state has this product's orientation.
       const bool bound = pr.init_kind == kInitBound;
       const float* add = (pr.s_add != nullptr && (!bound || g == 0)) ? pr.s_add + head_index : nullptr;
+      const bool own = pr.init_trans != 0;
       const float* src = nullptr;
       if (g > 0) {
         // the scanned prefix of segment g sits in the last share slot of segment g - 1
         const size_t head_ctas = static_cast<size_t>(nseg) * gridDim.x;
-        const size_t slot = bound ? static_cast<size_t>(bh) * pr.init_stride + (pr.bound_slot0 - g)
+        const size_t slot = bound ? static_cast<size_t>(bh) * pr.init_stride + (pr.bound_slot0 - g * pr.bound_step)
                                   : static_cast<size_t>(bh) * head_ctas + g * (head_ctas / (nseg - 1)) - 1;
         src = pr.init_base + slot * kFragElems;
       }
@@ -499,7 +515,8 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
       for (int jb = 0; jb < SBLK; ++jb) {
         const int cb = half * SBLK + jb;
         if (src != nullptr && row < DK) {
-          load_frag(src, cb, ra);
+          if (own) load_frag(src, cb, ra);
+          else load_frag_transposed(src, cb, ra);
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) ra[j] = 0u;
@@ -511,15 +528,15 @@ __device__ __noinline__ bool converter_prologue(const SegmentGeometry& p, const 
           for (int c = 0; c < 32; ++c)
             ra[c] = __float_as_uint(__uint_as_float(ra[c]) + __uint_as_float(rb[c]));
         }
-        if (keep != nullptr && row < DK) store_frag(keep, cb, ra);
-        ptx::tmem_st32(state + cb * 32, ra);
-        if (row < DK && sb_addr != 0) store_sb(cb, ra);
+        if (keep != nullptr && row < DK) store_frag_transposed(keep, cb, ra);
+        ptx::tmem_st32(lane_base + cfg::S_COL + cb * 32, ra);
+        if (row < DK) store_sb(cb, ra);
       }
     }
     ptx::tc_wait_st();
     ptx::fence_proxy_async_smem();
     ptx::tc_fence_before();
-    ptx::mbar_arrive(ready);
+    ptx::mbar_arrive(sb_ready);
   }
 
   return conv_ok;
@@ -608,8 +625,10 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   // Fused segments: every CTA loads a starting state (possibly all zeros), see phase B below.
   const bool fused = (mode == 0) && (p.fused != 0);
   const bool has_init = (mode == 0) && (fused || pr.s_init != nullptr);
-  // Phase A of the fused form (one problem a launch): this CTA's share of its segment's chunks. The
-  // last segment's sum is not needed by anyone.
+  // Phase A of the fused form: this CTA's share of its segment's chunks, in the scan order of the
+  // problem whose state is being summed. The last segment's sum is not needed by anyone.
+  const Problem& pre = p.prob[fused ? p.pre_prob : prob_idx];
+  const bool pre_desc = (pre.flags & kFlagDescending) != 0;
   int a_lo = 0, a_iter = 0, a_chunk0 = 0;
   if (fused && nseg > 1) {
     // The nseg - 1 segments whose sums are needed are shared by ALL CTAs of the head, `shares` per
@@ -704,7 +723,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   auto plain_chunk = [&](int i) { return exact0 && mem_chunk(i) == 0; };
   auto pre_mem_chunk = [&](int i) {
     const int c = a_chunk0 + a_lo + i;
-    return descending ? (p.nchunks - 1 - c) : c;
+    return pre_desc ? (p.nchunks - 1 - c) : c;
   };
   auto slot_addr = [&](int t) {
     return smem_base + static_cast<uint32_t>(t % NSLOT) * cfg::TILE_BYTES;
@@ -729,11 +748,12 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       const int s = t % NSLOT;
       const uint32_t ph = (t / NSLOT) & 1;
       if (!wait(empty_bar(s), ph ^ 1u)) break;
-      const bool phase_a = t < t0;  // k, v tiles, each on its own barrier
+      const bool phase_a = t < t0;  // k, v tiles of the summed problem, each on its own barrier
       const int tt = phase_a ? t : t - t0;
       const int i = phase_a ? (tt >> 1) : tt / tpc;
       const int which = phase_a ? 1 + (tt & 1) : tt - i * tpc + (mode == 0 ? 0 : 1);  // 0 q, 1 k, 2 v
-      const CUtensorMap* map = (which == 0) ? &pr.q : (which == 1 ? &pr.k : &pr.v);
+      const Problem& src = phase_a ? pre : pr;
+      const CUtensorMap* map = (which == 0) ? &src.q : (which == 1 ? &src.k : &src.v);
       const uint32_t dst = slot_addr(t);
       const int tok = (phase_a ? pre_mem_chunk(i) : mem_chunk(i)) * kChunk;
       const bool paired = mode == 0 && !phase_a;  // q and k of a chunk complete on q's barrier
@@ -993,20 +1013,20 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     // scan; then the starting state into TMEM and the operand buffer) lives in a function of its
     // own, so that its register needs stay out of the allocation of the loops below.
     PrologueArgs pa;
+    pa.prob_idx = prob_idx;
     pa.g = g;
     pa.nseg = nseg;
     pa.bh = bh;
     pa.a_iter = a_iter;
-    pa.state = tmem_base + cfg::S_COL;
+    pa.tmem_base = tmem_base;
     pa.sb_addr = sb_addr;
     pa.ost_addr = ost_addr;
     pa.s_full = s_full;
     pa.part_done = part_done;
     pa.grid_done = grid_done;
-    pa.ready = sb_ready;
-    pa.meet = true;
+    pa.sb_ready = sb_ready;
     pa.abort_flag = abort_flag;
-    const bool conv_ok = converter_prologue<DK, DV, HALF>(p, pr, pa);
+    const bool conv_ok = converter_prologue<DK, DV, HALF>(p, pa);
 
     // phase A, if it ran, used the first phase of s_full
     const uint32_t s_off = a_iter > 0 ? 1u : 0u;

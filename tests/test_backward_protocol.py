@@ -51,34 +51,25 @@ class Buffers(Model):
         return sorted(set(bad))
 
 
-def backward_kernel(n_iter, double, has_r, a_iter, to_final, wait_dv=True):
+def backward_kernel(n_iter, double, has_r, to_final, wait_dv=True):
     m = Buffers()
     conv, state, epi = ["convA", "convB"], ["stateA", "stateB"], ["epi0", "epi1"]  # two warps stand for each group
     roles = ["prod0", "prod1", "X"] + conv + state + epi
     nslot = 8 if double else 4
-    t0 = 2 * a_iter
     V, G, K, Q = range(4)
 
     def slot(i, w):  # slot and how often it was filled before, as slot_of() and use_of()
         if double:
-            return (t0 + 4 * i + w) % nslot, (t0 + 4 * i + w) // nslot
-        return (w - i) & 3, ((t0 + 3 - ((w - i) & 3)) >> 2) + i
+            return (4 * i + w) % nslot, (4 * i + w) // nslot
+        return (w - i) & 3, i
 
-    tiles = [(t % nslot, t // nslot) for t in range(t0)] + [slot(i, w) for i in range(n_iter) for w in range(4)]
+    tiles = [slot(i, w) for i in range(n_iter) for w in range(4)]
     for p in ("prod0", "prod1"):
         for s, use in tiles:
             if use > 0:
                 m.wait(p, f"empty@{s}", use - 1)
             m.arrive(p, f"full@{s}")
     X = "X"
-    for i in range(a_iter):
-        for t in (2 * i, 2 * i + 1):
-            m.wait(X, f"full@{t % nslot}", t // nslot)
-        for t in (2 * i, 2 * i + 1):
-            m.commit(X, f"empty@{t % nslot}")
-        if i == a_iter - 1:
-            m.commit(X, "r_full@")
-    r_off = int(a_iter > 0)
     m.wait(X, "s_loaded@", 0)
     alt = lambda name, n: (f"{name}@{n & 1}", n >> 1)  # noqa: E731
     place = lambda n: n & 1 if double else 0  # noqa: E731
@@ -143,15 +134,11 @@ def backward_kernel(n_iter, double, has_r, a_iter, to_final, wait_dv=True):
     m.commit(X, "drained@")
     m.wait(X, "drained@", 0)
     for c in conv:
-        if not double:
-            m.touch(c, "stage", -1)  # transposes of the states at the start
+        m.touch(c, "stage", -1)  # transposes of the states at the start
         m.touch(c, "S", (-1, 0))
         m.arrive(c, "s_loaded@")
         if has_r:
-            if a_iter:
-                m.wait(c, "r_full@", 0)
-            if not double:
-                m.touch(c, "stage", -1)
+            m.touch(c, "stage", -1)
             m.touch(c, "Rb", (0, 0))
             m.touch(c, "R", (-1, 0))
             m.arrive(c, "r_loaded@")
@@ -169,7 +156,7 @@ def backward_kernel(n_iter, double, has_r, a_iter, to_final, wait_dv=True):
             if not last or to_final:
                 if wait_dv:
                     m.wait(c, *alt("o_full", 3 * i + 1))
-                m.wait(c, "r_full@", i + r_off)
+                m.wait(c, "r_full@", i)
                 m.touch(c, "R", (i, 1))
                 m.touch(c, "Rb", (i + 1, 0))
                 if not last:
@@ -178,7 +165,7 @@ def backward_kernel(n_iter, double, has_r, a_iter, to_final, wait_dv=True):
         for n in range(3 * n_iter):
             m.wait(e, *alt("o_full", n))
             m.touch(e, f"O{place(n)}", (n, 1))
-            if not double and e == "epi0":  # (every warp has its own rows of the stage)
+            if e == "epi0":  # (every warp has its own rows of the stage)
                 m.touch(e, "stage", n)
             m.arrive(e, alt("o_free", n)[0])
     for r in roles:
@@ -204,11 +191,11 @@ def backward_kernel(n_iter, double, has_r, a_iter, to_final, wait_dv=True):
 
 @pytest.mark.parametrize("n_iter", [1, 2, 3, 7])
 @pytest.mark.parametrize("double", [False, True])
-@pytest.mark.parametrize("has_r,a_iter,to_final", [(0, 0, 0), (0, 0, 1), (1, 0, 0), (1, 0, 1), (1, 1, 0), (1, 4, 1)])
-def test_no_wait_is_overtaken_and_every_shared_buffer_has_one_user(n_iter, double, has_r, a_iter, to_final):
-    assert backward_kernel(n_iter, double, has_r, a_iter, to_final) == []
+@pytest.mark.parametrize("has_r,to_final", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_no_wait_is_overtaken_and_every_shared_buffer_has_one_user(n_iter, double, has_r, to_final):
+    assert backward_kernel(n_iter, double, has_r, to_final) == []
 
 
 def test_the_model_sees_a_copy_overwritten_under_a_product():
-    assert "disorder: Rb" in backward_kernel(3, False, 0, 0, 0, wait_dv=False)
-    assert "disorder: Rb" in backward_kernel(3, True, 1, 2, 0, wait_dv=False)
+    assert "disorder: Rb" in backward_kernel(3, False, 0, 0, wait_dv=False)
+    assert "disorder: Rb" in backward_kernel(3, True, 1, 0, wait_dv=False)
