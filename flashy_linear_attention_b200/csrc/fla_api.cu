@@ -711,6 +711,19 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
   return b;
 }
 
+// Unsegmented backward calls that give a head's three gradients one CTA (fla_backward_kernel) instead of
+// three. Such a CTA takes two to two and a half times as long for a chunk (64-wide: twice), so it pays where the
+// three need more than twice as many rounds over the SMs (64-wide: as many). Microseconds, three / one:
+//   128-wide, 16 chunks   74 heads 77 / 83   99: 107 / 85   128: 116 / 96   180: 159 / 174   222: 196 / 179   296: 251 / 203
+//    64-wide, 16 chunks   74 heads 63 / 62   99:  91 / 62   128:  80 / 56   180:  95 /  92   222: 117 /  93   296: 141 / 101
+// One chunk: 128 heads 20 / 12.5 and 23 / 12; 40 chunks, 512 heads: 1180 / 990 and 735 / 525.
+bool one_cta_backward(const FlaArgs* a, int sm_count) {
+  if (a->dk != a->dv || a->dk > 128) return false;
+  const long heads = static_cast<long>(a->batch) * a->heads;
+  auto rounds = [&](long ctas) { return (ctas + sm_count - 1) / sm_count; };
+  return a->dk > 64 ? rounds(3 * heads) > 2 * rounds(heads) : rounds(3 * heads) >= 2 * rounds(heads);
+}
+
 // Bytes of the boundary states a fused forward stores for a fused backward, or 0 when the pair of
 // calls does not run that way for these shapes.
 size_t seg_states_bytes(const FlaArgs* a, int sm_count, SegPlan* fwd_out, SegPlan* bwd_out) {
@@ -1291,12 +1304,6 @@ int run_backward(const FlaArgs* a, cudaStream_t stream) {
   return e == cudaSuccess ? FLA_OK : FLA_ERR_CUDA;
 }
 
-bool one_cta_backward_pays(int heads, int sm_count, int dim) {
-  if (const char* e = getenv("FLA_ONE_CTA")) return atoi(e) != 0;
-  (void)dim;
-  return heads > 2 * sm_count / 3;
-}
-
 }  // namespace
 
 extern "C" {
@@ -1382,6 +1389,7 @@ int fla_sm100_bwd_uses_final_state(const FlaArgs* a) {
   if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0) return 0;
   if (a->dk > 128 || a->dv > 128) return 0;
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
+  if (a->segments <= 1 && one_cta_backward(a, current_sm_count_early())) return 1;
   if (!(nchunks >= kSingleSweepMinChunks || (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP))) return 0;
   if (fla_sm100_seg_states_bytes(a) > 0) return 1;
   int nseg = a->segments > 0 ? a->segments
@@ -1480,9 +1488,8 @@ int fla_sm100_bwd(const FlaArgs* a) {
   int nseg = a->segments > 0 ? a->segments
                              : auto_segments(SplitForm::kBackward, a->batch * a->heads, nchunks, dev->sm_count, a->dk, a->dv);
   if (nseg > nchunks) nseg = nchunks;
-  if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks) && a->dk == a->dv &&
-      one_cta_backward_pays(a->batch * a->heads, dev->sm_count, a->dk))
-    return run_backward(a, stream);
+  // (Its dQ is no difference of two sums over a chunk, so the length rule of the single sweep is not its own.)
+  if (a->s_last != nullptr && nseg <= 1 && one_cta_backward(a, dev->sm_count)) return run_backward(a, stream);
   if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks)) {
     // The forward state after this call's tokens is known: dQ can walk the sequence in the same
     // descending order as dV and dK (state = total minus suffix), so the three products of a

@@ -16,6 +16,11 @@
 // D = 128 S, R, P and the accumulator fill its 512 columns. The states' 16-bit copies serve as MMA operands in
 // either direction (dV contracts over R's rows, dK over its columns) without a second copy.
 //
+// Bound by shared memory at D = 128: a chunk moves 1.0 MB of operands, states, tiles and staged outputs
+// through an SM, 8000 cycles at 128 bytes against 6300 of MMAs (three CTAs of fla_chunk_kernel: 1.25 MB); by the
+// issuer's waits and the conversions at D = 64. 128 heads, in one CTA each / three: 4096 x 128 186 / 220 us,
+// 8192 x 128 365 / 422 us, 4096 x 64 93 / 125 us. dQ's error against 64 bits 2.34e-3 / 2.40e-3.
+//
 // CTA layout (608 threads, one CTA per SM):
 //   warps 0, 18   TMA producers, each half of every tile (see fla_kernel.cuh)
 //   warp 1        MMA issuer (one elected lane) and TMEM owner
@@ -115,15 +120,15 @@ struct Walk {
   uint32_t start, step, jump;
 };
 template <bool TS>
-__device__ __forceinline__ void issue_group(uint32_t d, Walk a, Walk b, uint32_t idesc, uint32_t accumulate, int blocks) {
+__device__ __forceinline__ void issue_group(bool leader, uint32_t d, Walk a, Walk b, uint32_t idesc, uint32_t accumulate, int blocks) {
 #pragma unroll
   for (int blk = 0; blk < blocks; ++blk) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const uint32_t av = a.start + blk * a.jump + j * a.step, bv = b.start + blk * b.jump + j * b.step;
       const uint32_t add = (blk > 0 || j > 0) ? 1u : accumulate;
-      if (TS) ptx::mma_ts(d, av, bv, ptx::kDescHi, idesc, add);
-      else ptx::mma_ss(d, av, bv, ptx::kDescHi, idesc, add);
+      if (TS) ptx::mma_ts_on(leader, d, av, bv, ptx::kDescHi, idesc, add);
+      else ptx::mma_ss_on(leader, d, av, bv, ptx::kDescHi, idesc, add);
     }
   }
 }
@@ -244,7 +249,7 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_holder, 0);
 
   auto wait_uniform = [&](uint32_t bar_addr, uint32_t parity) {
     const int ok = ptx::mbar_wait(bar_addr, parity, abort_flag) ? 1 : 0;
@@ -264,17 +269,18 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
 
   if (warp == 0 || warp == 18) {
     // ================================================================ TMA producers
-    if (ptx::elect_one()) {
-      const int part = warp == 0 ? 0 : 1;
-      constexpr int kPartBytes = cfg::TILE_BYTES / 2;
-      const int part_col = cfg::G == 2 ? part * 64 : 0;
-      const int part_row = cfg::G == 2 ? 0 : part * cfg::LOAD_ROWS;
-      for (int t = 0; t < 4 * n_iter; ++t) {
-        const int i = t >> 2, w = t & 3;
-        const int s = slot_of(i, w);
-        if (!ptx::mbar_wait(empty_bar(s), (use_of(i, w) & 1) ^ 1u, abort_flag)) break;
-        const int tok = mem_chunk(i) * kChunk + part_row;
-        const CUtensorMap* map = w == V ? &p.v : w == G ? &p.g : w == K ? &p.k : &p.q;
+    const bool leader = ptx::elect_one();
+    const int part = warp == 0 ? 0 : 1;
+    constexpr int kPartBytes = cfg::TILE_BYTES / 2;
+    const int part_col = cfg::G == 2 ? part * 64 : 0;
+    const int part_row = cfg::G == 2 ? 0 : part * cfg::LOAD_ROWS;
+    for (int t = 0; t < 4 * n_iter; ++t) {
+      const int i = t >> 2, w = t & 3;
+      const int s = slot_of(i, w);
+      if (!wait_uniform(empty_bar(s), (use_of(i, w) & 1) ^ 1u)) break;
+      const int tok = mem_chunk(i) * kChunk + part_row;
+      const CUtensorMap* map = w == V ? &p.v : w == G ? &p.g : w == K ? &p.k : &p.q;
+      if (leader) {
         ptx::mbar_expect_tx(full_bar(s), kPartBytes);
         if (!(p.debug_withhold && t == 0))
           ptx::tma_load_4d(slot_addr(s) + part * kPartBytes, map, full_bar(s), part_col, tok, h, b);
@@ -282,6 +288,7 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
         // now. (128 heads x 8192: 396 us without, 376 with; at D = 64, two chunks deep, no difference.)
         if (D == 128 && i + 1 < n_iter) ptx::tma_prefetch_4d(map, part_col, tok - kChunk, h, b);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ================================================================ MMA issuer
@@ -291,31 +298,30 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
     constexpr uint32_t IDESC_XT = ptx::make_idesc(128, D, false, false, HALF);      // a X^T: contracts X's columns
     constexpr uint32_t IDESC_X = ptx::make_idesc(128, D, false, true, HALF);        // a X, P b: contracts rows
     const uint32_t tS = tmem_base + cfg::S_COL, tR = tmem_base + cfg::R_COL;
-    if (ptx::elect_one()) {
-    // One thread runs the role: a wait of a whole warp costs a vote, and there are two dozen of them a chunk.
-    auto wait = [&](uint32_t bar_addr, uint32_t parity) { return ptx::mbar_wait(bar_addr, parity, abort_flag); };
-    auto commit = [&](uint32_t bar_addr) { ptx::tc_commit(bar_addr); };
+    const bool leader = ptx::elect_one();
+    auto wait = [&](uint32_t bar_addr, uint32_t parity) { return wait_uniform(bar_addr, parity); };
+    auto commit = [&](uint32_t bar_addr) { ptx::tc_commit_on(leader, bar_addr); };
     // Operands: a chunk tile or a state's copy, contracted over its columns (K-major) or its rows (MN-major).
     constexpr int kStateGroup = D * 128;  // bytes between the 64-column groups of a state's copy
     auto columns = [](uint32_t addr, int group) { return Walk{ptx::desc_lo(addr, 16), 32u >> 4, static_cast<uint32_t>(group) >> 4}; };
     auto rows = [](uint32_t addr, int group) { return Walk{ptx::desc_lo(addr, group), 2048u >> 4, 8192u >> 4}; };
     auto scores = [&](int n, uint32_t a, uint32_t bt) {  // P = a b^T
-      issue_group<false>(tmem_base + cfg::p_col(n), columns(a, kGroupBytes), columns(bt, kGroupBytes), IDESC_P, 0u, D / 64);
+      issue_group<false>(leader, tmem_base + cfg::p_col(n), columns(a, kGroupBytes), columns(bt, kGroupBytes), IDESC_P, 0u, D / 64);
       commit(p_full(n));
     };
     // For D = 64 the instruction still spans 128 rows of the state; the upper 64 read whatever follows the a
     // tile in shared memory and land in tensor-memory lanes nobody reads.
     auto state_add = [&](uint32_t t_state, uint32_t a, uint32_t bt, uint32_t idesc, bool accumulate) {
-      issue_group<false>(t_state, rows(a, kGroupBytes), rows(bt, kGroupBytes), idesc, accumulate ? 1u : 0u, 2);
+      issue_group<false>(leader, t_state, rows(a, kGroupBytes), rows(bt, kGroupBytes), idesc, accumulate ? 1u : 0u, 2);
     };
     auto times_state_t = [&](int n, uint32_t a, uint32_t x) {  // O = a X^T
-      issue_group<false>(tmem_base + cfg::o_col(n), columns(a, kGroupBytes), columns(x, kStateGroup), IDESC_XT, 0u, D / 64);
+      issue_group<false>(leader, tmem_base + cfg::o_col(n), columns(a, kGroupBytes), columns(x, kStateGroup), IDESC_XT, 0u, D / 64);
     };
     auto times_state = [&](int n, uint32_t a, uint32_t x) {  // O = a X
-      issue_group<false>(tmem_base + cfg::o_col(n), columns(a, kGroupBytes), rows(x, kStateGroup), IDESC_X, 0u, D / 64);
+      issue_group<false>(leader, tmem_base + cfg::o_col(n), columns(a, kGroupBytes), rows(x, kStateGroup), IDESC_X, 0u, D / 64);
     };
     auto times_scores = [&](int n, uint32_t bt, bool accumulate) {  // O += P b, P in its 16-bit form (two halves)
-      issue_group<true>(tmem_base + cfg::o_col(n), Walk{tmem_base + cfg::p_col(n), 8u, 64u}, rows(bt, kGroupBytes), IDESC_X, accumulate ? 1u : 0u, 2);
+      issue_group<true>(leader, tmem_base + cfg::o_col(n), Walk{tmem_base + cfg::p_col(n), 8u, 64u}, rows(bt, kGroupBytes), IDESC_X, accumulate ? 1u : 0u, 2);
       commit(o_full(n));
     };
 
@@ -398,7 +404,6 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
     }
     // Nobody waits for the last releases; the barriers have to outlive them all the same.
     commit(drained);
-    }
   } else if (warp < 10) {
     // ================================================================ converters of the scores
     const int half = (warp - 2) >> 2;  // column half this group owns

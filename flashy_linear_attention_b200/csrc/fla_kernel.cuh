@@ -729,15 +729,15 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     return smem_base + static_cast<uint32_t>(t % NSLOT) * cfg::TILE_BYTES;
   };
 
-  // The waits of a role that one thread runs.
-  auto wait = [&](uint32_t bar, uint32_t parity) { return ptx::mbar_wait(bar, parity, abort_flag); };
+  bool issuer = false;  // the one lane of an issuer warp that executes tcgen05.mma / tcgen05.commit
 
   if (warp == 0 || warp == 15) {
     // ================================================================ TMA producers
-    // One thread of the warp runs the loop: a wait of the whole warp costs a vote. In mode 0 the q and k tiles of a chunk complete on the q tile's barrier.
+    // The whole warp runs the loop (so that addresses and coordinates stay warp-uniform); one
+    // elected lane issues. In mode 0 the q and k tiles of a chunk complete on the q tile's barrier.
     // Each producer loads its half of every tile: one 64-column group, or 64 of the 128 rows where
     // a tile is one group wide.
-    if (ptx::elect_one()) {
+    const bool leader = ptx::elect_one();
     const int part = warp == 0 ? 0 : 1;
     constexpr int kPartBytes = cfg::TILE_BYTES / 2;
     constexpr int kPartRows = cfg::LOAD_ROWS;
@@ -747,7 +747,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     for (int t = 0; t < n_tiles; ++t) {
       const int s = t % NSLOT;
       const uint32_t ph = (t / NSLOT) & 1;
-      if (!wait(empty_bar(s), ph ^ 1u)) break;
+      if (!wait_uniform(empty_bar(s), ph ^ 1u)) break;
       const bool phase_a = t < t0;  // k, v tiles of the summed problem, each on its own barrier
       const int tt = phase_a ? t : t - t0;
       const int i = phase_a ? (tt >> 1) : tt / tpc;
@@ -759,38 +759,44 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       const bool paired = mode == 0 && !phase_a;  // q and k of a chunk complete on q's barrier
       // barrier that the tile's bytes complete on, and the bytes armed on it at this point
       const uint32_t bar = (paired && which == 1) ? full_bar((t - 1) % NSLOT) : full_bar(s);
-      if (paired && which == 0) ptx::mbar_expect_tx(bar, 2 * kPartBytes);
-      if (!paired || which == 2) ptx::mbar_expect_tx(bar, kPartBytes);
-      // The k slot's own barrier is not waited on; complete its phase so that the parity of
-      // later ring passes stays in step.
-      if (paired && which == 1) ptx::mbar_arrive(full_bar(s));
-      if (!(p.debug_withhold && t == 0))
-        ptx::tma_load_4d(dst + part * kPartBytes, map, bar, part_col, tok + part_row, h, b);
-    }
+      if (leader) {
+        if (paired && which == 0) ptx::mbar_expect_tx(bar, 2 * kPartBytes);
+        if (!paired || which == 2) ptx::mbar_expect_tx(bar, kPartBytes);
+        // The k slot's own barrier is not waited on; complete its phase so that the parity of
+        // later ring passes stays in step.
+        if (paired && which == 1) ptx::mbar_arrive(full_bar(s));
+        if (!(p.debug_withhold && t == 0))
+          ptx::tma_load_4d(dst + part * kPartBytes, map, bar, part_col, tok + part_row, h, b);
+      }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // ================================================================ MMA issuer X
-    // S += K_i^T V_i, then P = Q_{i+1} K_{i+1}^T. One thread runs the role.
+    // S += K_i^T V_i, then P = Q_{i+1} K_{i+1}^T. The whole warp runs the loop with warp-uniform
+    // operands; one elected lane issues the tcgen05.mma / tcgen05.commit instructions.
     // Edges it waits on besides tile arrival:
     //   sb_ready(i-1)  the converters have read S of chunk i-1 out of TMEM      (before S += ..)
     //   p_read(i)      the converters have read P of chunk i out of TMEM        (before P = ..)
     //   o_full(i-1)    issuer Y's P V of chunk i-1 is done: that bf16 P buffer is reused by
     //                  the conversion of the tile written here
-    if (ptx::elect_one()) {
     constexpr uint32_t IDESC_QK = ptx::make_idesc(128, kChunk, false, false, HALF);  // P  = Q K^T
     constexpr uint32_t IDESC_KV_ADD = ptx::make_idesc(128, DV, true, true, HALF);    // S += K^T V
     constexpr uint32_t IDESC_KV_SUB = IDESC_KV_ADD | (1u << 13);               // S -= K^T V (A negated)
     const uint32_t IDESC_KV = tms ? IDESC_KV_SUB : IDESC_KV_ADD;
     const uint32_t tP = tmem_base + cfg::P_COL;
     const uint32_t tS = tmem_base + cfg::S_COL;
-    auto wait_tile = [&](int t) { return wait(full_bar(t % NSLOT), (t / NSLOT) & 1); };
-    auto release_tile = [&](int t) { ptx::tc_commit(empty_bar(t % NSLOT)); };
+    const bool leader = ptx::elect_one();
+    issuer = leader;
+    auto wait_tile = [&](int t) { return wait_uniform(full_bar(t % NSLOT), (t / NSLOT) & 1); };
+    auto release_tile = [&](int t) {
+      if (leader) ptx::tc_commit(empty_bar(t % NSLOT));
+    };
     // P = Q K^T of chunk i (both operands K-major, 16 columns of dk per instruction)
     auto issue_qk = [&](int i) {
       if (!wait_tile(t0 + 3 * i)) return false;  // covers the k tile too
       const uint32_t q_lo = ptx::desc_lo(slot_addr(t0 + 3 * i), 16);
       const uint32_t k_lo = ptx::desc_lo(slot_addr(t0 + 3 * i + 1), 16);
-      {
+      if (leader) {
 #pragma unroll
         for (int kk = 0; kk < DK / 16; ++kk) {
           const uint32_t off = ((kk >> 2) * kGroupBytes + (kk & 3) * 32) >> 4;
@@ -800,6 +806,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
       }
       release_tile(t0 + 3 * i);      // first of two arrivals on q (the other: issuer Y after Q Sb)
       release_tile(t0 + 3 * i + 1);  // first of two arrivals on k (the other: below, after K^T V)
+      __syncwarp();
       return true;
     };
     if (mode == 0) {
@@ -812,7 +819,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         const uint32_t k_lo = ptx::desc_lo(slot_addr(2 * i), kGroupBytes);
         const uint32_t v_lo = ptx::desc_lo(slot_addr(2 * i + 1), kGroupBytes);
         ptx::tc_fence_after();
-        {
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < kChunk / 16; ++kk) {
             ptx::mma_ss(tS, k_lo + kk * (2048 >> 4), v_lo + kk * (2048 >> 4), ptx::kDescHi,
@@ -825,7 +832,8 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           ptx::tc_commit(empty_bar((2 * i + 1) % NSLOT));
           if (i == a_iter - 1) ptx::tc_commit(s_full);
         }
-        }
+        __syncwarp();
+      }
       ok = ok && issue_qk(0);
       for (int i = 0; ok && i < n_iter; ++i) {
         // k, v MN-major: 64-column groups kGroupBytes apart
@@ -836,12 +844,12 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         // For DK = 64 the instruction still spans 128 rows; the upper 64 read whatever follows
         // the K tile in shared memory and land in TMEM lanes nobody reads.
         if (have_state) {
-          if (!wait(sb_ready, sb_waits & 1)) break;
+          if (!wait_uniform(sb_ready, sb_waits & 1)) break;
           ++sb_waits;
         }
         if (!wait_tile(t0 + 3 * i + 2)) break;
         ptx::tc_fence_after();
-        {
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < kChunk / 16; ++kk) {
             ptx::mma_ss(tS, k_lo + kk * (2048 >> 4), v_lo + kk * (2048 >> 4), ptx::kDescHi,
@@ -853,8 +861,8 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         release_tile(t0 + 3 * i + 2);  // first of two arrivals on v (the other: issuer Y after P V)
         // ---- score tile of the next chunk
         if (i + 1 < n_iter) {
-          if (!wait(p_read, i & 1)) break;
-          if (i >= 1 && !wait(((i - 1) & 1) ? o_full1 : o_full0, ((i - 1) >> 1) & 1)) break;
+          if (!wait_uniform(p_read, i & 1)) break;
+          if (i >= 1 && !wait_uniform(((i - 1) & 1) ? o_full1 : o_full0, ((i - 1) >> 1) & 1)) break;
           ptx::tc_fence_after();
           ok = issue_qk(i + 1);
         }
@@ -864,7 +872,7 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         if (!wait_tile(2 * i) || !wait_tile(2 * i + 1)) break;
         const uint32_t k_lo = ptx::desc_lo(slot_addr(2 * i), kGroupBytes);
         const uint32_t v_lo = ptx::desc_lo(slot_addr(2 * i + 1), kGroupBytes);
-        {
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < kChunk / 16; ++kk) {
             ptx::mma_ss(tS, k_lo + kk * (2048 >> 4), v_lo + kk * (2048 >> 4), ptx::kDescHi,
@@ -873,10 +881,9 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         }
         release_tile(2 * i);
         release_tile(2 * i + 1);
-        if (i == n_iter - 1) ptx::tc_commit(s_full);
-        }
-    }
-    ptx::tc_commit(drained_x);
+        if (leader && i == n_iter - 1) ptx::tc_commit(s_full);
+        __syncwarp();
+      }
     }
   } else if (warp == 14) {
     // ================================================================ MMA issuer Y
@@ -886,12 +893,14 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
     //   sb_ready(i-1) the bf16 state of chunk i-1 is in shared memory
     //   pb_ready(i)   the bf16 score tile of chunk i is in TMEM
     // and it signals qs_done(i) (the state buffer may be overwritten) and o_full(i).
-    if (mode == 0 && ptx::elect_one()) {
+    if (mode == 0) {
       constexpr uint32_t IDESC_PV = ptx::make_idesc(128, DV, false, true, HALF);  // O += Pb V
       constexpr uint32_t IDESC_QS = ptx::make_idesc(128, DV, false, true, HALF);  // O  = Q Sb
       const uint32_t tO0 = tmem_base + cfg::O_COL;
       const uint32_t sb_lo = ptx::desc_lo(sb_addr, DK * 128);  // MN-major, groups DK*128 B apart
-      auto wait_tile = [&](int t) { return wait(full_bar(t % NSLOT), (t / NSLOT) & 1); };
+      const bool leader = ptx::elect_one();
+      issuer = leader;
+      auto wait_tile = [&](int t) { return wait_uniform(full_bar(t % NSLOT), (t / NSLOT) & 1); };
       uint32_t sb_waits = 0;
       for (int i = 0; i < n_iter; ++i) {
         const uint32_t q_lo = ptx::desc_lo(slot_addr(t0 + 3 * i), 16);                // K-major
@@ -901,17 +910,17 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
         const uint32_t tPb = tmem_base + cfg::PB_COL + (i & 1) * 64;
         const uint32_t tO = tO0 + (cfg::O_BUFS == 2 ? (i & 1) * DV : 0);
         if (cfg::O_BUFS == 2) {
-          if (i >= 2 && !wait((i & 1) ? o_free1 : o_free0, ((i - 2) >> 1) & 1)) break;
+          if (i >= 2 && !wait_uniform((i & 1) ? o_free1 : o_free0, ((i - 2) >> 1) & 1)) break;
         } else {
-          if (i >= 1 && !wait(o_free0, (i - 1) & 1)) break;
+          if (i >= 1 && !wait_uniform(o_free0, (i - 1) & 1)) break;
         }
         if (have_state) {
-          if (!wait(sb_ready, sb_waits & 1)) break;
+          if (!wait_uniform(sb_ready, sb_waits & 1)) break;
           ++sb_waits;
         }
         if (!wait_tile(t0 + 3 * i)) break;
         ptx::tc_fence_after();
-        {
+        if (leader) {
           if (use_state) {
 #pragma unroll
             for (int kk = 0; kk < DK / 16; ++kk) {
@@ -923,10 +932,10 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           ptx::tc_commit(qs_done);
           ptx::tc_commit(empty_bar((t0 + 3 * i) % NSLOT));  // second arrival on q
         }
-        if (!wait((i & 1) ? pb_ready1 : pb_ready0, (i >> 1) & 1)) break;
+        if (!wait_uniform((i & 1) ? pb_ready1 : pb_ready0, (i >> 1) & 1)) break;
         if (!wait_tile(t0 + 3 * i + 2)) break;
         ptx::tc_fence_after();
-        {
+        if (leader) {
 #pragma unroll
           for (int kk = 0; kk < kChunk / 16; ++kk) {
             ptx::mma_ts(tO, tPb + kk * 8, v_lo + kk * (2048 >> 4), ptx::kDescHi, IDESC_PV,
@@ -935,8 +944,8 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
           ptx::tc_commit((i & 1) ? o_full1 : o_full0);
           ptx::tc_commit(empty_bar((t0 + 3 * i + 2) % NSLOT));  // second arrival on v
         }
-        }
-      ptx::tc_commit(drained_y);
+        __syncwarp();
+      }
     }
   } else if (warp < 10) {
     // ================================================================ converter groups A, B
@@ -1313,7 +1322,12 @@ fla_chunk_kernel(const __grid_constant__ KernelParams p) {
   __syncwarp();
   // The issuers' last instructions (S += K^T V of the last chunk, the releases of its tiles) have no
   // reader that waits for them; tensor memory and the barriers have to outlive them all the same.
-  if (warp == 1 || (warp == 14 && mode == 0)) wait_uniform(warp == 1 ? drained_x : drained_y, 0);
+  if (warp == 1 || (warp == 14 && mode == 0)) {
+    const uint32_t drained = warp == 1 ? drained_x : drained_y;
+    if (issuer) ptx::tc_commit(drained);
+    __syncwarp();
+    wait_uniform(drained, 0);
+  }
   if (*abort_flag) {
     // A wait gave up: let copies in flight land before the shared memory is released.
     __nanosleep(100000);

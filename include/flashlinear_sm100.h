@@ -83,9 +83,9 @@ typedef struct FlaArgs {
   float* r_final;
   /* Backward only, optional: the forward state AFTER this call's tokens (what the forward call
    * wrote to s_final). When given (and fla_sm100_bwd_uses_final_state() says so: the call is not
-   * split into segments or comes with seg_states, and the sequence is longer than 2048 tokens) dQ
-   * is computed in the same end-to-start sweep as dK and dV, which lets the three share every read
-   * of q, k, v, dO; s_init is then not needed. */
+   * split into segments or comes with seg_states, and the sequence is longer than 2048 tokens or there are
+   * heads enough for one CTA each) dQ is computed in the same end-to-start sweep as dK and dV, which lets the
+   * three share every read of q, k, v, dO; s_init then only says whether anything precedes the first token. */
   const float* s_last;
 
   /* Sequence segments per head (intra-GPU sequence split). 0 = pick automatically, 1 = none.
@@ -142,8 +142,8 @@ typedef struct FlaArgs {
  * launches apart. A process that replays many captured graphs on concurrent streams should set
  * this bit for all but one of the streams. */
 #define FLA_DEBUG_NO_FUSED_SEGMENTS 2u
-/* The backward uses s_last (dQ in the same end-to-start sweep as dK and dV) only for sequences
- * longer than 2048 tokens; on shorter ones that form is a little less accurate than the
+/* With a CTA per gradient the backward uses s_last (dQ in the same end-to-start sweep as dK and dV) only for
+ * sequences longer than 2048 tokens; on shorter ones that form is a little less accurate than the
  * two-direction form and saves nothing worth having. This bit lifts the length rule, for tests. */
 #define FLA_DEBUG_FORCE_SINGLE_SWEEP 4u
 
@@ -169,7 +169,7 @@ int fla_sm100_auto_segments(const FlaArgs* args, int pass);
 size_t fla_sm100_seg_states_bytes(const FlaArgs* args);
 /* 1 when fla_sm100_bwd for these shapes makes use of s_last (so that the forward should be asked
  * for s_final), 0 when it would ignore it: segmented backward without seg_states, sequences of at
- * most 2048 tokens, head dims above 128. */
+ * most 2048 tokens unless there are heads enough for one CTA each, head dims above 128. */
 int fla_sm100_bwd_uses_final_state(const FlaArgs* args);
 
 /* replaces linear_flash_wrapper_fwd / linear_flash_wrapper_fwd_smallv_hd

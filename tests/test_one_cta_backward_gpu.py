@@ -1,0 +1,150 @@
+"""fla_backward_kernel (the three gradients of a head in one CTA) against an evaluation in 64 bits: edges of its
+chunks, head dims and dtypes, states before and after, and which calls take it."""
+import ctypes
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _inputs(B, H, N, D, dtype, seed):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    q, k = (torch.nn.functional.elu(torch.randn(B, H, N, D, device=DEV, generator=gen)) + 1 for _ in range(2))
+    v, g = (torch.randn(B, H, N, D, device=DEV, generator=gen) for _ in range(2))
+    if dtype == torch.float16:
+        q = q / math.sqrt(D)
+    return [t.to(dtype) for t in (q, k, v, g)]
+
+
+def _exact(q, k, v, g, s0=None, r0=None):
+    q, k, v, g = (t.double() for t in (q, k, v, g))
+    p, dp = torch.tril(q @ k.mT), torch.tril(g @ v.mT)
+    dq, dk, dv = dp @ k, dp.mT @ q, p.mT @ g
+    if s0 is not None:
+        dq = dq + g @ s0.double().mT
+    if r0 is not None:
+        dk, dv = dk + v @ r0.double().mT, dv + k @ r0.double()
+    return dq, dk, dv, q.mT @ g + (0 if r0 is None else r0.double())
+
+
+# every gradient rounds its two operands of each kind, scores or state, and the result: three roundings of
+# 2^-9 (fp16: 2^-12) / sqrt(3) in norm; dq's and dk's score tiles have terms of both signs, which doubles theirs
+def _bound(dtype):
+    return (2.0**-9 if dtype == torch.bfloat16 else 2.0**-12) * math.sqrt((1 + 4 + 4) / 3)
+
+
+def _run(q, k, v, g, s_last, **kw):
+    from flashy_linear_attention_b200 import _lib, ops
+
+    grads = ops.causal_dot_product_bwd(g, q, k, v, s_last=s_last, segments=1, **kw)
+    assert _lib.load().fla_sm100_last_launch_count() == 1
+    torch.cuda.synchronize()
+    ops.check_status(torch.device(DEV))
+    return grads
+
+
+# one chunk, less than one, a ragged last one, the ring's second and third pass; 50 heads: the rule's edge at 64
+# columns, 99: at 128; 296 heads: two rounds
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,H,N,D", [(2, 50, 64, 128), (1, 99, 128, 128), (4, 25, 192, 83), (2, 64, 320, 96), (1, 100, 1216, 128),
+                                     (1, 50, 64, 64), (2, 32, 128, 40), (1, 64, 448, 64), (1, 60, 1216, 64), (2, 148, 192, 64)])
+def test_gradients_against_64_bits(B, H, N, D, dtype):
+    from flashlinear import LinearAttention
+    from flashy_linear_attention_b200 import ops
+
+    q, k, v, g = _inputs(B, H, N, D, dtype, N + D)
+    assert ops.backward_uses_final_state(q, v)
+    tq, tk, tv = (t.detach().requires_grad_(True) for t in (q, k, v))
+    got = torch.autograd.grad(LinearAttention.apply(tq, tk, tv), (tq, tk, tv), g)
+    ops.check_status(torch.device(DEV))
+    for name, x, want in zip(("dq", "dk", "dv"), got, _exact(q, k, v, g)):
+        rel = ((x.double() - want).norm() / want.norm()).item()
+        assert rel <= _bound(dtype), (name, rel)
+
+
+@pytest.mark.parametrize("with_s", [False, True])
+@pytest.mark.parametrize("with_r", [False, True])
+@pytest.mark.parametrize("H,N,D", [(100, 128, 128), (100, 576, 96), (64, 128, 64), (64, 576, 48)])
+def test_states_before_and_after(H, N, D, with_s, with_r):
+    q, k, v, g = _inputs(1, H, N, D, torch.bfloat16, N)
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    s0, r0 = (torch.randn(H, D, D, device=DEV, generator=gen) * 8 if w else None for w in (with_s, with_r))
+    s_last = (k[0].double().mT @ v[0].double() + (s0.double() if with_s else 0)).float()
+    r_final = torch.full((H, D, D), float("nan"), device=DEV)
+    got = _run(q, k, v, g, s_last, s_init=s0, r_init=r0, r_final=r_final)
+    want = _exact(q[0], k[0], v[0], g[0], s0, r0)
+    for name, x, w in zip(("dq", "dk", "dv"), got, want):
+        rel = ((x[0].double() - w).norm() / w.norm()).item()
+        assert rel <= _bound(torch.bfloat16), (name, rel)
+    # fp32 sums of N / 16 steps of 16 exact products
+    assert ((r_final.double() - want[3]).norm() / want[3].norm()).item() <= (N / 16 + 2) * 2.0**-24
+
+
+def test_strided_inputs_and_guard_bands():
+    """[B, H, N, D] views of [B, N, H, D] tensors; outputs' neighbours stay as they are."""
+    from flashy_linear_attention_b200 import _lib, ops
+    from flashy_linear_attention_b200._lib import FlaArgs
+
+    B, H, N, D = 1, 100, 200, 128
+    q, k, v, g = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in _inputs(B, H, N, D, torch.bfloat16, 3))
+    s_last = (k[0].double().mT @ v[0].double()).float()
+    frames = [torch.full((B, H, N + 4, D + 8), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
+    outs = [f[:, :, 2:N + 2, :D] for f in frames]
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = B, H, N, D, D
+    for name, t in zip(("q", "k", "v", "d_o", "d_q", "d_k", "d_v"), [q, k, v, g] + outs):
+        setattr(a, name, ops._desc(t))
+    a.s_last = s_last.data_ptr()
+    a.stream = torch.cuda.current_stream(DEV).cuda_stream
+    lib = _lib.load()
+    assert lib.fla_sm100_bwd(ctypes.byref(a)) == 0
+    torch.cuda.synchronize()
+    for f, o, w in zip(frames, outs, _exact(q, k, v, g)):
+        assert ((o.double() - w).norm() / w.norm()).item() <= _bound(torch.bfloat16)
+        o.fill_(7.0)
+        assert bool((f == 7.0).all())
+
+
+@pytest.mark.parametrize("heads,dim,one", [(49, 64, 0), (50, 64, 1), (98, 128, 0), (99, 128, 1), (148, 128, 1), (149, 128, 0),
+                                           (197, 128, 0), (198, 128, 1), (296, 128, 1), (149, 64, 1)])
+def test_calls_that_take_it_say_so_for_any_length(heads, dim, one):
+    from flashy_linear_attention_b200 import _lib
+    from flashy_linear_attention_b200._lib import FlaArgs
+
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, 256, dim, dim
+    assert _lib.load().fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == one
+    a.dv = dim // 2
+    assert _lib.load().fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == 0
+
+
+def test_a_tile_that_never_comes_ends_in_the_status_word():
+    from flashy_linear_attention_b200 import _lib, ops
+    from flashy_linear_attention_b200._lib import FLA_DEBUG_WITHHOLD_FIRST_TILE
+
+    q, k, v, g = _inputs(1, 100, 256, 128, torch.bfloat16, 5)
+    s_last = (k[0].double().mT @ v[0].double()).float()
+    want = _run(q, k, v, g, s_last)
+    a = _lib.FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, 100, 256, 128, 128
+    outs = [torch.empty_like(t) for t in (q, k, v)]
+    for name, t in zip(("q", "k", "v", "d_o", "d_q", "d_k", "d_v"), [q, k, v, g] + outs):
+        setattr(a, name, ops._desc(t))
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    a.s_last, a.status, a.wait_limit_us = s_last.data_ptr(), status.data_ptr(), 20000
+    a.stream = torch.cuda.current_stream(DEV).cuda_stream
+    a.debug_flags = FLA_DEBUG_WITHHOLD_FIRST_TILE
+    lib = _lib.load()
+    assert lib.fla_sm100_bwd(ctypes.byref(a)) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) & 1
+    recs = (ctypes.c_uint * (8 * 32))()
+    assert lib.fla_sm100_timeout_records(recs, 32) >= 1
+    status.zero_()
+    a.debug_flags = 0
+    assert lib.fla_sm100_bwd(ctypes.byref(a)) == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and all(torch.equal(x, y) for x, y in zip(outs, want))
