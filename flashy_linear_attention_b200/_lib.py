@@ -99,6 +99,8 @@ EXPORTED_SYMBOLS = (
     "fla_sm100_normalize_bwd_sweep",
     "fla_sm100_normalized_fused",
     "fla_sm100_normalized_fwd",
+    "fla_sm100_normalized_bwd_workspace_bytes",
+    "fla_sm100_normalized_bwd",
     "fla_sm100_taylor_dims",
     "fla_sm100_taylor_fwd",
     "fla_sm100_taylor_bwd",
@@ -174,6 +176,10 @@ def load() -> ctypes.CDLL:
     lib.fla_sm100_normalize_bwd_prepare.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_void_p, ctypes.c_void_p]
     lib.fla_sm100_normalize_bwd_sweep.restype = ctypes.c_int
     lib.fla_sm100_normalize_bwd_sweep.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_void_p]
+    lib.fla_sm100_normalized_bwd_workspace_bytes.restype = ctypes.c_size_t
+    lib.fla_sm100_normalized_bwd_workspace_bytes.argtypes = [ctypes.POINTER(FlaArgs)]
+    lib.fla_sm100_normalized_bwd.restype = ctypes.c_int
+    lib.fla_sm100_normalized_bwd.argtypes = [ctypes.POINTER(FlaArgs), ctypes.c_void_p]
     lib.fla_sm100_normalized_fused.restype = ctypes.c_int
     lib.fla_sm100_normalized_fused.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_normalized_fwd.restype = ctypes.c_int

@@ -541,6 +541,8 @@ int device_info(DeviceInfo** out) {
       norm_smem(reinterpret_cast<const void*>(fla::fla_backward_kernel<64, false>), fla::BwdCfg<64>::SMEM_BYTES);
       norm_smem(reinterpret_cast<const void*>(fla::fla_backward_kernel<64, true>), fla::BwdCfg<64>::SMEM_BYTES);
       norm_smem(reinterpret_cast<const void*>(fla::fla_backward_kernel<128, false>), fla::BwdCfg<128>::SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_backward_kernel<64, false, true>), fla::BwdCfg<64>::SMEM_BYTES);
+      norm_smem(reinterpret_cast<const void*>(fla::fla_backward_kernel<128, false, true>), fla::BwdCfg<128>::SMEM_BYTES);
       norm_smem(reinterpret_cast<const void*>(fla::fla_backward_kernel<128, true>), fla::BwdCfg<128>::SMEM_BYTES);
       norm_smem(reinterpret_cast<const void*>(fla::fla_taylor_attention_kernel<8>), fla::TaylorCfg<8>::SMEM_BYTES);
       norm_smem(reinterpret_cast<const void*>(fla::fla_taylor_attention_kernel<16>), fla::TaylorCfg<16>::SMEM_BYTES);
@@ -716,11 +718,15 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
 // three need more than twice as many rounds over the SMs (64-wide: as many). Microseconds, three / one:
 //   128-wide, 16 chunks   74 heads 77 / 83   99: 107 / 85   128: 116 / 96   180: 159 / 174   222: 196 / 179   296: 251 / 203
 //    64-wide, 16 chunks   74 heads 63 / 62   99:  91 / 62   128:  80 / 56   180:  95 /  92   222: 117 /  93   296: 141 / 101
-// One chunk: 128 heads 20 / 12.5 and 23 / 12; 40 chunks, 512 heads: 1180 / 990 and 735 / 525.
+// 40 chunks, 512 heads: 1180 / 990 and 735 / 525. It is the faster one for a single chunk too (128 heads 20 / 12.5
+// and 23 / 12), but a training step of that size is bound by the host (90 us; below eight chunks and
+// rounds the GPU needs less), and the final state that the forward then has to store is an allocation more (92.6
+// -> 96.3 us).
 bool one_cta_backward(const FlaArgs* a, int sm_count) {
   if (a->dk != a->dv || a->dk > 128) return false;
   const long heads = static_cast<long>(a->batch) * a->heads;
   auto rounds = [&](long ctas) { return (ctas + sm_count - 1) / sm_count; };
+  if (rounds(heads) * ((a->seqlen + fla::kChunk - 1) / fla::kChunk) < 8) return false;
   return a->dk > 64 ? rounds(3 * heads) > 2 * rounds(heads) : rounds(3 * heads) >= 2 * rounds(heads);
 }
 
@@ -1260,8 +1266,13 @@ void backward_products(const FlaArgs* a, Product* pq, Product* pv, Product* pk) 
   pk->ext_trans = 1;
 }
 
+// What the backward kernel's NORM variant takes beside the gradients, see BackwardParams.
+struct NormGradient {
+  const float *d, *zk, *zq;
+};
+
 // The three gradients of a head in one CTA: fla_backward_kernel. Needs s_last.
-int run_backward(const FlaArgs* a, cudaStream_t stream) {
+int run_backward(const FlaArgs* a, cudaStream_t stream, const NormGradient* norm = nullptr) {
   const int B = a->batch, H = a->heads, N = a->seqlen;
   const int tmpl = pick_template(a->dk, a->dv);
   fla::BackwardParams p;
@@ -1291,7 +1302,13 @@ int run_backward(const FlaArgs* a, cudaStream_t stream) {
   p.wait_limit_us = g_wait_limit_us;
   p.debug_withhold = g_debug_withhold;
   const dim3 grid(1, 1, B * H);
-  if (tmpl == 64) {
+  if (norm != nullptr) {
+    p.d = norm->d;
+    p.zk = norm->zk;
+    p.zq = norm->zq;
+    if (tmpl == 64) fla::fla_backward_kernel<64, false, true><<<grid, fla::kBwdThreads, fla::BwdCfg<64>::SMEM_BYTES, stream>>>(p);
+    else fla::fla_backward_kernel<128, false, true><<<grid, fla::kBwdThreads, fla::BwdCfg<128>::SMEM_BYTES, stream>>>(p);
+  } else if (tmpl == 64) {
     if (g_half) fla::fla_backward_kernel<64, true><<<grid, fla::kBwdThreads, fla::BwdCfg<64>::SMEM_BYTES, stream>>>(p);
     else fla::fla_backward_kernel<64, false><<<grid, fla::kBwdThreads, fla::BwdCfg<64>::SMEM_BYTES, stream>>>(p);
   } else {
@@ -1988,6 +2005,52 @@ int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den) {
   const NormLaunch norm = {eps, den};
   return run_products(&p, 1, a->batch, a->heads, a->seqlen, a->dk, a->dv, 1, nullptr, 0, a->status,
                       static_cast<cudaStream_t>(a->stream), *dev, false, 0, &norm);
+}
+
+// ---- the denominator's gradient inside the backward kernel
+size_t fla_sm100_normalized_bwd_workspace_bytes(const FlaArgs* a) {
+  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0 || a->dk <= 0 || a->dk != a->dv || a->dk > 128 ||
+      a->dk % 8 != 0 || a->seqlen % 4 != 0 || a->dtype != FLA_DTYPE_BF16 || a->segments > 1 ||
+      !one_cta_backward(a, current_sm_count_early()))
+    return 0;
+  const size_t nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
+  return 2 * static_cast<size_t>(a->batch) * a->heads * nchunks * a->dk * sizeof(float);
+}
+
+int fla_sm100_normalized_bwd(const FlaArgs* a, const float* dden) {
+  DeviceInfo* dev = nullptr;
+  g_last_launches = 0;
+  int rc = check_common(a, &dev);
+  if (rc) return rc;
+  if (dden == nullptr || a->s_last == nullptr) return FLA_ERR_INVALID;
+  if (a->s_init != nullptr || a->r_init != nullptr || a->r_final != nullptr) return FLA_ERR_UNSUPPORTED;
+  const size_t need = fla_sm100_normalized_bwd_workspace_bytes(a);
+  if (need == 0) return FLA_ERR_UNSUPPORTED;
+  if (a->workspace == nullptr || a->workspace_bytes < need) return FLA_ERR_WORKSPACE;
+  if (reinterpret_cast<uintptr_t>(a->workspace) % 16 != 0 || reinterpret_cast<uintptr_t>(dden) % 16 != 0) return FLA_ERR_ALIGNMENT;
+  if ((rc = check_operand(operand(a->q, a->dk), a->batch, a->heads)) || (rc = check_operand(operand(a->k, a->dk), a->batch, a->heads)))
+    return rc;
+  const int bh = a->batch * a->heads;
+  cudaStream_t stream = static_cast<cudaStream_t>(a->stream);
+  fla::NormParams p;
+  memset(&p, 0, sizeof(p));
+  p.q = norm_tensor(a->q);
+  p.k = norm_tensor(a->k);
+  p.dden = const_cast<float*>(dden);
+  p.heads = a->heads;
+  p.n = a->seqlen;
+  p.dk = a->dk;
+  p.dv = a->dv;
+  p.seg_len = fla::kChunk;
+  p.nseg = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
+  float* zk = static_cast<float*>(a->workspace);
+  float* zq = zk + static_cast<size_t>(bh) * p.nseg * a->dk;
+  if ((rc = launch_colsum(p, 0, zk, bh, stream)) || (rc = launch_colsum(p, 1, zq, bh, stream))) return rc;
+  fla::fla_chunk_prefix_kernel<<<dim3(bh, 2, 1), 128, 0, stream>>>(zk, zq, p.nseg, a->dk);
+  ++g_last_launches;
+  if (cudaGetLastError() != cudaSuccess) return FLA_ERR_CUDA;
+  const NormGradient norm = {dden, zk, zq};
+  return run_backward(a, stream, &norm);
 }
 
 int fla_sm100_product(const FlaArgs* a, int anticausal) {

@@ -47,6 +47,14 @@ struct BackwardParams {
   int* status;                // see KernelParams
   unsigned wait_limit_us;
   int debug_withhold;
+  // ---- NORM: the gradient of the attention's denominator in the same pass. With g the gradient of the product
+  // (dnum) and d_i that of the denominator of token i,
+  //     dQ_i += d_i sum_{j<=i} k_j,    dK_j += sum_{i>=j} d_i q_i.
+  // Inside the chunk d_i is a bias on the scores g_i . v_j of both, in fp32, before they are rounded; what
+  // comes from the other chunks is a vector per chunk, added in fp32 before the result is rounded.
+  const float* d;             // [bh][tokens]
+  const float* zk;            // [bh][chunks][dk]: sum of k over the chunks before
+  const float* zq;            // [bh][chunks][dk]: sum of d_i q_i over the chunks after
 };
 
 constexpr int kBwdThreads = 608;
@@ -173,7 +181,7 @@ __device__ __noinline__ void load_state(const float* src, int dim, uint32_t stat
   ptx::tc_fence_before();
 }
 
-template <int D, bool HALF>
+template <int D, bool HALF, bool NORM = false>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 fla_backward_kernel(const __grid_constant__ BackwardParams p) {
   using cfg = BwdCfg<D>;
@@ -433,16 +441,38 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       const int edge = upper ? lane - 1 : lane;
       const uint32_t flip = upper ? 0xffffffffu : 0u;
       const uint32_t src = lane_base + cfg::p_col(n) + half * 64;
+      const int tok0 = mem_chunk(n / 3) * kChunk;
+      const float* d = NORM ? p.d + static_cast<size_t>(bh) * p.n_tokens : nullptr;
+      float d_row = 0.f;
+      if (NORM && n % 3 == 2) {  // scores of dQ: a bias per row
+        const int tok = tok0 + quad * 32 + lane;
+        if (tok < p.n_tokens) d_row = __ldg(d + tok);
+      }
       if (!wait_tmem(p_full(n), (n >> 1) & 1)) break;
       if (!masked0 && !masked1) ptx::tmem_ld32x2(src, ra, src + 32, rb);
       else if (!masked0) ptx::tmem_ld32(src, ra);
       else if (!masked1) ptx::tmem_ld32(src + 32, rb);
-      auto convert_block = [&](int cb, bool masked, const uint32_t (&r)[32]) {
+      auto convert_block = [&](int cb, bool masked, uint32_t (&r)[32]) {
         uint32_t pk[16];
         if (masked) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) pk[j] = 0u;
         } else {
+          if (NORM && n % 3 == 0) {  // of dK: a bias per column (the token count is a multiple of 4)
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const int tok = tok0 + cb * 32 + j;
+              float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (tok < p.n_tokens) x = __ldg(reinterpret_cast<const float4*>(d + tok));
+              r[j] = __float_as_uint(__uint_as_float(r[j]) + x.x);
+              r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + x.y);
+              r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + x.z);
+              r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + x.w);
+            }
+          } else if (NORM) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + d_row);
+          }
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             pk[j] = ptx::pack16x2<HALF>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
@@ -474,6 +504,13 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       const CUtensorMap* map = which == 0 ? &p.dk : which == 1 ? &p.dv : &p.dq;
       const uint32_t stage = own_stage + (D == 64 ? which * kGroupBytes : 0);
       const uint32_t acc = lane_base + cfg::o_col(n);
+      const float* z = nullptr;  // NORM: what the other chunks add to this row, scaled by `scale`
+      float scale = 1.f;
+      if (NORM && which != 1) {
+        z = (which == 0 ? p.zq : p.zk) + (static_cast<size_t>(bh) * n_iter + mem_chunk(n / 3)) * p.dim;
+        const int tok = mem_chunk(n / 3) * kChunk + row;
+        if (which == 2) scale = tok < p.n_tokens ? __ldg(p.d + static_cast<size_t>(bh) * p.n_tokens + tok) : 0.f;
+      }
       // this warp's earlier stores have read the rows that are overwritten below
       if (lane == 0) ptx::bulk_wait_group_read0();
       __syncwarp();
@@ -482,7 +519,19 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
       for (int gg = 0; gg < cfg::G; ++gg) {  // one 64-column group at a time, as registers allow
         ptx::tmem_ld32x2(acc + gg * 64, ra, acc + gg * 64 + 32, rb);
         const uint32_t dst = stage + gg * kGroupBytes + row * 128;
-        auto store_half = [&](uint32_t j0, const uint32_t (&r)[32]) {
+        auto store_half = [&](uint32_t j0, uint32_t (&r)[32]) {
+          if (NORM && z != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const int c = gg * 64 + static_cast<int>(j0) * 8 + j;  // dk is a multiple of 8
+              float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (c < p.dim) x = __ldg(reinterpret_cast<const float4*>(z + c));
+              r[j] = __float_as_uint(__uint_as_float(r[j]) + scale * x.x);
+              r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) + scale * x.y);
+              r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) + scale * x.z);
+              r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) + scale * x.w);
+            }
+          }
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             ptx::st_shared_v4(dst + (((j0 + j) ^ swz) << 4),

@@ -158,6 +158,30 @@ fla_colsum_kernel(const NormParams p) {
   }
 }
 
+// Column sums per chunk -> sums over the chunks before (z = 0: of k) resp. after (z = 1: of dden_i q_i), in
+// place. A thread walks the chunks of one column, eight loads at a time.
+__global__ void __launch_bounds__(128) fla_chunk_prefix_kernel(float* zk, float* zq, int nchunks, int dk) {
+  const bool rev = blockIdx.y == 1;
+  float* base = (rev ? zq : zk) + static_cast<size_t>(blockIdx.x) * nchunks * dk;
+  for (int c = threadIdx.x; c < dk; c += 128) {
+    float run = 0.f;
+    for (int s0 = 0; s0 < nchunks; s0 += 8) {
+      float x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int s = s0 + j;
+        x[j] = s < nchunks ? base[static_cast<size_t>(rev ? nchunks - 1 - s : s) * dk + c] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int s = s0 + j;
+        if (s < nchunks) base[static_cast<size_t>(rev ? nchunks - 1 - s : s) * dk + c] = run;
+        run += x[j];
+      }
+    }
+  }
+}
+
 // Shared memory: kNormStages x (q tile, k tile, x tile) + Z [T][dkp] fp32
 __host__ __device__ inline size_t norm_fwd_smem_bytes(int dk, int dv, int tile) {
   const size_t dkp = (dk + 7) / 8 * 8, dvp = (dv + 7) / 8 * 8;

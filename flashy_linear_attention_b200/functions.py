@@ -197,6 +197,9 @@ class LinearAttentionNormalized(Function):
         q, k, v, out, den = saved[:5]
         s_final = saved[5] if ctx.has_state else None
         dnum, dden = ops.normalize_bwd_prepare(grad_output, out, den)
+        grads = ops.normalized_bwd(dnum, dden, q, k, v, s_final)
+        if grads is not None:
+            return grads + (None,)
         dq, dk, dv = ops.causal_dot_product_bwd(dnum, q, k, v, s_last=s_final, keep_padded=True)
         ops.normalize_bwd_sweep(q, k, dq, dk, dden)
         return dq, dk, dv, None

@@ -582,6 +582,32 @@ def normalized_fwd(q, k, v, eps: float, need_grad: bool):
     return out, den, s_final
 
 
+def normalized_bwd(dnum, dden, q, k, v, s_last):
+    """(dq, dk, dv) of the normalised attention from what normalize_bwd_prepare returned, with the denominator's
+    part formed in the product kernel, or None for calls that take product and normalize_bwd_sweep instead."""
+    if s_last is None or not all(t.dtype == torch.bfloat16 and t.shape == v.shape and t.device == v.device and _addressable(t)
+                                 for t in (dnum, q, k, v)):
+        return None
+    outs = [torch.empty_like(t) for t in (q, k, v)]
+    if not all(_addressable(t) for t in outs):
+        return None
+    with torch.cuda.device(q.device):
+        a = _norm_args(q, q.shape[-1], v.shape[-1])
+        a.debug_flags = _debug_flags
+        need = _lib.load().fla_sm100_normalized_bwd_workspace_bytes(ctypes.byref(a))
+        if need == 0:
+            return None
+        a.q, a.k, a.v, a.d_o = _desc(q), _desc(k), _desc(v), _desc(dnum)
+        a.d_q, a.d_k, a.d_v = (_desc(t) for t in outs)
+        a.s_last = s_last.data_ptr()
+        ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+        a.workspace, a.workspace_bytes = ws.data_ptr(), need
+        _norm_check(_lib.load().fla_sm100_normalized_bwd(ctypes.byref(a), dden.data_ptr()), "fla_sm100_normalized_bwd")
+    if os.environ.get("FLA_DEBUG", "0") == "1":
+        check_status(q.device)
+    return tuple(outs)
+
+
 def _taylor_on_chip(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> bool:
     """True for calls that the kernel on raw rows takes: those that pass the checks of the feature map and of
     the SmallVHD shapes, with values of 8 to 64 columns. What it does not take goes through the features in

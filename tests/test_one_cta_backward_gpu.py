@@ -46,11 +46,11 @@ def _run(q, k, v, g, s_last, **kw):
     return grads
 
 
-# one chunk, less than one, a ragged last one, the ring's second and third pass; 50 heads: the rule's edge at 64
-# columns, 99: at 128; 296 heads: two rounds
+# the shortest calls of the rule (eight chunks; two rounds: four), ragged last chunks, the ring's second and third
+# pass; 50 heads: the rule's edge at 64 columns, 99: at 128; 296 heads: two rounds
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("B,H,N,D", [(2, 50, 64, 128), (1, 99, 128, 128), (4, 25, 192, 83), (2, 64, 320, 96), (1, 100, 1216, 128),
-                                     (1, 50, 64, 64), (2, 32, 128, 40), (1, 64, 448, 64), (1, 60, 1216, 64), (2, 148, 192, 64)])
+@pytest.mark.parametrize("B,H,N,D", [(2, 50, 960, 128), (1, 99, 1024, 128), (4, 25, 1088, 83), (2, 64, 1344, 96), (1, 100, 1216, 128),
+                                     (1, 50, 960, 64), (2, 32, 1024, 40), (1, 64, 1472, 64), (1, 60, 1216, 64), (2, 148, 448, 64)])
 def test_gradients_against_64_bits(B, H, N, D, dtype):
     from flashlinear import LinearAttention
     from flashy_linear_attention_b200 import ops
@@ -67,7 +67,7 @@ def test_gradients_against_64_bits(B, H, N, D, dtype):
 
 @pytest.mark.parametrize("with_s", [False, True])
 @pytest.mark.parametrize("with_r", [False, True])
-@pytest.mark.parametrize("H,N,D", [(100, 128, 128), (100, 576, 96), (64, 128, 64), (64, 576, 48)])
+@pytest.mark.parametrize("H,N,D", [(100, 1024, 128), (100, 1096, 96), (64, 1024, 64), (64, 1100, 48)])
 def test_states_before_and_after(H, N, D, with_s, with_r):
     q, k, v, g = _inputs(1, H, N, D, torch.bfloat16, N)
     gen = torch.Generator(device=DEV).manual_seed(D)
@@ -88,7 +88,7 @@ def test_strided_inputs_and_guard_bands():
     from flashy_linear_attention_b200 import _lib, ops
     from flashy_linear_attention_b200._lib import FlaArgs
 
-    B, H, N, D = 1, 100, 200, 128
+    B, H, N, D = 1, 100, 1000, 128
     q, k, v, g = (t.transpose(1, 2).contiguous().transpose(1, 2) for t in _inputs(B, H, N, D, torch.bfloat16, 3))
     s_last = (k[0].double().mT @ v[0].double()).float()
     frames = [torch.full((B, H, N + 4, D + 8), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(3)]
@@ -110,26 +110,30 @@ def test_strided_inputs_and_guard_bands():
 
 @pytest.mark.parametrize("heads,dim,one", [(49, 64, 0), (50, 64, 1), (98, 128, 0), (99, 128, 1), (148, 128, 1), (149, 128, 0),
                                            (197, 128, 0), (198, 128, 1), (296, 128, 1), (149, 64, 1)])
-def test_calls_that_take_it_say_so_for_any_length(heads, dim, one):
+@pytest.mark.parametrize("tokens", [1024, 8192])
+def test_calls_that_take_it_say_so(heads, dim, one, tokens):
     from flashy_linear_attention_b200 import _lib
     from flashy_linear_attention_b200._lib import FlaArgs
 
     a = FlaArgs()
-    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, 256, dim, dim
-    assert _lib.load().fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == one
-    a.dv = dim // 2
-    assert _lib.load().fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == 0
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, tokens, dim, dim
+    uses = _lib.load().fla_sm100_bwd_uses_final_state
+    assert uses(ctypes.byref(a)) == (one or tokens > 2048)
+    a.seqlen = 256  # bound by the host: no state is stored
+    assert uses(ctypes.byref(a)) == 0
+    a.seqlen, a.dv = 1024, dim // 2
+    assert uses(ctypes.byref(a)) == 0
 
 
 def test_a_tile_that_never_comes_ends_in_the_status_word():
     from flashy_linear_attention_b200 import _lib, ops
     from flashy_linear_attention_b200._lib import FLA_DEBUG_WITHHOLD_FIRST_TILE
 
-    q, k, v, g = _inputs(1, 100, 256, 128, torch.bfloat16, 5)
+    q, k, v, g = _inputs(1, 100, 1024, 128, torch.bfloat16, 5)
     s_last = (k[0].double().mT @ v[0].double()).float()
     want = _run(q, k, v, g, s_last)
     a = _lib.FlaArgs()
-    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, 100, 256, 128, 128
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, 100, 1024, 128, 128
     outs = [torch.empty_like(t) for t in (q, k, v)]
     for name, t in zip(("q", "k", "v", "d_o", "d_q", "d_k", "d_v"), [q, k, v, g] + outs):
         setattr(a, name, ops._desc(t))
