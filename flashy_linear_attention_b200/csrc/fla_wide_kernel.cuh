@@ -149,7 +149,7 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_holder, 0);  // provably warp-uniform
+  const uint32_t tmem_base = *tmem_holder;
 
   auto wait_uniform = [&](uint32_t bar, uint32_t parity) {
     const int ok = ptx::mbar_wait(bar, parity, abort_flag) ? 1 : 0;
@@ -202,11 +202,6 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
               ptx::mbar_expect_tx(full_bar(s), kWideGroupBytes);
               ptx::tma_load_4d(group_addr(g), w == 0 ? &p.a : &p.b, full_bar(s), t * 128 + gg * 64,
                                tok, h, b);
-              // Slots are freed one chunk ahead at most: the next chunk's tile comes into L2 now, fetched by one of
-              // the slices that share it (128 heads x 2048, 160 / 32: 44.1 us without, 41.7 with; three pairs
-              // stream at the rate of HBM and lose: 280 / 64 72.4, 74.5 with).
-              if (NT == 2 && i + 1 < n_iter && static_cast<int>((g >> 1) % gridDim.x) == static_cast<int>(blockIdx.x))
-                ptx::tma_prefetch_4d(w == 0 ? &p.a : &p.b, t * 128 + gg * 64, mem_chunk(i + 1) * kWideChunk, h, b);
             }
           }
           if (!ok) break;
@@ -232,6 +227,13 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
       const bool have_state = i > 0;
       const int cs = i & 1;
       const uint32_t c_lo = ptx::desc_lo(c_addr + cs * kWideGroupBytes, kWideGroupBytes);  // MN-major
+      if (!wait_uniform(cfull_bar(cs), (i >> 1) & 1)) break;
+      if (i > 0) {
+        // the epilogue has drained O of chunk i-1; the converters have read S of chunk i-1 out of
+        // tensor memory and its bf16 copy is in shared memory
+        if (!wait_uniform(o_free, (i - 1) & 1)) break;
+        if (!wait_uniform(sb_ready, (i - 1) & 1)) break;
+      }
       for (int t = 0; t < NT; ++t) {
         const int groups = pair_groups(t);
         const int ga = tile_group(i, t, 0);
@@ -246,60 +248,51 @@ fla_wide_kernel(const __grid_constant__ WideParams p) {
         const uint32_t a_lo = ptx::desc_lo(group_addr(ga), 16);                // K-major
         const uint32_t b_lo = ptx::desc_lo(group_addr(gb), 16);                // K-major
         const uint32_t bt_lo = ptx::desc_lo(group_addr(gb), kWideGroupBytes);  // MN-major
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t off = ((kk >> 2) * kWideGroupBytes + (kk & 3) * 32) >> 4;
-          ptx::mma_ss_on(leader && kk < ksteps, tP, a_lo + off, b_lo + off, ptx::kDescHi, IDESC_P,
-                         (t > 0 || kk > 0) ? 1u : 0u);
-        }
-        if (t == NT - 1) ptx::tc_commit_on(leader, p_full);
-        if (t == 0) {
-          // Only now, behind the first pair's scores: the epilogue has drained O of chunk i-1, the converters
-          // have read S of chunk i-1 out of tensor memory and its bf16 copy is in shared memory. (Waiting before
-          // them: 32 heads x 4096 x 256 95 us, here 84. All pairs' scores first hold up the release of pair 0's
-          // slots: 99 - 101 us.)
-          ok = wait_uniform(cfull_bar(cs), (i >> 1) & 1) &&
-               (i == 0 || (wait_uniform(o_free, (i - 1) & 1) && wait_uniform(sb_ready, (i - 1) & 1)));
-          if (!ok) break;
-          ptx::tc_fence_after();
-        }
-        if (have_state) {
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
+        if (leader) {
+          for (int kk = 0; kk < ksteps; ++kk) {
             const uint32_t off = ((kk >> 2) * kWideGroupBytes + (kk & 3) * 32) >> 4;
-            ptx::mma_ss_on(leader && kk < ksteps, tO, a_lo + off, sb_lo + (t * 8 + kk) * (2048 >> 4), ptx::kDescHi,
-                           IDESC_AS, (t > 0 || kk > 0) ? 1u : 0u);
+            ptx::mma_ss(tP, a_lo + off, b_lo + off, ptx::kDescHi, IDESC_P, (t > 0 || kk > 0) ? 1u : 0u);
           }
-        }
-        // The instruction spans 128 state rows; rows past the loaded columns of b read whatever
-        // the slot holds and land in tensor-memory lanes nobody reads.
+          if (t == NT - 1) ptx::tc_commit(p_full);
+          if (have_state) {
+            for (int kk = 0; kk < ksteps; ++kk) {
+              const uint32_t off = ((kk >> 2) * kWideGroupBytes + (kk & 3) * 32) >> 4;
+              ptx::mma_ss(tO, a_lo + off, sb_lo + (t * 8 + kk) * (2048 >> 4), ptx::kDescHi, IDESC_AS,
+                          (t > 0 || kk > 0) ? 1u : 0u);
+            }
+          }
+          // The instruction spans 128 state rows; rows past the loaded columns of b read whatever
+          // the slot holds and land in tensor-memory lanes nobody reads.
 #pragma unroll
-        for (int kk = 0; kk < kWideChunk / 16; ++kk) {
-          ptx::mma_ss_on(leader, tS + t * 64, bt_lo + kk * (2048 >> 4), c_lo + kk * (2048 >> 4), ptx::kDescHi,
-                         IDESC_S, (have_state || kk > 0) ? 1u : 0u);
-        }
-        for (int gg = 0; gg < groups; ++gg) {
-          ptx::tc_commit_on(leader, empty_bar((ga + gg) % kWideSlots));
-          ptx::tc_commit_on(leader, empty_bar((gb + gg) % kWideSlots));
+          for (int kk = 0; kk < kWideChunk / 16; ++kk) {
+            ptx::mma_ss(tS + t * 64, bt_lo + kk * (2048 >> 4), c_lo + kk * (2048 >> 4), ptx::kDescHi,
+                        IDESC_S, (have_state || kk > 0) ? 1u : 0u);
+          }
+          for (int gg = 0; gg < groups; ++gg) {
+            ptx::tc_commit(empty_bar((ga + gg) % kWideSlots));
+            ptx::tc_commit(empty_bar((gb + gg) % kWideSlots));
+          }
         }
         __syncwarp();
       }
       if (!ok) break;
-      ptx::tc_commit_on(leader, s_full);  // S of chunk i complete, Sb no longer read
+      if (leader) ptx::tc_commit(s_full);  // S of chunk i complete, Sb no longer read
       __syncwarp();
       if (!wait_uniform(pb_ready, i & 1)) break;
       ptx::tc_fence_after();
+      if (leader) {
 #pragma unroll
-      for (int kk = 0; kk < kWideChunk / 16; ++kk) {
-        ptx::mma_ts_on(leader, tO, tPb + kk * 8, c_lo + kk * (2048 >> 4), ptx::kDescHi, IDESC_PC,
-                       (have_state || kk > 0) ? 1u : 0u);
+        for (int kk = 0; kk < kWideChunk / 16; ++kk) {
+          ptx::mma_ts(tO, tPb + kk * 8, c_lo + kk * (2048 >> 4), ptx::kDescHi, IDESC_PC,
+                      (have_state || kk > 0) ? 1u : 0u);
+        }
+        ptx::tc_commit(o_full);
+        ptx::tc_commit(cempty_bar(cs));
       }
-      ptx::tc_commit_on(leader, o_full);
-      ptx::tc_commit_on(leader, cempty_bar(cs));
       __syncwarp();
     }
     // Nobody waits for the last chunk's releases; the barriers have to outlive them all the same.
-    ptx::tc_commit_on(leader, drained);
+    if (leader) ptx::tc_commit(drained);
     __syncwarp();
     wait_uniform(drained, 0);
   } else if (warp < 10) {
