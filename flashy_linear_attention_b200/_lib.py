@@ -88,6 +88,7 @@ EXPORTED_SYMBOLS = (
     "fla_sm100_auto_segments",
     "fla_sm100_seg_states_bytes",
     "fla_sm100_bwd_uses_final_state",
+    "fla_sm100_bwd_one_cta",
     "fla_sm100_fwd",
     "fla_sm100_bwd",
     "fla_sm100_state",
@@ -148,6 +149,8 @@ def load() -> ctypes.CDLL:
     lib.fla_sm100_seg_states_bytes.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_bwd_uses_final_state.restype = ctypes.c_int
     lib.fla_sm100_bwd_uses_final_state.argtypes = [ctypes.POINTER(FlaArgs)]
+    lib.fla_sm100_bwd_one_cta.restype = ctypes.c_int
+    lib.fla_sm100_bwd_one_cta.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_fwd.restype = ctypes.c_int
     lib.fla_sm100_fwd.argtypes = [ctypes.POINTER(FlaArgs)]
     lib.fla_sm100_bwd.restype = ctypes.c_int

@@ -766,19 +766,20 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
 }
 
 // Unsegmented backward calls that give a head's three gradients one CTA (fla_backward_kernel) instead of
-// three. Such a CTA takes two to two and a half times as long for a chunk (64-wide: twice), so it pays where the
+// three. Its dQ takes the state before a chunk as the final state minus the sum over that chunk and all later
+// ones, like the single sweep's, and so it has the single sweep's length rule: in a short call dQ of a token depends
+// on no later one, and an Inf, a NaN or a row a thousand times larger further on must not reach it.
+// Such a CTA takes two to two and a half times as long for a chunk (64-wide: twice), so it pays where the
 // three need more than twice as many rounds over the SMs (64-wide: as many). Microseconds, three / one:
 //   128-wide, 16 chunks   74 heads 77 / 83   99: 107 / 85   128: 116 / 96   180: 159 / 174   222: 196 / 179   296: 251 / 203
 //    64-wide, 16 chunks   74 heads 63 / 62   99:  91 / 62   128:  80 / 56   180:  95 /  92   222: 117 /  93   296: 141 / 101
-// 40 chunks, 512 heads: 1180 / 990 and 735 / 525. It is the faster one for a single chunk too (128 heads 20 / 12.5
-// and 23 / 12), but a training step of that size is bound by the host (90 us; below eight chunks and
-// rounds the GPU needs less), and the final state that the forward then has to store is an allocation more (92.6
-// -> 96.3 us).
+// 40 chunks, 512 heads: 1180 / 990 and 735 / 525.
 bool one_cta_backward(const FlaArgs* a, int sm_count) {
-  if (a->dk != a->dv || a->dk > 128) return false;
+  if (a->dk != a->dv || a->dk > 128 || a->segments > 1) return false;
+  const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
+  if (nchunks < kSingleSweepMinChunks && !(a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP)) return false;
   const long heads = static_cast<long>(a->batch) * a->heads;
   auto rounds = [&](long ctas) { return (ctas + sm_count - 1) / sm_count; };
-  if (rounds(heads) * ((a->seqlen + fla::kChunk - 1) / fla::kChunk) < 8) return false;
   return a->dk > 64 ? rounds(3 * heads) > 2 * rounds(heads) : rounds(3 * heads) >= 2 * rounds(heads);
 }
 
@@ -1458,13 +1459,17 @@ int fla_sm100_bwd_uses_final_state(const FlaArgs* a) {
   if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0) return 0;
   if (a->dk > 128 || a->dv > 128) return 0;
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
-  if (a->segments <= 1 && one_cta_backward(a, current_sm_count_early())) return 1;
   if (!(nchunks >= kSingleSweepMinChunks || (a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP))) return 0;
   if (fla_sm100_seg_states_bytes(a) > 0) return 1;
   int nseg = a->segments > 0 ? a->segments
                              : auto_segments(SplitForm::kBackward, a->batch * a->heads, nchunks,
                                              current_sm_count_early(), a->dk, a->dv);
   return nseg <= 1 ? 1 : 0;
+}
+
+int fla_sm100_bwd_one_cta(const FlaArgs* a) {
+  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0 || a->dk <= 0) return 0;
+  return one_cta_backward(a, current_sm_count_early()) ? 1 : 0;
 }
 
 int fla_sm100_fwd(const FlaArgs* a) {
@@ -1557,7 +1562,6 @@ int fla_sm100_bwd(const FlaArgs* a) {
   int nseg = a->segments > 0 ? a->segments
                              : auto_segments(SplitForm::kBackward, a->batch * a->heads, nchunks, dev->sm_count, a->dk, a->dv);
   if (nseg > nchunks) nseg = nchunks;
-  // (Its dQ is no difference of two sums over a chunk, so the length rule of the single sweep is not its own.)
   if (a->s_last != nullptr && nseg <= 1 && one_cta_backward(a, dev->sm_count)) return run_backward(a, stream);
   if (a->s_last != nullptr && nseg <= 1 && single_sweep_allowed(nchunks)) {
     // The forward state after this call's tokens is known: dQ can walk the sequence in the same
@@ -2069,7 +2073,7 @@ int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den) {
 // 680 us with the kernels, 604 with this. Errors against 64 bits (dq, dk): 8.5e-3, 5.0e-3 -> 7.1e-3, 4.5e-3.
 size_t fla_sm100_normalized_bwd_workspace_bytes(const FlaArgs* a) {
   if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0 || a->dk <= 0 || a->dk != a->dv || a->dk > 128 ||
-      a->dk % 8 != 0 || a->seqlen % 4 != 0 || a->dtype != FLA_DTYPE_BF16 || a->segments > 1 ||
+      a->dk % 8 != 0 || a->seqlen % 4 != 0 || a->dtype != FLA_DTYPE_BF16 ||
       !one_cta_backward(a, current_sm_count_early()))
     return 0;
   const size_t nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;

@@ -717,9 +717,8 @@ def backward_uses_final_state(q: torch.Tensor, v: torch.Tensor) -> bool:
     """True when the backward of this shape can take the forward's final state (`s_last`) and sweep
     q, k, v, dO once for all three gradients: it runs unsegmented, or as one launch split at the
     forward's segment boundaries (then segment_states_buffer() is not None as well), and the
-    sequence is longer than 2048 tokens (shorter ones keep the two-direction form, which is a
-    little more accurate there) or there are heads enough for one CTA each (that form has no
-    difference of sums over a chunk)."""
+    sequence is longer than 2048 tokens (shorter ones keep the two-direction form, in which no later
+    token reaches dQ and which is a little more accurate there)."""
     B, H, N, dk = q.shape
     if dk > KERNEL_HEAD_DIM or v.shape[-1] > KERNEL_HEAD_DIM:
         return False

@@ -83,9 +83,12 @@ typedef struct FlaArgs {
   float* r_final;
   /* Backward only, optional: the forward state AFTER this call's tokens (what the forward call
    * wrote to s_final). When given (and fla_sm100_bwd_uses_final_state() says so: the call is not
-   * split into segments or comes with seg_states, and the sequence is longer than 2048 tokens or there are
-   * heads enough for one CTA each) dQ is computed in the same end-to-start sweep as dK and dV, which lets the
-   * three share every read of q, k, v, dO; s_init then only says whether anything precedes the first token. */
+   * split into segments or comes with seg_states, and the sequence is longer than 2048 tokens) dQ is
+   * computed in the same end-to-start sweep as dK and dV, which lets the three share every read of q, k,
+   * v, dO; s_init then only says whether anything precedes the first token. The state before a chunk is
+   * then s_last minus what follows: an Inf or NaN in k or v of a token makes dQ of all earlier chunks (but
+   * the first of a sequence) non-finite, and rows that are larger by orders of magnitude cost it accuracy.
+   * Calls of at most 2048 tokens sum dQ's state from the start, where no later token reaches it. */
   const float* s_last;
 
   /* Sequence segments per head (intra-GPU sequence split). 0 = pick automatically, 1 = none.
@@ -142,9 +145,9 @@ typedef struct FlaArgs {
  * launches apart. A process that replays many captured graphs on concurrent streams should set
  * this bit for all but one of the streams. */
 #define FLA_DEBUG_NO_FUSED_SEGMENTS 2u
-/* With a CTA per gradient the backward uses s_last (dQ in the same end-to-start sweep as dK and dV) only for
- * sequences longer than 2048 tokens; on shorter ones that form is a little less accurate than the
- * two-direction form and saves nothing worth having. This bit lifts the length rule, for tests. */
+/* The backward uses s_last (dQ in the same end-to-start sweep as dK and dV) only for sequences longer than
+ * 2048 tokens: in shorter ones dQ is summed from the start, see s_last. This bit lifts the length rule, for
+ * tests. */
 #define FLA_DEBUG_FORCE_SINGLE_SWEEP 4u
 
 /* Diagnostics for bit 0 of the status word: copies up to max_records records (8 words each) of the
@@ -169,8 +172,11 @@ int fla_sm100_auto_segments(const FlaArgs* args, int pass);
 size_t fla_sm100_seg_states_bytes(const FlaArgs* args);
 /* 1 when fla_sm100_bwd for these shapes makes use of s_last (so that the forward should be asked
  * for s_final), 0 when it would ignore it: segmented backward without seg_states, sequences of at
- * most 2048 tokens unless there are heads enough for one CTA each, head dims above 128. */
+ * most 2048 tokens, head dims above 128. */
 int fla_sm100_bwd_uses_final_state(const FlaArgs* args);
+/* 1 when fla_sm100_bwd, given s_last, computes the three gradients of a head in one CTA for these shapes (heads
+ * enough to fill the GPU that way, more than 2048 tokens), 0 when it takes a CTA for each. */
+int fla_sm100_bwd_one_cta(const FlaArgs* args);
 
 /* replaces linear_flash_wrapper_fwd / linear_flash_wrapper_fwd_smallv_hd
  * (flashlinear/kernels/linear_attn_kernels.py:310, linear_attn_kernels_smallv_hd.py:320) */

@@ -157,6 +157,24 @@ def test_host_pipeline_has_no_cpu_fallback():
         HostPipeline("cpu")
 
 
+@pytest.mark.parametrize("tokens", [128, 1024, 1984, 2048])
+@pytest.mark.parametrize("heads", [99, 128, 296, 512, 1100])
+@pytest.mark.parametrize("dim", [32, 64, 128])
+def test_short_backward_never_starts_from_the_final_state(heads, tokens, dim):
+    """Up to 2048 tokens dQ is summed from the start, whatever the number of heads (one late Inf would otherwise reach
+    dQ of all earlier tokens): neither the single sweep nor the form with one CTA a head is taken."""
+    from flashy_linear_attention_b200 import _lib
+
+    lib = _lib.load()
+    a = _lib.FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, tokens, dim, dim
+    assert lib.fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == 0
+    assert lib.fla_sm100_bwd_one_cta(ctypes.byref(a)) == 0
+    assert lib.fla_sm100_normalized_bwd_workspace_bytes(ctypes.byref(a)) == 0
+    a.seqlen = 2112
+    assert lib.fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == 1
+
+
 def test_segment_planning_queries_without_a_gpu():
     """How a call will be split is host arithmetic (148 SMs assumed when no device answers): the
     queries that size the caller's scratch must agree with each other for the shapes of the

@@ -9,6 +9,16 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
+@pytest.fixture
+def any_length():
+    """Lifts the rule that the kernel only runs above 2048 tokens."""
+    from flashy_linear_attention_b200 import _lib, ops
+
+    old = ops.set_debug_flags(_lib.FLA_DEBUG_FORCE_SINGLE_SWEEP)
+    yield
+    ops.set_debug_flags(old)
+
+
 def _inputs(B, H, N, D, bnhd):
     gen = torch.Generator(device=DEV).manual_seed(N + D)
 
@@ -23,7 +33,7 @@ def _inputs(B, H, N, D, bnhd):
 # the rule's edges in heads, ragged last chunks (a multiple of 4 tokens), whole and partly used tiles, two rounds
 @pytest.mark.parametrize("B,H,N,D,bnhd", [(1, 99, 1024, 128, False), (1, 100, 1100, 96, True), (2, 50, 1252, 128, True),
                                           (1, 50, 1024, 64, True), (1, 60, 1156, 40, False), (2, 148, 580, 64, False)])
-def test_against_64_bits(B, H, N, D, bnhd):
+def test_against_64_bits(any_length, B, H, N, D, bnhd):
     from flashy_linear_attention_b200 import ops
 
     q, k, v, dnum = _inputs(B, H, N, D, bnhd)
@@ -44,7 +54,7 @@ def test_against_64_bits(B, H, N, D, bnhd):
         assert rel <= cancel * 2.0**-9 * math.sqrt((1 + 4 + 4) / 3), (name, rel)
 
 
-def test_is_as_close_to_64_bits_as_the_separate_kernels():
+def test_is_as_close_to_64_bits_as_the_separate_kernels(any_length):
     from flashy_linear_attention_b200 import LinearAttentionNormalized, ops
 
     q, k, v, g = _inputs(1, 100, 1024, 128, False)
@@ -63,9 +73,9 @@ def test_is_as_close_to_64_bits_as_the_separate_kernels():
 
 
 @pytest.mark.parametrize("shape,dtype", [((1, 98, 1024, 128), torch.bfloat16), ((1, 100, 1024, 84), torch.bfloat16),
-                                         ((1, 100, 1022, 128), torch.bfloat16), ((1, 100, 256, 128), torch.bfloat16),
+                                         ((1, 100, 1022, 128), torch.bfloat16),
                                          ((1, 100, 1024, 128), torch.float16)])
-def test_calls_that_keep_the_separate_kernels(shape, dtype):
+def test_calls_that_keep_the_separate_kernels(any_length, shape, dtype):
     from flashy_linear_attention_b200 import ops
 
     q = torch.zeros(shape, dtype=dtype, device=DEV)
@@ -74,3 +84,12 @@ def test_calls_that_keep_the_separate_kernels(shape, dtype):
     s = torch.zeros(B * H, D, D, device=DEV)
     assert ops.normalized_bwd(q, dden, q, q, q, s) is None
     assert ops.normalized_bwd(q, dden, q, q, q, None) is None
+
+
+@pytest.mark.parametrize("tokens,inside", [(2048, False), (2052, True)])
+def test_short_calls_keep_the_separate_kernels(tokens, inside):
+    from flashy_linear_attention_b200 import ops
+
+    q = torch.zeros(1, 100, tokens, 128, dtype=torch.bfloat16, device=DEV)
+    grads = ops.normalized_bwd(q, torch.zeros(100, tokens, device=DEV), q, q, q, torch.zeros(100, 128, 128, device=DEV))
+    assert (grads is not None) == inside
