@@ -769,18 +769,35 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
 // three. Its dQ takes the state before a chunk as the final state minus the sum over that chunk and all later
 // ones, like the single sweep's, and so it has the single sweep's length rule: in a short call dQ of a token depends
 // on no later one, and an Inf, a NaN or a row a thousand times larger further on must not reach it.
-// Such a CTA takes two to two and a half times as long for a chunk (64-wide: twice), so it pays where the
-// three need more than twice as many rounds over the SMs (64-wide: as many). Microseconds, three / one:
-//   128-wide, 16 chunks   74 heads 77 / 83   99: 107 / 85   128: 116 / 96   180: 159 / 174   222: 196 / 179   296: 251 / 203
-//    64-wide, 16 chunks   74 heads 63 / 62   99:  91 / 62   128:  80 / 56   180:  95 /  92   222: 117 /  93   296: 141 / 101
-// 40 chunks, 512 heads: 1180 / 990 and 735 / 525.
-bool one_cta_backward(const FlaArgs* a, int sm_count) {
+// Such a CTA takes about twice as long for a chunk as one of three, so it pays where the three need more than twice
+// as many rounds over the SMs. Three / one, by heads, times of the backward at 2112 and 4096 tokens:
+//    64-wide   50 1.01 1.00 (8192: 0.98)  98 1.04 1.01   99 1.45 1.45   149 1.07 1.02 (8192: 1.00)  180 1.05 0.99   198 1.28 1.22   297 1.23 1.16
+//    32-wide   50 1.04 1.00   98 1.12 1.04   99 1.46 1.45   149 1.09 1.05   180 1.08 1.05   198 1.29 1.27   297 1.27 1.23
+//   128-wide   99 1.31 1.33   198 1.04 1.04   206 1.09 1.07   247 1.20 1.19   297 1.02 1.00   330 1.06 1.03   444 1.27 1.21
+//   112-wide   99 1.18 1.19   198 1.02 0.99   206 1.05 1.03   247 1.19 1.17   297 0.99 0.96   330 1.05 1.01   444 1.29 1.23
+//    72-wide   99 1.13 1.13   198 0.96 0.94   230 1.06 0.99   247 1.14 1.12   297 0.94 0.91   346 1.06 1.00   444 1.30 1.24
+// (us, 4096 tokens, 99 heads: 64-wide 125 / 87, 128-wide 199 / 159.) Below 64 as many rounds are enough. Above 64, in
+// more than one round, the three are held against their work and not their rounds, since CTAs of a last round that
+// is nearly empty run faster: 2.05 times the one's rounds; 2.3 where rows are an odd number of 16-byte pieces (72,
+// 88, 104, 120 columns), half a 32-byte sector.
+// norm: with the denominator's gradient inside, against one of the two forms above and kernels for that gradient.
+// Those are slow but for 64 and 128 columns, so that the other widths gain everywhere in the widest rule (1.0 to 1.5);
+// separate / inside for the whole step at 2112 and 4096 tokens:
+//    64-wide   50 0.96 0.89   98 0.99 1.00   99 1.10 1.11   180 0.98 0.97   198 1.05 1.04   297 1.08 1.03
+//   128-wide   99 1.03 1.04   198 0.97 0.97   214 1.00 1.00   230 1.04 1.02   297 0.98 0.98   346 1.03 1.03
+//    40-wide   50 1.13 1.09   149 1.20 1.19   96-wide   99 1.21 1.21   198 1.16 1.15   297 1.18 1.17
+bool one_cta_backward(const FlaArgs* a, int sm_count, bool norm = false) {
   if (a->dk != a->dv || a->dk > 128 || a->segments > 1) return false;
   const int nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   if (nchunks < kSingleSweepMinChunks && !(a->debug_flags & FLA_DEBUG_FORCE_SINGLE_SWEEP)) return false;
   const long heads = static_cast<long>(a->batch) * a->heads;
   auto rounds = [&](long ctas) { return (ctas + sm_count - 1) / sm_count; };
-  return a->dk > 64 ? rounds(3 * heads) > 2 * rounds(heads) : rounds(3 * heads) >= 2 * rounds(heads);
+  const long one = rounds(heads), three = rounds(3 * heads);
+  if (a->dk < 64) return three >= 2 * one;
+  if (three <= 2 * one) return false;
+  if (one == 1 || a->dk == 64 || (norm && a->dk != 128)) return true;
+  const bool odd_row = (a->dk + 7) / 8 % 2 != 0;
+  return 100 * 3 * heads >= (norm || odd_row ? 230 : 205) * one * sm_count;
 }
 
 // Bytes of the boundary states a fused forward stores for a fused backward, or 0 when the pair of
@@ -2074,7 +2091,7 @@ int fla_sm100_normalized_fwd(const FlaArgs* a, float eps, float* den) {
 size_t fla_sm100_normalized_bwd_workspace_bytes(const FlaArgs* a) {
   if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0 || a->dk <= 0 || a->dk != a->dv || a->dk > 128 ||
       a->dk % 8 != 0 || a->seqlen % 4 != 0 || a->dtype != FLA_DTYPE_BF16 ||
-      !one_cta_backward(a, current_sm_count_early()))
+      !one_cta_backward(a, current_sm_count_early(), true))
     return 0;
   const size_t nchunks = (a->seqlen + fla::kChunk - 1) / fla::kChunk;
   return 2 * static_cast<size_t>(a->batch) * a->heads * nchunks * a->dk * sizeof(float);
