@@ -305,7 +305,7 @@ std::optional<std::array<Tensor, 3>> backward(const Tensor& g, const Tensor& q, 
 bool taylor_covered(const Tensor& q, const Tensor& k, const Tensor& v) {
   const int64_t d = q.dim() == 4 ? q.size(3) : 0, dv = v.dim() == 4 ? v.size(3) : 0;
   return usable(q, q) && usable(k, q) && usable(v, q) && same_rows(q, k) && same_rows(q, v) && k.size(3) == d &&
-         (d == 8 || d == 16) && dv % 8 == 0 && dv <= 64 && q.scalar_type() == at::kBFloat16 && covered_dims(q, v);
+         (d == 8 || d == 16) && (dv == 8 || dv == 16 || dv == 32 || dv == 64) && q.scalar_type() == at::kBFloat16 && covered_dims(q, v);
 }
 std::optional<Tensor> taylor_forward(const Tensor& q, const Tensor& k, const Tensor& v, unsigned debug_flags, uintptr_t status) {
   if (!taylor_covered(q, k, v)) return std::nullopt;

@@ -212,28 +212,30 @@ class TaylorLinearAttention(Function):
     vec(x x^T) / (sqrt(2) sqrt(d))]`` (benchmark configuration 4: d = 16 -> 273 features), and its
     backward returns gradients with respect to the raw xq, xk and v.
 
-    The features are formed on chip and never exist in memory, in neither pass, and nothing but xq, xk and v
-    is kept for the backward (values wider than 64 columns, or of a width that is no multiple of 8, go through feature tensors in memory, in
-    both passes). The reference has no counterpart.
+    With values of 8, 16, 32 or 64 columns the features are formed on chip and never exist in memory, in neither
+    pass, and nothing but xq, xk and v is kept for the backward. Other powers of two go through feature tensors in memory,
+    which are kept; widths that are no power of two are refused (as by ``LinearAttentionSmallVHD``).
+    The reference has no counterpart.
     """
 
     @staticmethod
     @_autocast_to_bf16
     def forward(ctx: Any, xq, xk, v):
-        out = ops.taylor_forward(xq, xk, v)
-        if out is None:  # errors, and values wider than 64 columns
-            pq, pk = ops.taylor_features(xq), ops.taylor_features(xk)
-            ops.check_forward_preconditions(pq, v, smallv=True)
-            out = ops.causal_dot_product_fwd(pq, pk, v)
-        ctx.save_for_backward(xq, xk, v)
+        out, features = ops.taylor_forward(xq, xk, v), ()
+        if out is None:  # errors, and what does not run on chip
+            features = ops.taylor_features(xq), ops.taylor_features(xk)
+            ops.check_forward_preconditions(features[0], v, smallv=True)
+            out = ops.causal_dot_product_fwd(*features, v)
+        ctx.save_for_backward(xq, xk, v, *features)
         return out
 
     @staticmethod
     def backward(ctx: Any, grad_output):
-        xq, xk, v = ctx.saved_tensors
-        grads = ops.taylor_backward(grad_output, xq, xk, v)
-        if grads is not None:
-            return tuple(grads)
-        pq, pk = ops.taylor_features(xq), ops.taylor_features(xk)
-        dpq, dpk, dv = ops.causal_dot_product_bwd(grad_output, pq, pk, v, keep_padded=True)
+        xq, xk, v, *features = ctx.saved_tensors
+        if not features:
+            grads = ops.taylor_backward(grad_output, xq, xk, v)
+            if grads is not None:
+                return tuple(grads)
+            features = ops.taylor_features(xq), ops.taylor_features(xk)
+        dpq, dpk, dv = ops.causal_dot_product_bwd(grad_output, *features, v, keep_padded=True)
         return ops.taylor_features_bwd(dpq, xq), ops.taylor_features_bwd(dpk, xk), dv

@@ -610,7 +610,7 @@ def normalized_bwd(dnum, dden, q, k, v, s_last):
 
 def _taylor_on_chip(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> bool:
     """True for calls that the kernel on raw rows takes: those that pass the checks of the feature map and of
-    the SmallVHD shapes, with values of 8 to 64 columns. What it does not take goes through the features in
+    the SmallVHD shapes, with values of 8, 16, 32 or 64 columns. What it does not take goes through the features in
     memory, which report the errors."""
     if not all(t.is_cuda and t.device == xq.device and t.dtype == torch.bfloat16 and t.dim() == 4 for t in (xq, xk, v)):
         return False

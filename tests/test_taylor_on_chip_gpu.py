@@ -72,6 +72,32 @@ def test_every_path_to_the_kernel_gives_the_same(monkeypatch):
     assert ((wide[..., :64].double() - want[0].double()).norm() / want[0].double().norm()).item() < 2.0**-7
 
 
+# the narrowest and widest value widths on both sides of those that run on chip
+@pytest.mark.parametrize("d", [8, 16])
+@pytest.mark.parametrize("dv,kept", [(1, 2), (4, 2), (8, 0), (64, 0), (128, 2)])
+def test_features_in_memory_are_formed_once(d, dv, kept):
+    from flashy_linear_attention_b200 import TaylorLinearAttention
+
+    q, k, v, g = _inputs(1, 3, 320, d, dv)
+    tq, tk, tv = (t.requires_grad_(True) for t in (q, k, v))
+    out = TaylorLinearAttention.apply(tq, tk, tv)
+    assert len(out.grad_fn.saved_tensors) == 3 + kept
+    grads = torch.autograd.grad(out, (tq, tk, tv), g)
+    # as above, and with features in memory their gradients rounded too, each of which meets two terms
+    for name, got, want in zip(("out", "dxq", "dxk", "dv"), (out,) + grads, _exact(q, k, v, g)):
+        rel = ((got.double() - want).norm() / want.norm()).item()
+        assert rel <= math.sqrt(7) * 2.0**-9 / math.sqrt(3) * 1.5, (name, rel)
+
+
+@pytest.mark.parametrize("dv", [24, 40, 72])
+def test_value_widths_that_are_no_power_of_two_are_refused(dv):
+    from flashy_linear_attention_b200 import TaylorLinearAttention
+
+    q, k, v, _ = _inputs(1, 3, 320, 16, dv)
+    with pytest.raises(AssertionError, match="power of 2"):
+        TaylorLinearAttention.apply(q, k, v)
+
+
 @pytest.mark.parametrize("backward", [False, True])
 def test_a_tile_that_never_comes_ends_in_the_status_word(backward):
     from flashy_linear_attention_b200 import _lib, ops
