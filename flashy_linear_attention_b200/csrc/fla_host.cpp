@@ -349,6 +349,60 @@ std::optional<std::array<Tensor, 3>> taylor_backward(const Tensor& g, const Tens
   return std::array<Tensor, 3>{dq, dk, dv.full};
 }
 
+// The same through features in memory: out and the features of q and k, rows padded to a multiple of 8
+// elements; and the gradients from those. (Prepared in Python a training step took 200 us of the host.)
+struct FeatureDims {
+  int features, padded;
+};
+std::optional<FeatureDims> feature_dims(const Tensor& q, const Tensor& k, const Tensor& v) {
+  FeatureDims f;
+  if (!usable(q, q) || !usable(k, q) || !usable(v, q) || q.sizes() != k.sizes() || !same_rows(q, v) ||
+      q.scalar_type() != at::kBFloat16 || !covered_dims(q, v) ||
+      fla_sm100_taylor_dims(static_cast<int>(q.size(3)), &f.features, &f.padded) != FLA_OK)
+    return std::nullopt;
+  return f;
+}
+Tensor aligned_rows(const Tensor& x) {  // what the feature kernels read
+  const Tensor c = x.contiguous();
+  return reinterpret_cast<uintptr_t>(c.data_ptr()) % 16 == 0 ? c : c.clone();
+}
+std::optional<std::array<Tensor, 3>> taylor_forward_in_memory(const Tensor& q, const Tensor& k, const Tensor& v,
+                                                              unsigned debug_flags, uintptr_t status) {
+  const auto dims = feature_dims(q, k, v);
+  if (!dims.has_value()) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(q.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  auto features = [&](const Tensor& x) {
+    const Tensor rows = aligned_rows(x);
+    const Tensor phi = at::empty({x.size(0), x.size(1), x.size(2), dims->padded}, x.options());
+    check(fla_sm100_taylor_features(rows.data_ptr(), phi.data_ptr(), x.numel() / x.size(3), static_cast<int>(x.size(3)), stream),
+          "fla_sm100_taylor_features");
+    return phi.narrow(3, 0, dims->features);
+  };
+  const Tensor pq = features(q), pk = features(k);
+  const std::optional<Forward> r = forward(pq, pk, v, std::nullopt, 0, debug_flags, status);
+  if (!r.has_value()) return std::nullopt;
+  return std::array<Tensor, 3>{r->out, pq, pk};
+}
+std::optional<std::array<Tensor, 3>> taylor_backward_in_memory(const Tensor& g, const Tensor& q, const Tensor& k,
+                                                               const Tensor& v, const Tensor& pq, const Tensor& pk,
+                                                               unsigned debug_flags, uintptr_t status) {
+  const auto dims = feature_dims(q, k, v);
+  if (!dims.has_value()) return std::nullopt;
+  const auto r = backward(g, pq, pk, v, std::nullopt, std::nullopt, true, std::nullopt, debug_flags, status);
+  if (!r.has_value()) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(q.device());
+  void* stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+  auto raw = [&](const Tensor& dphi, const Tensor& x) {  // (dphi: fresh, its rows padded as those of the features)
+    const Tensor rows = aligned_rows(x), dx = at::empty(x.sizes(), x.options());
+    check(fla_sm100_taylor_features_bwd(dphi.data_ptr(), rows.data_ptr(), dx.data_ptr(), x.numel() / x.size(3),
+                                        static_cast<int>(x.size(3)), stream),
+          "fla_sm100_taylor_features_bwd");
+    return dx;
+  };
+  return std::array<Tensor, 3>{raw((*r)[0], q), raw((*r)[1], k), (*r)[2]};
+}
+
 // What is saved beside the repacked copy of an input that is not kept itself: an empty tensor that shares
 // its version count, for autograd to see that it was changed in place. (An inference tensor has none;
 // it is returned itself, and autograd refuses it as it always does.)
@@ -378,6 +432,8 @@ PYBIND11_MODULE(_hostcalls, m) {
   m.def("version_of", &version_of);
   m.def("taylor_forward", &taylor_forward, py::call_guard<py::gil_scoped_release>());
   m.def("taylor_backward", &taylor_backward, py::call_guard<py::gil_scoped_release>());
+  m.def("taylor_forward_in_memory", &taylor_forward_in_memory, py::call_guard<py::gil_scoped_release>());
+  m.def("taylor_backward_in_memory", &taylor_backward_in_memory, py::call_guard<py::gil_scoped_release>());
   m.def("backward", [](const Tensor& g, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& s_last,
                        const OptTensor& seg_states, bool keep_padded, const Strides& strides, unsigned debug_flags,
                        uintptr_t status) -> py::object {

@@ -214,7 +214,8 @@ class TaylorLinearAttention(Function):
 
     With values of 8, 16, 32 or 64 columns the features are formed on chip and never exist in memory, in neither
     pass, and nothing but xq, xk and v is kept for the backward. Other powers of two go through feature tensors in memory,
-    which are kept; widths that are no power of two are refused (as by ``LinearAttentionSmallVHD``).
+    which are kept, and so do few heads with many tokens at d = 8, where that is faster (see
+    ``ops._taylor_memory_is_faster``); widths that are no power of two are refused (as by ``LinearAttentionSmallVHD``).
     The reference has no counterpart.
     """
 
@@ -223,9 +224,9 @@ class TaylorLinearAttention(Function):
     def forward(ctx: Any, xq, xk, v):
         out, features = ops.taylor_forward(xq, xk, v), ()
         if out is None:  # errors, and what does not run on chip
-            features = ops.taylor_features(xq), ops.taylor_features(xk)
-            ops.check_forward_preconditions(features[0], v, smallv=True)
-            out = ops.causal_dot_product_fwd(*features, v)
+            out, *features = ops.taylor_forward_in_memory(xq, xk, v)
+            if ops._taylor_on_chip(xq, xk, v, backward=True):
+                features = ()
         ctx.save_for_backward(xq, xk, v, *features)
         return out
 
@@ -237,5 +238,4 @@ class TaylorLinearAttention(Function):
             if grads is not None:
                 return tuple(grads)
             features = ops.taylor_features(xq), ops.taylor_features(xk)
-        dpq, dpk, dv = ops.causal_dot_product_bwd(grad_output, *features, v, keep_padded=True)
-        return ops.taylor_features_bwd(dpq, xq), ops.taylor_features_bwd(dpk, xk), dv
+        return ops.taylor_backward_in_memory(grad_output, xq, xk, v, *features)

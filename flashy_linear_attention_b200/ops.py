@@ -608,15 +608,47 @@ def normalized_bwd(dnum, dden, q, k, v, s_last):
     return tuple(outs)
 
 
-def _taylor_on_chip(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> bool:
-    """True for calls that the kernel on raw rows takes: those that pass the checks of the feature map and of
-    the SmallVHD shapes, with values of 8, 16, 32 or 64 columns. What it does not take goes through the features in
-    memory, which report the errors."""
+def _taylor_rows(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> bool:
+    """True for tensors that pass the checks of the feature map, and whose lengths those of the SmallVHD shapes."""
     if not all(t.is_cuda and t.device == xq.device and t.dtype == torch.bfloat16 and t.dim() == 4 for t in (xq, xk, v)):
         return False
-    d, dv = xq.shape[-1], v.shape[-1]
+    d = xq.shape[-1]
     return (xq.shape == xk.shape and xq.shape[:3] == v.shape[:3] and xq.numel() > 0 and d in (8, 16)
-            and dv in (8, 16, 32, 64) and xq.shape[2] % (64 if d == 8 else 32) == 0)
+            and xq.shape[2] % (64 if d == 8 else 32) == 0)
+
+
+def _taylor_shapes(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> bool:
+    """The same, and the value width is one of the SmallVHD shapes."""
+    dv = v.shape[-1]
+    return _taylor_rows(xq, xk, v) and _next_pow2(dv) == dv <= _next_pow2(1 + xq.shape[-1] + xq.shape[-1] ** 2)
+
+
+def _taylor_memory_is_faster(d: int, heads: int, tokens: int, backward: bool) -> bool:
+    """The kernel on raw rows gives a head one CTA (backward: two) that walks all its chunks. 273 features (d = 16) in
+    memory are never split either, and never faster. 73 (d = 8) run in the kernels whose sequence is split over idle
+    SMs, and are faster for few heads and many tokens. Microseconds, n chunks of 128 tokens, h heads (1 to 48 heads,
+    4 to 512 chunks, 16 and 64 value columns):
+                  on chip         in memory
+        forward   4.5 + 1.16 n    27 + (0.04 + 0.0255 h) n
+        backward  4 + 1.91 n      50 + (0.05 + 0.109 h) n
+    in memory / on chip   1 head:   16 chunks 27 / 24 + 55 / 35    32: 29 / 41 + 57 / 66     512: 48 / 597 + 109 / 978
+                          4 heads:  32 chunks 29 / 43 + 63 / 66    64: 33 / 80 + 76 / 127    512: 86 / 598 + 292 / 980
+                         16 heads:  32 chunks 39 / 42 + 109 / 66   128: 85 / 154 + 292 / 250 512: 248 / 598 + 967 / 988
+                         32 heads:  64 chunks 88 / 80 + 257 / 128  128: 146 / 156 + 491 / 252 512: 486 / 607 + 1900 / 990
+    Where the backward is faster through memory, so is the forward."""
+    if d != 8:
+        return False
+    n = (tokens + 127) // 128
+    return (1.86 - 0.109 * heads) * n > 45.0 if backward else (1.12 - 0.0255 * heads) * n > 22.5
+
+
+def _taylor_on_chip(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor, backward: bool = False) -> bool:
+    """True for calls that the kernel on raw rows takes: values of 8, 16, 32 or 64 columns, unless features in memory are
+    the faster way. What it does not take goes through the features in memory, which report the errors."""
+    if not _taylor_rows(xq, xk, v) or v.shape[-1] not in (8, 16, 32, 64):
+        return False
+    B, H, N, d = xq.shape
+    return d != 8 or not _taylor_memory_is_faster(d, B * H, N, backward)
 
 
 def _taylor_call(name: str, xq, xk, v, **tensors) -> None:
@@ -652,7 +684,7 @@ def taylor_forward(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor) -> Optio
 def taylor_backward(grad_output: torch.Tensor, xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor):
     """Gradients of taylor_forward() with respect to xq, xk and v, or None as there."""
     g = grad_output
-    if not _taylor_on_chip(xq, xk, v) or g.shape != v.shape or g.dtype != v.dtype or g.device != v.device:
+    if not _taylor_on_chip(xq, xk, v, backward=True) or g.shape != v.shape or g.dtype != v.dtype or g.device != v.device:
         return None
     native = _lib.host()
     if native is not None:
@@ -668,6 +700,39 @@ def taylor_backward(grad_output: torch.Tensor, xq: torch.Tensor, xk: torch.Tenso
     return grads
 
 
+def _aligned_rows(x: torch.Tensor) -> torch.Tensor:
+    """`x` as the feature kernels read it: contiguous, from a 16-byte boundary on."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
+def taylor_forward_in_memory(xq: torch.Tensor, xk: torch.Tensor, v: torch.Tensor):
+    """(out, features of xq, features of xk): the same attention through features in memory."""
+    native = _lib.host() if xq.is_cuda else None
+    if native is not None and _taylor_shapes(xq, xk, v):
+        res = native.taylor_forward_in_memory(xq, xk, v, _debug_flags, _status_ptr(xq))
+        if res is not None:
+            if os.environ.get("FLA_DEBUG", "0") == "1":
+                check_status(xq.device)
+            return res
+    pq, pk = taylor_features(xq), taylor_features(xk)
+    check_forward_preconditions(pq, v, smallv=True)
+    return causal_dot_product_fwd(pq, pk, v), pq, pk
+
+
+def taylor_backward_in_memory(grad_output, xq, xk, v, pq, pk):
+    """Gradients of taylor_forward_in_memory() with respect to xq, xk and v."""
+    native = _lib.host() if xq.is_cuda else None
+    if native is not None and _taylor_shapes(xq, xk, v):
+        res = native.taylor_backward_in_memory(grad_output, xq, xk, v, pq, pk, _debug_flags, _status_ptr(xq))
+        if res is not None:
+            if os.environ.get("FLA_DEBUG", "0") == "1":
+                check_status(xq.device)
+            return tuple(res)
+    dpq, dpk, dv = causal_dot_product_bwd(grad_output, pq, pk, v, keep_padded=True)
+    return taylor_features_bwd(dpq, xq), taylor_features_bwd(dpk, xk), dv
+
+
 def taylor_features(x: torch.Tensor) -> torch.Tensor:
     """Second-order Taylor features phi(x) = [1, x / d^(1/4), vec(x x^T) / (sqrt(2) sqrt(d))] of raw
     x [B, H, N, d] (bf16, d = 8 or 16): a [B, H, N, 1 + d + d^2] view of rows padded to a multiple
@@ -678,7 +743,7 @@ def taylor_features(x: torch.Tensor) -> torch.Tensor:
     f, fp = ctypes.c_int(0), ctypes.c_int(0)
     if lib.fla_sm100_taylor_dims(d, ctypes.byref(f), ctypes.byref(fp)) != 0:
         raise NotImplementedError("flashlinear: Taylor features are built for raw head dims 8 and 16")
-    xc = x.contiguous()
+    xc = _aligned_rows(x)
     buf = torch.empty(x.shape[:-1] + (fp.value,), dtype=x.dtype, device=x.device)
     with torch.cuda.device(x.device):
         rc = lib.fla_sm100_taylor_features(xc.data_ptr(), buf.data_ptr(), xc.numel() // d, d,
@@ -704,7 +769,7 @@ def taylor_features_bwd(dphi: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
         buf = torch.zeros(dphi.shape[:-1] + (fp.value,), dtype=dphi.dtype, device=dphi.device)
         buf[..., :f.value] = dphi
         dphi = buf[..., :f.value]
-    xc = x.contiguous()
+    xc = _aligned_rows(x)
     dx = torch.empty_like(xc)
     with torch.cuda.device(x.device):
         rc = lib.fla_sm100_taylor_features_bwd(dphi.data_ptr(), xc.data_ptr(), dx.data_ptr(), rows, d,

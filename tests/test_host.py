@@ -356,3 +356,24 @@ def test_rule_of_the_fused_denominator(heads, tokens, fused, width):
     assert _lib.load().fla_sm100_normalized_fused(ctypes.byref(a)) == fused
     a.segments = 1
     assert _lib.load().fla_sm100_normalized_fused(ctypes.byref(a)) == 1
+
+
+# 73 features: the two lines in heads and tokens, and the sizes beside them that were timed on both sides
+@pytest.mark.parametrize("heads,tokens,forward,backward", [
+    (1, 2048, False, False), (1, 4096, True, True), (4, 4096, True, True), (8, 4096, True, False), (8, 8192, True, True),
+    (16, 3968, False, False), (16, 4096, True, False), (16, 65536, True, True), (24, 4096, False, False), (24, 8192, True, False),
+    (32, 8192, False, False), (32, 16384, True, False), (40, 16384, False, False), (48, 65536, False, False), (1, 128, False, False)])
+def test_raw_features_take_the_faster_way(heads, tokens, forward, backward):
+    from flashy_linear_attention_b200 import ops
+
+    assert ops._taylor_memory_is_faster(8, heads, tokens, False) == forward
+    assert ops._taylor_memory_is_faster(8, heads, tokens, True) == backward
+    assert not ops._taylor_memory_is_faster(16, heads, tokens, True) and not ops._taylor_memory_is_faster(16, heads, tokens, False)
+
+
+def test_where_the_backward_takes_features_from_memory_the_forward_does():
+    from flashy_linear_attention_b200 import ops
+
+    for heads in range(1, 200):
+        for tokens in range(64, 1 << 17, 64 * heads):
+            assert ops._taylor_memory_is_faster(8, heads, tokens, False) or not ops._taylor_memory_is_faster(8, heads, tokens, True)

@@ -89,6 +89,49 @@ def test_features_in_memory_are_formed_once(d, dv, kept):
         assert rel <= math.sqrt(7) * 2.0**-9 / math.sqrt(3) * 1.5, (name, rel)
 
 
+# d = 8: both passes through memory; the forward alone; neither
+@pytest.mark.parametrize("H,N,dv,bnhd,forward,kept", [(1, 4096, 64, True, False, 2), (3, 4160, 16, False, False, 2),
+                                                      (16, 4096, 32, True, False, 0), (16, 3968, 32, False, True, 0)])
+def test_few_long_heads_go_through_memory(H, N, dv, bnhd, forward, kept):
+    from flashy_linear_attention_b200 import TaylorLinearAttention, ops
+
+    q, k, v, g = _inputs(1, H, N, 8, dv, bnhd)
+    assert (ops.taylor_forward(q, k, v) is not None) == forward
+    tq, tk, tv = (t.detach().requires_grad_(True) for t in (q, k, v))
+    out = TaylorLinearAttention.apply(tq, tk, tv)
+    assert len(out.grad_fn.saved_tensors) == 3 + kept
+    grads = torch.autograd.grad(out, (tq, tk, tv), g)
+    ops.check_status(torch.device(DEV))
+    assert out.stride() == torch.empty_like(v).stride() and grads[2].stride() == torch.empty_like(v).stride()
+    for name, got, want in zip(("out", "dxq", "dxk", "dv"), (out,) + grads, _exact(q, k, v, g)):
+        assert got.shape == want.shape
+        rel = ((got.double() - want).norm() / want.norm()).item()
+        assert rel <= math.sqrt(7) * 2.0**-9 / math.sqrt(3) * 1.5, (name, rel)
+
+
+@pytest.mark.parametrize("d,dv", [(8, 64), (16, 128), (8, 4)])
+def test_every_path_through_memory_gives_the_same(d, dv, monkeypatch):
+    """The calls prepared in Python instead of in the native host code, rows of other strides or off a 16-byte
+    boundary, an expanded gradient."""
+    from flashy_linear_attention_b200 import _lib, ops
+
+    def both(q, k, v, g):
+        out, pq, pk = ops.taylor_forward_in_memory(q, k, v)
+        return (out,) + tuple(ops.taylor_backward_in_memory(g, q, k, v, pq, pk))
+
+    q, k, v, g = _inputs(2, 3, 320, d, dv)
+    want = both(q, k, v, g)
+    flat = torch.empty(q.numel() + 1, device=DEV, dtype=torch.bfloat16)
+    off = flat[1:].view_as(q).copy_(q)
+    assert off.is_contiguous() and off.data_ptr() % 16 != 0
+    turned = k.transpose(1, 2).contiguous().transpose(1, 2)
+    ones = torch.ones(1, 1, 1, 1, device=DEV, dtype=torch.bfloat16).expand(2, 3, 320, dv)
+    other, spread = both(off, turned, v, g), both(q, k, v, ones)
+    monkeypatch.setattr(_lib, "_host", False)
+    for a, b in ((want, other), (want, both(q, k, v, g)), (want, both(off, turned, v, g)), (spread, both(q, k, v, ones.contiguous()))):
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
 @pytest.mark.parametrize("dv", [24, 40, 72])
 def test_value_widths_that_are_no_power_of_two_are_refused(dv):
     from flashy_linear_attention_b200 import TaylorLinearAttention
