@@ -585,18 +585,22 @@ def normalized_fwd(q, k, v, eps: float, need_grad: bool):
 def normalized_bwd(dnum, dden, q, k, v, s_last):
     """(dq, dk, dv) of the normalised attention from what normalize_bwd_prepare returned, with the denominator's
     part formed in the product kernel, or None for calls that take product and normalize_bwd_sweep instead."""
-    if s_last is None or not all(t.dtype == torch.bfloat16 and t.shape == v.shape and t.device == v.device and _addressable(t)
-                                 for t in (dnum, q, k, v)):
+    if s_last is None:
+        return None
+    a = FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = *q.shape, v.shape[-1]
+    a.debug_flags = _debug_flags
+    need = _lib.load().fla_sm100_normalized_bwd_workspace_bytes(ctypes.byref(a))
+    # (asked before anything is allocated: most calls with a final state have too few heads)
+    if need == 0 or not all(t.dtype == torch.bfloat16 and t.shape == v.shape and t.device == v.device and _addressable(t)
+                            for t in (dnum, q, k, v)):
         return None
     outs = [torch.empty_like(t) for t in (q, k, v)]
     if not all(_addressable(t) for t in outs):
         return None
     with torch.cuda.device(q.device):
-        a = _norm_args(q, q.shape[-1], v.shape[-1])
-        a.debug_flags = _debug_flags
-        need = _lib.load().fla_sm100_normalized_bwd_workspace_bytes(ctypes.byref(a))
-        if need == 0:
-            return None
+        a.stream = torch.cuda.current_stream(q.device).cuda_stream
+        a.status = _status_word(q.device).data_ptr()
         a.q, a.k, a.v, a.d_o = _desc(q), _desc(k), _desc(v), _desc(dnum)
         a.d_q, a.d_k, a.d_v = (_desc(t) for t in outs)
         a.s_last = s_last.data_ptr()

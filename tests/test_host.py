@@ -377,3 +377,14 @@ def test_where_the_backward_takes_features_from_memory_the_forward_does():
     for heads in range(1, 200):
         for tokens in range(64, 1 << 17, 64 * heads):
             assert ops._taylor_memory_is_faster(8, heads, tokens, False) or not ops._taylor_memory_is_faster(8, heads, tokens, True)
+
+
+def test_a_call_for_the_separate_kernels_allocates_nothing(monkeypatch):
+    """The denominator's gradient inside the product kernel is refused before any tensor is made (or a GPU needed)."""
+    from flashy_linear_attention_b200 import ops
+
+    q = torch.zeros(1, 16, 2176, 64, dtype=torch.bfloat16)
+    s_last = torch.zeros(16, 64, 64)
+    for name in ("empty", "empty_like"):
+        monkeypatch.setattr(torch, name, lambda *a, **k: pytest.fail("allocated"))
+    assert ops.normalized_bwd(q, None, q, q, q, s_last) is None
