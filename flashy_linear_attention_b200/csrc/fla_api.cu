@@ -424,7 +424,9 @@ __global__ void fla_pad_rows_kernel(const __grid_constant__ PadBatch batch, long
 // row's end, in two. Within a row they start at an arbitrary 2-byte offset and are fetched like the
 // pad kernel's; a piece that crosses a row end takes its elements one by one. Bound by instruction
 // issue before it is by HBM: with one thread per 32-bit word (a division per 4 bytes) 24 MB took
-// 19.7 us at d = 83, with 16-byte pieces 14.7 us (12.2 us a tensor with three in one launch). WIDE: rows and the source are 4-byte and the
+// 19.7 us at d = 83, with 16-byte pieces 14.7 us (12.2 us a tensor with three in one launch). (A variant that brought a
+// block's rows into shared memory first gained 0.4 to 1 us on tensors of up to 25,000 rows of 73 columns or more and
+// lost on the others: 142,848 rows of 83 14.9 -> 15.4 us, of 273 32.6 -> 36.9, 524,288 of 9 16.9 -> 26.7.) WIDE: rows and the source are 4-byte and the
 // destination 16-byte aligned; else element loads and stores throughout.
 template <bool WIDE>
 __global__ void fla_unpad_rows_kernel(const __grid_constant__ PadBatch batch, long long rows, int d, int dpad) {
@@ -479,58 +481,6 @@ __global__ void fla_unpad_rows_kernel(const __grid_constant__ PadBatch batch, lo
           if (j < n) bdst[e0 + j] = x[j];
       }
     }
-  }
-}
-
-// The same for rows of 8 to kUnpadMaxRow elements and 16-byte aligned tensors: a block's padded rows come into shared
-// memory in 16-byte pieces, and a thread puts a destination piece together from 32-bit words there: eight
-// consecutive elements, or, where the row ends inside, those up to the end and the rest from `gap` elements
-// further on. Without the element-by-element path that nearly every warp has some lanes in: 24 MB at d = 83 in
-// 13.8 us, 15.4 with the kernel above, which keeps longer rows and other alignments.
-constexpr int kUnpadMaxRow = 384;
-__global__ void __launch_bounds__(256) fla_unpad_rows_staged_kernel(const __grid_constant__ PadBatch batch, long long rows, int d, int dpad) {
-  __shared__ uint4 stage[kPadRowsPerBlock * kUnpadMaxRow / 8 + 1];
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(stage);
-  const uint4* __restrict__ src = static_cast<const uint4*>(batch.src[blockIdx.y]);
-  unsigned short* __restrict__ dst = static_cast<unsigned short*>(batch.dst[blockIdx.y]);
-  const int gap = dpad - d, pieces = dpad >> 3;
-  for (long long blk = blockIdx.x; blk * kPadRowsPerBlock < rows; blk += gridDim.x) {
-    const long long row0 = blk * kPadRowsPerBlock;
-    const int nrows = static_cast<int>(min(static_cast<long long>(kPadRowsPerBlock), rows - row0));
-    for (int i = threadIdx.x; i < nrows * pieces; i += 256) stage[i] = __ldg(src + row0 * pieces + i);
-    __syncthreads();
-    unsigned short* bdst = dst + row0 * d;  // 64 d bytes a block: as aligned as the tensor itself
-    const int total = nrows * d;
-    for (int e0 = threadIdx.x * 8; e0 < total; e0 += 256 * 8) {
-      const int r = e0 / d, c = e0 - r * d;
-      const int s0 = e0 + r * gap;  // source element
-      // elements s, s + 1, ... in pairs (reads at most one word past the last row: there is one)
-      auto fetch = [&](int s, uint32_t (&x)[4]) {
-        uint32_t w[5];
-#pragma unroll
-        for (int j = 0; j < 5; ++j) w[j] = words[(s >> 1) + j];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) x[j] = __funnelshift_r(w[j], w[j + 1], (s & 1) * 16);
-      };
-      uint32_t x[4];
-      fetch(s0, x);
-      const int left = d - c;  // elements up to the row's end
-      if (left < 8) {
-        uint32_t y[4];
-        fetch(min(s0 + gap, nrows * dpad - 8), y);  // (the last row has no next: nothing of y is used)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          x[j] = left <= 2 * j ? y[j] : left == 2 * j + 1 ? __byte_perm(x[j], y[j], 0x7610) : x[j];
-      }
-      if (e0 + 8 <= total) {
-        *reinterpret_cast<uint4*>(bdst + e0) = make_uint4(x[0], x[1], x[2], x[3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (e0 + j < total) bdst[e0 + j] = static_cast<unsigned short>(x[j >> 1] >> ((j & 1) * 16));
-      }
-    }
-    __syncthreads();  // the stage is refilled
   }
 }
 
@@ -1823,22 +1773,19 @@ int fla_sm100_unpad_rows_batch(const void* const* src, void* const* dst, int cou
   if (src == nullptr || dst == nullptr || count <= 0 || rows <= 0 || d <= 0 || dpad < d) return FLA_ERR_INVALID;
   if (count > kPadMaxTensors) return FLA_ERR_UNSUPPORTED;
   PadBatch batch = {};
-  bool wide = dpad % 2 == 0, staged = dpad % 8 == 0 && d >= 8 && dpad <= kUnpadMaxRow;
+  bool wide = dpad % 2 == 0;
   for (int i = 0; i < count; ++i) {
     if (src[i] == nullptr || dst[i] == nullptr) return FLA_ERR_INVALID;
     if (reinterpret_cast<uintptr_t>(dst[i]) % 4 != 0 || reinterpret_cast<uintptr_t>(src[i]) % 2 != 0)
       return FLA_ERR_ALIGNMENT;
     wide = wide && reinterpret_cast<uintptr_t>(dst[i]) % 16 == 0 && reinterpret_cast<uintptr_t>(src[i]) % 4 == 0;
-    staged = staged && reinterpret_cast<uintptr_t>(dst[i]) % 16 == 0 && reinterpret_cast<uintptr_t>(src[i]) % 16 == 0;
     batch.src[i] = src[i];
     batch.dst[i] = dst[i];
   }
   const int blocks = static_cast<int>(
       std::min<long long>((rows + kPadRowsPerBlock - 1) / kPadRowsPerBlock, 148 * 32));
   const dim3 grid(blocks, count, 1);
-  if (staged)
-    fla_unpad_rows_staged_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(batch, rows, d, dpad);
-  else if (wide)
+  if (wide)
     fla_unpad_rows_kernel<true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(batch, rows, d, dpad);
   else
     fla_unpad_rows_kernel<false><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(batch, rows, d, dpad);

@@ -1,4 +1,4 @@
-"""The row unpad kernels at the limits of the staged one."""
+"""The row unpad kernel: odd widths, blocks of rows, alignments."""
 import pytest
 import torch
 
@@ -6,8 +6,8 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
-# the widths and row counts around the staged kernel's limits (8 and 384 elements, 32 rows a block), and tensors
-# that are only 4-byte aligned, which it does not take
+# narrow, ordinary and wide rows, row counts around a block's, and tensors that are only 4-byte aligned, which are
+# written element by element
 @pytest.mark.parametrize("d", [7, 9, 11, 83, 273, 383, 385])
 @pytest.mark.parametrize("rows", [1, 31, 33, 1000])
 @pytest.mark.parametrize("offset", [0, 2])
