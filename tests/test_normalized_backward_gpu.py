@@ -30,9 +30,11 @@ def _inputs(B, H, N, D, bnhd):
     return draw(True), draw(True), draw(False), draw(False)
 
 
-# the rule's edges in heads, ragged last chunks (a multiple of 4 tokens), whole and partly used tiles, two rounds
+# the rule's edges in heads, ragged last chunks (a multiple of 4 tokens), whole and partly used tiles, two rounds;
+# one, two and three chunks
 @pytest.mark.parametrize("B,H,N,D,bnhd", [(1, 99, 1024, 128, False), (1, 100, 1100, 96, True), (2, 50, 1252, 128, True),
-                                          (1, 99, 1024, 64, True), (1, 50, 1024, 56, True), (1, 60, 1156, 40, False), (2, 148, 580, 64, False)])
+                                          (1, 99, 1024, 64, True), (1, 50, 1024, 56, True), (1, 60, 1156, 40, False), (2, 148, 580, 64, False),
+                                          (1, 99, 64, 128, False), (1, 99, 192, 64, True), (1, 100, 324, 96, False)])
 def test_against_64_bits(any_length, B, H, N, D, bnhd):
     from flashy_linear_attention_b200 import ops
 

@@ -103,6 +103,40 @@ def test_states_before_and_after(any_length, H, N, D, with_s, with_r):
     assert ((r_final.double() - want[3]).norm() / want[3].norm()).item() <= (N / 16 + 2) * 2.0**-24
 
 
+@pytest.mark.parametrize("with_s", [False, True])
+@pytest.mark.parametrize("H,N,D", [(100, 1024, 128), (99, 1100, 64)])
+def test_state_after_without_its_update(any_length, H, N, D, with_s):
+    """r_init and no r_final: the R of the last chunk walked is never formed."""
+    q, k, v, g = _inputs(1, H, N, D, torch.bfloat16, N)
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    s0, r0 = (torch.randn(H, D, D, device=DEV, generator=gen) * 8 if w else None for w in (with_s, True))
+    s_last = (k[0].double().mT @ v[0].double() + (s0.double() if with_s else 0)).float()
+    got = _run(q, k, v, g, s_last, s_init=s0, r_init=r0)
+    for name, x, w in zip(("dq", "dk", "dv"), got, _exact(q[0], k[0], v[0], g[0], s0, r0)):
+        rel = ((x[0].double() - w).norm() / w.norm()).item()
+        assert rel <= _bound(torch.bfloat16), (name, rel)
+
+
+# one, two and three chunks: the first is the exact one, R is not formed, a state's copy is used once, a slot of the
+# ring is filled a first and a second time; 445 heads: more than two rounds
+@pytest.mark.parametrize("states", [False, True])
+@pytest.mark.parametrize("H,N,D", [(99, 64, 128), (99, 128, 64), (100, 192, 128), (100, 250, 64), (99, 320, 96), (50, 384, 48),
+                                   (445, 192, 128), (445, 320, 64)])
+def test_few_chunks(any_length, H, N, D, states):
+    q, k, v, g = _inputs(1, H, N, D, torch.bfloat16, N)
+    gen = torch.Generator(device=DEV).manual_seed(D)
+    s0, r0 = (torch.randn(H, D, D, device=DEV, generator=gen) * 8 if states else None for _ in range(2))
+    s_last = (k[0].double().mT @ v[0].double() + (s0.double() if states else 0)).float()
+    r_final = torch.full((H, D, D), float("nan"), device=DEV) if states else None
+    got = _run(q, k, v, g, s_last, s_init=s0, r_init=r0, r_final=r_final)
+    want = _exact(q[0], k[0], v[0], g[0], s0, r0)
+    for name, x, w in zip(("dq", "dk", "dv"), got, want):
+        rel = ((x[0].double() - w).norm() / w.norm()).item()
+        assert rel <= _bound(torch.bfloat16), (name, rel)
+    if states:  # fp32 sums of N / 16 steps of 16 exact products
+        assert ((r_final.double() - want[3]).norm() / want[3].norm()).item() <= (N / 16 + 2) * 2.0**-24
+
+
 def test_strided_inputs_and_guard_bands():
     """[B, H, N, D] views of [B, N, H, D] tensors; outputs' neighbours stay as they are."""
     from flashy_linear_attention_b200 import _lib, ops

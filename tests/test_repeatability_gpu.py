@@ -7,10 +7,13 @@ issuer that the fp32 score tile had been read directly behind its tensor-memory 
 in 10^4 launches (at the first chunk of a CTA, where the issuer is already polling that barrier) the
 next chunk's score MMA overwrote columns whose load was still in flight; 32 rows of one chunk were
 then off by a few per cent of the tensor's maximum, within a tolerance-based check more often than
-not. The shapes below are the ones that showed it: the 64-wide kernel with the single-sweep backward
+not. The shapes that showed it: the 64-wide kernel with the single-sweep backward
 (most often), the 16-head share of the headline job (both passes fused cooperative launches) and a
-sequence shard that starts from a given state in both directions.
+sequence shard that starts from a given state in both directions. The later kernels (one CTA for a head's
+gradients, with and without the denominator's, and the features formed on chip) are held to the same.
 """
+import ctypes
+
 import pytest
 import torch
 
@@ -47,12 +50,17 @@ def _repeat(fn, repeats, batch):
     return {n: c for n, c in zip(NAMES, differing.tolist()) if c}
 
 
-@pytest.mark.parametrize("shape,repeats", [((8, 16, 4096, 64), 20000), ((1, 16, 8192, 128), 12000)],
-                         ids=["B8_H16_N4096_D64", "B1_H16_N8192_D128_fused"])
-def test_forward_and_single_sweep_backward_repeat_bit_for_bit(shape, repeats):
-    from flashy_linear_attention_b200 import ops
+# one CTA a head at 64 and 128 columns; three at 64; three split at the forward's segments
+@pytest.mark.parametrize("shape,repeats,one_cta", [((8, 16, 4096, 64), 20000, 1), ((1, 128, 2176, 128), 12000, 1),
+                                                   ((1, 98, 4096, 64), 20000, 0), ((1, 16, 8192, 128), 12000, 0)],
+                         ids=["B8_H16_N4096_D64", "B1_H128_N2176_D128", "B1_H98_N4096_D64", "B1_H16_N8192_D128_fused"])
+def test_forward_and_single_sweep_backward_repeat_bit_for_bit(shape, repeats, one_cta):
+    from flashy_linear_attention_b200 import _lib, ops
 
     B, H, N, D = shape
+    a = _lib.FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = B, H, N, D, D
+    assert _lib.load().fla_sm100_bwd_one_cta(ctypes.byref(a)) == one_cta
     q, k, v, dy = _inputs(B, H, N, D)
     s_final = torch.empty(B * H, D, D, dtype=torch.float32, device=DEV)
     seg_states = ops.segment_states_buffer(q, v)
@@ -94,3 +102,31 @@ def test_sequence_shard_with_states_from_both_sides_repeats_bit_for_bit():
         return (out,) + tuple(grads)
 
     assert _repeat(step, 4000, batch=16) == {}
+
+
+@pytest.mark.parametrize("H,N,D", [(128, 2176, 128), (128, 2304, 64), (100, 2116, 96)])
+def test_denominator_inside_the_backward_repeats_bit_for_bit(H, N, D):
+    from flashy_linear_attention_b200 import ops
+
+    q, k, v, dnum = _inputs(1, H, N, D, seed=7)
+    gen = torch.Generator(device=DEV).manual_seed(8)
+    dden = torch.randn(H, N, device=DEV, generator=gen)
+    s_last = torch.empty(H, D, D, dtype=torch.float32, device=DEV)
+    ops.causal_dot_product_fwd(q, k, v, s_final=s_last)
+    assert ops.normalized_bwd(dnum, dden, q, k, v, s_last) is not None
+    assert _repeat(lambda: ops.normalized_bwd(dnum, dden, q, k, v, s_last), 6000, batch=16) == {}
+
+
+# more CTAs than SMs in the backward, and fewer; a ragged last chunk
+@pytest.mark.parametrize("H,N,d,dv", [(128, 1024, 16, 64), (100, 1056, 16, 32), (160, 1088, 8, 64), (8, 1024, 8, 16)])
+def test_features_on_chip_repeat_bit_for_bit(H, N, d, dv):
+    from flashy_linear_attention_b200 import ops
+
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    q, k, v, dy = (torch.randn(1, H, N, w, device=DEV, generator=gen).bfloat16() for w in (d, d, dv, dv))
+    assert ops.taylor_forward(q, k, v) is not None
+
+    def step():
+        return (ops.taylor_forward(q, k, v),) + tuple(ops.taylor_backward(dy, q, k, v))
+
+    assert _repeat(step, 8000, batch=16) == {}
