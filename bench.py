@@ -48,10 +48,11 @@ UNIT = "Mtokens/s"
 PARITY_TOL = 2e-2
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the forward and the backward launch
-# of one cfg3 step: a constant, not a measurement of the run that prints it. It comes from an ncu
-# capture of the same grids at half the sequence length (518.1 + 952.6 MB), doubled: the traffic of
-# these launches grows in proportion to N. Other workloads report null.
-NCU_TRAFFIC_BYTES_PER_STEP = {"cfg3": 2.941e9}
+# of one cfg3 step on one GPU (fla_chunk_kernel<128,128>, fla_backward_kernel<128>): a constant, not a
+# measurement of the run that prints it. It comes from an ncu capture of the same grids at half the sequence
+# length (516.3 + 913.5 MB), doubled: the traffic of these launches grows in proportion to N. Other
+# workloads report null.
+NCU_TRAFFIC_BYTES_PER_STEP = {"cfg3": 2.860e9}
 
 
 def measured_peaks():
@@ -74,6 +75,21 @@ def measured_tensor_peak():
         return float(p["bf16_tflops_sustained"]), "measured sustained (MEASURED_PEAKS.json)"
     except Exception:
         return 1400.0, "fallback (1.4 PFLOP/s sustained, earlier measurement on this pool)"
+
+
+def kernel_names(B, H, N, dk, dv):
+    """The kernels of one step with head dims up to 128 (these heads and tokens on one GPU)."""
+    import ctypes
+
+    from flashy_linear_attention_b200 import _lib
+
+    a = _lib.FlaArgs()
+    a.batch, a.heads, a.seqlen, a.dk, a.dv = B, H, N, dk, dv
+    d = 64 if max(dk, dv) <= 64 else 128
+    chunk = f"fla_chunk_kernel<{d},{d}>"
+    if _lib.load().fla_sm100_bwd_one_cta(ctypes.byref(a)):
+        return f"{chunk} (fwd launch), fla_backward_kernel<{d}> (bwd launch)"
+    return f"{chunk} (fwd launch + bwd launch)"
 
 
 def algorithmic_flops(B, H, N, dk, dv, chunk=128):
@@ -792,7 +808,7 @@ def main():
             "gpu_launches": head["launches_per_step"] * steps,
             "clocks": head["clocks"],
             "roofline": {
-                "bound": "hbm", "kernel": (f"fla_chunk_kernel<{max(dk, dv)},{max(dk, dv)}> (fwd launch + bwd launch)"
+                "bound": "hbm", "kernel": (kernel_names(Bl, Hl, Nl, dk, dv)
                                              if max(dk, dv) <= 128 else
                                              "fla_pad_rows_kernel x2, fla_wide_kernel<3> (fwd, dV), "
                                              "fla_chunk_kernel<128,128> on 128-column output slices (dQ, dK)"),

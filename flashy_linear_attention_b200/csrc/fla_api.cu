@@ -1,8 +1,9 @@
 // C ABI of libflashlinear_sm100.so (declared in include/flashlinear_sm100.h).
 //
-// Forward and backward of causal linear attention are expressed with ONE device kernel,
+// Forward and backward of causal linear attention up to 128 columns are expressed with one product,
 // fla_chunk_kernel (fla_kernel.cuh), which computes  out_i = sum_{j<=i} (a_i . b_j) c_j  (or the
-// anti-causal sum j>=i). With a=q, b=k, c=v this is the forward output
+// anti-causal sum j>=i); long calls of many heads take fla_backward_kernel (fla_backward.cuh), wider heads
+// fla_wide_kernel (fla_wide_kernel.cuh). With a=q, b=k, c=v this is the forward output
 // (flashlinear/kernels/linear_attn_kernels.py:74-82); the gradients of
 // flashlinear/kernels/linear_attn_kernels.py:179-197 and :291-299 are the same product with
 // permuted operands:

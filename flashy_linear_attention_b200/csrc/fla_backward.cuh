@@ -16,10 +16,14 @@
 // D = 128 S, R, P and the accumulator fill its 512 columns. The states' 16-bit copies serve as MMA operands in
 // either direction (dV contracts over R's rows, dK over its columns) without a second copy.
 //
-// Bound by shared memory at D = 128: a chunk moves 1.0 MB of operands, states, tiles and staged outputs
-// through an SM, 8000 cycles at 128 bytes against 6300 of MMAs (three CTAs of fla_chunk_kernel: 1.25 MB); by the
-// issuer's waits and the conversions at D = 64. 128 heads, in one CTA each / three: 4096 x 128 186 / 220 us,
-// 8192 x 128 365 / 422 us, 4096 x 64 93 / 125 us. dQ's error against 64 bits 2.34e-3 / 2.40e-3.
+// At D = 128 a chunk moves 1.0 MB of operands, states, tiles and staged outputs through an SM's shared memory, at
+// least 8000 cycles at 128 bytes, against 6300 of MMAs (three CTAs of fla_chunk_kernel: 1.25 MB). It takes
+// 10600 to 11200 (346 - 365 us for 64 chunks): the rest are waits for tiles and score conversions that nothing
+// covers with one score tile and one accumulator. At D = 64 5700 cycles, the issuer's waits and the
+// conversions. (Counters: tensor pipe 64 % and 53 % of active cycles, DRAM 62 % and 55 % of its peak.)
+// 128 heads, in one CTA each / three: 4096 x 128 186 / 220 us, 8192 x 128 365 / 422 us, 4096 x 64 93 / 125 us.
+// NORM 4096 x 128: 308 us, its loads of d and the chunk vectors lie behind the waits for the tiles they go with
+// (tensor pipe 33 %, DRAM 36 %). dQ's error against 64 bits 2.34e-3 / 2.40e-3.
 //
 // CTA layout (608 threads, one CTA per SM):
 //   warps 0, 18   TMA producers, each half of every tile (see fla_kernel.cuh)
@@ -293,7 +297,8 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
         if (!(p.debug_withhold && t == 0))
           ptx::tma_load_4d(slot_addr(s) + part * kPartBytes, map, full_bar(s), part_col, tok, h, b);
         // At D = 128 a slot is free only shortly before its tile is wanted: the tile after that comes into L2
-        // now. (128 heads x 8192: 396 us without, 376 with; at D = 64, two chunks deep, no difference.)
+        // now. (128 heads x 8192, an earlier state of the kernel: 396 us without, 376 with; at D = 64, two chunks
+        // deep, no difference.)
         if (D == 128 && i + 1 < n_iter) ptx::tma_prefetch_4d(map, part_col, tok - kChunk, h, b);
       }
       __syncwarp();
@@ -511,7 +516,8 @@ fla_backward_kernel(const __grid_constant__ BackwardParams p) {
         const int tok = mem_chunk(n / 3) * kChunk + row;
         if (which == 2) scale = tok < p.n_tokens ? __ldg(p.d + static_cast<size_t>(bh) * p.n_tokens + tok) : 0.f;
       }
-      // this warp's earlier stores have read the rows that are overwritten below
+      // this warp's earlier stores have read the rows that are overwritten below (at D = 64 too all of them are
+      // waited for, although each gradient has a stage of its own)
       if (lane == 0) ptx::bulk_wait_group_read0();
       __syncwarp();
       if (!wait_tmem(o_full(n), (n >> 1) & 1)) break;

@@ -23,6 +23,9 @@
 // conversions unrolled per mask the same work took 42 and 144 us instead of 32 and 96).
 // 128 heads x 2048 tokens, d = 16, 64 value columns: forward 32 us and backward 96, against 130 and 355 through
 // features in memory; relative error against 64 bits 2.3e-3 (out), 2.6e-3 (dq, dk), there 2.4e-3 and 3.1e-3.
+// (Counters: issue slots 39 % and 33 % busy, tensor pipe 38 % and 32 % of active cycles, DRAM 20 % and 13 %.) A head has one
+// CTA, resp. two, whatever its length: few heads leave SMs idle, at d = 16 with less time all the same (1 head x 8192:
+// 103 + 174 us against 240 + 353), at d = 8 not, see the caller's rule.
 //
 // CTA layout (576 threads, one CTA per SM):
 //   warp 0        TMA producer: a and b tiles, two stages

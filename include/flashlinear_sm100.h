@@ -317,7 +317,7 @@ int fla_sm100_normalized_fused(const FlaArgs* args);
 int fla_sm100_normalized_fwd(const FlaArgs* args, float eps, float* den);
 /* The backward with the denominator's gradient inside: what fla_sm100_bwd on d_o = dnum followed by
  * normalize_bwd_sweep gives, with that gradient added in fp32 before dQ and dK are rounded. For bf16 calls
- * with dk = dv <= 128, a multiple of 8, a sequence length that is a multiple of 4, and heads enough for one CTA
+ * with dk = dv <= 128, a multiple of 8, more than 2048 tokens, a multiple of 4, and heads enough for one CTA
  * each; needs s_last, and scratch in args->workspace: normalized_bwd_workspace_bytes() is 0 for calls it does
  * not take (FLA_ERR_UNSUPPORTED). dden as normalize_bwd_prepare wrote it, 16-byte aligned. */
 size_t fla_sm100_normalized_bwd_workspace_bytes(const FlaArgs* args);
