@@ -727,10 +727,11 @@ SegPlan backward_aligned_plan(const FlaArgs* a, int sm_count, const SegPlan& f) 
 //   128-wide   99 1.31 1.33   198 1.04 1.04   206 1.09 1.07   247 1.20 1.19   297 1.02 1.00   330 1.06 1.03   444 1.27 1.21
 //   112-wide   99 1.18 1.19   198 1.02 0.99   206 1.05 1.03   247 1.19 1.17   297 0.99 0.96   330 1.05 1.01   444 1.29 1.23
 //    72-wide   99 1.13 1.13   198 0.96 0.94   230 1.06 0.99   247 1.14 1.12   297 0.94 0.91   346 1.06 1.00   444 1.30 1.24
-// (us, 4096 tokens, 99 heads: 64-wide 125 / 87, 128-wide 199 / 159.) Below 64 as many rounds are enough. Above 64, in
-// more than one round, the three are held against their work and not their rounds, since CTAs of a last round that
-// is nearly empty run faster: 2.05 times the one's rounds; 2.3 where rows are an odd number of 16-byte pieces (72,
-// 88, 104, 120 columns), half a 32-byte sector.
+// (us, 4096 tokens, 99 heads: 64-wide 125 / 87, 128-wide 199 / 159.) Below 64 as many rounds are enough; at 64 they
+// are up to 24 chunks (2560 tokens: 1.00 to 1.03; 16384: 0.98). Above 64, in more than one round, the three are held
+// against their work and not their rounds, since CTAs of a last round that is nearly empty run faster: from three
+// rounds of the one on, 2.05 times those; where rows are an odd number of 16-byte pieces (72, 88, 104, 120
+// columns: half a 32-byte sector), from two on, 2.3 times.
 // norm: with the denominator's gradient inside, against one of the two forms above and kernels for that gradient.
 // Those are slow but for 64 and 128 columns, so that the other widths gain everywhere in the widest rule (1.0 to 1.5);
 // separate / inside for the whole step at 2112 and 4096 tokens:
@@ -744,10 +745,11 @@ bool one_cta_backward(const FlaArgs* a, int sm_count, bool norm = false) {
   const long heads = static_cast<long>(a->batch) * a->heads;
   auto rounds = [&](long ctas) { return (ctas + sm_count - 1) / sm_count; };
   const long one = rounds(heads), three = rounds(3 * heads);
-  if (a->dk < 64) return three >= 2 * one;
+  if (a->dk < 64 || (a->dk == 64 && !norm && nchunks <= 24)) return three >= 2 * one;
   if (three <= 2 * one) return false;
   if (one == 1 || a->dk == 64 || (norm && a->dk != 128)) return true;
   const bool odd_row = (a->dk + 7) / 8 % 2 != 0;
+  if (one == 2 && !norm && !odd_row) return true;
   return 100 * 3 * heads >= (norm || odd_row ? 230 : 205) * one * sm_count;
 }
 

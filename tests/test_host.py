@@ -178,10 +178,10 @@ def test_short_backward_never_starts_from_the_final_state(heads, tokens, dim):
 # heads, head dim, one CTA a head, the same with the denominator's gradient inside: both sides of every line
 @pytest.mark.parametrize("heads,dim,one,norm", [
     (49, 56, 0, 0), (50, 56, 1, 1), (197, 56, 1, 1), (98, 64, 0, 0), (99, 64, 1, 1), (148, 64, 1, 1), (149, 64, 0, 0), (197, 64, 0, 0),
-    (198, 64, 1, 1), (98, 128, 0, 0), (99, 128, 1, 1), (148, 128, 1, 1), (149, 128, 0, 0), (202, 128, 0, 0), (203, 128, 1, 0),
+    (198, 64, 1, 1), (98, 128, 0, 0), (99, 128, 1, 1), (148, 128, 1, 1), (149, 128, 0, 0), (197, 128, 0, 0), (198, 128, 1, 0),
     (226, 128, 1, 0), (227, 128, 1, 1), (303, 128, 0, 0), (304, 128, 1, 0), (341, 128, 1, 1), (98, 72, 0, 0), (99, 72, 1, 1),
-    (197, 72, 0, 0), (198, 72, 0, 1), (226, 72, 0, 1), (227, 72, 1, 1), (340, 72, 0, 1), (341, 72, 1, 1), (198, 96, 0, 1), (203, 96, 1, 1),
-    (226, 83, 0, 0), (227, 83, 1, 0), (203, 90, 1, 0)])
+    (197, 72, 0, 0), (198, 72, 0, 1), (226, 72, 0, 1), (227, 72, 1, 1), (340, 72, 0, 1), (341, 72, 1, 1), (198, 96, 1, 1), (303, 112, 0, 1), (304, 112, 1, 1),
+    (226, 83, 0, 0), (227, 83, 1, 0), (198, 90, 1, 0)])
 def test_which_heads_get_one_cta_for_their_gradients(heads, dim, one, norm):
     from flashy_linear_attention_b200 import _lib
 
@@ -189,6 +189,8 @@ def test_which_heads_get_one_cta_for_their_gradients(heads, dim, one, norm):
     a = _lib.FlaArgs()
     a.batch, a.heads, a.seqlen, a.dk, a.dv = 1, heads, 4096, dim, dim
     assert lib.fla_sm100_bwd_one_cta(ctypes.byref(a)) == one
+    a.seqlen = 3072  # the line of 64 columns in tokens
+    assert lib.fla_sm100_bwd_one_cta(ctypes.byref(a)) == (one or (dim == 64 and heads >= 50))
     assert (lib.fla_sm100_normalized_bwd_workspace_bytes(ctypes.byref(a)) > 0) == norm
     assert lib.fla_sm100_bwd_uses_final_state(ctypes.byref(a)) == 1
 
